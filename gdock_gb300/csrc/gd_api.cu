@@ -596,8 +596,12 @@ gd_status gd_complex_create(gd_context *ctx, const gd_atoms *rec, const gd_atoms
       // softcore_lj_potential's per-pair constants (src/fitness.rs:58-63)
       const double eps = std::sqrt(t_eps[a] * t_eps[b]);
       const double r6 = powi6(t_rmin[a] + t_rmin[b]);
-      tab64[a * nt + b] = TypePair64{r6, 0.5 * r6, eps, 0.0};
       const double inv2 = r6 > 0.0 ? 2.0 / r6 : 0.0;
+      // an R6 that vanishes (or is not a number or infinite) gives the
+      // reference's 0 (or NaN) times eps at every distance
+      if (!std::isfinite(r6)) tab64[a * nt + b] = TypePair64{NAN, 4.0 * eps};
+      else if (r6 < 1e-150) tab64[a * nt + b] = TypePair64{r6 == 0.0 ? -0.0 : 0.0, 0.0 * eps};
+      else tab64[a * nt + b] = TypePair64{inv2, 4.0 * eps};
       tab32[a * nt + b] = TypePair32{r6 > 0.0 && inv2 < FLT_MAX ? static_cast<float>(inv2) : FLT_MAX,
                                      static_cast<float>(4.0 * eps)};
       if (eps > 50.0) cx->need_clamp = true;
@@ -710,6 +714,33 @@ gd_status gd_complex_create(gd_context *ctx, const gd_atoms *rec, const gd_atoms
     }
   }
   cx->K = static_cast<int>(rl.size());
+
+  // The FP64 form adds its terms as 128-bit integers with as many fraction
+  // bits as the largest possible sum leaves room for: pairs x the deepest well
+  // (50 where clamped), pairs x the largest charge product (d2 > 1), atoms x
+  // the largest burial energy.
+  {
+    double eps = 0.0, qr = 0.0, ql = 0.0, des = 0.0;
+    for (const TypePair64 &t : tab64)
+      if (std::isfinite(t.eps4)) eps = std::max(eps, std::fabs(t.eps4));
+    for (int i = 0; i < rec->n; ++i)
+      if (std::isfinite(rec->charge[i])) qr = std::max(qr, std::fabs(rec->charge[i]));
+    for (int j = 0; j < lig->n; ++j)
+      if (std::isfinite(lig->charge[j])) ql = std::max(ql, std::fabs(lig->charge[j]));
+    for (const std::vector<double> *v : {&rdes, &ldes})
+      for (double d : *v)
+        if (std::isfinite(d)) des = std::max(des, std::fabs(d));
+    auto bits = [](double largest, double terms) {
+      int e = 0, m = 0;
+      std::frexp(largest, &e);
+      std::frexp(terms, &m);
+      return largest > 0.0 ? std::min(124 - e - m, 1000) : 0;
+    };
+    const double pairs = std::max(1.0, static_cast<double>(rec->n) * lig->n);
+    cx->fx_vdw = bits(eps, pairs);
+    cx->fx_elec = bits(std::isfinite(qr * ql) ? qr * ql : DBL_MAX, pairs);
+    cx->fx_desolv = bits(des, static_cast<double>(rec->n) + lig->n + 1.0);
+  }
 
   gd_status s;
   UploadPack pack;

@@ -1,6 +1,6 @@
 // Device helpers shared by the scoring kernels: bulk-copy/mbarrier
 // primitives (inline PTX), the exact pose transform, exact squared distance,
-// compensated and warp sums, and the per-pose AIR/record epilogue.
+// warp sums, and the per-pose AIR/record epilogue.
 #pragma once
 
 #include "gd_internal.cuh"
@@ -109,53 +109,44 @@ static __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-// Block-wide FP64 sum of three values; result valid in thread 0.
-template <int NT>
-__device__ __forceinline__ void block_sum3(double &a, double &b, double &c, double *s_red) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  a = warp_sum(a);
-  b = warp_sum(b);
-  c = warp_sum(c);
-  if (lane == 0) {
-    s_red[warp * 3 + 0] = a;
-    s_red[warp * 3 + 1] = b;
-    s_red[warp * 3 + 2] = c;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    a = b = c = 0.0;
-    for (int w = 0; w < NT / 32; ++w) {
-      a += s_red[w * 3 + 0];
-      b += s_red[w * 3 + 1];
-      c += s_red[w * 3 + 2];
+// FP32 squared distance of a receptor atom and a ligand atom (both relative to O).
+static __device__ __forceinline__ float d2f(const float4 &r, float lx, float ly, float lz) {
+  const float dx = __fsub_rn(r.x, lx), dy = __fsub_rn(r.y, ly), dz = __fsub_rn(r.z, lz);
+  return __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
+}
+
+// AIR energy and satisfied-restraint count (src/fitness.rs:205-267,
+// src/restraints.rs:11-40) by one warp: one restraint per lane, summed in
+// restraint order.
+static __device__ __forceinline__ void warp_air(const ScoreParams &p, const gd_pose_frame &f, int pose, int lane,
+                                                double &air, int &sat) {
+  air = 0.0;
+  sat = 0;
+  for (int r0 = 0; r0 < p.K; r0 += 32) {
+    double term = 0.0;
+    int ok = 0;
+    const int r = r0 + lane;
+    if (r < p.K) {
+      const D4 a = p.restr_rec[r];
+      double X, Y, Z;
+      ligand_atom(p, f, pose, p.restr_lig[r], X, Y, Z);
+      const double dist = sqrt(exact_d2(a.x, a.y, a.z, X, Y, Z));
+      double v = 0.0;
+      if (dist < 0.0) v = __dsub_rn(0.0, dist);
+      else if (dist > 7.0) v = __dsub_rn(dist, 7.0);
+      term = __dmul_rn(__dmul_rn(10.0, v), v);
+      ok = dist <= 7.0;
+    }
+    for (int k = 0; k < 32 && r0 + k < p.K; ++k) {
+      air = __dadd_rn(air, __shfl_sync(kFull, term, k));
+      sat += __shfl_sync(kFull, ok, k);
     }
   }
 }
 
-// AIR energy and satisfied-restraint count in restraint order
-// (src/fitness.rs:205-267, src/restraints.rs:11-40); one thread.
-static __device__ void air_terms(const ScoreParams &p, const gd_pose_frame &f, int pose, double &air, int &sat) {
-  air = 0.0;
-  sat = 0;
-  for (int r = 0; r < p.K; ++r) {
-    const D4 a = p.restr_rec[r];
-    double X, Y, Z;
-    ligand_atom(p, f, pose, p.restr_lig[r], X, Y, Z);
-    const double dist = sqrt(exact_d2(a.x, a.y, a.z, X, Y, Z));
-    double v = 0.0;
-    if (dist < 0.0) v = __dsub_rn(0.0, dist);
-    else if (dist > 7.0) v = __dsub_rn(dist, 7.0);
-    air = __dadd_rn(air, __dmul_rn(__dmul_rn(10.0, v), v));
-    if (dist <= 7.0) ++sat;
-  }
-}
-
 // Final per-pose record (src/chromosome.rs:111-127).
-static __device__ void write_pose(const ScoreParams &p, int pose, double vdw, double elec, double desolv,
-                           const gd_pose_frame &f) {
-  double air;
-  int sat;
-  air_terms(p, f, pose, air, sat);
+static __device__ __forceinline__ void write_pose(const ScoreParams &p, int pose, double vdw, double elec,
+                                                  double desolv, double air, int sat) {
   const double ratio = p.K > 0 ? static_cast<double>(sat) / static_cast<double>(p.K) : 0.0;
   gd_pose_energy o;
   o.vdw = vdw;

@@ -774,10 +774,10 @@ extern "C" gd_status gd_ga_run(gd_context *ctx, gd_complex *const *complexes, in
         if (ss != GD_OK) return ss;
       } else {
         // plain form: one FP64 launch per job; finished jobs are skipped on
-        // the device by the GA step, so their scores stay final
+        // the device, so their scores stay final
         for (int j = 0; j < jobs; ++j) {
           gd_status ss = launch_score(complexes[j], descs[j].frames, nullptr, n, GD_PREC_F64, descs[j].out, st,
-                                      c.max_displacement);
+                                      c.max_displacement, descs[j].skip);
           if (ss != GD_OK) return ss;
         }
       }

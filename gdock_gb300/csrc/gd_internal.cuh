@@ -17,13 +17,12 @@ struct alignas(32) D4 {
   double x, y, z, w;
 };
 
-// Receptor atoms per tile staged in shared memory by one bulk (TMA) copy.
+// The receptor's arrays are padded to a multiple of this many atoms.
 constexpr int kTile = 256;
-// Receptor atoms per segment of the FP32 kernel's ring: the receptor is
-// stored as spatially compact segments of this many atoms, each with a
-// bounding sphere.
+// Receptor atoms per segment (a stage of the FP32 kernel's ring, a unit of the
+// FP64 kernel): the receptor is stored as spatially compact segments of this
+// many atoms, each with a bounding sphere.
 constexpr int kRecSeg = 64;
-constexpr int kStages = 3;
 // Upper bounds of a device-side wait before it gives up: polls and wall time.
 constexpr uint32_t kSpinLimit = 1u << 26;
 constexpr uint64_t kWaitLimitNs = 2000000000ull;
@@ -58,8 +57,9 @@ struct GaJobState {
 // rewritten as eps (q^2 - 2q) = 4 eps x (x - 1) with q = 2x and
 // x = 1 / (r^6 * 2/R6 + 1), R6 = (Rmin_i + Rmin_j)^6, eps = sqrt(eps_i eps_j).
 struct TypePair32 { float inv2, eps4; };  // 2/R6 (FLT_MAX when R6 = 0), 4 eps
-// FP64 form: R6, alpha*R6 (alpha = 0.5), eps.
-struct TypePair64 { double r6, hr6, eps, pad; };
+// FP64 form of the same: 2/R6 (0 with eps4 = 0 eps when R6 vanishes: no
+// energy, whatever the distance; -0 when it is exactly zero), 4 eps.
+struct alignas(16) TypePair64 { double inv2, eps4; };
 
 // Exact FP64 thresholds on the squared distance d2 = dx*dx + dy*dy + dz*dz,
 // so that d2-comparisons make the same decisions as the reference's
@@ -80,7 +80,7 @@ struct ScoreParams {
   const int4 *rec_meta16;   // (type, serial, 0, 0): the FP32 kernel's copy, as wide as a position
   const double *rec_desolv; // [nr * 11] energy contribution at burial count 0..10
   const float4 *rec_seg;    // per kRecSeg-atom segment: bounding sphere (centre - O, radius) FP32
-  int nr, n_tiles, nseg;
+  int nr, nseg;
   // ligand in slot order (spatially compact runs of 32 atoms)
   const int *lig_perm;      // slot position -> original atom index
   const D4 *lig_slot_sph;   // per 32-atom slot: bounding sphere in the positioned frame (centre, radius)
@@ -95,6 +95,8 @@ struct ScoreParams {
   const TypePair64 *tab64;
   int nt;
   int need_clamp;           // some |eps_ij| may exceed the [-50, 500] clamp
+  // FP64 form: fraction bits of the exact sums of vdW, Coulomb and desolvation
+  int fx_vdw, fx_elec, fx_desolv;
   // restraints: receptor CA coordinates and ligand CA atom index
   const D4 *restr_rec; // (x, y, z, -) of the receptor CA
   const int *restr_lig;     // ligand CA index (slot order)
@@ -148,6 +150,7 @@ struct gd_complex {
   gd_weights w{};
   bool serial_overlap = false;
   bool need_clamp = false;
+  int fx_vdw = 0, fx_elec = 0, fx_desolv = 0;  // fraction bits of the FP64 form's exact sums
   double cx = 0, cy = 0, cz = 0, ox = 0, oy = 0, oz = 0;
   double rec_extent = 0;  // max |x - O| over receptor atoms (inf-norm)
   double lig_radius = 0;  // max |x - c| over ligand atoms (Euclidean)
@@ -201,7 +204,8 @@ Thresholds make_thresholds(double contact_cutoff);
 void make_frame(const double *g, gd_pose_frame *f);
 void guard_widths(const gd_complex *cx, double max_disp, float *gv, float *ge, float *gd);
 gd_status launch_score(gd_complex *cx, const gd_pose_frame *d_frames, const double *d_models, int n,
-                       gd_precision prec, gd_pose_energy *d_out, cudaStream_t stream, double max_disp);
+                       gd_precision prec, gd_pose_energy *d_out, cudaStream_t stream, double max_disp,
+                       const int *skip = nullptr);
 void free_cluster_cache(gd_complex *cx);
 // A small sphere enclosing n points (x[i], y[i], z[i]) for i = idx[k], or
 // i = k when idx is null; the radius is the largest distance from the

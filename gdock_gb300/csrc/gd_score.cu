@@ -6,15 +6,26 @@
 // src/chromosome.rs:79-83; energies src/fitness.rs:57-302; per-pose
 // combination src/chromosome.rs:110-127.
 //
-// k_score_f64: one pose per CTA iteration of a persistent grid.  Receptor
-// atoms are streamed through shared memory in tiles of kTile atoms by bulk
-// (TMA) copies into a kStages-deep ring guarded by mbarriers with bounded
-// waits; the receptor stream is the same for every pose, so the ring runs
-// continuously across the poses a CTA owns.  Each thread holds S ligand atoms
-// of the current pose (atoms tid, tid+NT, ... of the chunk) in registers
-// after transforming them in FP64 with the reference's operation order, so
-// coordinates are bit-identical to gdock's.  Every pair is evaluated in FP64
-// (no culling), with decisions against exact thresholds on d2.
+// k_score_f64: one pose per thread-block cluster of 1 to 16 CTAs.
+//   1. The ligand's atoms are moved in FP64 with the reference's operation
+//      order (coordinates bit-identical to gdock's) into shared memory, each
+//      CTA of the cluster a share, the others copied from its shared memory.
+//   2. Work units of one 32-atom ligand slot x some blocks of 32 receptor
+//      atoms are taken by the cluster's warps from one counter.  A unit finds
+//      its pairs within reach in FP32 (bounding spheres of the slot and of the
+//      receptor segments, then each pair's distance, all with the FP32 guard
+//      band added, so that only pairs whose every term is exactly zero are
+//      dropped) and lists them in shared memory; every 32 listed pairs are
+//      evaluated in FP64, one per lane: near pairs (within 12 A) every term,
+//      far ones Coulomb only.  Decisions are exact: the squared distance's
+//      high word settles them, and pairs next to a cutoff are decided on d2
+//      in the reference's operation order against the exact thresholds.
+//   3. Every term is added as a 128-bit fixed-point integer.  Integer sums are
+//      exact, so the energies do not depend on which lane, warp or CTA took
+//      which pair, nor on the launch's other poses; the integer adds issue
+//      beside the FP64 pipe, which is the bound.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cmath>
 
@@ -23,212 +34,484 @@
 namespace gd {
 namespace {
 
-struct SmemLayout {
-  size_t pos, meta, bars, tab, frame, red, rcnt, total;
+namespace cg = cooperative_groups;
+
+constexpr int kNT = 256;              // threads per CTA of k_score_f64
+constexpr int kNW = kNT / 32;
+constexpr int kLigBits = 10;
+constexpr int kLigCap = 1 << kLigBits;  // ligand atoms held in shared memory at once (longer ligands: in turns)
+constexpr int kRows = 4;              // rows searched per step
+constexpr int kQueue = 32 * (kRows + 1);  // listed pairs per warp and kind: 31 left over + 32 of each row
+constexpr int kGrainMax = 4;          // 32-atom receptor blocks of a unit, at most
+constexpr int kMaxCluster = 16;
+constexpr int kTinyHi = 0x2b000000;   // high word of 2^-335: below it r^6 may underflow
+
+struct F64Smem {
+  size_t x, y, z, q, fx, fy, fz, lt, sph, rcnt, lcnt, queue, red, nf, frame, misc, total;
 };
 
-template <typename PosT>
-__host__ __device__ inline SmemLayout smem_layout(int nt, int nr, int nthreads, size_t tab_entry) {
-  SmemLayout L;
+__host__ __device__ inline F64Smem f64_smem(int nr, int nl) {
+  F64Smem L;
   size_t o = 0;
-  auto al = [&](size_t a) { o = (o + a - 1) / a * a; };
-  L.pos = o;
-  o += sizeof(PosT) * kStages * kTile;
-  al(16);
-  L.meta = o;
-  o += sizeof(int2) * kStages * kTile;
-  al(16);
-  L.bars = o;
-  o += 8 * 8;
-  al(16);
-  L.tab = o;
-  o += tab_entry * nt * nt;
-  al(16);
-  L.frame = o;
-  o += sizeof(gd_pose_frame);
-  al(16);
-  L.red = o;
-  o += sizeof(double) * 3 * (nthreads / 32);
-  al(16);
-  L.rcnt = o;
-  o += sizeof(uint32_t) * nr;
-  al(16);
+  const size_t cap = nl < kLigCap ? (static_cast<size_t>(nl) + 31) / 32 * 32 : kLigCap;
+  auto take = [&](size_t b) {
+    const size_t at = o;
+    o += (b + 15) / 16 * 16;
+    return at;
+  };
+  L.x = take(8 * cap);
+  L.y = take(8 * cap);
+  L.z = take(8 * cap);
+  L.q = take(8 * cap);
+  L.fx = take(4 * cap);
+  L.fy = take(4 * cap);
+  L.fz = take(4 * cap);
+  L.lt = take(cap);
+  L.sph = take(sizeof(float4) * (cap / 32));
+  L.rcnt = take(2 * (static_cast<size_t>(nr) + 1));  // 16-bit burial counts, two a word
+  L.lcnt = take(2 * (static_cast<size_t>(nl) + 1));
+  L.queue = take(2 * sizeof(uint32_t) * kQueue * kNW);
+  L.red = take(3 * sizeof(__int128) * kNW);
+  L.nf = take(3 * sizeof(double) * kNW);
+  L.frame = take(sizeof(gd_pose_frame));
+  L.misc = take(32);  // next unit, satisfied restraints, AIR energy
   L.total = o;
   return L;
 }
 
-// Producer side of the receptor ring: tile q of the CTA's sequence.
-template <typename PosT>
-__device__ __forceinline__ void issue_tile(long long q, int n_tiles, const PosT *g_pos, const int2 *g_meta,
-                                           PosT *s_pos, int2 *s_meta, uint64_t *s_full) {
-  const int st = static_cast<int>(q % kStages);
-  const int t = static_cast<int>(q % n_tiles);
-  mbar_expect_tx(&s_full[st], kTile * (sizeof(PosT) + sizeof(int2)));
-  bulk_g2s(&s_pos[st * kTile], g_pos + static_cast<size_t>(t) * kTile, kTile * sizeof(PosT), &s_full[st]);
-  bulk_g2s(&s_meta[st * kTile], g_meta + static_cast<size_t>(t) * kTile, kTile * sizeof(int2), &s_full[st]);
+// 1/d by one third-order step x (1 + e + e^2), e = 1 - d x (the Householder
+// series of the reciprocal), on the hardware's approximation x, whose
+// relative error is at most 2^-23: the remaining error e^3 lies below the
+// FP64 rounding.  Three FP64 multiply-adds; FP64 issues at 1/64 of the FP32
+// rate on this part, and a correctly rounded division costs about ten.
+__device__ __forceinline__ double rcp64(double d) {
+  double x;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
+  double e = __fma_rn(-d, x, 1.0);
+  e = __fma_rn(e, e, e);
+  return __fma_rn(x, e, x);
 }
 
-// After an abort: wait (bounded) for copies still in flight, then return.
-__device__ void drain(uint64_t *s_full, long long q_from, long long q_to) {
-  for (long long q = q_from; q < q_to; ++q) mbar_wait(&s_full[q % kStages], static_cast<uint32_t>((q / kStages) & 1));
+// Exact sum of FP64 values as a fixed-point integer with 2^-bits resolution
+// (bits leaves room for the largest possible sum); values that are not finite
+// are kept apart (they decide the result).
+struct ExactSum {
+  __int128 v = 0;
+  double nf = 0.0;
+  __device__ __forceinline__ void add(double x, int bits) {
+    const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(x));
+    const int e = static_cast<int>(b >> 52) & 0x7ff;
+    if (e == 0) return;  // zero (a subnormal is far below the resolution)
+    if (e == 0x7ff) {
+      nf += x;
+      return;
+    }
+    const unsigned long long m = (b & 0xfffffffffffffull) | 0x10000000000000ull;
+    const int sh = e - 1075 + bits;
+    const unsigned __int128 t = sh >= 0 ? static_cast<unsigned __int128>(m) << min(sh, 74)
+                                        : static_cast<unsigned __int128>(m >> min(-sh, 63));
+    v += static_cast<long long>(b) < 0 ? -static_cast<__int128>(t) : static_cast<__int128>(t);
+  }
+  __device__ __forceinline__ void add(const ExactSum &o) {
+    v += o.v;
+    nf += o.nf;
+  }
+  __device__ __forceinline__ ExactSum shfl_xor(int o) const {
+    ExactSum r;
+    const unsigned long long lo = __shfl_xor_sync(kFull, static_cast<unsigned long long>(v), o);
+    const long long hi = __shfl_xor_sync(kFull, static_cast<long long>(v >> 64), o);
+    r.v = (static_cast<__int128>(hi) << 64) | lo;
+    r.nf = __shfl_xor_sync(kFull, nf, o);
+    return r;
+  }
+  __device__ double value(int bits) const {
+    if (nf != 0.0) return nf;  // inf or NaN
+    const double hi = static_cast<double>(static_cast<long long>(v >> 64)),
+                 lo = static_cast<double>(static_cast<unsigned long long>(v));
+    return ldexp(hi * 18446744073709551616.0 + lo, -bits);
+  }
+};
+
+// min(count, 10) is all that is read: a count that has reached 10 is left
+// alone, which also keeps the 16 bits from overflowing (at most 10 + one
+// concurrent add of each of the CTA's threads).
+__device__ __forceinline__ void bury(uint32_t *cnt, int i) {
+  const int sh = (i & 1) * 16;
+  if (((*reinterpret_cast<volatile uint32_t *>(cnt + (i >> 1)) >> sh) & 0xffffu) < 10u) atomicAdd(cnt + (i >> 1), 1u << sh);
 }
 
-// --------------------------------------------------------------- FP64 ----
+// d2 next to the squared cutoff t: its high word is t's or a neighbour of it
+// (a relative 2^-20 to either side), which covers the few ulps between a
+// fused d2 and the reference's.
+__device__ __forceinline__ bool near_hi(int hi, double t) {
+  return static_cast<unsigned>(hi - (__double2hiint(t) - 1)) <= 2u;
+}
 
-template <int NT, int S, bool SERIAL, bool CLAMP>
-__global__ void __launch_bounds__(NT) k_score_f64(const ScoreParams p) {
+// The pair's decisions in the reference's arithmetic: bit 0 vdW, 1 burial, 2
+// Coulomb.  Kept out of line: a handful of pairs in a million come here, and
+// inlined as predicated instructions they took a third of the FP64 pipe.
+__device__ __noinline__ int exact_decisions(const Thresholds &t, double rx, double ry, double rz, double lx, double ly,
+                                            double lz) {
+  const double d2 = exact_d2(rx, ry, rz, lx, ly, lz);
+  return (d2 > 0.0 && d2 < t.vdw_lt) | (d2 < t.desolv_lt) << 1 | (d2 > t.elec_gt && d2 < t.elec_lt) << 2;
+}
+
+template <bool SERIAL, bool CLAMP>
+struct PairEval {
+  const ScoreParams &p;
+  const double *x, *y, *z, *q;
+  const uint8_t *lt;
+  uint32_t *rcnt, *lcnt;
+  int base;  // ligand atom of the shared arrays' first entry
+
+  // one listed pair per lane (on): w = receptor atom, ligand entry
+  template <bool NEAR>
+  __device__ __forceinline__ void eval(bool on, uint32_t w, ExactSum &vdw, ExactSum &elec) const {
+    if (!on) return;
+    const int ri = static_cast<int>(w >> kLigBits), k = static_cast<int>(w & (kLigCap - 1));
+    const double2 *rp = reinterpret_cast<const double2 *>(p.rec_pos64 + ri);
+    const double2 rxy = __ldg(rp), rzq = __ldg(rp + 1);
+    const double lx = x[k], ly = y[k], lz = z[k];
+    const double dx = rxy.x - lx, dy = rxy.y - ly, dz = rzq.x - lz;
+    const double d2 = __fma_rn(dz, dz, __fma_rn(dy, dy, dx * dx));
+    const int hi = __double2hiint(d2);
+    if (!NEAR) {
+      bool pe = hi < __double2hiint(p.thr.elec_lt);
+      if (near_hi(hi, p.thr.elec_lt)) pe = exact_decisions(p.thr, rxy.x, rxy.y, rzq.x, lx, ly, lz) & 4;
+      if (pe) elec.add(rzq.y * q[k] * rcp64(d2), p.fx_elec);
+      return;
+    }
+    // (a zero, a tiny or an undefined d2 takes the exact tests too)
+    bool pv = hi < __double2hiint(p.thr.vdw_lt), pd = hi < __double2hiint(p.thr.desolv_lt);
+    bool pe = hi > __double2hiint(p.thr.elec_gt) && hi < __double2hiint(p.thr.elec_lt);
+    if (near_hi(hi, p.thr.vdw_lt) | near_hi(hi, p.thr.desolv_lt) | near_hi(hi, p.thr.elec_gt) |
+        near_hi(hi, p.thr.elec_lt) | (hi < kTinyHi)) {  // hi < 0: NaN
+      const int d = exact_decisions(p.thr, rxy.x, rxy.y, rzq.x, lx, ly, lz);
+      pv = d & 1;
+      pd = d & 2;
+      pe = d & 4;
+      // where r^6 underflows and R6 is zero, the reference's ratio is 0 / 0
+      if (pv && d2 * d2 * d2 == 0.0 &&
+          __double_as_longlong(__ldg(&p.tab64[__ldg(p.rec_meta + ri).x + lt[k]].inv2)) < 0)
+        vdw.nf = NAN;
+    }
+    const int2 m = __ldg(p.rec_meta + ri);
+    if (SERIAL) pv = pv && m.y != __ldg(p.lig_serial + base + k);
+    if (pd) {
+      bury(rcnt, ri);
+      bury(lcnt, base + k);
+    }
+    if (pv) {
+      // softcore_lj_potential (src/fitness.rs:57-70) as 4 eps (x^2 - x) with
+      // x = 1 / (r^6 2/R6 + 1), half the reference's ratio
+      const double2 tp = __ldg(reinterpret_cast<const double2 *>(p.tab64) + m.x + lt[k]);
+      const double u = rcp64(__fma_rn(d2 * d2 * d2, tp.x, 1.0));
+      double v = tp.y * __fma_rn(u, u, -u);
+      if (CLAMP) v = v < -50.0 ? -50.0 : (v > 500.0 ? 500.0 : v);
+      vdw.add(v, p.fx_vdw);
+    }
+    // elec_energy term (src/fitness.rs:296) without its constant, which
+    // multiplies the pose's sum
+    if (pe) elec.add(rzq.y * q[k] * rcp64(d2), p.fx_elec);
+  }
+};
+
+// What bounds it: the FP64 pipe, two lanes' operations per clock and SM.  The
+// form that evaluated every pair spent about 35 of them on each pair, though
+// only 13 % of the pairs of a scan have a term; a listed pair costs 18 (near)
+// or 11 (far), and the FP32 search runs beside the FP64 pipe.  On receptors of
+// 2,538 and ligands of 1,280 atoms: 2,048 poses 348 -> 28.7 ms, 150 poses
+// 29.0 -> 2.38 ms; one pose of 411 x 649 atoms 1,746 -> 89 us a call.
+template <bool SERIAL, bool CLAMP>
+__global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const int grain) {
+  if (p.skip && *p.skip) return;
   extern __shared__ __align__(128) unsigned char smem[];
-  const SmemLayout L = smem_layout<D4>(p.nt, p.nr, NT, sizeof(D4));
-  D4 *s_pos = reinterpret_cast<D4 *>(smem + L.pos);
-  int2 *s_meta = reinterpret_cast<int2 *>(smem + L.meta);
-  uint64_t *s_full = reinterpret_cast<uint64_t *>(smem + L.bars);
-  D4 *s_tab = reinterpret_cast<D4 *>(smem + L.tab);
+  const F64Smem L = f64_smem(p.nr, p.nl);
+  double *s_x = reinterpret_cast<double *>(smem + L.x), *s_y = reinterpret_cast<double *>(smem + L.y),
+         *s_z = reinterpret_cast<double *>(smem + L.z), *s_q = reinterpret_cast<double *>(smem + L.q);
+  float *s_fx = reinterpret_cast<float *>(smem + L.fx), *s_fy = reinterpret_cast<float *>(smem + L.fy),
+        *s_fz = reinterpret_cast<float *>(smem + L.fz);
+  uint8_t *s_lt = smem + L.lt;
+  float4 *s_sph = reinterpret_cast<float4 *>(smem + L.sph);
+  uint32_t *s_rcnt = reinterpret_cast<uint32_t *>(smem + L.rcnt), *s_lcnt = reinterpret_cast<uint32_t *>(smem + L.lcnt);
   gd_pose_frame *s_frame = reinterpret_cast<gd_pose_frame *>(smem + L.frame);
-  double *s_red = reinterpret_cast<double *>(smem + L.red);
-  uint32_t *s_rcnt = reinterpret_cast<uint32_t *>(smem + L.rcnt);
+  __int128 *s_red = reinterpret_cast<__int128 *>(smem + L.red);
+  double *s_nf = reinterpret_cast<double *>(smem + L.nf);
+  int *s_next = reinterpret_cast<int *>(smem + L.misc), *s_sat = s_next + 1;
+  double *s_air = reinterpret_cast<double *>(smem + L.misc + 8);
 
-  const int tid = threadIdx.x, lane = tid & 31;
-  if (tid == 0) {
-    for (int s = 0; s < kStages; ++s) mbar_init(&s_full[s], 1);
-    fence_mbar_init();
-  }
-  for (int i = tid; i < p.nt * p.nt; i += NT) {
-    const TypePair64 t = p.tab64[i];
-    s_tab[i] = D4{t.r6, t.hr6, t.eps, 0.0};
-  }
-  for (int i = tid; i < p.nr; i += NT) s_rcnt[i] = 0;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int nc = static_cast<int>(cluster.num_blocks()), rank = static_cast<int>(cluster.block_rank());
+  const int pose = static_cast<int>(blockIdx.x) / nc;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned lt_mask = (1u << lane) - 1u;
+  uint32_t *q_near = reinterpret_cast<uint32_t *>(smem + L.queue) + warp * 2 * kQueue, *q_far = q_near + kQueue;
+
+  if (!p.models && tid < 16)
+    reinterpret_cast<double *>(s_frame)[tid] = reinterpret_cast<const double *>(p.frames + pose)[tid];
+  for (int i = tid; i < (p.nr + 1) / 2; i += kNT) s_rcnt[i] = 0;
+  for (int i = tid; i < (p.nl + 1) / 2; i += kNT) s_lcnt[i] = 0;
+  if (tid == 0) *s_next = 0;
   __syncthreads();
+  const gd_pose_frame &f = *s_frame;
 
-  constexpr int kChunk = NT * S;
-  const int nchunks = (p.nl + kChunk - 1) / kChunk;
-  const int my_poses =
-      (static_cast<int>(blockIdx.x) < p.n_poses) ? (p.n_poses - 1 - static_cast<int>(blockIdx.x)) / gridDim.x + 1 : 0;
-  const long long Q = static_cast<long long>(my_poses) * nchunks * p.n_tiles;
-  if (tid == 0)
-    for (long long q = 0; q < Q && q < kStages; ++q)
-      issue_tile(q, p.n_tiles, p.rec_pos64, p.rec_meta, s_pos, s_meta, s_full);
+  // FP32 reach of the elec and vdW cutoffs with their guard bands.  The tests
+  // below are written so that an undefined comparison (coordinates beyond
+  // FP32) and an infinite band keep the pair for the FP64 decision.
+  const float lim_e = 225.0f + p.guard_e, lim_v = 144.0f + p.guard_v;
+  const float reach = sqrtf(225.01f + 2.0f * p.guard_e) + 0.01f;
+  const int nblk = (p.nr + 31) / 32, ngrp = (nblk + grain - 1) / grain;
+  ExactSum vdw, elec;
+  int first = 0;  // unit counter at the start of this turn
 
-  const double vdw_lt = p.thr.vdw_lt, elec_gt = p.thr.elec_gt, elec_lt = p.thr.elec_lt, des_lt = p.thr.desolv_lt;
-  long long q = 0;
-  for (int k = 0; k < my_poses; ++k) {
-    const int pose = static_cast<int>(blockIdx.x) + k * static_cast<int>(gridDim.x);
-    if (!p.models && tid < 16)
-      reinterpret_cast<double *>(s_frame)[tid] = reinterpret_cast<const double *>(p.frames + pose)[tid];
-    __syncthreads();
-    const gd_pose_frame f = *s_frame;
-    double vdw_t = 0.0, elec_t = 0.0, desolv_t = 0.0;
-
-    for (int ch = 0; ch < nchunks; ++ch) {
-      double lx[S], ly[S], lz[S], lq[S];
-      int lt[S], lser[S], lcnt[S];
-#pragma unroll
-      for (int s = 0; s < S; ++s) {
-        const int j = ch * kChunk + s * NT + tid;
-        lcnt[s] = 0;
-        if (j < p.nl) {
-          ligand_atom(p, f, pose, j, lx[s], ly[s], lz[s]);
-          lq[s] = p.lig_q[j];
-          lt[s] = p.lig_type[j];
-          if (!GD_DCHECK(p.err, lt[s] >= 0 && lt[s] < p.nt, 22)) lt[s] = 0;
-          lser[s] = SERIAL ? p.lig_serial[j] : 0;
-        } else {
-          lx[s] = ly[s] = lz[s] = 1.0e30;
-          lq[s] = 0.0;
-          lt[s] = 0;
-          lser[s] = 0;
-        }
+  const int turns = (p.nl + kLigCap - 1) / kLigCap, turn = turns ? ((p.nl + turns - 1) / turns + 31) / 32 * 32 : 0;
+  for (int l0 = 0; l0 < p.nl; l0 += turn) {
+    const int nl = min(turn, p.nl - l0), nslot = (nl + 31) / 32, nunit = nslot * ngrp;
+    // the CTA's share of the slots: one warp per slot, one atom per lane
+    for (int s = rank + nc * warp; s < nslot; s += nc * kNW) {
+      const int k = s * 32 + lane, j = l0 + k;
+      const bool on = k < nl;
+      float fx = 0.0f, fy = 0.0f, fz = 0.0f;
+      if (on) {
+        double X, Y, Z;
+        ligand_atom(p, f, pose, j, X, Y, Z);
+        s_x[k] = X;
+        s_y[k] = Y;
+        s_z[k] = Z;
+        fx = static_cast<float>(X - p.ox);
+        fy = static_cast<float>(Y - p.oy);
+        fz = static_cast<float>(Z - p.oz);
+        s_fx[k] = fx;
+        s_fy[k] = fy;
+        s_fz[k] = fz;
       }
-      for (int t = 0; t < p.n_tiles; ++t, ++q) {
-        const int st = static_cast<int>(q % kStages);
-        const bool ok = __all_sync(kFull, mbar_wait(&s_full[st], static_cast<uint32_t>((q / kStages) & 1)));
-        const int base = t * kTile;
-        const int cnt = min(kTile, p.nr - base);
-        if (ok) {
-          for (int a = 0; a < cnt; ++a) {
-            const D4 r = s_pos[st * kTile + a];
-            int2 m = s_meta[st * kTile + a];
-            if (!GD_DCHECK(p.err, m.x >= 0 && m.x + p.nt <= p.nt * p.nt, 20)) m.x = 0;
-            int rc = 0;
+      // a sphere around the slot: centre of its bounding box, farthest atom
+      float lo[3] = {on ? fx : 3.0e38f, on ? fy : 3.0e38f, on ? fz : 3.0e38f},
+            hi[3] = {on ? fx : -3.0e38f, on ? fy : -3.0e38f, on ? fz : -3.0e38f};
 #pragma unroll
-            for (int s = 0; s < S; ++s) {
-              const double d2 = exact_d2(r.x, r.y, r.z, lx[s], ly[s], lz[s]);
-              bool pv = d2 > 0.0 && d2 < vdw_lt;
-              if (SERIAL) pv = pv && (m.y != lser[s]);
-              const bool pe = d2 > elec_gt && d2 < elec_lt;
-              const bool pd = d2 < des_lt;
-              if (__any_sync(kFull, pv)) {
-                // softcore_lj_potential (src/fitness.rs:57-70) with r^6 from d2
-                const D4 tp = s_tab[m.x + lt[s]];
-                const double d4 = d2 * d2;
-                const double r6 = d2 * d4;
-                const double ratio = tp.x / (r6 + tp.y);
-                double v = tp.z * (ratio * ratio - 2.0 * ratio);
-                if (CLAMP) v = v < -50.0 ? -50.0 : (v > 500.0 ? 500.0 : v);
-                vdw_t += pv ? v : 0.0;
-              }
-              if (__any_sync(kFull, pe)) {
-                // elec_energy term (src/fitness.rs:296): k*(q1*q2)/r^2
-                const double e = (332.0636 * (r.w * lq[s])) / d2;
-                elec_t += pe ? e : 0.0;
-              }
-              lcnt[s] += pd;
-              rc += pd;
-            }
-            const int tot = __reduce_add_sync(kFull, rc);
-            if (lane == 0 && tot && GD_DCHECK(p.err, base + a < p.nr, 21))
-              atomicAdd(&s_rcnt[base + a], static_cast<uint32_t>(tot));
-          }
-        }
-        if (__syncthreads_or(!ok)) {
-          if (tid == 0) {
-            atomicExch(p.err, kDevTimeout);
-            drain(s_full, q, (q + kStages < Q ? q + kStages : Q));
-          }
-          return;
-        }
-        if (tid == 0 && q + kStages < Q) issue_tile(q + kStages, p.n_tiles, p.rec_pos64, p.rec_meta, s_pos, s_meta, s_full);
-      }
+      for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-      for (int s = 0; s < S; ++s) {
-        const int j = ch * kChunk + s * NT + tid;
-        if (j < p.nl) desolv_t += p.lig_desolv[static_cast<size_t>(j) * 11 + min(lcnt[s], 10)];
+        for (int a = 0; a < 3; ++a) {
+          lo[a] = fminf(lo[a], __shfl_xor_sync(kFull, lo[a], o));
+          hi[a] = fmaxf(hi[a], __shfl_xor_sync(kFull, hi[a], o));
+        }
+      const float cx = 0.5f * (lo[0] + hi[0]), cy = 0.5f * (lo[1] + hi[1]), cz = 0.5f * (lo[2] + hi[2]);
+      float rr = on ? sqrtf((fx - cx) * (fx - cx) + (fy - cy) * (fy - cy) + (fz - cz) * (fz - cz)) : 0.0f;
+      const bool odd = __any_sync(kFull, !(rr < 3.0e38f));  // not finite: a sphere that keeps everything
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) rr = fmaxf(rr, __shfl_xor_sync(kFull, rr, o));
+      if (lane == 0) s_sph[s] = make_float4(cx, cy, cz, odd ? INFINITY : rr * 1.0001f + 0.01f);
+    }
+    for (int k = tid; k < nl; k += kNT) {
+      int t = p.lig_type[l0 + k];
+      if (!GD_DCHECK(p.err, t >= 0 && t < p.nt, 22)) t = 0;
+      s_lt[k] = static_cast<uint8_t>(t);
+      s_q[k] = p.lig_q[l0 + k];
+    }
+    if (nc > 1) {
+      // the other CTAs' slots, out of their shared memory
+      cluster.sync();
+      for (int s = warp; s < nslot; s += kNW) {
+        const int o = s % nc;
+        if (o == rank) continue;
+        const int k = s * 32 + lane;
+        if (k < nl) {
+          s_x[k] = *cluster.map_shared_rank(s_x + k, o);
+          s_y[k] = *cluster.map_shared_rank(s_y + k, o);
+          s_z[k] = *cluster.map_shared_rank(s_z + k, o);
+          s_fx[k] = *cluster.map_shared_rank(s_fx + k, o);
+          s_fy[k] = *cluster.map_shared_rank(s_fy + k, o);
+          s_fz[k] = *cluster.map_shared_rank(s_fz + k, o);
+        }
+        if (lane == 0) s_sph[s] = *cluster.map_shared_rank(s_sph + s, o);
       }
     }
-    for (int i = tid; i < p.nr; i += NT) {
-      desolv_t += p.rec_desolv[static_cast<size_t>(i) * 11 + min(s_rcnt[i], 10u)];
-      s_rcnt[i] = 0;
-    }
-    block_sum3<NT>(vdw_t, elec_t, desolv_t, s_red);
-    if (tid == 0) write_pose(p, pose, vdw_t, elec_t, desolv_t, f);
     __syncthreads();
+
+    const PairEval<SERIAL, CLAMP> ev{p, s_x, s_y, s_z, s_q, s_lt, s_rcnt, s_lcnt, l0};
+    int *next = nc > 1 ? cluster.map_shared_rank(s_next, 0) : s_next;
+    int nn = 0, nf = 0;  // listed near and far pairs of this warp
+    for (;;) {
+      int u = 0;
+      if (lane == 0) u = atomicAdd(next, 1);
+      u = __shfl_sync(kFull, u, 0) - first;
+      if (u >= nunit) break;
+      const int slot = u / ngrp, b0 = u % ngrp * grain, b1 = min(nblk, b0 + grain);
+      const int k = slot * 32 + lane;
+      const bool on = k < nl;
+      const float lx = on ? s_fx[k] : 0.0f, ly = on ? s_fy[k] : 0.0f, lz = on ? s_fz[k] : 0.0f;
+      const float4 sp = s_sph[slot];
+      const float lim_s = sp.w + reach, lim_s2 = lim_s * lim_s;
+#pragma unroll 1
+      for (int b = b0; b < b1; ++b) {
+        {
+          const float4 sg = __ldg(&p.rec_seg[b >> 1]);
+          const float dx = sg.x - sp.x, dy = sg.y - sp.y, dz = sg.z - sp.z;
+          const float lim = sg.w + sp.w + reach + 0.1f + 1e-3f * (sg.w + sp.w);
+          if (dx * dx + dy * dy + dz * dz > lim * lim) {
+            b |= 1;  // the segment's second block too
+            continue;
+          }
+        }
+        // rows: receptor atoms within reach of the slot's sphere
+        const int a0 = b * 32;
+        bool keep = a0 + lane < p.nr;
+        if (keep) {
+          const float4 r = __ldg(&p.rec_pos32[a0 + lane]);
+          const float dx = r.x - sp.x, dy = r.y - sp.y, dz = r.z - sp.z;
+          keep = !(dx * dx + dy * dy + dz * dz > lim_s2);
+        }
+        unsigned rows = __ballot_sync(kFull, keep);
+        // kRows rows a step (past the last: a row that lists nothing), so that
+        // their loads and votes overlap
+        while (rows) {
+          int a[kRows];
+          float d2[kRows];
+#pragma unroll
+          for (int i = 0; i < kRows; ++i) {
+            a[i] = rows ? a0 + __ffs(rows) - 1 : -1;
+            rows &= rows - 1;
+            d2[i] = d2f(__ldg(&p.rec_pos32[max(a[i], a0)]), lx, ly, lz);
+          }
+#pragma unroll
+          for (int i = 0; i < kRows; ++i) {
+            const bool reached = on && a[i] >= 0 && !(d2[i] > lim_e), close = reached && !(d2[i] > lim_v);
+            const unsigned Mn = __ballot_sync(kFull, close), Mf = __ballot_sync(kFull, reached && !close);
+            const uint32_t e = static_cast<uint32_t>(a[i]) << kLigBits | static_cast<uint32_t>(k);
+            if (close) q_near[nn + __popc(Mn & lt_mask)] = e;
+            else if (reached) q_far[nf + __popc(Mf & lt_mask)] = e;
+            nn += __popc(Mn);
+            nf += __popc(Mf);
+          }
+          if (nn >= 32 || nf >= 32) {
+            __syncwarp();
+            for (; nn >= 32; nn -= 32) ev.template eval<true>(true, q_near[nn - 32 + lane], vdw, elec);
+            for (; nf >= 32; nf -= 32) ev.template eval<false>(true, q_far[nf - 32 + lane], vdw, elec);
+            __syncwarp();
+          }
+        }
+      }
+    }
+    // the rest of both lists, together when they fit one round (the near
+    // evaluation decides every term itself)
+    __syncwarp();
+    if (nn + nf <= 32) {
+      ev.template eval<true>(lane < nn + nf, lane < nn ? q_near[lane] : q_far[lane - nn], vdw, elec);
+    } else {
+      ev.template eval<true>(lane < nn, q_near[lane], vdw, elec);
+      ev.template eval<false>(lane < nf, q_far[lane], vdw, elec);
+    }
+    __syncwarp();
+    // every warp of the cluster drew one unit number past the last
+    first += nunit + nc * kNW;
+    if (l0 + turn < p.nl) {
+      if (nc > 1) cluster.sync();  // nobody reads this turn's ligand atoms any more
+      else __syncthreads();
+    }
   }
+
+  // AIR: one restraint per lane, summed in restraint order (bit-identical)
+  if (rank == 0 && warp == 0) {
+    double air;
+    int sat;
+    warp_air(p, f, pose, lane, air, sat);
+    if (lane == 0) {
+      *s_air = air;
+      *s_sat = sat;
+    }
+  }
+  if (nc > 1) cluster.sync();
+  else __syncthreads();
+  // desolvation from the cluster's summed burial counts, a share per CTA
+  ExactSum desolv;
+  for (int side = 0; side < 2; ++side) {
+    const int n = side ? p.nl : p.nr;
+    const double *tab = side ? p.lig_desolv : p.rec_desolv;
+    uint32_t *cnt = side ? s_lcnt : s_rcnt;
+    for (int i = rank * kNT + tid; i < n; i += nc * kNT) {
+      unsigned c = 0;
+      for (int r = 0; r < nc; ++r) {
+        const uint32_t *o = nc > 1 ? cluster.map_shared_rank(cnt, r) : cnt;
+        c += (o[i >> 1] >> ((i & 1) * 16)) & 0xffffu;
+      }
+      desolv.add(tab[static_cast<size_t>(i) * 11 + min(c, 10u)], p.fx_desolv);
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    vdw.add(vdw.shfl_xor(o));
+    elec.add(elec.shfl_xor(o));
+    desolv.add(desolv.shfl_xor(o));
+  }
+  if (lane == 0) {
+    s_red[warp * 3] = vdw.v;
+    s_red[warp * 3 + 1] = elec.v;
+    s_red[warp * 3 + 2] = desolv.v;
+    s_nf[warp * 3] = vdw.nf;
+    s_nf[warp * 3 + 1] = elec.nf;
+    s_nf[warp * 3 + 2] = desolv.nf;
+  }
+  if (nc > 1) cluster.sync();
+  else __syncthreads();
+  if (rank == 0 && tid < 32) {
+    ExactSum t[3];
+    for (int w = lane; w < nc * kNW; w += 32)
+      for (int c = 0; c < 3; ++c) {
+        const int at = (w % kNW) * 3 + c;
+        t[c].v += nc > 1 ? *cluster.map_shared_rank(s_red + at, w / kNW) : s_red[at];
+        t[c].nf += nc > 1 ? *cluster.map_shared_rank(s_nf + at, w / kNW) : s_nf[at];
+      }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      for (int c = 0; c < 3; ++c) t[c].add(t[c].shfl_xor(o));
+    if (lane == 0)
+      write_pose(p, pose, t[0].value(p.fx_vdw), 332.0636 * t[1].value(p.fx_elec), t[2].value(p.fx_desolv), *s_air, *s_sat);
+  }
+  if (nc > 1) cluster.sync();  // the shared memory read above stays until here
 }
 
 // ------------------------------------------------------------ dispatch ----
 
-constexpr int kNT = 256;
-
 template <typename Kern>
-cudaError_t launch_kernel(Kern kern, int n, size_t smem, int sm_count, cudaStream_t stream, const ScoreParams &p,
-                          int *grid_out) {
+cudaError_t launch_f64(Kern kern, const ScoreParams &p, int sm_count, cudaStream_t stream) {
+  const size_t smem = f64_smem(p.nr, p.nl).total;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return e;
-  int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kNT, smem);
-  if (e != cudaSuccess) return e;
-  if (per_sm < 1) return cudaErrorInvalidConfiguration;
-  const int grid = std::max(1, std::min(n, per_sm * sm_count));
-  if (grid_out) *grid_out = grid;
-  kern<<<grid, kNT, smem, stream>>>(p);
-  return cudaGetLastError();
-}
-
-template <int S>
-cudaError_t launch_f64(const ScoreParams &p, bool serial, bool clamp, size_t smem, int sm, cudaStream_t st) {
-  if (!serial && !clamp) return launch_kernel(k_score_f64<kNT, S, false, false>, p.n_poses, smem, sm, st, p, nullptr);
-  if (serial && !clamp) return launch_kernel(k_score_f64<kNT, S, true, false>, p.n_poses, smem, sm, st, p, nullptr);
-  if (!serial && clamp) return launch_kernel(k_score_f64<kNT, S, false, true>, p.n_poses, smem, sm, st, p, nullptr);
-  return launch_kernel(k_score_f64<kNT, S, true, true>, p.n_poses, smem, sm, st, p, nullptr);
+  // CTAs per pose: eight for every SM over the launch (poses differ widely in
+  // work), as far as a cluster and the pose's blocks go; blocks per unit: 32
+  // units or more for every warp, so that the last ones leave few warps
+  // waiting.  Half the CTAs and units four times as large took 3.97 ms instead
+  // of 3.25 on 150 poses of 2,538 x 1,280 atoms (warps waiting at the end of
+  // their pose).
+  const long long slots = std::max(1, (std::min(p.nl, kLigCap) + 31) / 32), blocks = std::max(1, (p.nr + 31) / 32);
+  int nc = 1;
+  while (nc < kMaxCluster && static_cast<long long>(p.n_poses) * nc * 2 <= 8LL * sm_count && slots * blocks > 4 * kNW * nc)
+    nc *= 2;
+  const int grain = static_cast<int>(std::max(1LL, std::min<long long>(kGrainMax, slots * blocks / (32LL * kNW * nc))));
+  if (nc > 8) {
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.blockDim = dim3(kNT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  for (;; nc /= 2) {
+    at.val.clusterDim.x = static_cast<unsigned>(nc);
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(static_cast<unsigned>(p.n_poses) * nc);
+    if (nc == 1) break;
+    // a cluster this large may not fit beside the shared memory it needs
+    int fit = 0;
+    if (cudaOccupancyMaxActiveClusters(&fit, kern, &cfg) == cudaSuccess && fit > 0) break;
+    (void)cudaGetLastError();
+  }
+  if (nc == 1) cfg.numAttrs = 0;
+  return cudaLaunchKernelEx(&cfg, kern, p, grain);
 }
 
 }  // namespace
@@ -242,7 +525,6 @@ ScoreParams make_params(gd_complex *cx, const gd_pose_frame *d_frames, const dou
   p.rec_meta16 = cx->rec_meta16;
   p.rec_desolv = cx->rec_desolv;
   p.nr = cx->nr;
-  p.n_tiles = cx->nr_pad / kTile;
   p.lig_perm = cx->lig_perm;
   p.lig_slot_sph = cx->lig_slot_sph;
   p.rec_seg = cx->rec_seg;
@@ -263,6 +545,9 @@ ScoreParams make_params(gd_complex *cx, const gd_pose_frame *d_frames, const dou
   p.oz = cx->oz;
   p.tab32 = cx->tab32;
   p.tab64 = cx->tab64;
+  p.fx_vdw = cx->fx_vdw;
+  p.fx_elec = cx->fx_elec;
+  p.fx_desolv = cx->fx_desolv;
   p.nt = cx->nt;
   p.need_clamp = cx->need_clamp;
   p.restr_rec = cx->restr_rec;
@@ -283,23 +568,25 @@ ScoreParams make_params(gd_complex *cx, const gd_pose_frame *d_frames, const dou
 }
 
 gd_status launch_score(gd_complex *cx, const gd_pose_frame *d_frames, const double *d_models, int n,
-                       gd_precision prec, gd_pose_energy *d_out, cudaStream_t stream, double max_disp) {
+                       gd_precision prec, gd_pose_energy *d_out, cudaStream_t stream, double max_disp,
+                       const int *skip) {
   gd_context *ctx = cx->ctx;
   if (n <= 0) return GD_OK;
-  const ScoreParams p = make_params(cx, d_frames, d_models, n, d_out, max_disp);
+  ScoreParams p = make_params(cx, d_frames, d_models, n, d_out, max_disp);
+  p.skip = skip;
   const bool serial = cx->serial_overlap, clamp = cx->need_clamp;
   if (prec == GD_PREC_F32)
     return launch_score_batch_f32(ctx, std::vector<ScoreParams>{p}, serial, clamp,
                                   ctx->tune_f32_slots ? ctx->tune_f32_slots : kDefaultF32Tune, stream);
+  // the band is first order in the coordinates' FP32 rounding: beyond 1 A^2
+  // (coordinates some 40,000 A from the origin, or not finite) FP32 drops
+  // nothing and every pair is decided in FP64
+  if (!(p.guard_e <= 1.0f)) p.guard_e = p.guard_v = INFINITY;
   cudaError_t e;
-  const size_t smem = smem_layout<D4>(p.nt, p.nr, kNT, sizeof(D4)).total;
-  const int S = std::max(1, std::min(4, (p.nl + kNT - 1) / kNT));
-  switch (S) {
-    case 1: e = launch_f64<1>(p, serial, clamp, smem, ctx->sm_count, stream); break;
-    case 2: e = launch_f64<2>(p, serial, clamp, smem, ctx->sm_count, stream); break;
-    case 3: e = launch_f64<3>(p, serial, clamp, smem, ctx->sm_count, stream); break;
-    default: e = launch_f64<4>(p, serial, clamp, smem, ctx->sm_count, stream); break;
-  }
+  if (serial) e = clamp ? launch_f64(k_score_f64<true, true>, p, ctx->sm_count, stream)
+                        : launch_f64(k_score_f64<true, false>, p, ctx->sm_count, stream);
+  else e = clamp ? launch_f64(k_score_f64<false, true>, p, ctx->sm_count, stream)
+                 : launch_f64(k_score_f64<false, false>, p, ctx->sm_count, stream);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "score kernel launch");
   return GD_OK;
 }

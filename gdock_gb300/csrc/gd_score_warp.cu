@@ -175,11 +175,6 @@ __device__ __forceinline__ void count_if_lt64(int &a, int &b, float d2) {
       : "f"(d2));
 }
 
-__device__ __forceinline__ float d2f(const float4 &r, float lx, float ly, float lz) {
-  const float dx = __fsub_rn(r.x, lx), dy = __fsub_rn(r.y, ly), dz = __fsub_rn(r.z, lz);
-  return __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
-}
-
 // soft-core LJ in FP32 (src/fitness.rs:57-70): eps*(q^2 - 2q) with
 // q = R6/(r^6 + R6/2), evaluated as 4 eps x (x - 1) = 4 eps (x^2 - x),
 // x = q/2 = 1/(r^6 2/R6 + 1); at d2 = 0 it is exactly 0
@@ -810,42 +805,10 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_score_f32w(const BatchPar
     const double vdw_t = static_cast<double>(warp_sum_ll(vdw_i)) * 0x1p-32;
     const double elec_t = static_cast<double>(warp_sum_ll(elec_i)) * 0x1p-32;
     desolv_t = warp_sum(desolv_t);
-    // AIR: one restraint per lane, summed in restraint order
-    double air = 0.0;
-    int sat = 0;
-    for (int r0 = 0; r0 < p.K; r0 += 32) {
-      double term = 0.0;
-      int ok = 0;
-      const int r = r0 + lane;
-      if (r < p.K) {
-        const D4 a = p.restr_rec[r];
-        double X, Y, Z;
-        ligand_atom(p, f, pose, p.restr_lig[r], X, Y, Z);
-        const double dist = sqrt(exact_d2(a.x, a.y, a.z, X, Y, Z));
-        double v = 0.0;
-        if (dist < 0.0) v = __dsub_rn(0.0, dist);
-        else if (dist > 7.0) v = __dsub_rn(dist, 7.0);
-        term = __dmul_rn(__dmul_rn(10.0, v), v);
-        ok = dist <= 7.0;
-      }
-      for (int k = 0; k < 32 && r0 + k < p.K; ++k) {
-        air = __dadd_rn(air, __shfl_sync(kFull, term, k));
-        sat += __shfl_sync(kFull, ok, k);
-      }
-    }
-    if (lane == 0) {
-      const double ratio = p.K > 0 ? static_cast<double>(sat) / static_cast<double>(p.K) : 0.0;
-      gd_pose_energy o;
-      o.vdw = vdw_t;
-      o.elec = elec_t;
-      o.desolv = desolv_t;
-      o.air = air;
-      o.restraint_penalty = __dmul_rn(__dsub_rn(1.0, ratio), static_cast<double>(p.K));
-      o.fitness = __dadd_rn(
-          __dadd_rn(__dadd_rn(__dmul_rn(p.wv, vdw_t), __dmul_rn(p.we, elec_t)), __dmul_rn(p.wd, desolv_t)),
-          __dmul_rn(p.wa, air));
-      p.out[pose] = o;
-    }
+    double air;
+    int sat;
+    warp_air(p, f, pose, lane, air, sat);
+    if (lane == 0) write_pose(p, pose, vdw_t, elec_t, desolv_t, air, sat);
     __syncwarp();
   }
 }

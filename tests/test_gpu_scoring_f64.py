@@ -1,0 +1,75 @@
+"""The plain FP64 form where its work split can go wrong: sizes around the
+32-atom slots, blocks and segments and around the ligand atoms held at once,
+launches of one pose to several hundred (clusters of sixteen CTAs down to
+one), coordinates that FP32 cannot resolve and poses that are not finite.
+
+Tolerance: 1e-12 relative to max(|E|, 1 kcal/mol), the bound of the other FP64
+tests (the terms differ from the oracle's by a few FP64 roundings each); the
+same pose gives the same bits in every launch."""
+import numpy as np
+import pytest
+
+import gdock_gb300 as gd
+from gdock_gb300 import synth
+from test_gpu_scoring import F64_TOL, _first_atoms, check
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def big():
+    return synth.make_complex(60, 300, 8, seed=41)
+
+
+@pytest.mark.parametrize("nr,nl", [(1, 1), (31, 33), (32, 32), (33, 31), (64, 65), (65, 1023), (97, 1024), (128, 1025),
+                                   (300, 2050)])
+def test_sizes_and_launches(oracle, big, nr, nl):
+    rec, lig = _first_atoms(big.receptor, nr), _first_atoms(big.ligand, nl)
+    lig = gd.position_ligand(rec, lig)
+    genes = synth.random_genes(np.random.default_rng(nr + nl), 320, max_displacement=9.0)
+    cx = gd.Complex(rec, lig, big.restraint_pairs)
+    all_of = cx.score_poses(genes)
+    check(all_of[:12], oracle.score_poses(rec, lig, big.restraint_pairs, genes[:12]), F64_TOL)
+    for n in (1, 2, 11, 40, 170):
+        assert cx.score_poses(genes[:n]).tobytes() == all_of[:n].tobytes(), n
+    models = np.stack([np.stack(oracle.apply_genes(lig, g), axis=1) for g in genes[:12]])
+    assert cx.score_models(models).tobytes() == all_of[:12].tobytes()
+
+
+@pytest.mark.parametrize("shift", [3000.0, 1.0e5, 3.0e9])
+def test_far_from_the_origin(oracle, big, shift):
+    """Coordinates far from zero, up to where FP32 cannot tell atoms apart."""
+    rec, lig = _first_atoms(big.receptor, 120), _first_atoms(big.ligand, 90)
+    rec = rec.with_coords(rec.x + shift, rec.y - shift, rec.z)
+    lig = gd.position_ligand(rec, lig)
+    genes = synth.random_genes(np.random.default_rng(3), 6, max_displacement=9.0)
+    genes[3, 3] = 2.0 * shift  # a pose far away widens the others' bands, too
+    cx = gd.Complex(rec, lig, [])
+    check(cx.score_poses(genes), oracle.score_poses(rec, lig, [], genes), F64_TOL)
+
+
+def check_nan(e, ref):
+    """check(), with the oracle's NaN and infinities where it has them."""
+    for k, name in enumerate(("fitness", "vdw", "elec", "desolv", "air", "restraint_penalty")):
+        np.testing.assert_allclose(e[name], ref[:, k], rtol=F64_TOL, atol=F64_TOL, err_msg=name)
+
+
+def test_poses_that_are_not_finite(oracle, big):
+    rec, lig = _first_atoms(big.receptor, 120), _first_atoms(big.ligand, 90)
+    lig = gd.position_ligand(rec, lig)
+    genes = synth.random_genes(np.random.default_rng(4), 6, max_displacement=9.0)
+    genes[1, 3], genes[2, 0], genes[4, 4] = np.inf, np.nan, 1.0e300
+    cx = gd.Complex(rec, lig, big.restraint_pairs)
+    check_nan(cx.score_poses(genes), oracle.score_poses(rec, lig, big.restraint_pairs, genes))
+
+
+def test_coincident_atoms_and_vanishing_radii(oracle):
+    """Atoms on top of each other (a distance of zero has no vdW and no
+    Coulomb term but buries) and Rmin/2 of zero (no vdW energy, but the
+    reference's 0 / 0 where r^6 underflows)."""
+    from conftest import make_mol, tatom
+    rec = make_mol([tatom(float(k), 0, 0, "O", charge=0.5, rmin2=0.0 if k % 2 else 1.8, serial=1 + k) for k in range(5)])
+    lig = make_mol([tatom(float(k), 0, 0, "N", charge=-0.25, rmin2=0.0 if k < 3 else 2.0, serial=100 + k) for k in range(5)])
+    cx = gd.Complex(rec, lig, [])
+    xyz = np.stack([lig.xyz(), lig.xyz() + 1.0e-160, lig.xyz() + [0.0, 1.0e-9, 0.0]])
+    check_nan(cx.score_models(xyz), oracle.score_models(rec, lig, [], xyz))
