@@ -109,6 +109,45 @@ static __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
+// Exact sum of FP64 values as a fixed-point integer with 2^-bits resolution
+// (bits leaves room for the largest sum expected); values that are not finite,
+// or of more than 2^(kMaxShift + 53 - bits), are kept apart in FP64.
+template <int kMaxShift = 70>
+struct ExactSum {
+  __int128 v = 0;
+  double nf = 0.0;
+  __device__ __forceinline__ void add(double x, int bits) {
+    const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(x));
+    const int e = static_cast<int>(b >> 52) & 0x7ff;
+    if (e == 0) return;  // zero (a subnormal is far below the resolution)
+    const int sh = e - 1075 + bits;
+    if (e == 0x7ff || sh > kMaxShift) {
+      nf += x;
+      return;
+    }
+    const unsigned long long m = (b & 0xfffffffffffffull) | 0x10000000000000ull;
+    const unsigned __int128 t = sh >= 0 ? static_cast<unsigned __int128>(m) << sh
+                                        : static_cast<unsigned __int128>(m >> min(-sh, 63));
+    v += static_cast<long long>(b) < 0 ? -static_cast<__int128>(t) : static_cast<__int128>(t);
+  }
+  // every lane: the sum over the warp
+  __device__ __forceinline__ void warp_total() {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long lo = __shfl_xor_sync(kFull, static_cast<unsigned long long>(v), o);
+      const long long hi = __shfl_xor_sync(kFull, static_cast<long long>(v >> 64), o);
+      v += (static_cast<__int128>(hi) << 64) | lo;
+    }
+    if (__any_sync(kFull, __double_as_longlong(nf) != 0)) nf = warp_sum(nf);
+  }
+  __device__ __forceinline__ double value(int bits) const {
+    const double hi = static_cast<double>(static_cast<long long>(v >> 64)),
+                 lo = static_cast<double>(static_cast<unsigned long long>(v));
+    const double s = ldexp(hi * 18446744073709551616.0 + lo, -bits);
+    return nf != 0.0 ? nf + s : s;
+  }
+};
+
 // FP32 squared distance of a receptor atom and a ligand atom (both relative to O).
 static __device__ __forceinline__ float d2f(const float4 &r, float lx, float ly, float lz) {
   const float dx = __fsub_rn(r.x, lx), dy = __fsub_rn(r.y, ly), dz = __fsub_rn(r.z, lz);

@@ -14,9 +14,12 @@
 //     interface), and the receptor atoms whose contact with it has a native
 //     identity (a docked contact counts once when it is native); ligand atoms
 //     with none of these are left out.
-// Device (k_dockq): one warp per pose; each ligand atom moved once, exactly
-// (FP64, the reference's operation order); distances sqrt(d2) with d2 in the
-// reference's order; contact decisions against the exact d2 threshold of 5 A.
+// Device (k_dockq): the lanes of one warp (or of eight, for few poses) take a
+// pose's ligand atoms; per atom the difference from its partner is one chain
+// of fused multiply-adds, the distance its square root, the sums exact integer
+// ones; contacts are decided in FP32 outside a guard band and exactly (the
+// reference's transform and threshold) inside it, and distances that
+// cancellation would spoil (below 1/4 A) are redone in the reference's order.
 //   rmsd  = sqrt(sum over pairs of distance / |reference|)    (src/evaluator.rs:86-103;
 //   irmsd = likewise over the interface pairings               the sum is of distances)
 //   fnat  = docked native contacts / |native contacts|
@@ -38,9 +41,13 @@ struct gd_evaluator {
   int n_p = 0;                            // native-identity (receptor atom, ligand atom) pairs
   int64_t counts[GD_EVAL_COUNTS] = {};    // as gd_evaluator_counts reports them
   const int *u_slot = nullptr;            // [n_u] device slot of each such ligand atom (interface atoms first)
-  const D4 *u_ref = nullptr, *u_iref = nullptr;  // [n_u] paired reference atom (w = 1) or none (w = 0)
-  const int *u_pbeg = nullptr;            // [n_u + 1] CSR offsets into p_rec
+  int n_if = 0;                           // the first n_if of them have an i-RMSD partner or native contacts
+  const D4 *u_x0 = nullptr;               // [n_u] ligand atom relative to the rotation centre
+  const D4 *u_ref = nullptr;              // [n_u] paired reference atom (w = 1) or none (w = 0)
+  const D4 *u_iref = nullptr;             // [n_if] likewise; w = 2: the same atom as u_ref
+  const int *u_pbeg = nullptr;            // [n_if + 1] CSR offsets into p_rec
   const D4 *p_rec = nullptr;              // [n_p] receptor atoms whose contact with the ligand atom is native
+  const float4 *p_rec32 = nullptr;        // [n_p] the same, FP32 relative to the origin O
   double thr5 = 0.0;
   void *block = nullptr;
   size_t bytes = 0;
@@ -52,60 +59,195 @@ namespace {
 struct EvalParams {
   ScoreParams p;  // ligand arrays, frames and the rotation centre
   const int *u_slot, *u_pbeg;
-  const D4 *u_ref, *u_iref, *p_rec;
-  int n_u, n_ref, n_iref, n_native;
+  const D4 *u_x0, *u_ref, *u_iref, *p_rec;
+  const float4 *p_rec32;
+  int n_u, n_if, n_ref, n_iref, n_native;
   double thr5;
+  float extent;     // bounds |coordinate - O| of receptor and ligand atoms before the displacement
   const int *skip;  // nonzero: no work (a finished GA job); may be null
   gd_dock_metrics *out;
 };
 
-constexpr int kEvalWarps = 4;
+constexpr int kEvalWarps = 8;
+constexpr int kEvalCtas = 2;    // resident per SM (registers)
+// distance sums: a resolution of 2^-96 A (at the native pose the distances
+// are rounding noise of some 1e-15 A), 2^31 A of room, single distances from
+// 2^14 A on kept apart
+constexpr int kDistBits = 96;
+using DistSum = ExactSum<57>;
 
-// One warp per pose; each lane moves its ligand atoms once and uses each for
-// the L-RMSD pairing, the i-RMSD pairing and its native-identity contacts.
-__global__ void __launch_bounds__(kEvalWarps * 32) k_dockq(const EvalParams e) {
-  const int lane = threadIdx.x & 31;
-  const int pose = blockIdx.x * kEvalWarps + (threadIdx.x >> 5);
-  if (pose >= e.p.n_poses || (e.skip && *e.skip)) return;
-  gd_pose_frame f;
-  {
-    const double *src = reinterpret_cast<const double *>(e.p.frames + pose);
-    double *dst = reinterpret_cast<double *>(&f);
-#pragma unroll
-    for (int k = 0; k < 16; ++k) dst[k] = src[k];
-  }
-  double sl = 0.0, si = 0.0;
-  int common = 0;
-  for (int u = lane; u < e.n_u; u += 32) {
-    double X, Y, Z;
-    int slot = e.u_slot[u];
-    if (!GD_DCHECK(e.p.err, slot >= 0 && slot < e.p.nl, 40)) slot = 0;
-    ligand_atom(e.p, f, pose, slot, X, Y, Z);
-    const D4 r = e.u_ref[u], q = e.u_iref[u];
-    // ligand atom first, as atom1.distance_to(atom2) (src/evaluator.rs:96-100)
-    if (r.w != 0.0) sl += sqrt(exact_d2(X, Y, Z, r.x, r.y, r.z));
-    if (q.w != 0.0) si += sqrt(exact_d2(X, Y, Z, q.x, q.y, q.z));
-    const int k1 = e.u_pbeg[u + 1];
-    for (int k = e.u_pbeg[u]; k < k1; ++k) {
-      const D4 a = e.p_rec[k];  // receptor atom first, as calculate_contacts (src/evaluator.rs:150-152)
-      common += exact_d2(a.x, a.y, a.z, X, Y, Z) <= e.thr5;
+// The distance of ligand atom `slot` and (rx, ry, rz) as the reference forms
+// it (exact transform, distance_to): out of line, few atoms come here.
+__device__ __noinline__ double exact_distance(const ScoreParams &p, const gd_pose_frame &f, int pose, int slot,
+                                              double rx, double ry, double rz) {
+  double X, Y, Z;
+  ligand_atom(p, f, pose, slot, X, Y, Z);
+  return sqrt(exact_d2(X, Y, Z, rx, ry, rz));  // ligand atom first (src/evaluator.rs:96-100)
+}
+
+// The reference's contact decision (receptor atom first, src/evaluator.rs:150-152).
+__device__ __noinline__ bool exact_contact(const ScoreParams &p, const gd_pose_frame &f, int pose, int slot, const D4 &a,
+                                           double thr5) {
+  double X, Y, Z;
+  ligand_atom(p, f, pose, slot, X, Y, Z);
+  return exact_d2(a.x, a.y, a.z, X, Y, Z) <= thr5;
+}
+
+// sqrt(d2) for d2 in [1/16, 2^900): s (1 - e)^(-1/2) by its Taylor series to
+// the second order on the hardware's approximation y of d2^(-1/2), with
+// s = d2 y and e = 1 - s y (about 2^-20, so that the next term lies below the
+// FP64 rounding): five FP64 operations.
+__device__ __forceinline__ double sqrt64(double d2) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d2));
+  const double s = d2 * y, e = __fma_rn(-s, y, 1.0);
+  return __fma_rn(s, e * __fma_rn(e, 0.375, 0.5), s);
+}
+
+// What bounds it: the FP64 pipe.  The reference's transform, difference,
+// square and correctly rounded root cost about 60 FP64 operations per atom;
+// this form takes 12 for the difference, 3 and 5 for square and root and adds
+// in integers.  WPP warps per pose: one where the poses fill the GPU, else the
+// whole CTA (150 poses of one warp each kept 38 of the 152 SMs waiting on
+// FP64 latency).
+// 65,536 poses of 2,538 x 1,280 atoms (the whole call, host frames and copies
+// included) 10.8 -> 4.32 ms; the kernel on 150 poses of 1,074 x 741 atoms 99 ->
+// 18 us.
+template <int WPP>
+__global__ void __launch_bounds__(kEvalWarps * 32, kEvalCtas) k_dockq(const EvalParams e) {
+  if (e.skip && *e.skip) return;
+  __shared__ gd_pose_frame s_f[kEvalWarps / WPP];
+  __shared__ __int128 s_sum[kEvalWarps][2];
+  __shared__ double s_nf[kEvalWarps][2];
+  __shared__ int s_common[kEvalWarps];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int step = gridDim.x * (kEvalWarps / WPP);
+  const int t0 = WPP == 1 ? lane : static_cast<int>(threadIdx.x);
+  gd_pose_frame &f = s_f[WPP == 1 ? warp : 0];
+  // lane k keeps the k-th pose's sums until the warp has 32 of them: the
+  // divisions and roots of the metrics then run on all lanes
+  DistSum my_l, my_i;
+  int my_common = 0, my_pose = -1, held = 0;
+  auto finish = [&]() {
+    if (my_pose >= 0) {
+      // src/evaluator.rs:68-84, without contraction into fused multiply-adds
+      const double sl = my_l.value(kDistBits), si = my_i.value(kDistBits);
+      const double rmsd = e.n_ref ? __dsqrt_rn(__ddiv_rn(sl, static_cast<double>(e.n_ref))) : 0.0;
+      const double irmsd = e.n_iref ? __dsqrt_rn(__ddiv_rn(si, static_cast<double>(e.n_iref))) : 0.0;
+      const double fnat = e.n_native ? __ddiv_rn(static_cast<double>(my_common), static_cast<double>(e.n_native)) : 0.0;
+      const double a = __ddiv_rn(irmsd, 1.5), b = __ddiv_rn(rmsd, 8.5);
+      const double is = __ddiv_rn(1.0, __dadd_rn(1.0, __dmul_rn(a, a)));
+      const double ls = __ddiv_rn(1.0, __dadd_rn(1.0, __dmul_rn(b, b)));
+      const double dockq = __ddiv_rn(__dadd_rn(__dadd_rn(fnat, is), ls), 3.0);
+      e.out[my_pose] = gd_dock_metrics{rmsd, irmsd, fnat, dockq};
+    }
+    my_pose = -1;
+    held = 0;
+  };
+  for (int pose = blockIdx.x * (kEvalWarps / WPP) + (WPP == 1 ? warp : 0); pose < e.p.n_poses; pose += step) {
+    if (WPP == 1) __syncwarp();
+    else __syncthreads();
+    if (t0 < 16) reinterpret_cast<double *>(&f)[t0] = reinterpret_cast<const double *>(e.p.frames + pose)[t0];
+    if (WPP == 1) __syncwarp();
+    else __syncthreads();
+    // moved atom = R x0 + (centre + displacement)
+    const double m00 = f.ca * f.cb, m01 = f.m01, m02 = f.m02, m10 = f.sa * f.cb, m11 = f.m11, m12 = f.m12;
+    const double m20 = -f.sb, m21 = f.cb * f.sg, m22 = f.cb * f.cg;
+    const double tx = e.p.cx + f.dx, ty = e.p.cy + f.dy, tz = e.p.cz + f.dz;
+    // the FP32 guard band of the contact test, as for the contact bitmaps
+    // (M bounds the coordinates; twice it covers the sum that forms them)
+    const float M = 2.0f * (e.extent + fmaxf(fabsf(static_cast<float>(f.dx)),
+                                             fmaxf(fabsf(static_cast<float>(f.dy)), fabsf(static_cast<float>(f.dz)))));
+    const float guard = 4.0f * (17.33f * (2.0f * M + 5.0f) + 100.0f) * 0x1p-24f + 1e-6f;
+    const bool band_ok = guard < 1.0f;
+    DistSum sl, si;
+    int common = 0;
+#pragma unroll 1
+    for (int u = t0; u < e.n_u; u += 32 * WPP) {
+      const D4 a = e.u_x0[u], r = e.u_ref[u];
+      auto from = [&](const D4 &q, double &dx, double &dy, double &dz) {
+        dx = __fma_rn(m00, a.x, __fma_rn(m01, a.y, __fma_rn(m02, a.z, tx - q.x)));
+        dy = __fma_rn(m10, a.x, __fma_rn(m11, a.y, __fma_rn(m12, a.z, ty - q.y)));
+        dz = __fma_rn(m20, a.x, __fma_rn(m21, a.y, __fma_rn(m22, a.z, tz - q.z)));
+      };
+      auto distance = [&](const D4 &q, double dx, double dy, double dz) {
+        const double d2 = __fma_rn(dz, dz, __fma_rn(dy, dy, dx * dx));
+        const int hi = __double2hiint(d2);
+        if (hi < 0x3fb00000 || hi >= 0x78300000) {  // below 1/16, or from 2^900 (and NaN) on
+          int slot = e.u_slot[u];
+          if (!GD_DCHECK(e.p.err, slot >= 0 && slot < e.p.nl, 40)) slot = 0;
+          return exact_distance(e.p, f, pose, slot, q.x, q.y, q.z);
+        }
+        return sqrt64(d2);
+      };
+      double dx, dy, dz;
+      from(r, dx, dy, dz);
+      double d = 0.0;
+      if (r.w != 0.0) {
+        d = distance(r, dx, dy, dz);
+        sl.add(d, kDistBits);
+      }
+      if (u < e.n_if) {
+        const D4 q = e.u_iref[u];
+        if (q.w == 2.0) {
+          si.add(d, kDistBits);
+        } else if (q.w != 0.0) {
+          double ex, ey, ez;
+          from(q, ex, ey, ez);
+          si.add(distance(q, ex, ey, ez), kDistBits);
+        }
+        int k = e.u_pbeg[u];
+        const int k1 = e.u_pbeg[u + 1];
+        if (k < k1) {
+          const float lx = static_cast<float>(dx) + static_cast<float>(r.x - e.p.ox),
+                      ly = static_cast<float>(dy) + static_cast<float>(r.y - e.p.oy),
+                      lz = static_cast<float>(dz) + static_cast<float>(r.z - e.p.oz);
+          for (; k < k1; ++k) {
+            const float t = d2f(__ldg(&e.p_rec32[k]), lx, ly, lz) - 25.0f;
+            bool hit = t < 0.0f;
+            if (!(band_ok && fabsf(t) > guard)) {
+              int slot = e.u_slot[u];
+              if (!GD_DCHECK(e.p.err, slot >= 0 && slot < e.p.nl, 40)) slot = 0;
+              hit = exact_contact(e.p, f, pose, slot, e.p_rec[k], e.thr5);
+            }
+            common += hit;
+          }
+        }
+      }
+    }
+    sl.warp_total();
+    si.warp_total();
+    common = __reduce_add_sync(kFull, common);
+    if (WPP > 1) {
+      if (lane == 0) {
+        s_sum[warp][0] = sl.v;
+        s_sum[warp][1] = si.v;
+        s_nf[warp][0] = sl.nf;
+        s_nf[warp][1] = si.nf;
+        s_common[warp] = common;
+      }
+      __syncthreads();
+      if (warp == 0) {
+        for (int w = 1; w < WPP; ++w) {
+          sl.v += s_sum[w][0];
+          si.v += s_sum[w][1];
+          sl.nf += s_nf[w][0];
+          si.nf += s_nf[w][1];
+          common += s_common[w];
+        }
+      }
+    }
+    if (WPP == 1 || warp == 0) {
+      if (lane == held) {
+        my_l = sl;
+        my_i = si;
+        my_common = common;
+        my_pose = pose;
+      }
+      if (++held == 32) finish();
     }
   }
-  sl = warp_sum(sl);
-  si = warp_sum(si);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) common += __shfl_xor_sync(kFull, common, o);
-  if (lane == 0) {
-    // src/evaluator.rs:68-84, without contraction into fused multiply-adds
-    const double rmsd = e.n_ref ? __dsqrt_rn(__ddiv_rn(sl, static_cast<double>(e.n_ref))) : 0.0;
-    const double irmsd = e.n_iref ? __dsqrt_rn(__ddiv_rn(si, static_cast<double>(e.n_iref))) : 0.0;
-    const double fnat = e.n_native ? __ddiv_rn(static_cast<double>(common), static_cast<double>(e.n_native)) : 0.0;
-    const double a = __ddiv_rn(irmsd, 1.5), b = __ddiv_rn(rmsd, 8.5);
-    const double is = __ddiv_rn(1.0, __dadd_rn(1.0, __dmul_rn(a, a)));
-    const double ls = __ddiv_rn(1.0, __dadd_rn(1.0, __dmul_rn(b, b)));
-    const double dockq = __ddiv_rn(__dadd_rn(__dadd_rn(fnat, is), ls), 3.0);
-    e.out[pose] = gd_dock_metrics{rmsd, irmsd, fnat, dockq};
-  }
+  if (WPP == 1 || warp == 0) finish();
 }
 
 double host_dist(double ax, double ay, double az, double bx, double by, double bz) {
@@ -124,17 +266,30 @@ gd_status launch_dockq(gd_evaluator *ev, const gd_pose_frame *d_frames, int n, g
   ep.p = make_params(ev->cx, d_frames, nullptr, n, nullptr, 0.0);
   ep.u_slot = ev->u_slot;
   ep.u_pbeg = ev->u_pbeg;
+  ep.u_x0 = ev->u_x0;
   ep.u_ref = ev->u_ref;
   ep.u_iref = ev->u_iref;
   ep.p_rec = ev->p_rec;
+  ep.p_rec32 = ev->p_rec32;
   ep.n_u = ev->n_u;
+  ep.n_if = ev->n_if;
   ep.n_ref = ev->n_ref;
   ep.n_iref = ev->n_iref;
   ep.n_native = ev->n_native;
   ep.thr5 = ev->thr5;
+  const gd_complex *cx = ev->cx;
+  const double m = std::max(cx->rec_extent, cx->lig_radius + std::max({std::fabs(cx->cx - cx->ox), std::fabs(cx->cy - cx->oy),
+                                                                      std::fabs(cx->cz - cx->oz)})) + 1.0;
+  ep.extent = static_cast<float>(m * (1.0 + 1e-6));
   ep.skip = skip;
   ep.out = d_out;
-  k_dockq<<<(n + kEvalWarps - 1) / kEvalWarps, kEvalWarps * 32, 0, stream>>>(ep);
+  // one warp per pose when the poses give every resident warp one, else a CTA
+  // per pose
+  const int warps = kEvalCtas * kEvalWarps * ev->ctx->sm_count;
+  if (n >= warps)
+    k_dockq<1><<<std::min((n + kEvalWarps - 1) / kEvalWarps, warps / kEvalWarps), kEvalWarps * 32, 0, stream>>>(ep);
+  else
+    k_dockq<kEvalWarps><<<n, kEvalWarps * 32, 0, stream>>>(ep);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? GD_OK : cuda_fail(ev->ctx, e, "evaluator launch");
 }
@@ -215,21 +370,35 @@ gd_status gd_evaluator_create(gd_complex *cx, const gd_atoms *reference, const u
     return group(x) != group(y) ? group(x) < group(y) : cx->h_lig_slot[x] < cx->h_lig_slot[y];
   });
   const int nu = static_cast<int>(order.size());
-  std::vector<int> u_slot(nu), u_pbeg(nu + 1, 0);
-  std::vector<D4> u_ref(nu), u_iref(nu), p_rec;
+  int n_if = 0;
+  while (n_if < nu && group(order[n_if]) == 0) ++n_if;
+  std::vector<int> u_slot(nu), u_pbeg(n_if + 1, 0);
+  std::vector<D4> u_x0(nu), u_ref(nu), u_iref(n_if), p_rec;
+  std::vector<float4> p_rec32;
   p_rec.reserve(n_p);
+  p_rec32.reserve(n_p);
   for (int u = 0; u < nu; ++u) {
     const int j = order[u];
     u_slot[u] = cx->h_lig_slot[j];
+    u_x0[u] = D4{cx->h_lx[j] - cx->cx, cx->h_ly[j] - cx->cy, cx->h_lz[j] - cx->cz, 0.0};
     u_ref[u] = l_ref[j];
+    if (u >= n_if) continue;
     u_iref[u] = l_iref[j];
-    for (int a : l_rec[j]) p_rec.push_back(D4{cx->h_rx[a], cx->h_ry[a], cx->h_rz[a], 0.0});
+    if (l_ref[j].w != 0.0 && l_iref[j].w != 0.0 && l_ref[j].x == l_iref[j].x && l_ref[j].y == l_iref[j].y &&
+        l_ref[j].z == l_iref[j].z)
+      u_iref[u].w = 2.0;
+    for (int a : l_rec[j]) {
+      p_rec.push_back(D4{cx->h_rx[a], cx->h_ry[a], cx->h_rz[a], 0.0});
+      p_rec32.push_back(make_float4(static_cast<float>(cx->h_rx[a] - cx->ox), static_cast<float>(cx->h_ry[a] - cx->oy),
+                                    static_cast<float>(cx->h_rz[a] - cx->oz), 0.0f));
+    }
     u_pbeg[u + 1] = static_cast<int>(p_rec.size());
   }
   gd_evaluator *ev = new gd_evaluator();
   ev->cx = cx;
   ev->ctx = ctx;
   ev->n_u = nu;
+  ev->n_if = n_if;
   ev->n_ref = nf;
   ev->n_iref = static_cast<int>(ref_i.size());
   ev->n_native = n_native;
@@ -240,9 +409,10 @@ gd_status gd_evaluator_create(gd_complex *cx, const gd_atoms *reference, const u
                                        static_cast<int64_t>(std::min(lig_i.size(), ref_i.size())), n_p};
   std::copy(cnt, cnt + GD_EVAL_COUNTS, ev->counts);
   auto al = [](size_t b) { return (std::max<size_t>(b, 1) + 255) / 256 * 256; };
-  const size_t b_slot = al(sizeof(int) * nu), b_beg = al(sizeof(int) * (nu + 1)), b_ref = al(sizeof(D4) * nu),
-               b_prec = al(sizeof(D4) * p_rec.size());
-  ev->bytes = b_slot + b_beg + 2 * b_ref + b_prec;
+  const size_t b_slot = al(sizeof(int) * nu), b_beg = al(sizeof(int) * (n_if + 1)), b_ref = al(sizeof(D4) * nu),
+               b_iref = al(sizeof(D4) * n_if), b_prec = al(sizeof(D4) * p_rec.size()),
+               b_prec32 = al(sizeof(float4) * p_rec32.size());
+  ev->bytes = b_slot + b_beg + 2 * b_ref + b_iref + b_prec + b_prec32;
   gd_status s = dev_alloc(ctx, ev->bytes, &ev->block);
   if (s != GD_OK) {
     delete ev;
@@ -257,10 +427,12 @@ gd_status gd_evaluator_create(gd_complex *cx, const gd_atoms *reference, const u
     return d;
   };
   ev->u_slot = reinterpret_cast<const int *>(put(u_slot.data(), sizeof(int) * nu, b_slot));
-  ev->u_pbeg = reinterpret_cast<const int *>(put(u_pbeg.data(), sizeof(int) * (nu + 1), b_beg));
+  ev->u_pbeg = reinterpret_cast<const int *>(put(u_pbeg.data(), sizeof(int) * (n_if + 1), b_beg));
+  ev->u_x0 = reinterpret_cast<const D4 *>(put(u_x0.data(), sizeof(D4) * nu, b_ref));
   ev->u_ref = reinterpret_cast<const D4 *>(put(u_ref.data(), sizeof(D4) * nu, b_ref));
-  ev->u_iref = reinterpret_cast<const D4 *>(put(u_iref.data(), sizeof(D4) * nu, b_ref));
+  ev->u_iref = reinterpret_cast<const D4 *>(put(u_iref.data(), sizeof(D4) * n_if, b_iref));
   ev->p_rec = reinterpret_cast<const D4 *>(put(p_rec.data(), sizeof(D4) * p_rec.size(), b_prec));
+  ev->p_rec32 = reinterpret_cast<const float4 *>(put(p_rec32.data(), sizeof(float4) * p_rec32.size(), b_prec32));
   const cudaError_t e = cudaMemcpy(ev->block, h.data(), ev->bytes, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     dev_free(ctx, ev->block, ev->bytes);

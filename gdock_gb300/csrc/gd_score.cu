@@ -92,46 +92,6 @@ __device__ __forceinline__ double rcp64(double d) {
   return __fma_rn(x, e, x);
 }
 
-// Exact sum of FP64 values as a fixed-point integer with 2^-bits resolution
-// (bits leaves room for the largest possible sum); values that are not finite
-// are kept apart (they decide the result).
-struct ExactSum {
-  __int128 v = 0;
-  double nf = 0.0;
-  __device__ __forceinline__ void add(double x, int bits) {
-    const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(x));
-    const int e = static_cast<int>(b >> 52) & 0x7ff;
-    if (e == 0) return;  // zero (a subnormal is far below the resolution)
-    if (e == 0x7ff) {
-      nf += x;
-      return;
-    }
-    const unsigned long long m = (b & 0xfffffffffffffull) | 0x10000000000000ull;
-    const int sh = e - 1075 + bits;
-    const unsigned __int128 t = sh >= 0 ? static_cast<unsigned __int128>(m) << min(sh, 74)
-                                        : static_cast<unsigned __int128>(m >> min(-sh, 63));
-    v += static_cast<long long>(b) < 0 ? -static_cast<__int128>(t) : static_cast<__int128>(t);
-  }
-  __device__ __forceinline__ void add(const ExactSum &o) {
-    v += o.v;
-    nf += o.nf;
-  }
-  __device__ __forceinline__ ExactSum shfl_xor(int o) const {
-    ExactSum r;
-    const unsigned long long lo = __shfl_xor_sync(kFull, static_cast<unsigned long long>(v), o);
-    const long long hi = __shfl_xor_sync(kFull, static_cast<long long>(v >> 64), o);
-    r.v = (static_cast<__int128>(hi) << 64) | lo;
-    r.nf = __shfl_xor_sync(kFull, nf, o);
-    return r;
-  }
-  __device__ double value(int bits) const {
-    if (nf != 0.0) return nf;  // inf or NaN
-    const double hi = static_cast<double>(static_cast<long long>(v >> 64)),
-                 lo = static_cast<double>(static_cast<unsigned long long>(v));
-    return ldexp(hi * 18446744073709551616.0 + lo, -bits);
-  }
-};
-
 // min(count, 10) is all that is read: a count that has reached 10 is left
 // alone, which also keeps the 16 bits from overflowing (at most 10 + one
 // concurrent add of each of the CTA's threads).
@@ -166,7 +126,7 @@ struct PairEval {
 
   // one listed pair per lane (on): w = receptor atom, ligand entry
   template <bool NEAR>
-  __device__ __forceinline__ void eval(bool on, uint32_t w, ExactSum &vdw, ExactSum &elec) const {
+  __device__ __forceinline__ void eval(bool on, uint32_t w, ExactSum<> &vdw, ExactSum<> &elec) const {
     if (!on) return;
     const int ri = static_cast<int>(w >> kLigBits), k = static_cast<int>(w & (kLigCap - 1));
     const double2 *rp = reinterpret_cast<const double2 *>(p.rec_pos64 + ri);
@@ -261,7 +221,7 @@ __global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const
   const float lim_e = 225.0f + p.guard_e, lim_v = 144.0f + p.guard_v;
   const float reach = sqrtf(225.01f + 2.0f * p.guard_e) + 0.01f;
   const int nblk = (p.nr + 31) / 32, ngrp = (nblk + grain - 1) / grain;
-  ExactSum vdw, elec;
+  ExactSum<> vdw, elec;
   int first = 0;  // unit counter at the start of this turn
 
   const int turns = (p.nl + kLigCap - 1) / kLigCap, turn = turns ? ((p.nl + turns - 1) / turns + 31) / 32 * 32 : 0;
@@ -423,7 +383,7 @@ __global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const
   if (nc > 1) cluster.sync();
   else __syncthreads();
   // desolvation from the cluster's summed burial counts, a share per CTA
-  ExactSum desolv;
+  ExactSum<> desolv;
   for (int side = 0; side < 2; ++side) {
     const int n = side ? p.nl : p.nr;
     const double *tab = side ? p.lig_desolv : p.rec_desolv;
@@ -437,12 +397,9 @@ __global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const
       desolv.add(tab[static_cast<size_t>(i) * 11 + min(c, 10u)], p.fx_desolv);
     }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    vdw.add(vdw.shfl_xor(o));
-    elec.add(elec.shfl_xor(o));
-    desolv.add(desolv.shfl_xor(o));
-  }
+  vdw.warp_total();
+  elec.warp_total();
+  desolv.warp_total();
   if (lane == 0) {
     s_red[warp * 3] = vdw.v;
     s_red[warp * 3 + 1] = elec.v;
@@ -454,16 +411,14 @@ __global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const
   if (nc > 1) cluster.sync();
   else __syncthreads();
   if (rank == 0 && tid < 32) {
-    ExactSum t[3];
+    ExactSum<> t[3];
     for (int w = lane; w < nc * kNW; w += 32)
       for (int c = 0; c < 3; ++c) {
         const int at = (w % kNW) * 3 + c;
         t[c].v += nc > 1 ? *cluster.map_shared_rank(s_red + at, w / kNW) : s_red[at];
         t[c].nf += nc > 1 ? *cluster.map_shared_rank(s_nf + at, w / kNW) : s_nf[at];
       }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-      for (int c = 0; c < 3; ++c) t[c].add(t[c].shfl_xor(o));
+    for (int c = 0; c < 3; ++c) t[c].warp_total();
     if (lane == 0)
       write_pose(p, pose, t[0].value(p.fx_vdw), 332.0636 * t[1].value(p.fx_elec), t[2].value(p.fx_desolv), *s_air, *s_sat);
   }

@@ -261,7 +261,8 @@ gd_status gd_evaluator_counts(const gd_evaluator *ev, int64_t *counts);
 /* Population::eval_metrics (src/population.rs:63-71): calc_metrics of the
  * ligand moved by each of n gene vectors (6 doubles each), FP64 on the GPU;
  * out[n].  Contact decisions and fnat are exact; rmsd and irmsd differ from
- * the reference's sequential sums only by summation order. */
+ * the reference's sequential sums by FP64 rounding (their distances are summed
+ * exactly; those below 1/4 A are formed in the reference's order). */
 gd_status gd_evaluate_poses(gd_evaluator *ev, const double *genes, int32_t n, gd_dock_metrics *out);
 /* gd_evaluate_poses on device-resident frames (gd_make_frames layout) into
  * device-resident metrics, asynchronously on `stream` (NULL = the context's
