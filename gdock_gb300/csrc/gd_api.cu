@@ -622,6 +622,7 @@ gd_status gd_complex_create(gd_context *ctx, const gd_atoms *rec, const gd_atoms
   cx->nr_pad = ((rec->n + kTile - 1) / kTile) * kTile;
   std::vector<float4> rp32(cx->nr_pad, make_float4(1e9f, 1e9f, 1e9f, 0.f));
   std::vector<D4> rp64(cx->nr_pad, D4{1e30, 1e30, 1e30, 0.0});
+  std::vector<FixAtom> rfix(cx->nr_pad, FixAtom{0, 0, 0, 0.0});
   std::vector<int2> rmeta(cx->nr_pad, make_int2(0, 0));
   std::vector<int4> rmeta16(cx->nr_pad, make_int4(0, 0, 0, 0));
   std::vector<double> rdes(static_cast<size_t>(std::max(rec->n, 1)) * 11, 0.0);
@@ -634,6 +635,14 @@ gd_status gd_complex_create(gd_context *ctx, const gd_atoms *rec, const gd_atoms
     rp32[k] = make_float4(static_cast<float>(rec->x[i] - o[0]), static_cast<float>(rec->y[i] - o[1]),
                           static_cast<float>(rec->z[i] - o[2]), static_cast<float>(332.0636 * rec->charge[i]));
     rp64[k] = D4{rec->x[i], rec->y[i], rec->z[i], rec->charge[i]};
+    {
+      const double m = std::max({std::fabs(rec->x[i]), std::fabs(rec->y[i]), std::fabs(rec->z[i])});
+      const bool fin = std::isfinite(rec->x[i]) && std::isfinite(rec->y[i]) && std::isfinite(rec->z[i]);
+      cx->abs_max = fin ? std::max(cx->abs_max, m) : INFINITY;
+      if (fin && m <= kFixMax)
+        rfix[k] = FixAtom{std::llrint(std::ldexp(rec->x[i], kFixBits)), std::llrint(std::ldexp(rec->y[i], kFixBits)),
+                          std::llrint(std::ldexp(rec->z[i], kFixBits)), rec->charge[i]};
+    }
     rmeta[k] = make_int2(rtype[i] * nt, rec->serial[i]);
     rmeta16[k] = make_int4(rtype[i] * nt, rec->serial[i], 0, 0);
     desolv_row(rec->element[i], rec->vdw_radius[i], &rdes[static_cast<size_t>(k) * 11]);
@@ -673,6 +682,10 @@ gd_status gd_complex_create(gd_context *ctx, const gd_atoms *rec, const gd_atoms
     rad = std::max(rad, std::sqrt(dx * dx + dy * dy + dz * dz));
   }
   cx->lig_radius = rad;
+  {
+    const double m = std::max({std::fabs(c[0]), std::fabs(c[1]), std::fabs(c[2])}) + rad;
+    cx->abs_max = std::isfinite(m) ? std::max(cx->abs_max, m) : INFINITY;
+  }
   // bounding sphere of each 32-atom slot in the positioned frame: a pose moves
   // it rigidly, so its transformed centre and the same radius bound the
   // slot's atoms in every pose
@@ -746,6 +759,7 @@ gd_status gd_complex_create(gd_context *ctx, const gd_atoms *rec, const gd_atoms
   UploadPack pack;
   pack.add(rp32, &cx->rec_pos32);
   pack.add(rp64, &cx->rec_pos64);
+  pack.add(rfix, &cx->rec_fix);
   pack.add(rmeta, &cx->rec_meta);
   pack.add(rmeta16, &cx->rec_meta16);
   pack.add(rdes, &cx->rec_desolv);

@@ -17,6 +17,15 @@ struct alignas(32) D4 {
   double x, y, z, w;
 };
 
+// One receptor atom of the FP64 kernel: coordinates as integers of 2^-kFixBits
+// A and the charge.
+struct alignas(32) FixAtom {
+  long long x, y, z;
+  double q;
+};
+constexpr int kFixBits = 51;
+constexpr double kFixMax = 4000.0;  // |coordinate| up to which the integers are used (they hold 4,096)
+
 // The receptor's arrays are padded to a multiple of this many atoms.
 constexpr int kTile = 256;
 // Receptor atoms per segment (a stage of the FP32 kernel's ring, a unit of the
@@ -76,6 +85,8 @@ struct ScoreParams {
   // receptor, sorted by atom type, padded to a multiple of kTile
   const float4 *rec_pos32;  // (x-O, y-O, z-O, 332.0636*q) FP32
   const D4 *rec_pos64; // (x, y, z, q) FP64
+  const FixAtom *rec_fix;   // the same as integers
+  int fix;                  // every coordinate of the launch lies within kFixMax
   const int2 *rec_meta;     // (type, serial)
   const int4 *rec_meta16;   // (type, serial, 0, 0): the FP32 kernel's copy, as wide as a position
   const double *rec_desolv; // [nr * 11] energy contribution at burial count 0..10
@@ -157,6 +168,8 @@ struct gd_complex {
   // device arrays
   float4 *rec_pos32 = nullptr;
   D4 *rec_pos64 = nullptr;
+  gd::FixAtom *rec_fix = nullptr;
+  double abs_max = 0;     // max |x| over receptor atoms and (ligand centroid + radius); inf when not finite
   int2 *rec_meta = nullptr;
   int4 *rec_meta16 = nullptr;
   double *rec_desolv = nullptr;

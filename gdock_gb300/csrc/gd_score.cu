@@ -10,8 +10,7 @@
 //   1. The ligand's atoms are moved in FP64 with the reference's operation
 //      order (coordinates bit-identical to gdock's) into shared memory, each
 //      CTA of the cluster a share, the others copied from its shared memory.
-//   2. Work units of one 32-atom ligand slot x some blocks of 32 receptor
-//      atoms are taken by the cluster's warps from one counter.  A unit finds
+//   2. Work units of one 32-atom ligand slot x a run of receptor atoms are taken by the cluster's warps from one counter.  A unit finds
 //      its pairs within reach in FP32 (bounding spheres of the slot and of the
 //      receptor segments, then each pair's distance, all with the FP32 guard
 //      band added, so that only pairs whose every term is exactly zero are
@@ -42,7 +41,7 @@ constexpr int kLigBits = 10;
 constexpr int kLigCap = 1 << kLigBits;  // ligand atoms held in shared memory at once (longer ligands: in turns)
 constexpr int kRows = 4;              // rows searched per step
 constexpr int kQueue = 32 * (kRows + 1);  // listed pairs per warp and kind: 31 left over + 32 of each row
-constexpr int kGrainMax = 4;          // 32-atom receptor blocks of a unit, at most
+constexpr int kRowsMin = 8, kRowsMax = 128;  // receptor atoms of a unit (a power of two)
 constexpr int kMaxCluster = 16;
 constexpr int kTinyHi = 0x2b000000;   // high word of 2^-335: below it r^6 may underflow
 
@@ -100,26 +99,48 @@ __device__ __forceinline__ void bury(uint32_t *cnt, int i) {
   if (((*reinterpret_cast<volatile uint32_t *>(cnt + (i >> 1)) >> sh) & 0xffffu) < 10u) atomicAdd(cnt + (i >> 1), 1u << sh);
 }
 
-// d2 next to the squared cutoff t: its high word is t's or a neighbour of it
-// (a relative 2^-20 to either side), which covers the few ulps between a
-// fused d2 and the reference's.
+// A pair's d2 in the reference's arithmetic and its decisions: bit 0 vdW, 1
+// burial, 2 Coulomb, 3: r^6 underflows and R6 is zero, where the reference's
+// ratio is 0 / 0.  Kept out of line: a handful of pairs in a million come
+// here, and inlined as predicated instructions they took a third of the FP64
+// pipe.
+struct ExactPair {
+  double d2;
+  int flags;
+};
+__device__ __noinline__ ExactPair exact_pair(const ScoreParams &p, const gd_pose_frame &f, int pose, int ri, int j) {
+  const D4 r = p.rec_pos64[ri];
+  double X, Y, Z;
+  ligand_atom(p, f, pose, j, X, Y, Z);
+  const double d2 = exact_d2(r.x, r.y, r.z, X, Y, Z);
+  const Thresholds &t = p.thr;
+  ExactPair e{d2, (d2 > 0.0 && d2 < t.vdw_lt) | (d2 < t.desolv_lt) << 1 | (d2 > t.elec_gt && d2 < t.elec_lt) << 2};
+  if ((e.flags & 1) && d2 * d2 * d2 == 0.0 && signbit(p.tab64[p.rec_meta[ri].x + p.lig_type[j]].inv2)) e.flags |= 8;
+  return e;
+}
+
+// A double's high word next to that of the squared cutoff t (a relative 2^-20
+// to either side: more than the few ulps between a fused d2 and the
+// reference's).
 __device__ __forceinline__ bool near_hi(int hi, double t) {
   return static_cast<unsigned>(hi - (__double2hiint(t) - 1)) <= 2u;
 }
+// A fixed-point d2's high word (2^-24 A^2) next to that of the squared cutoff
+// c2: within 6e-8 A^2, where integers and doubles differ by some 1e-14.
+__device__ __forceinline__ bool near_fix(unsigned hw, unsigned c2) { return hw - ((c2 << 24) - 1u) <= 1u; }
 
-// The pair's decisions in the reference's arithmetic: bit 0 vdW, 1 burial, 2
-// Coulomb.  Kept out of line: a handful of pairs in a million come here, and
-// inlined as predicated instructions they took a third of the FP64 pipe.
-__device__ __noinline__ int exact_decisions(const Thresholds &t, double rx, double ry, double rz, double lx, double ly,
-                                            double lz) {
-  const double d2 = exact_d2(rx, ry, rz, lx, ly, lz);
-  return (d2 > 0.0 && d2 < t.vdw_lt) | (d2 < t.desolv_lt) << 1 | (d2 > t.elec_gt && d2 < t.elec_lt) << 2;
-}
-
-template <bool SERIAL, bool CLAMP>
+// FIX: d2 from integer coordinates.  The differences and the three squares are
+// exact and d2 is truncated below 2^-56 A^2, so its error is the coordinates'
+// rounding to 2^-52 A, less than theirs as doubles above 4 A.  It takes about
+// 45 integer instructions a pair, which issue beside the FP64 pipe, in place of
+// 6 FP64 ones.
+template <bool FIX, bool SERIAL, bool CLAMP>
 struct PairEval {
   const ScoreParams &p;
-  const double *x, *y, *z, *q;
+  const gd_pose_frame &f;
+  int pose;
+  const void *x, *y, *z;  // FIX: integers, else doubles
+  const double *q;
   const uint8_t *lt;
   uint32_t *rcnt, *lcnt;
   int base;  // ligand atom of the shared arrays' first entry
@@ -129,61 +150,98 @@ struct PairEval {
   __device__ __forceinline__ void eval(bool on, uint32_t w, ExactSum<> &vdw, ExactSum<> &elec) const {
     if (!on) return;
     const int ri = static_cast<int>(w >> kLigBits), k = static_cast<int>(w & (kLigCap - 1));
-    const double2 *rp = reinterpret_cast<const double2 *>(p.rec_pos64 + ri);
-    const double2 rxy = __ldg(rp), rzq = __ldg(rp + 1);
-    const double lx = x[k], ly = y[k], lz = z[k];
-    const double dx = rxy.x - lx, dy = rxy.y - ly, dz = rzq.x - lz;
-    const double d2 = __fma_rn(dz, dz, __fma_rn(dy, dy, dx * dx));
-    const int hi = __double2hiint(d2);
-    if (!NEAR) {
-      bool pe = hi < __double2hiint(p.thr.elec_lt);
-      if (near_hi(hi, p.thr.elec_lt)) pe = exact_decisions(p.thr, rxy.x, rxy.y, rzq.x, lx, ly, lz) & 4;
-      if (pe) elec.add(rzq.y * q[k] * rcp64(d2), p.fx_elec);
-      return;
+    double rq, d2;
+    bool pv, pd, pe, rare;
+    if (FIX) {
+      const longlong2 *rp = reinterpret_cast<const longlong2 *>(p.rec_fix + ri);
+      const longlong2 rxy = __ldg(rp), rzq = __ldg(rp + 1);
+      rq = __longlong_as_double(rzq.y);
+      const long long d[3] = {rxy.x - static_cast<const long long *>(x)[k], rxy.y - static_cast<const long long *>(y)[k],
+                              rzq.x - static_cast<const long long *>(z)[k]};
+      long long H = 0, M = 0;
+      unsigned lo = 0;
+      // d = h 2^32 + l with a signed l: d^2 = h^2 2^64 + h l 2^33 + l^2
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const int l = static_cast<int>(d[a]);
+        const int h = static_cast<int>(d[a] >> 32) + static_cast<int>(static_cast<unsigned>(l) >> 31);
+        H += static_cast<long long>(h) * h;
+        M += static_cast<long long>(h) * l;
+        lo += static_cast<unsigned>(__mulhi(l, l)) >> 2;  // three of them fit 32 bits
+      }
+      const unsigned long long D = (static_cast<unsigned long long>(H) << 18) + (M >> 13) + (lo >> 12);  // 2^-56 A^2
+      const unsigned hw = static_cast<unsigned>(D >> 32);
+      // to a double, rounded: the leading bit at 63 - n (n = 0 from 128 A^2 on)
+      const int n = NEAR ? __clz(hw) : 0;
+      const unsigned long long m = D << n;
+      d2 = __longlong_as_double(static_cast<long long>((m >> 11) + ((m >> 10) & 1)) +
+                                (static_cast<long long>(1029 - n) << 52));
+      pe = hw < (225u << 24);
+      rare = near_fix(hw, 225u);
+      if (NEAR) {
+        pv = hw < (144u << 24);
+        pd = hw < (64u << 24);
+        pe = pe && hw >= (1u << 24);
+        rare = rare | near_fix(hw, 144u) | near_fix(hw, 64u) | near_fix(hw, 1u) | (hw == 0u);
+      }
+    } else {
+      const double2 *rp = reinterpret_cast<const double2 *>(p.rec_pos64 + ri);
+      const double2 rxy = __ldg(rp), rzq = __ldg(rp + 1);
+      rq = rzq.y;
+      const double dx = rxy.x - static_cast<const double *>(x)[k], dy = rxy.y - static_cast<const double *>(y)[k],
+                   dz = rzq.x - static_cast<const double *>(z)[k];
+      d2 = __fma_rn(dz, dz, __fma_rn(dy, dy, dx * dx));
+      const int hi = __double2hiint(d2);
+      pe = hi < __double2hiint(p.thr.elec_lt);
+      rare = near_hi(hi, p.thr.elec_lt);
+      if (NEAR) {
+        pv = hi < __double2hiint(p.thr.vdw_lt);
+        pd = hi < __double2hiint(p.thr.desolv_lt);
+        pe = pe && hi > __double2hiint(p.thr.elec_gt);
+        // a zero, a tiny or an undefined d2 (NaN: hi < 0) takes the exact tests too
+        rare = rare | near_hi(hi, p.thr.vdw_lt) | near_hi(hi, p.thr.desolv_lt) | near_hi(hi, p.thr.elec_gt) | (hi < kTinyHi);
+      }
     }
-    // (a zero, a tiny or an undefined d2 takes the exact tests too)
-    bool pv = hi < __double2hiint(p.thr.vdw_lt), pd = hi < __double2hiint(p.thr.desolv_lt);
-    bool pe = hi > __double2hiint(p.thr.elec_gt) && hi < __double2hiint(p.thr.elec_lt);
-    if (near_hi(hi, p.thr.vdw_lt) | near_hi(hi, p.thr.desolv_lt) | near_hi(hi, p.thr.elec_gt) |
-        near_hi(hi, p.thr.elec_lt) | (hi < kTinyHi)) {  // hi < 0: NaN
-      const int d = exact_decisions(p.thr, rxy.x, rxy.y, rzq.x, lx, ly, lz);
-      pv = d & 1;
-      pd = d & 2;
-      pe = d & 4;
-      // where r^6 underflows and R6 is zero, the reference's ratio is 0 / 0
-      if (pv && d2 * d2 * d2 == 0.0 &&
-          __double_as_longlong(__ldg(&p.tab64[__ldg(p.rec_meta + ri).x + lt[k]].inv2)) < 0)
-        vdw.nf = NAN;
+    if (rare) {
+      const ExactPair e = exact_pair(p, f, pose, ri, base + k);
+      d2 = e.d2;
+      pv = e.flags & 1;
+      pd = e.flags & 2;
+      pe = e.flags & 4;
+      if (e.flags & 8) vdw.nf = NAN;
     }
-    const int2 m = __ldg(p.rec_meta + ri);
-    if (SERIAL) pv = pv && m.y != __ldg(p.lig_serial + base + k);
-    if (pd) {
-      bury(rcnt, ri);
-      bury(lcnt, base + k);
-    }
-    if (pv) {
-      // softcore_lj_potential (src/fitness.rs:57-70) as 4 eps (x^2 - x) with
-      // x = 1 / (r^6 2/R6 + 1), half the reference's ratio
-      const double2 tp = __ldg(reinterpret_cast<const double2 *>(p.tab64) + m.x + lt[k]);
-      const double u = rcp64(__fma_rn(d2 * d2 * d2, tp.x, 1.0));
-      double v = tp.y * __fma_rn(u, u, -u);
-      if (CLAMP) v = v < -50.0 ? -50.0 : (v > 500.0 ? 500.0 : v);
-      vdw.add(v, p.fx_vdw);
+    if (NEAR) {
+      const int2 m = __ldg(p.rec_meta + ri);
+      if (SERIAL) pv = pv && m.y != __ldg(p.lig_serial + base + k);
+      if (pd) {
+        bury(rcnt, ri);
+        bury(lcnt, base + k);
+      }
+      if (pv) {
+        // softcore_lj_potential (src/fitness.rs:57-70) as 4 eps (x^2 - x) with
+        // x = 1 / (r^6 2/R6 + 1), half the reference's ratio
+        const double2 tp = __ldg(reinterpret_cast<const double2 *>(p.tab64) + m.x + lt[k]);
+        const double u = rcp64(__fma_rn(d2 * d2 * d2, tp.x, 1.0));
+        double v = tp.y * __fma_rn(u, u, -u);
+        if (CLAMP) v = v < -50.0 ? -50.0 : (v > 500.0 ? 500.0 : v);
+        vdw.add(v, p.fx_vdw);
+      }
     }
     // elec_energy term (src/fitness.rs:296) without its constant, which
     // multiplies the pose's sum
-    if (pe) elec.add(rzq.y * q[k] * rcp64(d2), p.fx_elec);
+    if (pe) elec.add(rq * q[k] * rcp64(d2), p.fx_elec);
   }
 };
 
 // What bounds it: the FP64 pipe, two lanes' operations per clock and SM.  The
 // form that evaluated every pair spent about 35 of them on each pair, though
 // only 13 % of the pairs of a scan have a term; a listed pair costs 18 (near)
-// or 11 (far), and the FP32 search runs beside the FP64 pipe.  On receptors of
-// 2,538 and ligands of 1,280 atoms: 2,048 poses 348 -> 28.7 ms, 150 poses
-// 29.0 -> 2.38 ms; one pose of 411 x 649 atoms 1,746 -> 89 us a call.
-template <bool SERIAL, bool CLAMP>
-__global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const int grain) {
+// or 11 (far), and the FP32 search runs beside the FP64 pipe; d2 from integers
+// takes another 6 off.  On receptors of 2,538 and ligands of 1,280 atoms: 2,048
+// poses 348 -> 28.7 -> 18.0 ms (every pair; listed pairs; integers), 150 poses
+// 29.0 -> 2.38 -> 1.72 ms; one pose of 411 x 649 atoms 1,746 -> 89 -> 75 us a call.
+template <bool FIX, bool SERIAL, bool CLAMP>
+__global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const int unit_rows) {
   if (p.skip && *p.skip) return;
   extern __shared__ __align__(128) unsigned char smem[];
   const F64Smem L = f64_smem(p.nr, p.nl);
@@ -220,7 +278,7 @@ __global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const
   // FP32) and an infinite band keep the pair for the FP64 decision.
   const float lim_e = 225.0f + p.guard_e, lim_v = 144.0f + p.guard_v;
   const float reach = sqrtf(225.01f + 2.0f * p.guard_e) + 0.01f;
-  const int nblk = (p.nr + 31) / 32, ngrp = (nblk + grain - 1) / grain;
+  const int ngrp = (p.nr + unit_rows - 1) / unit_rows;
   ExactSum<> vdw, elec;
   int first = 0;  // unit counter at the start of this turn
 
@@ -235,12 +293,21 @@ __global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const
       if (on) {
         double X, Y, Z;
         ligand_atom(p, f, pose, j, X, Y, Z);
-        s_x[k] = X;
-        s_y[k] = Y;
-        s_z[k] = Z;
         fx = static_cast<float>(X - p.ox);
         fy = static_cast<float>(Y - p.oy);
         fz = static_cast<float>(Z - p.oz);
+        if (FIX) {
+          // (a coordinate that is not a number: no pair has a term)
+          if (!(fabsf(fx) + fabsf(fy) + fabsf(fz) < 3.0e38f)) fx = INFINITY;
+          constexpr double kOne = 1LL << kFixBits;
+          s_x[k] = __longlong_as_double(__double2ll_rn(X * kOne));
+          s_y[k] = __longlong_as_double(__double2ll_rn(Y * kOne));
+          s_z[k] = __longlong_as_double(__double2ll_rn(Z * kOne));
+        } else {
+          s_x[k] = X;
+          s_y[k] = Y;
+          s_z[k] = Z;
+        }
         s_fx[k] = fx;
         s_fy[k] = fy;
         s_fz[k] = fz;
@@ -288,7 +355,7 @@ __global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const
     }
     __syncthreads();
 
-    const PairEval<SERIAL, CLAMP> ev{p, s_x, s_y, s_z, s_q, s_lt, s_rcnt, s_lcnt, l0};
+    const PairEval<FIX, SERIAL, CLAMP> ev{p, f, pose, s_x, s_y, s_z, s_q, s_lt, s_rcnt, s_lcnt, l0};
     int *next = nc > 1 ? cluster.map_shared_rank(s_next, 0) : s_next;
     int nn = 0, nf = 0;  // listed near and far pairs of this warp
     for (;;) {
@@ -296,26 +363,25 @@ __global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const
       if (lane == 0) u = atomicAdd(next, 1);
       u = __shfl_sync(kFull, u, 0) - first;
       if (u >= nunit) break;
-      const int slot = u / ngrp, b0 = u % ngrp * grain, b1 = min(nblk, b0 + grain);
+      const int slot = u / ngrp, r0 = u % ngrp * unit_rows, r1 = min(p.nr, r0 + unit_rows);
       const int k = slot * 32 + lane;
       const bool on = k < nl;
       const float lx = on ? s_fx[k] : 0.0f, ly = on ? s_fy[k] : 0.0f, lz = on ? s_fz[k] : 0.0f;
       const float4 sp = s_sph[slot];
       const float lim_s = sp.w + reach, lim_s2 = lim_s * lim_s;
 #pragma unroll 1
-      for (int b = b0; b < b1; ++b) {
+      for (int a0 = r0 & ~31; a0 < r1; a0 += 32) {
         {
-          const float4 sg = __ldg(&p.rec_seg[b >> 1]);
+          const float4 sg = __ldg(&p.rec_seg[a0 / kRecSeg]);
           const float dx = sg.x - sp.x, dy = sg.y - sp.y, dz = sg.z - sp.z;
           const float lim = sg.w + sp.w + reach + 0.1f + 1e-3f * (sg.w + sp.w);
           if (dx * dx + dy * dy + dz * dz > lim * lim) {
-            b |= 1;  // the segment's second block too
+            a0 |= 32;  // the segment's second half too
             continue;
           }
         }
         // rows: receptor atoms within reach of the slot's sphere
-        const int a0 = b * 32;
-        bool keep = a0 + lane < p.nr;
+        bool keep = a0 + lane >= r0 && a0 + lane < r1;
         if (keep) {
           const float4 r = __ldg(&p.rec_pos32[a0 + lane]);
           const float dx = r.x - sp.x, dy = r.y - sp.y, dz = r.z - sp.z;
@@ -432,17 +498,25 @@ cudaError_t launch_f64(Kern kern, const ScoreParams &p, int sm_count, cudaStream
   const size_t smem = f64_smem(p.nr, p.nl).total;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return e;
-  // CTAs per pose: eight for every SM over the launch (poses differ widely in
-  // work), as far as a cluster and the pose's blocks go; blocks per unit: 32
-  // units or more for every warp, so that the last ones leave few warps
-  // waiting.  Half the CTAs and units four times as large took 3.97 ms instead
-  // of 3.25 on 150 poses of 2,538 x 1,280 atoms (warps waiting at the end of
-  // their pose).
-  const long long slots = std::max(1, (std::min(p.nl, kLigCap) + 31) / 32), blocks = std::max(1, (p.nr + 31) / 32);
+  // CTAs per pose: the more the fewer poses there are, as far as the pose's
+  // rows (receptor atom x ligand slot) go round.  Poses differ widely in work,
+  // so splitting them pays beyond the point where they fill the SMs, the less
+  // so the more CTAs a cluster must find places for at once.  Measured on
+  // 2,538 x 1,280 atoms, us at 1 / 2 / 4 / 8 / 16 CTAs: 40 poses 3695 / 1937 /
+  // 1028 / 657 / 640, 300 poses 4930 / 3879 / 3312 / 3150 / 3786, 1,200 poses
+  // 12547 / 11307 / 11067 / 11648 / 14676; on 411 x 649 atoms 2,400 poses 3242 /
+  // 3062 / 3265 / 3809 / 5719, 9,600 poses 10759 / 10954 / 12225 / 14601 / 22295.
+  const long long rows = static_cast<long long>(std::max(1, (std::min(p.nl, kLigCap) + 31) / 32)) * std::max(1, p.nr);
+  constexpr int kPerSm[] = {64, 32, 16, 4};  // CTAs per SM up to which poses are split in 2, 4, 8, 16
   int nc = 1;
-  while (nc < kMaxCluster && static_cast<long long>(p.n_poses) * nc * 2 <= 8LL * sm_count && slots * blocks > 4 * kNW * nc)
-    nc *= 2;
-  const int grain = static_cast<int>(std::max(1LL, std::min<long long>(kGrainMax, slots * blocks / (32LL * kNW * nc))));
+  for (int k = 0; k < 4 && nc < kMaxCluster; ++k)
+    if (static_cast<long long>(p.n_poses) * (2 << k) <= static_cast<long long>(kPerSm[k]) * sm_count &&
+        rows > 64 * kNW * (2 << k))
+      nc = 2 << k;
+  // rows per unit: 32 units or more for every warp, so that the last ones
+  // leave few warps waiting (8 to 128 units a warp made no difference)
+  int unit_rows = kRowsMin;
+  while (unit_rows < kRowsMax && rows >= 2LL * unit_rows * 32 * kNW * nc) unit_rows *= 2;
   if (nc > 8) {
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
@@ -466,7 +540,7 @@ cudaError_t launch_f64(Kern kern, const ScoreParams &p, int sm_count, cudaStream
     (void)cudaGetLastError();
   }
   if (nc == 1) cfg.numAttrs = 0;
-  return cudaLaunchKernelEx(&cfg, kern, p, grain);
+  return cudaLaunchKernelEx(&cfg, kern, p, unit_rows);
 }
 
 }  // namespace
@@ -476,6 +550,8 @@ ScoreParams make_params(gd_complex *cx, const gd_pose_frame *d_frames, const dou
   ScoreParams p{};
   p.rec_pos32 = cx->rec_pos32;
   p.rec_pos64 = cx->rec_pos64;
+  p.rec_fix = cx->rec_fix;
+  p.fix = cx->abs_max + max_disp <= kFixMax;
   p.rec_meta = cx->rec_meta;
   p.rec_meta16 = cx->rec_meta16;
   p.rec_desolv = cx->rec_desolv;
@@ -538,10 +614,18 @@ gd_status launch_score(gd_complex *cx, const gd_pose_frame *d_frames, const doub
   // nothing and every pair is decided in FP64
   if (!(p.guard_e <= 1.0f)) p.guard_e = p.guard_v = INFINITY;
   cudaError_t e;
-  if (serial) e = clamp ? launch_f64(k_score_f64<true, true>, p, ctx->sm_count, stream)
-                        : launch_f64(k_score_f64<true, false>, p, ctx->sm_count, stream);
-  else e = clamp ? launch_f64(k_score_f64<false, true>, p, ctx->sm_count, stream)
-                 : launch_f64(k_score_f64<false, false>, p, ctx->sm_count, stream);
+  const int sm = ctx->sm_count;
+  if (p.fix) {
+    if (serial) e = clamp ? launch_f64(k_score_f64<true, true, true>, p, sm, stream)
+                          : launch_f64(k_score_f64<true, true, false>, p, sm, stream);
+    else e = clamp ? launch_f64(k_score_f64<true, false, true>, p, sm, stream)
+                   : launch_f64(k_score_f64<true, false, false>, p, sm, stream);
+  } else {
+    if (serial) e = clamp ? launch_f64(k_score_f64<false, true, true>, p, sm, stream)
+                          : launch_f64(k_score_f64<false, true, false>, p, sm, stream);
+    else e = clamp ? launch_f64(k_score_f64<false, false, true>, p, sm, stream)
+                   : launch_f64(k_score_f64<false, false, false>, p, sm, stream);
+  }
   if (e != cudaSuccess) return cuda_fail(ctx, e, "score kernel launch");
   return GD_OK;
 }

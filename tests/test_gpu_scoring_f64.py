@@ -36,14 +36,16 @@ def test_sizes_and_launches(oracle, big, nr, nl):
     assert cx.score_models(models).tobytes() == all_of[:12].tobytes()
 
 
-@pytest.mark.parametrize("shift", [3000.0, 1.0e5, 3.0e9])
-def test_far_from_the_origin(oracle, big, shift):
-    """Coordinates far from zero, up to where FP32 cannot tell atoms apart."""
+@pytest.mark.parametrize("shift,far", [(3000.0, True), (3890.0, False), (3990.0, False), (1.0e5, True), (3.0e9, True)])
+def test_far_from_the_origin(oracle, big, shift, far):
+    """Coordinates far from zero: on both sides of the 4,000 A up to which the
+    distances come from integers, and up to where FP32 cannot tell atoms apart."""
     rec, lig = _first_atoms(big.receptor, 120), _first_atoms(big.ligand, 90)
     rec = rec.with_coords(rec.x + shift, rec.y - shift, rec.z)
     lig = gd.position_ligand(rec, lig)
     genes = synth.random_genes(np.random.default_rng(3), 6, max_displacement=9.0)
-    genes[3, 3] = 2.0 * shift  # a pose far away widens the others' bands, too
+    if far:
+        genes[3, 3] = 2.0 * shift  # a pose far away widens the others' bands, too
     cx = gd.Complex(rec, lig, [])
     check(cx.score_poses(genes), oracle.score_poses(rec, lig, [], genes), F64_TOL)
 
