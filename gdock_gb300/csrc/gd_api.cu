@@ -665,6 +665,7 @@ gd_status gd_complex_create(gd_context *ctx, const gd_atoms *rec, const gd_atoms
   const std::vector<int> perm = slot_order(lig->x, lig->y, lig->z, lig->n);
   std::vector<int> inv(lig->n);
   std::vector<double> lx(lig->n), ly(lig->n), lz(lig->n), lq(lig->n);
+  std::vector<D4> lrel(lig->n);
   std::vector<int> lser(lig->n), ltp(lig->n);
   std::vector<double> ldes(static_cast<size_t>(std::max(lig->n, 1)) * 11, 0.0);
   double rad = 0.0;
@@ -675,6 +676,7 @@ gd_status gd_complex_create(gd_context *ctx, const gd_atoms *rec, const gd_atoms
     ly[k] = lig->y[j];
     lz[k] = lig->z[j];
     lq[k] = lig->charge[j];
+    lrel[k] = D4{lig->x[j] - c[0], lig->y[j] - c[1], lig->z[j] - c[2], lig->charge[j]};
     lser[k] = lig->serial[j];
     ltp[k] = ltype[j];
     desolv_row(lig->element[j], lig->vdw_radius[j], &ldes[static_cast<size_t>(k) * 11]);
@@ -694,7 +696,7 @@ gd_status gd_complex_create(gd_context *ctx, const gd_atoms *rec, const gd_atoms
     const int s1 = std::min(lig->n, s0 + 32);
     double cs[3], r;
     enclosing_ball(lx.data() + s0, ly.data() + s0, lz.data() + s0, nullptr, s1 - s0, cs, r);
-    lslot[s0 / 32] = D4{cs[0], cs[1], cs[2], r * (1.0 + 1e-6) + 0.01};
+    lslot[s0 / 32] = D4{cs[0] - c[0], cs[1] - c[1], cs[2] - c[2], r * (1.0 + 1e-6) + 0.01};
   }
   {
     // equal receptor/ligand serials (vdW pairs skipped): disjoint serial
@@ -767,6 +769,7 @@ gd_status gd_complex_create(gd_context *ctx, const gd_atoms *rec, const gd_atoms
   pack.add(ly, &cx->lig_y);
   pack.add(lz, &cx->lig_z);
   pack.add(lq, &cx->lig_q);
+  pack.add(lrel, &cx->lig_rel);
   pack.add(ltp, &cx->lig_type);
   pack.add(lser, &cx->lig_serial);
   pack.add(ldes, &cx->lig_desolv);

@@ -94,7 +94,8 @@ struct ScoreParams {
   int nr, nseg;
   // ligand in slot order (spatially compact runs of 32 atoms)
   const int *lig_perm;      // slot position -> original atom index
-  const D4 *lig_slot_sph;   // per 32-atom slot: bounding sphere in the positioned frame (centre, radius)
+  const D4 *lig_slot_sph;   // per 32-atom slot: bounding sphere (centre relative to the rotation centre, radius)
+  const D4 *lig_rel;        // ligand atoms relative to the rotation centre, and their charge
   const double *lig_x, *lig_y, *lig_z;
   const double *lig_q;
   const int *lig_type, *lig_serial;
@@ -182,7 +183,8 @@ struct gd_complex {
   int *restr_lig = nullptr;
   int *lig_perm = nullptr;  // slot position -> original ligand atom index
   float4 *rec_seg = nullptr;  // receptor segment spheres (FP32, relative to O)
-  D4 *lig_slot_sph = nullptr;  // ligand slot spheres (positioned frame)
+  D4 *lig_slot_sph = nullptr;  // ligand slot spheres (relative to the rotation centre)
+  D4 *lig_rel = nullptr;       // ligand atoms relative to the rotation centre, and their charge
   int nseg = 0;
   std::vector<void *> allocs;
   uint64_t bytes = 0;

@@ -558,6 +558,7 @@ ScoreParams make_params(gd_complex *cx, const gd_pose_frame *d_frames, const dou
   p.nr = cx->nr;
   p.lig_perm = cx->lig_perm;
   p.lig_slot_sph = cx->lig_slot_sph;
+  p.lig_rel = cx->lig_rel;
   p.rec_seg = cx->rec_seg;
   p.nseg = cx->nseg;
   p.lig_x = cx->lig_x;

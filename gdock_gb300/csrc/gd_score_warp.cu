@@ -233,6 +233,46 @@ __device__ __forceinline__ bool near_band(float d2, float gv, float ge, float gd
   return (fabsf(__fsub_rn(fabsf(te), 112.0f)) < ge) | (fabsf(tv) < gv) | (fabsf(__fsub_rn(d2, 64.0f)) < gdd);
 }
 
+// Ligand coordinates relative to the FP32 origin O, in FP64, as the FP32 images
+// are rounded from: one chain of multiply-adds on the precomputed offset from
+// the rotation centre, 9 FP64 operations in place of the 31 of the reference's
+// order, from which it differs by some 1e-15 A (decisions inside the guard
+// bands take the exact coordinates).  FP64 issues at 1/64 of the FP32 rate, and
+// with receptor parts every part's item moves its ligand atoms: 150 poses of
+// 1,074 x 741 atoms apart from each other took 147 us, 58 of them the FP64
+// pipe's; with this and without the items that have no segment in reach, 97 us.
+__device__ __forceinline__ void relative_atom(const ScoreParams &p, const gd_pose_frame &f, const D4 &r, double &x,
+                                              double &y, double &z) {
+  const double tx = (p.cx + f.dx) - p.ox, ty = (p.cy + f.dy) - p.oy, tz = (p.cz + f.dz) - p.oz;
+  x = __fma_rn(f.ca * f.cb, r.x, __fma_rn(f.m01, r.y, __fma_rn(f.m02, r.z, tx)));
+  y = __fma_rn(f.sa * f.cb, r.x, __fma_rn(f.m11, r.y, __fma_rn(f.m12, r.z, ty)));
+  z = __fma_rn(-f.sb, r.x, __fma_rn(f.cb * f.sg, r.y, __fma_rn(f.cb * f.cg, r.z, tz)));
+}
+__device__ __forceinline__ float3 atom32(const ScoreParams &p, const gd_pose_frame &f, int pose, int j) {
+  double x, y, z;
+  if (p.models) {
+    ligand_atom(p, f, pose, j, x, y, z);
+    x -= p.ox;
+    y -= p.oy;
+    z -= p.oz;
+  } else {
+    relative_atom(p, f, p.lig_rel[j], x, y, z);
+  }
+  return make_float3(static_cast<float>(x), static_cast<float>(y), static_cast<float>(z));
+}
+
+// Warp-wide minimum and maximum, one instruction each.
+__device__ __forceinline__ float warp_min(float v) {
+  float r;
+  asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ float warp_max(float v) {
+  float r;
+  asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+
 // Corrections of one pair's FP32 contributions after its FP64 re-decision.
 struct FixOut {
   float dv, de;
@@ -406,10 +446,9 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_score_f32w(const BatchPar
         float4 v = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
         if (sl * 32 < p.nl) {
           const D4 sp = p.lig_slot_sph[sl];
-          double X, Y, Z;
-          transform_atom(f, p.cx, p.cy, p.cz, sp.x, sp.y, sp.z, X, Y, Z);
-          v = make_float4(static_cast<float>(X - p.ox), static_cast<float>(Y - p.oy), static_cast<float>(Z - p.oz),
-                          static_cast<float>(sp.w));
+          double x, y, z;
+          relative_atom(p, f, sp, x, y, z);
+          v = make_float4(static_cast<float>(x), static_cast<float>(y), static_cast<float>(z), static_cast<float>(sp.w));
         }
         s_ssph[lane] = v;
       }
@@ -444,276 +483,272 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_score_f32w(const BatchPar
         __syncwarp();
       }
       auto seg_at = [&](int k) { return listed ? static_cast<int>(s_segl[k]) : rpart + k * R; };
-      if (lane == 0)
-        for (int k = 0; k < nk && k < kWS; ++k)
-          if (!(bp.drop_copy && item == 0 && ch == ch0 && k == 0))
-            issue_seg(q + k, seg_at(k), p, s_pos, s_meta, s_bar);
-      q_issued = q + min(nk, kWS);
-      float lx[S], ly[S], lz[S], lq[S];
-      int lt[S], lser[S], lcnt[S];
-#pragma unroll
-      for (int s = 0; s < S; ++s) {
-        const int j = ch * kChunk + s * 32 + lane;
-        lcnt[s] = 0;
-        const bool on = j < p.nl;
-        if (on) {
-          double X, Y, Z;
-          ligand_atom(p, f, pose, j, X, Y, Z);
-          lx[s] = static_cast<float>(X - p.ox);
-          ly[s] = static_cast<float>(Y - p.oy);
-          lz[s] = static_cast<float>(Z - p.oz);
-          lq[s] = static_cast<float>(p.lig_q[j]);
-          lt[s] = p.lig_type[j];
-          if (!GD_DCHECK(bp.err, lt[s] >= 0 && lt[s] < p.nt, 6)) lt[s] = 0;
-          lser[s] = SERIAL ? p.lig_serial[j] : 0;
-        } else {
-          // far from every receptor atom, including the padding at +1e9
-          lx[s] = ly[s] = lz[s] = -1.0e9f;
-          lq[s] = 0.0f;
-          lt[s] = 0;
-          lser[s] = 0;
-        }
-        // bounding sphere of the slot's 32 atoms: with a rigid pose the
-        // precomputed small enclosing sphere moved with it (s_ssph, smaller
-        // than the centroid's sphere), else the centroid's of these atoms
-        const unsigned on_mask = __ballot_sync(kFull, on);
-        float cx = 0.0f, cy = 0.0f, cz = 0.0f, rr = 0.0f;
-        if (!cull) {
-          cx = on ? lx[s] : 0.f, cy = on ? ly[s] : 0.f, cz = on ? lz[s] : 0.f;
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) {
-            cx += __shfl_xor_sync(kFull, cx, o);
-            cy += __shfl_xor_sync(kFull, cy, o);
-            cz += __shfl_xor_sync(kFull, cz, o);
-          }
-          const float inv = on_mask ? 1.0f / static_cast<float>(__popc(on_mask)) : 0.0f;
-          cx *= inv;
-          cy *= inv;
-          cz *= inv;
-          rr = on ? sqrtf((lx[s] - cx) * (lx[s] - cx) + (ly[s] - cy) * (ly[s] - cy) + (lz[s] - cz) * (lz[s] - cz))
-                  : 0.0f;
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) rr = fmaxf(rr, __shfl_xor_sync(kFull, rr, o));
-        }
-        // axis-aligned bounding box of the same atoms (half-widths widened
-        // like the radius so that FP32 rounding never shrinks it)
-        float lo_x = on ? lx[s] : 3.0e38f, lo_y = on ? ly[s] : 3.0e38f, lo_z = on ? lz[s] : 3.0e38f;
-        float hi_x = on ? lx[s] : -3.0e38f, hi_y = on ? ly[s] : -3.0e38f, hi_z = on ? lz[s] : -3.0e38f;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          lo_x = fminf(lo_x, __shfl_xor_sync(kFull, lo_x, o));
-          lo_y = fminf(lo_y, __shfl_xor_sync(kFull, lo_y, o));
-          lo_z = fminf(lo_z, __shfl_xor_sync(kFull, lo_z, o));
-          hi_x = fmaxf(hi_x, __shfl_xor_sync(kFull, hi_x, o));
-          hi_y = fmaxf(hi_y, __shfl_xor_sync(kFull, hi_y, o));
-          hi_z = fmaxf(hi_z, __shfl_xor_sync(kFull, hi_z, o));
-        }
-        if (lane == 0) {
-          s_blob[s] = !on_mask ? make_float4(0.0f, 0.0f, 0.0f, -1.0e30f)
-                               : (cull ? s_ssph[s] : make_float4(cx, cy, cz, rr * 1.0001f + 0.01f));
-          if (on_mask) {
-            s_box[2 * s] = make_float4(0.5f * (lo_x + hi_x), 0.5f * (lo_y + hi_y), 0.5f * (lo_z + hi_z),
-                                       0.5f * (hi_x - lo_x) * 1.0001f + 0.01f);
-            s_box[2 * s + 1] = make_float4(0.5f * (hi_y - lo_y) * 1.0001f + 0.01f,
-                                           0.5f * (hi_z - lo_z) * 1.0001f + 0.01f, 0.0f, 0.0f);
-          } else {
-            s_box[2 * s] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            s_box[2 * s + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          }
-        }
-      }
-      __syncwarp();
-      // phase-1 role of this lane: row (slot my_s, atom my_a of each 8-atom round)
-      const float4 myb = my_s < S ? s_blob[my_s] : make_float4(0.0f, 0.0f, 0.0f, -1.0e30f);
-      const float mlim = myb.w + reach;
-      const float mlim2 = (myb.w >= 0.0f) ? mlim * mlim : -1.0f;  // empty slot: no row kept
-      const float mnear = myb.w + reach_v, mnear2 = mnear * mnear;
       long long fv = 0, fe = 0;  // this item's vdW and Coulomb sums, 2^-32 fixed point
-      // per segment: flagged steps (high 16 bits) and recorded near rows (low 16)
-      int seg_cnt = 0;
-      for (int kk = 0; kk < nk; ++kk, ++q) {
-        const int g = seg_at(kk);
-        const int st = static_cast<int>(q % kWS);
-        const bool ok = __all_sync(kFull, mbar_wait(&s_bar[st], static_cast<uint32_t>((q / kWS) & 1)));
-        if (!ok) {
-          failed = true;
-          break;
-        }
-        const int gbase = g * kSeg;
-        const int na = min(kSeg, p.nr - gbase);
-        const int sbase = st * kSeg;
-
-        // Phase 1: lane (slot, atom) tests one row against the slot's sphere.
-        // Kept rows go to the slot's list: far rows (Coulomb only) from the
-        // front, near rows from the back; each run is padded with the far
-        // dummy atom to whole steps.
-        int nf_mine = 0, nn_mine = 0;  // far / near rows of this lane's slot
-        uint16_t *my_list = s_list + my_s * kList;
-        for (int b0 = 0; b0 < na; b0 += kBlk) {
-          const float4 ra = s_pos[sbase + b0 + my_a];  // atoms past nr are padding far away
-          const float dx = ra.x - myb.x, dy = ra.y - myb.y, dz = ra.z - myb.z;
-          const float dc2 = dx * dx + dy * dy + dz * dz;
-          // distance from the atom to the slot's box: a second lower bound on
-          // every pair distance of the row (either bound may drop the row or
-          // make it far)
-          const float4 bx0 = s_box[2 * (my_s & (kMaxS - 1))], bx1 = s_box[2 * (my_s & (kMaxS - 1)) + 1];
-          const float ex = fmaxf(fabsf(ra.x - bx0.x) - bx0.w, 0.0f), ey = fmaxf(fabsf(ra.y - bx0.y) - bx1.x, 0.0f),
-                      ez = fmaxf(fabsf(ra.z - bx0.z) - bx1.y, 0.0f);
-          const float db2 = ex * ex + ey * ey + ez * ez;
-          const bool keep = dc2 < mlim2 && db2 < reach2, nearr = dc2 < mnear2 && db2 < reach_v2;
-          const unsigned Mf = __ballot_sync(kFull, keep && !nearr), Mn = __ballot_sync(kFull, keep && nearr);
-          const uint16_t idx = static_cast<uint16_t>(sbase + b0 + my_a);
-          // at most na <= kSeg rows per slot: far rows fill [0, nf), near rows
-          // (kList - nn, kList - 1], with room for both paddings in between
-          const int pf = nf_mine + __popc(Mf & my_group & lt_mask), pn = kList - 1 - nn_mine - __popc(Mn & my_group & lt_mask);
-          if (keep && !nearr && GD_DCHECK(bp.err, pf >= 0 && pf < kList, 1)) my_list[pf] = idx;
-          if (keep && nearr && GD_DCHECK(bp.err, pn >= 0 && pn < kList, 2)) my_list[pn] = idx;
-
-          nf_mine += __popc(Mf & my_group);
-          nn_mine += __popc(Mn & my_group);
-        }
-        if (my_s < S && my_a < kAtoms &&
-            GD_DCHECK(bp.err, nf_mine + my_a < kList && kList - 1 - nn_mine - my_a >= 0, 3)) {
-          my_list[nf_mine + my_a] = static_cast<uint16_t>(kFar);
-          my_list[kList - 1 - nn_mine - my_a] = static_cast<uint16_t>(kFar);
-        }
-        __syncwarp();
-
-        // Phase 2: every term of the kept rows, kAtoms rows per step
-        float av = 0.0f, ae = 0.0f;  // ae: corrections from FP64 re-decisions (charge included)
+      int lcnt[S];
+#pragma unroll
+      for (int s = 0; s < S; ++s) lcnt[s] = 0;
+      // an item without a segment in reach (the usual one of a pose apart from
+      // the receptor, and of a receptor part) ends here
+      if (nk > 0) {
+        if (lane == 0)
+          for (int k = 0; k < nk && k < kWS; ++k)
+            if (!(bp.drop_copy && item == 0 && ch == ch0 && k == 0))
+              issue_seg(q + k, seg_at(k), p, s_pos, s_meta, s_bar);
+        q_issued = q + min(nk, kWS);
+        float lx[S], ly[S], lz[S], lq[S];
+        int lt[S], lser[S];
 #pragma unroll
         for (int s = 0; s < S; ++s) {
-          float aes = 0.0f;  // sum of q_r / d2 over this slot's kept pairs
-          const int nf = __shfl_sync(kFull, nf_mine, s * 8), nn = __shfl_sync(kFull, nn_mine, s * 8);
-          const uint16_t *lst = s_list + s * kList;
-          // far rows: Coulomb only
-#pragma unroll 1
-          for (int k0 = 0; k0 < nf; k0 += kAtoms) {
-            int ix[kAtoms];
-            float4 r[kAtoms];
+          const int j = ch * kChunk + s * 32 + lane;
+          const bool on = j < p.nl;
+          if (on) {
+            const float3 c = atom32(p, f, pose, j);
+            lx[s] = c.x;
+            ly[s] = c.y;
+            lz[s] = c.z;
+            lq[s] = static_cast<float>(p.lig_rel[j].w);
+            lt[s] = p.lig_type[j];
+            if (!GD_DCHECK(bp.err, lt[s] >= 0 && lt[s] < p.nt, 6)) lt[s] = 0;
+            lser[s] = SERIAL ? p.lig_serial[j] : 0;
+          } else {
+            // far from every receptor atom, including the padding at +1e9
+            lx[s] = ly[s] = lz[s] = -1.0e9f;
+            lq[s] = 0.0f;
+            lt[s] = 0;
+            lser[s] = 0;
+          }
+          // bounding sphere of the slot's 32 atoms: with a rigid pose the
+          // precomputed small enclosing sphere moved with it (s_ssph, smaller
+          // than the centroid's sphere), else the centroid's of these atoms
+          const unsigned on_mask = __ballot_sync(kFull, on);
+          float cx = 0.0f, cy = 0.0f, cz = 0.0f, rr = 0.0f;
+          if (!cull) {
+            cx = on ? lx[s] : 0.f, cy = on ? ly[s] : 0.f, cz = on ? lz[s] : 0.f;
 #pragma unroll
-            for (int i = 0; i < kAtoms; ++i) {
-              ix[i] = lst[k0 + i];
-              if (!GD_DCHECK(bp.err, ix[i] <= kFar, 4)) ix[i] = kFar;
-              r[i] = s_pos[ix[i]];
+            for (int o = 16; o > 0; o >>= 1) {
+              cx += __shfl_xor_sync(kFull, cx, o);
+              cy += __shfl_xor_sync(kFull, cy, o);
+              cz += __shfl_xor_sync(kFull, cz, o);
             }
-            bool amb = false;
-#pragma unroll
-            for (int i = 0; i < kAtoms; ++i) pair32_elec(r[i], lx[s], ly[s], lz[s], ge, aes, amb);
-            if (__any_sync(kFull, amb)) {  // at most one entry per step: <= 4 * 18 per segment
-              if (lane == 0 && GD_DCHECK(bp.err, (seg_cnt >> 16) < kMaxS * kList, 7))
-                s_fixq[seg_cnt >> 16] = static_cast<uint16_t>(k0 | (s << 8));
-              seg_cnt += 1 << 16;
+            const float inv = on_mask ? 1.0f / static_cast<float>(__popc(on_mask)) : 0.0f;
+            cx *= inv;
+            cy *= inv;
+            cz *= inv;
+            rr = on ? sqrtf((lx[s] - cx) * (lx[s] - cx) + (ly[s] - cy) * (ly[s] - cy) + (lz[s] - cz) * (lz[s] - cz))
+                    : 0.0f;
+            rr = warp_max(rr);
+          }
+          // axis-aligned bounding box of the same atoms (half-widths widened
+          // like the radius so that FP32 rounding never shrinks it)
+          const float lo_x = warp_min(on ? lx[s] : 3.0e38f), lo_y = warp_min(on ? ly[s] : 3.0e38f),
+                      lo_z = warp_min(on ? lz[s] : 3.0e38f);
+          const float hi_x = warp_max(on ? lx[s] : -3.0e38f), hi_y = warp_max(on ? ly[s] : -3.0e38f),
+                      hi_z = warp_max(on ? lz[s] : -3.0e38f);
+          if (lane == 0) {
+            s_blob[s] = !on_mask ? make_float4(0.0f, 0.0f, 0.0f, -1.0e30f)
+                                 : (cull ? s_ssph[s] : make_float4(cx, cy, cz, rr * 1.0001f + 0.01f));
+            if (on_mask) {
+              s_box[2 * s] = make_float4(0.5f * (lo_x + hi_x), 0.5f * (lo_y + hi_y), 0.5f * (lo_z + hi_z),
+                                         0.5f * (hi_x - lo_x) * 1.0001f + 0.01f);
+              s_box[2 * s + 1] = make_float4(0.5f * (hi_y - lo_y) * 1.0001f + 0.01f,
+                                             0.5f * (hi_z - lo_z) * 1.0001f + 0.01f, 0.0f, 0.0f);
+            } else {
+              s_box[2 * s] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+              s_box[2 * s + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             }
           }
-          // near rows: every term; the first step may start in the padding
+        }
+        __syncwarp();
+        // phase-1 role of this lane: row (slot my_s, atom my_a of each 8-atom round)
+        const float4 myb = my_s < S ? s_blob[my_s] : make_float4(0.0f, 0.0f, 0.0f, -1.0e30f);
+        const float mlim = myb.w + reach;
+        const float mlim2 = (myb.w >= 0.0f) ? mlim * mlim : -1.0f;  // empty slot: no row kept
+        const float mnear = myb.w + reach_v, mnear2 = mnear * mnear;
+        // per segment: flagged steps (high 16 bits) and recorded near rows (low 16)
+        int seg_cnt = 0;
+        for (int kk = 0; kk < nk; ++kk, ++q) {
+          const int g = seg_at(kk);
+          const int st = static_cast<int>(q % kWS);
+          const bool ok = __all_sync(kFull, mbar_wait(&s_bar[st], static_cast<uint32_t>((q / kWS) & 1)));
+          if (!ok) {
+            failed = true;
+            break;
+          }
+          const int gbase = g * kSeg;
+          const int na = min(kSeg, p.nr - gbase);
+          const int sbase = st * kSeg;
+
+          // Phase 1: lane (slot, atom) tests one row against the slot's sphere.
+          // Kept rows go to the slot's list: far rows (Coulomb only) from the
+          // front, near rows from the back; each run is padded with the far
+          // dummy atom to whole steps.
+          int nf_mine = 0, nn_mine = 0;  // far / near rows of this lane's slot
+          uint16_t *my_list = s_list + my_s * kList;
+          for (int b0 = 0; b0 < na; b0 += kBlk) {
+            const float4 ra = s_pos[sbase + b0 + my_a];  // atoms past nr are padding far away
+            const float dx = ra.x - myb.x, dy = ra.y - myb.y, dz = ra.z - myb.z;
+            const float dc2 = dx * dx + dy * dy + dz * dz;
+            // distance from the atom to the slot's box: a second lower bound on
+            // every pair distance of the row (either bound may drop the row or
+            // make it far)
+            const float4 bx0 = s_box[2 * (my_s & (kMaxS - 1))], bx1 = s_box[2 * (my_s & (kMaxS - 1)) + 1];
+            const float ex = fmaxf(fabsf(ra.x - bx0.x) - bx0.w, 0.0f), ey = fmaxf(fabsf(ra.y - bx0.y) - bx1.x, 0.0f),
+                        ez = fmaxf(fabsf(ra.z - bx0.z) - bx1.y, 0.0f);
+            const float db2 = ex * ex + ey * ey + ez * ez;
+            const bool keep = dc2 < mlim2 && db2 < reach2, nearr = dc2 < mnear2 && db2 < reach_v2;
+            const unsigned Mf = __ballot_sync(kFull, keep && !nearr), Mn = __ballot_sync(kFull, keep && nearr);
+            const uint16_t idx = static_cast<uint16_t>(sbase + b0 + my_a);
+            // at most na <= kSeg rows per slot: far rows fill [0, nf), near rows
+            // (kList - nn, kList - 1], with room for both paddings in between
+            const int pf = nf_mine + __popc(Mf & my_group & lt_mask), pn = kList - 1 - nn_mine - __popc(Mn & my_group & lt_mask);
+            if (keep && !nearr && GD_DCHECK(bp.err, pf >= 0 && pf < kList, 1)) my_list[pf] = idx;
+            if (keep && nearr && GD_DCHECK(bp.err, pn >= 0 && pn < kList, 2)) my_list[pn] = idx;
+
+            nf_mine += __popc(Mf & my_group);
+            nn_mine += __popc(Mn & my_group);
+          }
+          if (my_s < S && my_a < kAtoms &&
+              GD_DCHECK(bp.err, nf_mine + my_a < kList && kList - 1 - nn_mine - my_a >= 0, 3)) {
+            my_list[nf_mine + my_a] = static_cast<uint16_t>(kFar);
+            my_list[kList - 1 - nn_mine - my_a] = static_cast<uint16_t>(kFar);
+          }
+          __syncwarp();
+
+          // Phase 2: every term of the kept rows, kAtoms rows per step
+          float av = 0.0f, ae = 0.0f;  // ae: corrections from FP64 re-decisions (charge included)
+#pragma unroll
+          for (int s = 0; s < S; ++s) {
+            float aes = 0.0f;  // sum of q_r / d2 over this slot's kept pairs
+            const int nf = __shfl_sync(kFull, nf_mine, s * 8), nn = __shfl_sync(kFull, nn_mine, s * 8);
+            const uint16_t *lst = s_list + s * kList;
+            // far rows: Coulomb only
 #pragma unroll 1
-          for (int k0 = kList - (nn + kAtoms - 1) / kAtoms * kAtoms; k0 < kList; k0 += kAtoms) {
-            int ix[kAtoms];
-            float4 r[kAtoms];
-            int rt[kAtoms], rs[kAtoms], rc[kAtoms];
-#pragma unroll
-            for (int i = 0; i < kAtoms; ++i) {
-              ix[i] = lst[k0 + i];
-              if (!GD_DCHECK(bp.err, ix[i] <= kFar, 4)) ix[i] = kFar;
-              r[i] = s_pos[ix[i]];
-              const int4 mt = s_meta[ix[i]];
-              rt[i] = mt.x;
-              if (!GD_DCHECK(bp.err, rt[i] >= 0 && rt[i] + lt[s] < p.nt * p.nt, 5)) rt[i] = 0;
-              rs[i] = mt.y;
-              rc[i] = 0;
-            }
-            bool amb = false;
-#pragma unroll
-            for (int i = 0; i < kAtoms; ++i)
-              pair32<SERIAL, CLAMP>(r[i], rt[i], rs[i], tab, lx[s], ly[s], lz[s], lt[s], lser[s], gv, ge, gdd, av,
-                                    aes, lcnt[s], rc[i], amb);
-            if (__any_sync(kFull, amb)) {  // at most one entry per step: <= 4 * 18 per segment
-              if (lane == 0 && GD_DCHECK(bp.err, (seg_cnt >> 16) < kMaxS * kList, 7))
-                s_fixq[seg_cnt >> 16] = static_cast<uint16_t>(k0 | (s << 8));
-              seg_cnt += 1 << 16;
-            }
-            // receptor burial counts of the step's rows: their ballots are
-            // recorded here and added up once per segment (below); a step
-            // with no pair within 8 A (about half of them) records nothing
-            int any_rc = 0;
-#pragma unroll
-            for (int i = 0; i < kAtoms; ++i) any_rc |= rc[i];
-            if (__any_sync(kFull, any_rc != 0)) {
+            for (int k0 = 0; k0 < nf; k0 += kAtoms) {
+              int ix[kAtoms];
+              float4 r[kAtoms];
 #pragma unroll
               for (int i = 0; i < kAtoms; ++i) {
-                const unsigned bm = __ballot_sync(kFull, rc[i] != 0);
-                if (lane == i && GD_DCHECK(bp.err, (seg_cnt & 0xffff) + i < kMaxS * kList, 8)) {
-                  s_cmask[(seg_cnt & 0xffff) + i] = bm;
-                  s_cidx[(seg_cnt & 0xffff) + i] = static_cast<uint16_t>(ix[i]);
-                }
+                ix[i] = lst[k0 + i];
+                if (!GD_DCHECK(bp.err, ix[i] <= kFar, 4)) ix[i] = kFar;
+                r[i] = s_pos[ix[i]];
               }
-              seg_cnt += kAtoms;
+              bool amb = false;
+#pragma unroll
+              for (int i = 0; i < kAtoms; ++i) pair32_elec(r[i], lx[s], ly[s], lz[s], ge, aes, amb);
+              if (__any_sync(kFull, amb)) {  // at most one entry per step: <= 4 * 18 per segment
+                if (lane == 0 && GD_DCHECK(bp.err, (seg_cnt >> 16) < kMaxS * kList, 7))
+                  s_fixq[seg_cnt >> 16] = static_cast<uint16_t>(k0 | (s << 8));
+                seg_cnt += 1 << 16;
+              }
             }
-          }
-          ae = __fmaf_rn(aes, lq[s], ae);
-        }
-        __syncwarp();
-        // FP64 re-decisions of the flagged steps' pairs in the guard band
-        const int nfix = seg_cnt >> 16, ncm = seg_cnt & 0xffff;
+            // near rows: every term; the first step may start in the padding
 #pragma unroll 1
-        for (int t = 0; t < nfix; ++t) {
-          const int e = s_fixq[t], k0 = e & 255, s = e >> 8;
-          const int j = ch * kChunk + s * 32 + lane;
-          if (j >= p.nl) continue;
-          double X, Y, Z;
-          ligand_atom(p, f, pose, j, X, Y, Z);
-          // the lane's FP32 coordinates, as in the chunk set-up
-          const float fx = static_cast<float>(X - p.ox), fy = static_cast<float>(Y - p.oy),
-                      fz = static_cast<float>(Z - p.oz);
-          const float fq = static_cast<float>(p.lig_q[j]);
-          const int ft = p.lig_type[j], fs = SERIAL ? p.lig_serial[j] : 0;
+            for (int k0 = kList - (nn + kAtoms - 1) / kAtoms * kAtoms; k0 < kList; k0 += kAtoms) {
+              int ix[kAtoms];
+              float4 r[kAtoms];
+              int rt[kAtoms], rs[kAtoms], rc[kAtoms];
+#pragma unroll
+              for (int i = 0; i < kAtoms; ++i) {
+                ix[i] = lst[k0 + i];
+                if (!GD_DCHECK(bp.err, ix[i] <= kFar, 4)) ix[i] = kFar;
+                r[i] = s_pos[ix[i]];
+                const int4 mt = s_meta[ix[i]];
+                rt[i] = mt.x;
+                if (!GD_DCHECK(bp.err, rt[i] >= 0 && rt[i] + lt[s] < p.nt * p.nt, 5)) rt[i] = 0;
+                rs[i] = mt.y;
+                rc[i] = 0;
+              }
+              bool amb = false;
+#pragma unroll
+              for (int i = 0; i < kAtoms; ++i)
+                pair32<SERIAL, CLAMP>(r[i], rt[i], rs[i], tab, lx[s], ly[s], lz[s], lt[s], lser[s], gv, ge, gdd, av,
+                                      aes, lcnt[s], rc[i], amb);
+              if (__any_sync(kFull, amb)) {  // at most one entry per step: <= 4 * 18 per segment
+                if (lane == 0 && GD_DCHECK(bp.err, (seg_cnt >> 16) < kMaxS * kList, 7))
+                  s_fixq[seg_cnt >> 16] = static_cast<uint16_t>(k0 | (s << 8));
+                seg_cnt += 1 << 16;
+              }
+              // receptor burial counts of the step's rows: their ballots are
+              // recorded here and added up once per segment (below); a step
+              // with no pair within 8 A (about half of them) records nothing
+              int any_rc = 0;
+#pragma unroll
+              for (int i = 0; i < kAtoms; ++i) any_rc |= rc[i];
+              if (__any_sync(kFull, any_rc != 0)) {
+#pragma unroll
+                for (int i = 0; i < kAtoms; ++i) {
+                  const unsigned bm = __ballot_sync(kFull, rc[i] != 0);
+                  if (lane == i && GD_DCHECK(bp.err, (seg_cnt & 0xffff) + i < kMaxS * kList, 8)) {
+                    s_cmask[(seg_cnt & 0xffff) + i] = bm;
+                    s_cidx[(seg_cnt & 0xffff) + i] = static_cast<uint16_t>(ix[i]);
+                  }
+                }
+                seg_cnt += kAtoms;
+              }
+            }
+            ae = __fmaf_rn(aes, lq[s], ae);
+          }
+          __syncwarp();
+          // FP64 re-decisions of the flagged steps' pairs in the guard band
+          const int nfix = seg_cnt >> 16, ncm = seg_cnt & 0xffff;
 #pragma unroll 1
-          for (int i = 0; i < kAtoms; ++i) {
-            const int ixi = s_list[s * kList + k0 + i];
-            if (ixi == kFar || !GD_DCHECK(bp.err, ixi < kFar, 4)) continue;
-            const float4 ri = s_pos[ixi];
-            if (!near_band(d2f(ri, fx, fy, fz), gv, ge, gdd)) continue;
-            const int4 mt = s_meta[ixi];
-            const FixOut fo = fix_pair<SERIAL, CLAMP>(p, X, Y, Z, ri, gbase + ixi - sbase, mt.x, mt.y, fx, fy, fz, fq,
-                                                      ft, fs);
-            av += fo.dv;
-            ae += fo.de;
-            if (fo.dl) {
-              s_lfix[s * 32 + lane] += fo.dl;
-              atomicAdd(&s_rc[ixi - sbase], fo.dl);
+          for (int t = 0; t < nfix; ++t) {
+            const int e = s_fixq[t], k0 = e & 255, s = e >> 8;
+            const int j = ch * kChunk + s * 32 + lane;
+            if (j >= p.nl) continue;
+            double X, Y, Z;
+            ligand_atom(p, f, pose, j, X, Y, Z);
+            // the lane's FP32 coordinates, as in the chunk set-up
+            const float3 c32 = atom32(p, f, pose, j);
+            const float fx = c32.x, fy = c32.y, fz = c32.z, fq = static_cast<float>(p.lig_rel[j].w);
+            const int ft = p.lig_type[j], fs = SERIAL ? p.lig_serial[j] : 0;
+#pragma unroll 1
+            for (int i = 0; i < kAtoms; ++i) {
+              const int ixi = s_list[s * kList + k0 + i];
+              if (ixi == kFar || !GD_DCHECK(bp.err, ixi < kFar, 4)) continue;
+              const float4 ri = s_pos[ixi];
+              if (!near_band(d2f(ri, fx, fy, fz), gv, ge, gdd)) continue;
+              const int4 mt = s_meta[ixi];
+              const FixOut fo = fix_pair<SERIAL, CLAMP>(p, X, Y, Z, ri, gbase + ixi - sbase, mt.x, mt.y, fx, fy, fz, fq,
+                                                        ft, fs);
+              av += fo.dv;
+              ae += fo.de;
+              if (fo.dl) {
+                s_lfix[s * 32 + lane] += fo.dl;
+                atomicAdd(&s_rc[ixi - sbase], fo.dl);
+              }
             }
           }
-        }
-        // receptor burial counts of the near rows (the far atom's ballots are 0)
-        for (int t = lane; t < ncm; t += 32) {
-          const unsigned bm = s_cmask[t];
-          if (bm) atomicAdd(&s_rc[s_cidx[t] - sbase], __popc(bm));
-        }
-        seg_cnt = 0;
-        fv += fx_energy(av, bp.err);
-        fe += fx_energy(ae, bp.err);
-        __syncwarp();
-        // receptor burial counts of this segment into the per-item counters
-        for (int i = lane; i < na; i += 32) {
-          const int c = s_rc[i];
-          if (c) {
-            if (SPLIT) {
-              // a count never exceeds the ligand's atoms (< 65,536 in split
-              // launches), so the two halves of a word never carry into each other
-              const int a = gbase + i;
-              if (GD_DCHECK(bp.err, a < bp.max_nr, 10))
-                atomicAdd(&bp.pcount[static_cast<size_t>(gp) * ((bp.max_nr + 1) >> 1) + (a >> 1)],
-                          static_cast<unsigned>(c) << ((a & 1) * 16));
-            }
-            else bump_count(cnt, gbase + i, c);
-            s_rc[i] = 0;
+          // receptor burial counts of the near rows (the far atom's ballots are 0)
+          for (int t = lane; t < ncm; t += 32) {
+            const unsigned bm = s_cmask[t];
+            if (bm) atomicAdd(&s_rc[s_cidx[t] - sbase], __popc(bm));
           }
-        }
-        __syncwarp();
-        if (lane == 0 && kk + kWS < nk) {
-          issue_seg(q + kWS, seg_at(kk + kWS), p, s_pos, s_meta, s_bar);
-          q_issued = q + kWS + 1;
+          seg_cnt = 0;
+          fv += fx_energy(av, bp.err);
+          fe += fx_energy(ae, bp.err);
+          __syncwarp();
+          // receptor burial counts of this segment into the per-item counters
+          for (int i = lane; i < na; i += 32) {
+            const int c = s_rc[i];
+            if (c) {
+              if (SPLIT) {
+                // a count never exceeds the ligand's atoms (< 65,536 in split
+                // launches), so the two halves of a word never carry into each other
+                const int a = gbase + i;
+                if (GD_DCHECK(bp.err, a < bp.max_nr, 10))
+                  atomicAdd(&bp.pcount[static_cast<size_t>(gp) * ((bp.max_nr + 1) >> 1) + (a >> 1)],
+                            static_cast<unsigned>(c) << ((a & 1) * 16));
+              }
+              else bump_count(cnt, gbase + i, c);
+              s_rc[i] = 0;
+            }
+          }
+          __syncwarp();
+          if (lane == 0 && kk + kWS < nk) {
+            issue_seg(q + kWS, seg_at(kk + kWS), p, s_pos, s_meta, s_bar);
+            q_issued = q + kWS + 1;
+          }
         }
       }
       if (failed) break;
@@ -778,21 +813,36 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_score_f32w(const BatchPar
         if (R == 1) {
           desolv_t += __ldcg(bp.part + (static_cast<size_t>(gp) * bp.max_chunks + c) * 96 + 64 + lane);
         } else {
-          double dc = 0.0;
+          double dc = 0.0, t[S];
+#pragma unroll
           for (int s = 0; s < S; ++s) {
             const int j = c * kChunk + s * 32 + lane;
+            t[s] = 0.0;
             if (j < p.nl) {
               const unsigned n = __ldcg(&bp.lcount[static_cast<size_t>(gp) * bp.max_nl + j]);
-              dc += p.lig_desolv[static_cast<size_t>(j) * 11 + (n < 10u ? n : 10u)];
+              t[s] = p.lig_desolv[static_cast<size_t>(j) * 11 + (n < 10u ? n : 10u)];
             }
           }
+#pragma unroll
+          for (int s = 0; s < S; ++s) dc += t[s];
           desolv_t += dc;
         }
       }
-      for (int i = lane; i < p.nr; i += 32) {
-        const unsigned w = __ldcg(&bp.pcount[static_cast<size_t>(gp) * ((bp.max_nr + 1) >> 1) + (i >> 1)]);
-        const unsigned c = (w >> ((i & 1) * 16)) & 0xffffu;
-        desolv_t += p.rec_desolv[static_cast<size_t>(i) * 11 + (c < 10u ? c : 10u)];
+      // four rounds' loads in flight, added in order
+      for (int i0 = 0; i0 < p.nr; i0 += 128) {
+        double t[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int i = i0 + u * 32 + lane;
+          t[u] = 0.0;
+          if (i < p.nr) {
+            const unsigned w = __ldcg(&bp.pcount[static_cast<size_t>(gp) * ((bp.max_nr + 1) >> 1) + (i >> 1)]);
+            const unsigned c = (w >> ((i & 1) * 16)) & 0xffffu;
+            t[u] = p.rec_desolv[static_cast<size_t>(i) * 11 + (c < 10u ? c : 10u)];
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) desolv_t += t[u];
       }
     } else {
       // receptor burial -> desolvation; reset the counters for the next item
