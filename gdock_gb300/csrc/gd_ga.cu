@@ -20,6 +20,7 @@
 // evolve.  One generation is captured as a CUDA graph and replayed.
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstring>
 #include <vector>
 
@@ -104,34 +105,45 @@ void draw_initial(Rng &rng, const gd_ga_cfg &c, double *genes) {
 // entries in the reference's operation order).
 // slots (may be null): the k-th group of n poses belongs to slot slots[k / n]
 // (the server's resident jobs); else pose k belongs to job job_of[k].
-__global__ void k_frames(const double *genes, gd_pose_frame *frames, const int *job_of, const GaJobState *state,
-                         int total, const int *slots, int n) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= total) return;
-  const int job = slots ? slots[t / n] : job_of[t];
-  const int k = slots ? job * n + t % n : t;
-  if (state[job].stop) return;
+// Four lanes per pose, one angle each (FP64 sines are some sixty operations on
+// a pipe of two lanes a clock and SM), in CTAs of two warps so that a
+// population spreads over the SMs: 150 poses 8.5 -> 5.0 us.
+constexpr int kFrameThreads = 64;
+__global__ void __launch_bounds__(kFrameThreads) k_frames(const double *genes, gd_pose_frame *frames, const int *job_of,
+                                                          const GaJobState *state, int total, const int *slots, int n) {
+  const int i = blockIdx.x * kFrameThreads + threadIdx.x, t = i >> 2, c = i & 3;
+  int k = 0;
+  bool on = t < total;
+  if (on) {
+    const int job = slots ? slots[t / n] : job_of[t];
+    k = slots ? job * n + t % n : t;
+    on = !state[job].stop;
+  }
   const double *g = genes + 6 * static_cast<size_t>(k);
-  double sa, ca, sb, cb, sg, cg;
-  sincos(g[0], &sa, &ca);
-  sincos(g[1], &sb, &cb);
-  sincos(g[2], &sg, &cg);
-  gd_pose_frame f;
-  f.ca = ca;
-  f.sa = sa;
-  f.cb = cb;
-  f.sb = sb;
-  f.cg = cg;
-  f.sg = sg;
-  f.m01 = __dadd_rn(__dmul_rn(-sa, cg), __dmul_rn(__dmul_rn(ca, sb), sg));
-  f.m02 = __dadd_rn(__dmul_rn(sa, sg), __dmul_rn(__dmul_rn(ca, sb), cg));
-  f.m11 = __dadd_rn(__dmul_rn(ca, cg), __dmul_rn(__dmul_rn(sa, sb), sg));
-  f.m12 = __dadd_rn(__dmul_rn(-ca, sg), __dmul_rn(__dmul_rn(sa, sb), cg));
-  f.dx = g[3];
-  f.dy = g[4];
-  f.dz = g[5];
-  f.pad[0] = f.pad[1] = f.pad[2] = 0.0;
-  frames[k] = f;
+  double sn = 0.0, cs = 0.0;
+  if (on && c < 3) sincos(g[c], &sn, &cs);
+  const double sa = __shfl_sync(kFull, sn, 0, 4), sb = __shfl_sync(kFull, sn, 1, 4), sg = __shfl_sync(kFull, sn, 2, 4);
+  const double ca = __shfl_sync(kFull, cs, 0, 4), cb = __shfl_sync(kFull, cs, 1, 4), cg = __shfl_sync(kFull, cs, 2, 4);
+  if (!on) return;
+  // each lane stores a quarter of the frame
+  D4 q;
+  if (c == 0) {
+    q = D4{ca, sa, cb, sb};
+  } else if (c == 1) {
+    q = D4{cg, sg, __dadd_rn(__dmul_rn(-sa, cg), __dmul_rn(__dmul_rn(ca, sb), sg)),
+                     __dadd_rn(__dmul_rn(sa, sg), __dmul_rn(__dmul_rn(ca, sb), cg))};
+  } else if (c == 2) {
+    q = D4{__dadd_rn(__dmul_rn(ca, cg), __dmul_rn(__dmul_rn(sa, sb), sg)),
+                     __dadd_rn(__dmul_rn(-ca, sg), __dmul_rn(__dmul_rn(sa, sb), cg)), g[3], g[4]};
+  } else {
+    q = D4{g[5], 0.0, 0.0, 0.0};
+  }
+  static_assert(sizeof(gd_pose_frame) == 4 * sizeof(D4) && offsetof(gd_pose_frame, m01) == 48 &&
+                    offsetof(gd_pose_frame, m11) == 64 && offsetof(gd_pose_frame, dx) == 80,
+                "the quarters of a frame");
+  double2 *out = reinterpret_cast<double2 *>(reinterpret_cast<double *>(frames + k) + 4 * c);
+  out[0] = make_double2(q.x, q.y);
+  out[1] = make_double2(q.z, q.w);
 }
 
 struct GaStepParams {
@@ -173,27 +185,42 @@ __device__ __forceinline__ bool hof_similar(const double *a, const double *b) {
   return true;
 }
 
+constexpr int kGaThreads = 512;  // threads of k_ga_step
+// k_ga_step runs kGaThreads working threads, which meet at barrier 1, and one
+// more warp for the generation's report, which does not.
+__device__ __forceinline__ void ga_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kGaThreads) : "memory"); }
+constexpr int kMirrorMax = 1024;  // populations up to this size are mirrored in FP32 for the Hall of Fame
+constexpr size_t kGaSmemPlain = 24 * 1024;  // dynamic shared memory that needs no raised limit beside the static part
 constexpr int kHofChunk = 32;    // candidates pre-checked per round (one per lane)
 constexpr int kHofNewMax = 32;   // entries a round may add before the pre-check is redone
 constexpr int kHofF32Max = 512;  // entries mirrored in FP32 for the pre-filter
 
-// FP32 pre-filter of hof_similar: true only where the exact FP64 test says
-// "not similar": some angle differs by more than 0.2 and less than
-// 2 pi - 0.2 (so also by more than 0.2 across the wrap), or some
-// displacement by more than 2, each by a margin (1e-4 + 1e-6 (|a| + |b|))
-// far above the FP32 rounding of both values and of their difference.
-__device__ __forceinline__ bool hof_far32(const float *a, const float *b) {
+// FP32 pre-filter of hof_similar: 0 only where the exact FP64 test says "not
+// similar" (some angle differs by more than 0.2 and less than 2 pi - 0.2, so
+// also by more than 0.2 across the wrap, or some displacement by more than 2),
+// 1 only where it says "similar" (every angle within 0.2, directly or across
+// the wrap, and every displacement within 2), each by a margin (1e-4 +
+// 1e-6 (|a| + |b|)) far above the FP32 rounding of both values and of their
+// difference; else 2.
+__device__ __forceinline__ int hof_test32(const float *a, const float *b) {
+  bool sure = true;
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     const float d = fabsf(a[i] - b[i]), mg = 1e-4f + 1e-6f * (fabsf(a[i]) + fabsf(b[i]));
-    if (d > 0.2f + mg && d < 6.0831853f - mg) return true;
+    if (d > 0.2f + mg && d < 6.0831853f - mg) return 0;
+    sure = sure && (d < 0.2f - mg || d > 6.0831853f + mg);
   }
 #pragma unroll
   for (int i = 3; i < 6; ++i) {
     const float d = fabsf(a[i] - b[i]), mg = 1e-4f + 1e-6f * (fabsf(a[i]) + fabsf(b[i]));
-    if (d > 2.0f + mg) return true;
+    if (d > 2.0f + mg) return 0;
+    sure = sure && d < 2.0f - mg;
   }
-  return false;
+  return sure ? 1 : 2;
+}
+__device__ __forceinline__ bool hof_similar_any(const float *a32, const float *b32, const double *a, const double *b) {
+  const int t = hof_test32(a32, b32);
+  return t == 2 ? hof_similar(a, b) : t == 1;
 }
 
 __device__ __forceinline__ bool genes_equal(const double *a, const double *b) {
@@ -228,16 +255,16 @@ __device__ void hof_update(const GaStepParams &P, GaJobState &st, int job, int g
     s_ctl[2] = st.hof_n;
     s_ctl[3] = st.hof_sorted;
   }
-  __syncthreads();
+  ga_sync();
   for (;;) {
     const int base = s_ctl[0], cnt0 = s_ctl[2];
     if (base >= n || s_ctl[1] >= c.hof_top_k) break;
     const int end = min(base + kHofChunk, n);
-    const int nw = blockDim.x >> 5, w = tid >> 5;
+    const int nw = kGaThreads >> 5, w = tid >> 5;
     const bool f32 = cnt0 <= kHofF32Max;
     if (f32)
-      for (int i = tid; i < 6 * cnt0; i += blockDim.x) s_hf[i] = __double2float_rn(H[i / 6].genes[i % 6]);
-    __syncthreads();
+      for (int i = tid; i < 6 * cnt0; i += kGaThreads) s_hf[i] = __double2float_rn(H[i / 6].genes[i % 6]);
+    ga_sync();
     {
       int cs = 0;
       if (base + lane < end) {
@@ -250,11 +277,11 @@ __device__ void hof_update(const GaStepParams &P, GaJobState &st, int job, int g
           g32[i] = __double2float_rn(g[i]);
         }
         for (int e = w; e < cnt0; e += nw)
-          if (!(f32 && hof_far32(g32, s_hf + 6 * e))) cs += hof_similar(g, H[e].genes);
+          cs += f32 ? hof_similar_any(g32, s_hf + 6 * e, g, H[e].genes) : hof_similar(g, H[e].genes);
       }
       s_part[tid] = cs;
     }
-    __syncthreads();
+    ga_sync();
     if (tid < 32) {
       {
         int cs = 0;
@@ -342,12 +369,89 @@ __device__ void hof_update(const GaStepParams &P, GaJobState &st, int job, int g
         s_ctl[3] = sorted;
       }
     }
-    __syncthreads();
+    ga_sync();
   }
   if (tid == 0) {
     st.hof_n = s_ctl[2];
     st.hof_sorted = s_ctl[3];
   }
+}
+
+// hof_update when no prune can come up (the entries held and top_k more fit)
+// and the entries fit the FP32 mirror: then a candidate goes in when it is
+// similar neither to an entry held at the start nor to one added before it in
+// this generation.  A warp per candidate tests the entries held; then, add by
+// add, all threads drop the candidates similar to the new entry.  (One warp
+// walking rounds of 32 candidates took 35 to 50 us of a generation of 150.)
+__device__ void hof_append(const GaStepParams &P, GaJobState &st, int job, int gen, const double *G, const double *f,
+                           const int *order, uint8_t *s_drop, int *s_ctl, float *s_hf, float *s_pf) {
+  const gd_ga_cfg &c = P.cfg;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = c.pop_size, cnt0 = st.hof_n;
+  gd_hof_entry *H = P.hof + static_cast<size_t>(job) * (c.hof_max_size + 1);
+  // FP32 mirrors, gene by gene (conversions run on the FP64 pipe: once each)
+  for (int i = tid; i < 6 * cnt0; i += kGaThreads) s_hf[i % 6 * kHofF32Max + i / 6] = __double2float_rn(H[i / 6].genes[i % 6]);
+  for (int i = tid; i < 6 * n; i += kGaThreads) s_pf[i] = __double2float_rn(G[i]);
+  ga_sync();
+  for (int r = warp; r < n; r += kGaThreads / 32) {
+    const int k = order[r];
+    float g32[6];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) g32[i] = s_pf[6 * k + i];
+    bool sim = false;
+    for (int e0 = 0; e0 < cnt0 && !sim; e0 += 32) {
+      const int e = e0 + lane;
+      bool hit = false;
+      if (e < cnt0) {
+        float h32[6];
+#pragma unroll
+        for (int i = 0; i < 6; ++i) h32[i] = s_hf[i * kHofF32Max + e];
+        hit = hof_similar_any(g32, h32, G + 6 * k, H[e].genes);
+      }
+      sim = __any_sync(kFull, hit);
+    }
+    if (lane == 0) s_drop[r] = sim;
+  }
+  ga_sync();
+  int from = 0, cnt = cnt0;
+  for (int added = 0; added < c.hof_top_k; ++added) {
+    if (warp == 0) {
+      // the first candidate left, as the next entry
+      int r0 = n;
+      for (int b = from & ~31; b < n; b += 32) {
+        const int r = b + lane;
+        const unsigned m = __ballot_sync(kFull, r >= from && r < n && !s_drop[r]);
+        if (m) {
+          r0 = b + __ffs(m) - 1;
+          break;
+        }
+      }
+      if (r0 < n && GD_DCHECK(P.err, cnt < c.hof_max_size + 1, 50)) {
+        gd_hof_entry &x = H[cnt];
+        const int k = order[r0];
+        if (lane < 6) x.genes[lane] = G[6 * k + lane];
+        else if (lane == 6) x.fitness = f[k];
+        else if (lane == 7) x.generation = gen;
+        else if (lane == 8) x.pad = 0;
+      }
+      if (lane == 0) s_ctl[0] = r0;
+    }
+    ga_sync();
+    const int r0 = s_ctl[0];
+    if (r0 >= n) break;
+    ++cnt;
+    from = r0 + 1;
+    if (added + 1 < c.hof_top_k) {
+      const int a = order[r0];
+      for (int r = from + tid; r < n; r += kGaThreads) {
+        if (s_drop[r]) continue;
+        const int k = order[r];
+        if (hof_similar_any(s_pf + 6 * k, s_pf + 6 * a, G + 6 * k, G + 6 * a)) s_drop[r] = 1;
+      }
+    }
+    ga_sync();
+  }
+  ga_sync();
+  if (tid == 0) st.hof_n = cnt;
 }
 
 // Sort keys of fitness values: unsigned order = the order of the values,
@@ -365,7 +469,7 @@ __device__ __forceinline__ unsigned long long asc_key(double f) {
 __device__ void bitonic_sort(unsigned long long *key, int *idx, int P) {
   for (int k = 2; k <= P; k <<= 1)
     for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int t = threadIdx.x; t < P / 2; t += blockDim.x) {
+      for (int t = threadIdx.x; t < P / 2; t += kGaThreads) {
         const int i = ((t & ~(j - 1)) << 1) | (t & (j - 1)), l = i | j;
         const unsigned long long a = key[i], b = key[l];
         const int ia = idx[i], ib = idx[l];
@@ -377,8 +481,40 @@ __device__ void bitonic_sort(unsigned long long *key, int *idx, int P) {
           idx[l] = ia;
         }
       }
-      __syncthreads();
+      ga_sync();
     }
+}
+
+// order = the indices of keys [0, n) ascending by key then index.  Up to a
+// thread per entry each is placed by the number of entries before it (two
+// threads an entry where they suffice): 256 entries took 36 barrier-separated
+// sorting stages, 4 us; larger populations keep the bitonic sort.
+__device__ void sort_order(unsigned long long *key, int *order, int n, int P) {
+  const int nt = kGaThreads, tid = threadIdx.x;
+  ga_sync();
+  if (n <= nt) {
+    const int per = 2 * n <= nt ? 2 : 1, e = tid / per, h = tid % per;
+    const int q0 = h * ((n + 1) / 2), q1 = per == 2 && h == 0 ? (n + 1) / 2 : n;
+    int rank = 0;
+    if (e < n) {
+      const unsigned long long k = key[e];
+#pragma unroll 8
+      for (int q = q0; q < q1; ++q) {
+        const unsigned long long o = key[q];
+        rank += o < k || (o == k && q < e);
+      }
+    }
+    if (per == 2) rank += __shfl_xor_sync(kFull, rank, 1);
+    if (e < n && h == 0) order[rank] = e;
+    ga_sync();
+    return;
+  }
+  for (int k = tid; k < P; k += nt) {
+    if (k >= n) key[k] = ~0ull;
+    order[k] = k;
+  }
+  ga_sync();
+  bitonic_sort(key, order, P);
 }
 
 __host__ __device__ inline int pow2_at_least(int n) {
@@ -390,27 +526,43 @@ __host__ __device__ inline int pow2_at_least(int n) {
 // dynamic shared memory of k_ga_step for a population of n
 inline size_t ga_step_smem(int n) {
   const size_t p2 = static_cast<size_t>(pow2_at_least(n));
-  return sizeof(double) * n + sizeof(unsigned long long) * p2 + sizeof(int) * (n + p2);
+  return sizeof(double) * n + sizeof(unsigned long long) * p2 + sizeof(int) * (n + p2) +
+         (n <= kMirrorMax ? 6 * sizeof(float) * n : 0) + static_cast<size_t>(n);
+}
+
+// f64::rem_euclid(v, 2 pi) (src/chromosome.rs:66): fmod is exact, and so are v
+// itself and v -+ 2 pi (Sterbenz) where it equals them.
+__device__ __forceinline__ double wrap_angle(double v) {
+  const double two_pi = 6.283185307179586;
+  const double m = fabs(v);
+  double r = m < two_pi ? v : (m < 2.0 * two_pi ? copysign(__dsub_rn(m, two_pi), v) : fmod(v, two_pi));
+  if (r < 0.0) r = __dadd_rn(r, two_pi);
+  return r;
 }
 
 // One CTA per job: the reference loop's bookkeeping for the fitness just
 // computed (with the Hall of Fame), then evolve.  The stable orders of the
 // population (elitism, Hall of Fame, best of the generation) and of the
-// offspring are bitonic sorts of integer keys: FP64 comparisons run at a
-// small fraction of the integer rate on this part, and the O(n^2) rank
-// counts they replace took 29 ms per generation at 4,096 poses.
-__global__ void __launch_bounds__(256) k_ga_step(const GaStepParams P) {
+// offspring are sorts of integer keys: FP64 comparisons run at a small
+// fraction of the integer rate on this part, and the O(n^2) rank counts they
+// replace took 29 ms per generation at 4,096 poses.
+// What bounds it: latency (one CTA; chains of loads and barriers).  150 poses
+// with Hall of Fame and metrics: 70 -> 30 us (cold caches).
+__global__ void __launch_bounds__(kGaThreads + 32) k_ga_step(const GaStepParams P) {
   extern __shared__ __align__(16) unsigned char smem[];
   const gd_ga_cfg &c = P.cfg;
-  const int job = P.slots ? P.slots[blockIdx.x] : static_cast<int>(blockIdx.x), tid = threadIdx.x, nt = blockDim.x;
+  const int job = P.slots ? P.slots[blockIdx.x] : static_cast<int>(blockIdx.x), tid = threadIdx.x;
+  constexpr int nt = kGaThreads;
   const int n = c.pop_size, m = 2 * (n / 2), P2 = pow2_at_least(n);
   double *f = reinterpret_cast<double *>(smem);                            // [n] fitness of the population
   unsigned long long *kb = reinterpret_cast<unsigned long long *>(f + n);  // [P2] sort keys
   int *sel = reinterpret_cast<int *>(kb + P2);                             // [n] tournament winners
   int *order = sel + n;                                                    // [P2] sort indices
+  float *s_pf = reinterpret_cast<float *>(order + P2);                     // [n][6] genes (n <= kMirrorMax)
+  uint8_t *s_drop = reinterpret_cast<uint8_t *>(s_pf + (n <= kMirrorMax ? 6 * n : 0));  // [n] candidates out
   __shared__ double s_eg[64 * 6];                  // elites' genes, staged before the population is overwritten
-  __shared__ int s_evolve, s_hof, s_gen, s_final, s_nan;
-  __shared__ int s_csim[kHofChunk], s_hctl[4], s_hpart[256];  // Hall of Fame rounds
+  __shared__ int s_evolve, s_hof, s_gen, s_final, s_nan, s_best;
+  __shared__ int s_csim[kHofChunk], s_hctl[4], s_hpart[kGaThreads];  // Hall of Fame rounds
   __shared__ double s_hnew[kHofNewMax * 6];
   __shared__ float s_hf[kHofF32Max * 6];
   GaJobState &st = P.state[job];
@@ -420,22 +572,39 @@ __global__ void __launch_bounds__(256) k_ga_step(const GaStepParams P) {
     s_final = st.gen >= c.max_generations;
     s_nan = 0;
   }
-  for (int k = tid; k < n; k += nt) f[k] = E[k].fitness;
   __syncthreads();
   if (s_final) {
     // the evaluation just done was of the final population: stop here
     if (tid == 0) st.stop = 2;
     return;
   }
+  const bool report = P.metrics && P.eval_on[job];
+  if (tid >= nt) {
+    // the generation's metrics: the best pose's and the mean DockQ as a
+    // left-to-right sum (src/commands/run.rs:388,449-451): a chain of n FP64
+    // adds, 9 us at 150, beside the other warps' work
+    if (!report) return;
+    const gd_dock_metrics *M = P.metrics + static_cast<size_t>(job) * n;
+    double sum = 0.0;
+#pragma unroll 8
+    for (int k = 0; k < n; ++k) sum += M[k].dockq;
+    asm volatile("bar.sync 2, %0;" ::"n"(kGaThreads + 32) : "memory");  // s_gen, s_best
+    if (tid == nt) {
+      const size_t jg = static_cast<size_t>(job) * c.max_generations + s_gen;
+      P.best_metrics[jg] = M[s_best];
+      P.mean_dockq[jg] = sum / static_cast<double>(n);
+    }
+    return;
+  }
   // stable ascending order of the population (src/population.rs:76-82 for
   // the elites, src/commands/run.rs:195-201 for the Hall of Fame)
-  for (int k = tid; k < P2; k += nt) {
-    if (k < n && f[k] != f[k]) s_nan = 1;
-    kb[k] = k < n ? asc_key(f[k]) : ~0ull;
-    order[k] = k;
+  for (int k = tid; k < n; k += nt) {
+    const double e = E[k].fitness;
+    f[k] = e;
+    if (e != e) s_nan = 1;
+    kb[k] = asc_key(e);
   }
-  __syncthreads();
-  bitonic_sort(kb, order, P2);
+  sort_order(kb, order, n, P2);
   if (tid == 0) {
     const int gen = st.gen;
     s_gen = gen;
@@ -449,18 +618,9 @@ __global__ void __launch_bounds__(256) k_ga_step(const GaStepParams P) {
       for (int k = 1; k < n; ++k)
         if (f[bi] > f[k]) bi = k;
     }
+    s_best = bi;
     const double best = f[bi];
     P.history[static_cast<size_t>(job) * c.max_generations + gen] = best;
-    if (P.metrics && P.eval_on[job]) {
-      // the generation's metrics: the best pose's and the mean DockQ as a
-      // left-to-right sum (src/commands/run.rs:388,449-451)
-      const gd_dock_metrics *M = P.metrics + static_cast<size_t>(job) * n;
-      const size_t jg = static_cast<size_t>(job) * c.max_generations + gen;
-      P.best_metrics[jg] = M[bi];
-      double sum = 0.0;
-      for (int k = 0; k < n; ++k) sum += M[k].dockq;
-      P.mean_dockq[jg] = sum / static_cast<double>(n);
-    }
     if (gen > 0) {  // convergence window (src/commands/run.rs:400-409)
       const double imp = (st.last_best - best) / fabs(st.last_best);
       if (imp < c.convergence_threshold) st.stagnant += 1;
@@ -475,13 +635,20 @@ __global__ void __launch_bounds__(256) k_ga_step(const GaStepParams P) {
       s_evolve = 1;
     }
   }
-  __syncthreads();
-  if (!s_evolve && !s_hof) return;
+  ga_sync();
+  if (report) asm volatile("bar.arrive 2, %0;" ::"n"(kGaThreads + 32) : "memory");
   double *G = P.genes + static_cast<size_t>(job) * n * 6;
   const int ne = c.elitism < n ? c.elitism : n;
-  if (s_hof) hof_update(P, st, job, s_gen, G, f, order, s_csim, s_hnew, s_hctl, s_hpart, s_hf);
+  if (s_hof) {
+    const int held = st.hof_n;
+    ga_sync();
+    if (n <= kMirrorMax && held <= kHofF32Max && held + min(c.hof_top_k, n) <= c.hof_max_size)
+      hof_append(P, st, job, s_gen, G, f, order, s_drop, s_hctl, s_hf, s_pf);
+    else
+      hof_update(P, st, job, s_gen, G, f, order, s_csim, s_hnew, s_hctl, s_hpart, s_hf);
+  }
   if (!s_evolve) return;
-  const int gen = st.gen - 1;  // draws of the generation being evolved
+  const int gen = s_gen;  // draws of the generation being evolved
   const size_t jg = static_cast<size_t>(job) * c.max_generations + gen;
   const int *tour = P.tour + jg * c.tournament_size * n;
   const int *perm = P.perm + jg * n;
@@ -500,46 +667,39 @@ __global__ void __launch_bounds__(256) k_ga_step(const GaStepParams P) {
   }
   // elites: the first ne of the stable order
   for (int i = tid; i < ne * 6; i += nt) s_eg[i] = G[6 * order[i / 6] + i % 6];
-  __syncthreads();
+  ga_sync();
   // shuffle + crossover + mutation (src/population.rs:88-107, src/ga.rs:7-39,
-  // src/chromosome.rs:56-77); the offspring's carried fitness goes straight
-  // into descending sort keys
-  const double two_pi = 6.283185307179586;
-  for (int p = tid; p < n / 2; p += nt) {
+  // src/chromosome.rs:56-77), a thread per pair and gene; the offspring's
+  // carried fitness goes straight into descending sort keys
+  for (int i = tid; i < 6 * (n / 2); i += nt) {
+    const int p = i / 6, g = i % 6;
     const int a = sel[perm[2 * p]], b = sel[perm[2 * p + 1]];
-    for (int g = 0; g < 6; ++g) {
-      const double ga = G[6 * a + g], gb = G[6 * b + g];
-      const bool sw = cu[6 * p + g] <= c.crossover_rate;
-      double o[2] = {sw ? gb : ga, sw ? ga : gb};
-      for (int h = 0; h < 2; ++h) {
-        const int k = 2 * p + h;
-        if (mu[6 * k + g] <= c.mutation_rate) {
-          double v = __dadd_rn(o[h], mz[6 * k + g]);
-          if (g < 3) {
-            double r = fmod(v, two_pi);  // f64::rem_euclid
-            if (r < 0.0) r = __dadd_rn(r, two_pi);
-            v = r;
-          } else {
-            v = v < -c.max_displacement ? -c.max_displacement : (v > c.max_displacement ? c.max_displacement : v);
-          }
-          o[h] = v;
-        }
-        T[6 * k + g] = o[h];
+    const double ga = G[6 * a + g], gb = G[6 * b + g];
+    const bool sw = cu[i] <= c.crossover_rate;
+    const double o[2] = {sw ? gb : ga, sw ? ga : gb};
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int k = 2 * p + h;
+      double v = o[h];
+      if (mu[6 * k + g] <= c.mutation_rate) {
+        v = __dadd_rn(v, mz[6 * k + g]);
+        if (g < 3) v = wrap_angle(v);
+        else v = v < -c.max_displacement ? -c.max_displacement : (v > c.max_displacement ? c.max_displacement : v);
       }
+      T[6 * k + g] = v;
     }
-    kb[2 * p] = ~asc_key(f[a]);
-    kb[2 * p + 1] = ~asc_key(f[b]);
+    if (g == 0) {
+      kb[2 * p] = ~asc_key(f[a]);
+      kb[2 * p + 1] = ~asc_key(f[b]);
+    }
   }
-  for (int k = m + tid; k < P2; k += nt) kb[k] = ~0ull;
-  for (int k = tid; k < P2; k += nt) order[k] = k;
-  __syncthreads();
   // stable descending order by the carried fitness; elites over the first
   // slots (src/population.rs:110-118)
-  bitonic_sort(kb, order, P2);
-  for (int r = ne + tid; r < m; r += nt) {
-    const int k = order[r];
+  sort_order(kb, order, m, P2);
+  for (int i = 6 * ne + tid; i < 6 * m; i += nt) {
+    const int k = order[i / 6];
     if (!GD_DCHECK(P.err, k >= 0 && k < m, 52)) continue;
-    for (int g = 0; g < 6; ++g) G[6 * r + g] = T[6 * k + g];
+    G[i] = T[6 * k + i % 6];
   }
   for (int i = tid; i < ne * 6; i += nt) G[i] = s_eg[i];
 }
@@ -766,7 +926,7 @@ extern "C" gd_status gd_ga_run(gd_context *ctx, gd_complex *const *complexes, in
     cudaStream_t st = ctx->stream;
     auto generation = [&]() -> gd_status {
       const int total = static_cast<int>(jn);
-      k_frames<<<(total + 255) / 256, 256, 0, st>>>(R.genes, R.frames, R.job_of, R.state, total, nullptr, n);
+      k_frames<<<(4 * total + kFrameThreads - 1) / kFrameThreads, kFrameThreads, 0, st>>>(R.genes, R.frames, R.job_of, R.state, total, nullptr, n);
       cudaError_t ee = cudaGetLastError();
       if (ee != cudaSuccess) return cuda_fail(ctx, ee, "frames kernel");
       if (prec == GD_PREC_F32) {
@@ -788,11 +948,11 @@ extern "C" gd_status gd_ga_run(gd_context *ctx, gd_complex *const *complexes, in
                                         R.metrics + static_cast<size_t>(j) * n, &R.state[j].stop, st);
             if (ss != GD_OK) return ss;
           }
-      k_ga_step<<<jobs, 256, ga_smem, st>>>(P);
+      k_ga_step<<<jobs, kGaThreads + 32, ga_smem, st>>>(P);
       ee = cudaGetLastError();
       return ee == cudaSuccess ? GD_OK : cuda_fail(ctx, ee, "GA step kernel");
     };
-    if (ga_smem > 48 * 1024) cudaFuncSetAttribute(k_ga_step, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (ga_smem > kGaSmemPlain) cudaFuncSetAttribute(k_ga_step, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                   static_cast<int>(ga_smem));
     const int iters = G + 1;  // G evolutions + the evaluation of the final population
     if (use_graph && prec == GD_PREC_F32) {
@@ -1229,7 +1389,7 @@ gd_status server_tick(gd_server *S, int *active_out) {
     S->dirty = false;
     const int total = active * n;
     cudaEventRecord(S->ev0, st);
-    k_frames<<<(total + 255) / 256, 256, 0, st>>>(R.genes, R.frames, R.job_of, R.state, total, S->d_slots, n);
+    k_frames<<<(4 * total + kFrameThreads - 1) / kFrameThreads, kFrameThreads, 0, st>>>(R.genes, R.frames, R.job_of, R.state, total, S->d_slots, n);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(ctx, e, "frames kernel");
     if (S->cfg.precision == GD_PREC_F32) {
@@ -1259,9 +1419,9 @@ gd_status server_tick(gd_server *S, int *active_out) {
     P.slots = S->d_slots;
     P.cfg = c;
     const size_t ga_smem = ga_step_smem(n);
-    if (ga_smem > 48 * 1024)
+    if (ga_smem > kGaSmemPlain)
       cudaFuncSetAttribute(k_ga_step, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(ga_smem));
-    k_ga_step<<<active, 256, ga_smem, st>>>(P);
+    k_ga_step<<<active, kGaThreads + 32, ga_smem, st>>>(P);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(ctx, e, "GA step kernel");
     cudaEventRecord(S->ev1, st);
     e = cudaMemcpyAsync(S->h_states, R.state, sizeof(GaJobState) * J, cudaMemcpyDeviceToHost, st);
