@@ -108,10 +108,8 @@ gd_status ensure_batch_scratch(gd_context *ctx, size_t dev_bytes) {
   return GD_OK;
 }
 
-gd_status check_device_error(gd_context *ctx) {
-  int h = 0;
-  cudaError_t e = cudaMemcpy(&h, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return cuda_fail(ctx, e, "reading the device error word");
+// The status of a device error word that has been read (and is cleared when set).
+static gd_status error_status(gd_context *ctx, int h) {
   if (h == kDevOk) return GD_OK;
   cudaMemset(ctx->d_err, 0, sizeof(int));
   if (h == kDevTimeout) return fail(ctx, GD_ERR_TIMEOUT, "a device-side wait exceeded its spin limit");
@@ -123,6 +121,20 @@ gd_status check_device_error(gd_context *ctx) {
     return fail(ctx, GD_ERR_CUDA, "device index check failed at site " + std::to_string(h - kDevBoundsBase) +
                                       " (debug library)");
   return fail(ctx, GD_ERR_CUDA, "device error code " + std::to_string(h));
+}
+
+gd_status check_device_error(gd_context *ctx) {
+  int h = 0;
+  cudaError_t e = cudaMemcpy(&h, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost);
+  if (e != cudaSuccess) return cuda_fail(ctx, e, "reading the device error word");
+  return error_status(ctx, h);
+}
+
+gd_status finish_stream(gd_context *ctx, cudaStream_t stream, const char *what) {
+  cudaError_t e = cudaMemcpyAsync(ctx->h_err, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+  if (e != cudaSuccess) return cuda_fail(ctx, e, what);
+  return error_status(ctx, *ctx->h_err);
 }
 
 // Smallest double x with sqrt(x) >= c: then sqrt(d2) < c  <=>  d2 < x.
@@ -321,23 +333,24 @@ static std::vector<int> slot_order(const double *x, const double *y, const doubl
   return order;
 }
 
-// Receptor atoms grouped into spatially compact segments of kRecSeg (the FP32
-// kernel's ring stage): recursive bisection along the longest extent of the
-// bounding box, the left part always a whole number of segments, so every
-// segment but the last is full; inside a segment the bisection goes on down
-// to compact runs of 8 (one row-test round).  Deterministic (a stable sort
-// per level).  Returns order[k] = original index of the atom at position k.
-static std::vector<int> segment_order(const double *x, const double *y, const double *z, int n) {
+}  // namespace gd
+
+// Points grouped into spatially compact runs of `unit`: recursive bisection
+// along the longest extent of the bounding box, the left part always a whole
+// number of runs, so every run but the last is full; inside a run the bisection
+// goes on down to compact runs of `sub`.  Deterministic (a stable sort per
+// level).  Returns order[k] = original index of the point at position k.
+std::vector<int> gd::compact_runs(const double *x, const double *y, const double *z, int n, int unit, int sub) {
   std::vector<int> order(n);
   for (int i = 0; i < n; ++i) order[i] = i;
   struct Span { int lo, hi, unit; };
-  std::vector<Span> pending{{0, n, kRecSeg}};
+  std::vector<Span> pending{{0, n, unit}};
   while (!pending.empty()) {
     const Span sp = pending.back();
     pending.pop_back();
     const int m = sp.hi - sp.lo;
     if (m <= sp.unit) {
-      if (sp.unit > 8 && m > 8) pending.push_back({sp.lo, sp.hi, 8});
+      if (sp.unit > sub && m > sub) pending.push_back({sp.lo, sp.hi, sub});
       continue;
     }
     double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
@@ -357,8 +370,6 @@ static std::vector<int> segment_order(const double *x, const double *y, const do
   }
   return order;
 }
-
-}  // namespace gd
 
 // The centre starts at the centroid and moves toward the farthest point with
 // steps 1/(i + 1) (Badoiu and Clarkson's iteration for the minimum enclosing
@@ -467,6 +478,13 @@ gd_status gd_context_create(int32_t device, uint64_t hbm_budget_bytes, gd_contex
   }
   ctx->d_err = static_cast<int *>(p);
   cudaMemset(ctx->d_err, 0, sizeof(int));
+  if (cudaMallocHost(reinterpret_cast<void **>(&ctx->h_err), 256) != cudaSuccess) {
+    cudaFree(ctx->d_err);
+    cudaStreamDestroy(ctx->stream);
+    delete ctx;
+    return GD_ERR_OOM;
+  }
+  ctx->h_info = ctx->h_err + 16;
   *out = ctx;
   return GD_OK;
 }
@@ -479,6 +497,7 @@ gd_status gd_context_destroy(gd_context *ctx) {
   if (ctx->d_batch) cudaFree(ctx->d_batch);
   if (ctx->h_pinned) cudaFreeHost(ctx->h_pinned);
   if (ctx->d_err) cudaFree(ctx->d_err);
+  if (ctx->h_err) cudaFreeHost(ctx->h_err);
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);
   cudaStreamDestroy(ctx->stream);
@@ -629,7 +648,8 @@ gd_status gd_complex_create(gd_context *ctx, const gd_atoms *rec, const gd_atoms
   double ext = 0.0;
   // receptor in compact segments (sums are order-free; the burial tables
   // follow the same order)
-  const std::vector<int> rperm = segment_order(rec->x, rec->y, rec->z, rec->n);
+  // (segments of the FP32 kernel's ring stage, runs of one row-test round)
+  const std::vector<int> rperm = compact_runs(rec->x, rec->y, rec->z, rec->n, kRecSeg, 8);
   for (int k = 0; k < rec->n; ++k) {
     const int i = rperm[k];
     rp32[k] = make_float4(static_cast<float>(rec->x[i] - o[0]), static_cast<float>(rec->y[i] - o[1]),

@@ -136,6 +136,7 @@ struct gd_context {
   cudaStream_t stream = nullptr;
   int sm_count = 0;
   int *d_err = nullptr;
+  int *h_err = nullptr, *h_info = nullptr;  // pinned: the error word as last read; small results of a call
   std::string last_error;
   // grow-only scratch: device and pinned host staging
   void *d_scratch = nullptr;
@@ -150,10 +151,10 @@ struct gd_context {
   int tune_split = 0;      // GD_TUNE_SPLIT: 0 automatic, 1 whole poses, 2 always split
   int tune_fault = 0;      // GD_TUNE_FAULT: 1 = drop one stage copy (failure-detection tests)
   int tune_fcc = 0;        // GD_TUNE_FCC: 0 automatic, 1 bitsets, 2 contact postings
-  int tune_contacts = 0;   // GD_TUNE_CONTACTS: 0 automatic (bitmaps where possible), 1 per-residue lists
+  int tune_contacts = 0;   // GD_TUNE_CONTACTS: 0 automatic (k_contacts where possible), 1 k_contacts_rl
   int tune_rparts = 0;     // GD_TUNE_RPARTS: 0 automatic, 1..8 receptor parts per ligand chunk (split mode)
   int last_fcc = 0;        // GD_INFO_LAST_FCC: pair counts of the last device clustering (1 bitsets, 2 postings)
-  int last_contacts = 0;   // GD_INFO_LAST_CONTACTS: kernel of the last contact pass (1 lists, 2 bitmaps)
+  int last_contacts = 0;   // GD_INFO_LAST_CONTACTS: kernel of the last contact pass (1 k_contacts_rl, 2 k_contacts)
 };
 
 struct gd_complex {
@@ -215,6 +216,9 @@ gd_status dev_alloc(gd_context *ctx, uint64_t bytes, void **p);
 void dev_free(gd_context *ctx, void *p, uint64_t bytes);
 gd_status ensure_scratch(gd_context *ctx, size_t dev_bytes, size_t pinned_bytes);
 gd_status check_device_error(gd_context *ctx);
+// Wait for the stream and report its errors, the device error word (read on
+// the same stream, before the wait) included.
+gd_status finish_stream(gd_context *ctx, cudaStream_t stream, const char *what);
 Thresholds make_thresholds(double contact_cutoff);
 void make_frame(const double *g, gd_pose_frame *f);
 void guard_widths(const gd_complex *cx, double max_disp, float *gv, float *ge, float *gd);
@@ -227,6 +231,7 @@ void free_cluster_cache(gd_complex *cx);
 // returned centre, so every point is enclosed (gd_api.cu).
 void enclosing_ball(const double *x, const double *y, const double *z, const int *idx, int n, double c[3],
                     double &r);
+std::vector<int> compact_runs(const double *x, const double *y, const double *z, int n, int unit, int sub);
 gd_status ensure_batch_scratch(gd_context *ctx, size_t dev_bytes);
 ScoreParams make_params(gd_complex *cx, const gd_pose_frame *d_frames, const double *d_models, int n,
                         gd_pose_energy *d_out, double max_disp);

@@ -126,11 +126,11 @@ gd_status gd_context_destroy(gd_context *ctx);
  *                      when the contacts are spread over many poses, at most
  *                      16,384 poses).  Clusters are identical either way.
  *   GD_TUNE_CONTACTS:  contact pass of gd_pose_contacts: 0 = automatic (the
- *                      per-pose residue-pair bitmaps of the clustering path
- *                      whenever receptor and ligand are single chains that
- *                      share no residue, else per-residue contact lists),
- *                      1 = per-residue contact lists always.  Both decide
- *                      every atom pair exactly; the keys are identical.
+ *                      clustering path's, which decides in FP32 outside a
+ *                      guard band, whenever receptor and ligand are single
+ *                      chains that share no residue, else the one that decides
+ *                      every pair in FP64), 1 = the FP64 one always.  Both
+ *                      decide every atom pair exactly; the keys are identical.
  *   GD_TUNE_RPARTS:    receptor parts per ligand chunk of a split FP32
  *                      launch: 0 = automatic (more than one only when the
  *                      launch has too few (pose, chunk) items to fill the
@@ -140,7 +140,8 @@ gd_status gd_context_destroy(gd_context *ctx);
  *   GD_INFO_LAST_FCC:      pair counts of the context's last device
  *                          clustering: 1 bitsets, 2 postings, 0 none yet.
  *   GD_INFO_LAST_CONTACTS: contact pass of the last gd_pose_contacts or
- *                          gd_cluster: 1 lists, 2 bitmaps, 0 none yet. */
+ *                          gd_cluster: 1 the FP64 one, 2 the clustering
+ *                          path's, 0 none yet. */
 enum { GD_TUNE_F32_SLOTS = 0, GD_TUNE_SPLIT = 1, GD_TUNE_FAULT = 2, GD_TUNE_FCC = 3, GD_TUNE_CONTACTS = 4,
        GD_TUNE_RPARTS = 5,
        GD_INFO_LAST_FCC = 16, GD_INFO_LAST_CONTACTS = 17 };

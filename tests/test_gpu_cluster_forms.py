@@ -1,0 +1,67 @@
+"""Clustering where its kernels change form: pose counts around the FCC tiles
+and the greedy pass's one CTA or cluster of CTAs, ratios exactly at the
+cutoffs, residues of more atoms than a half warp, a warp or the staging takes,
+and poses with more contacts than their lists first have room for.  Contacts
+and clusters equal the oracle's exactly."""
+import numpy as np
+import pytest
+
+import gdock_gb300 as gd
+from conftest import make_mol, tatom
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [1, 16, 17, 33, 512, 513, 886, 887, 1024, 1025, 1300])
+@pytest.mark.parametrize("min_size", [1, 4])
+def test_pose_counts(oracle, n, min_size):
+    """Sets of 5 to 40 contacts around a few prototypes: many pairs at exactly
+    60 % and 45 % common contacts, large clusters and singletons."""
+    rng = np.random.default_rng(n)
+    protos = [rng.choice(300, 20, replace=False) for _ in range(5)]
+    sets = []
+    for k in range(n):
+        p = protos[k % 5]
+        common = p[: int(rng.choice([20, 15, 12, 9, 6]))] if k % 7 else rng.choice(300, int(rng.integers(0, 20)), replace=False)
+        sets.append(np.unique(np.concatenate([common, rng.integers(300, 400, int(rng.choice([0, 5, 8])))])).astype(np.int64))
+    cfg = gd.ClusteringConfig(min_cluster_size=min_size)
+    assert [(r.center_idx, r.members) for r in gd.cluster_sets(sets, cfg)] == oracle.cluster(sets, min_size=min_size)
+
+
+def residues(rng, sizes, chain, centre):
+    atoms = []
+    for k, m in enumerate(sizes):
+        at = centre + rng.normal(0.0, 5.0, 3)
+        atoms += [tatom(*(at + rng.normal(0.0, 1.5, 3)), "C", resseq=k + 1, serial=len(atoms) + 1, chain=chain)
+                  for _ in range(m)]
+    return make_mol(atoms)
+
+
+@pytest.mark.parametrize("rec,lig", [([16, 17, 1, 40, 8] * 7, [8, 16, 17, 33] * 4), ([5] * 40, [64, 64, 64, 3, 64]),
+                                     ([20] * 9, [65, 4, 4]), ([7], [9])])
+def test_large_residues(oracle, rec, lig):
+    rng = np.random.default_rng(len(rec))
+    R, L = residues(rng, rec, "A", np.zeros(3)), residues(rng, lig, "B", np.zeros(3))
+    genes = np.concatenate([rng.uniform(0, 6.28, (24, 3)), rng.normal(0, 7.0, (24, 3))], axis=1)
+    cx = gd.Complex(R, L, [])
+    sets = [oracle.pose_contacts(R, L, g) for g in genes]
+    for a, b in zip(cx.pose_contacts(genes), sets):
+        np.testing.assert_array_equal(a, b)
+    got = cx.cluster(genes, gd.ClusteringConfig(min_cluster_size=1))
+    assert [(r.center_idx, r.members) for r in got] == oracle.cluster(sets, min_size=1)
+
+
+def test_more_contacts_than_room(oracle):
+    """Every residue of one molecule against every one of the other: 6,400
+    contacts a pose."""
+    rng = np.random.default_rng(1)
+    R, L = residues(rng, [1] * 80, "A", np.zeros(3)), residues(rng, [1] * 80, "B", np.zeros(3))
+    R, L = (m.with_coords(m.x * 0.1, m.y * 0.1, m.z * 0.1) for m in (R, L))
+    genes = np.concatenate([rng.uniform(0, 6.28, (40, 3)), rng.normal(0, 0.5, (40, 3))], axis=1)
+    genes[30:, 3] += 4.0
+    cx = gd.Complex(R, L, [])
+    sets = [oracle.pose_contacts(R, L, g) for g in genes]
+    assert max(len(s) for s in sets) > 2048
+    for a, b in zip(cx.pose_contacts(genes), sets):
+        np.testing.assert_array_equal(a, b)
+    assert [(r.center_idx, r.members) for r in cx.cluster(genes)] == oracle.cluster(sets)
