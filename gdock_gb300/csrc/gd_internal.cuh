@@ -88,7 +88,6 @@ struct ScoreParams {
   const FixAtom *rec_fix;   // the same as integers
   int fix;                  // every coordinate of the launch lies within kFixMax
   const int2 *rec_meta;     // (type, serial)
-  const int4 *rec_meta16;   // (type, serial, 0, 0): the FP32 kernel's copy, as wide as a position
   const double *rec_desolv; // [nr * 11] energy contribution at burial count 0..10
   const float4 *rec_seg;    // per kRecSeg-atom segment: bounding sphere (centre - O, radius) FP32
   int nr, nseg;
@@ -173,7 +172,6 @@ struct gd_complex {
   gd::FixAtom *rec_fix = nullptr;
   double abs_max = 0;     // max |x| over receptor atoms and (ligand centroid + radius); inf when not finite
   int2 *rec_meta = nullptr;
-  int4 *rec_meta16 = nullptr;
   double *rec_desolv = nullptr;
   double *lig_x = nullptr, *lig_y = nullptr, *lig_z = nullptr, *lig_q = nullptr;
   int *lig_type = nullptr, *lig_serial = nullptr;

@@ -553,7 +553,6 @@ ScoreParams make_params(gd_complex *cx, const gd_pose_frame *d_frames, const dou
   p.rec_fix = cx->rec_fix;
   p.fix = cx->abs_max + max_disp <= kFixMax;
   p.rec_meta = cx->rec_meta;
-  p.rec_meta16 = cx->rec_meta16;
   p.rec_desolv = cx->rec_desolv;
   p.nr = cx->nr;
   p.lig_perm = cx->lig_perm;

@@ -7,11 +7,11 @@
 //
 // Per work item a warp
 //   1. copies the complex's descriptor and the pose frame to its shared memory;
-//   2. for each chunk of 32*S ligand atoms: transforms them exactly (FP64, the
-//      reference's operation order, src/structure.rs:80-131), keeps FP32
-//      copies in registers (S slots of 32 atoms, one per lane; the ligand is
-//      stored in spatially compact slot order) and a bounding sphere and box
-//      per slot;
+//   2. for each chunk of 32*S ligand atoms: moves them in FP64 (one
+//      multiply-add chain a coordinate; src/structure.rs:80-131), keeps FP32
+//      copies in shared memory (S slots of 32 atoms, one per lane; the ligand
+//      is stored in spatially compact slot order) and a bounding sphere and
+//      box per slot;
 //   3. streams the receptor through its own two-stage shared-memory ring,
 //      each stage filled by one bulk (TMA) copy of a 64-atom segment and
 //      guarded by a per-warp mbarrier with a bounded wait; the receptor is
@@ -24,12 +24,20 @@
 //      sphere or box is dropped (every pair of it contributes exactly
 //      nothing), one beyond the 12 A reach is a far row (Coulomb only); kept
 //      rows go to per-slot lists in shared memory;
-//   5. evaluates the kept rows four at a time (independent FP32 chains):
-//      soft-core LJ, Coulomb, burial counts and guard-band tests for near
-//      rows, Coulomb and its band for far rows;
+//   5. evaluates the kept rows four at a time (independent FP32 chains), the
+//      last one or two of a slot two at a time: soft-core LJ, Coulomb, burial
+//      counts and guard-band tests for near rows, Coulomb and its band for far
+//      rows.  The kernel issues on 85 % of its cycles and no other unit is
+//      near its limit, so instructions per row set its time: the slots' FP32
+//      atoms lie in shared memory behind one loop (not one unrolled copy a
+//      slot), and a list entry already holds the shared address of the row's
+//      position and its row of the pair table.  That took 150 poses of
+//      2,538 x 1,280 atoms from 419 to 376 us and 65,536 of them from 83.4
+//      to 81.4 ms;
 //   6. re-decides in FP64, once per segment, the pairs of flagged steps whose
 //      FP32 d2 lies within the guard band of a cutoff (1, 8, 12, 15 A), so
-//      all decisions equal the FP64 ones;
+//      all decisions equal the FP64 ones; a flagged step computes exact
+//      coordinates only for the pairs that lie in a band;
 //   7. reduces exactly: each segment's FP32 vdW and Coulomb partials become
 //      2^-32 fixed-point integers summed per lane (integer sums do not depend
 //      on their order, so neither do the energies on how segments, chunks and
@@ -43,6 +51,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "gd_device.cuh"
@@ -71,7 +80,6 @@ struct BatchParams {
   int gcount_stride;              // bytes per warp in gcounts
   int smem_cnt;                   // bytes per warp of shared-memory counters (0: use gcounts)
   int max_nr;                     // largest receptor of the batch
-  int warp_smem;                  // bytes of shared memory per warp
   int *err;
   // split mode: a work item is one ligand chunk of a pose; the chunk that
   // finishes a pose last reduces its per-chunk partials
@@ -90,32 +98,39 @@ struct BatchParams {
 };
 
 struct WarpSmem {
-  size_t pos, meta, list, fixq, cmask, cidx, lfix, bars, desc, frame, blob, box, rc, ssph, segl, cnt, total;
+  size_t pos, meta, list, fixq, cmask, cstep, lig, lt, lcnt, bars, desc, frame, blob, box, rc, ssph, segl, cnt, total;
 };
 
-__host__ __device__ inline WarpSmem warp_layout(int smem_cnt) {
+// atoms: rows per step of the kernel variant
+__host__ __device__ inline WarpSmem warp_layout(int smem_cnt, int atoms) {
   WarpSmem L;
   size_t o = 0;
   auto al = [&](size_t a) { o = (o + a - 1) / a * a; };
+  const size_t steps = kMaxS * (kList / atoms + 2);  // of a segment, at most
   L.pos = o;
   o += sizeof(float4) * (kWS * kSeg + 1);  // + the far dummy atom
   al(16);
-  L.meta = o;  // at a fixed distance from pos: one address serves both
-  o += sizeof(int4) * (kWS * kSeg + 1);
+  L.meta = o;
+  o += sizeof(int2) * (kWS * kSeg + 1);
   al(16);
-  L.list = o;
-  o += sizeof(uint16_t) * kMaxS * kList;
+  L.list = o;   // kept rows per slot: shared address of the position << 12 | type row
+  o += sizeof(uint32_t) * kMaxS * kList;
   al(16);
-  L.fixq = o;
-  o += sizeof(uint16_t) * kMaxS * kList;  // at most one entry per step of a segment
+  L.fixq = o;   // flagged steps
+  o += sizeof(uint16_t) * steps;
   al(16);
-  L.cmask = o;  // per near row of the segment: lanes with d2 < 64 (ballot)
+  L.cmask = o;  // per recorded near row of the segment: lanes with d2 < 64 (ballot)
   o += sizeof(unsigned) * kMaxS * kList;
   al(16);
-  L.cidx = o;   // ... and its receptor atom (stage index)
-  o += sizeof(uint16_t) * kMaxS * kList;
+  L.cstep = o;  // ... and per recorded step its place in the lists
+  o += sizeof(uint16_t) * steps;
   al(16);
-  L.lfix = o;
+  L.lig = o;    // the chunk's ligand atoms (x, y, z, charge), their types and burial counts
+  o += sizeof(float4) * kMaxS * 32;
+  L.lt = o;
+  o += sizeof(uint16_t) * kMaxS * 32;
+  al(16);
+  L.lcnt = o;
   o += sizeof(int) * kMaxS * 32;
   al(16);
   L.bars = o;
@@ -144,13 +159,13 @@ __host__ __device__ inline WarpSmem warp_layout(int smem_cnt) {
   return L;
 }
 
-__device__ __forceinline__ void issue_seg(long long q, int seg, const ScoreParams &p, float4 *s_pos, int4 *s_meta,
+__device__ __forceinline__ void issue_seg(long long q, int seg, const ScoreParams &p, float4 *s_pos, int2 *s_meta,
                                           uint64_t *s_bar) {
   const int st = static_cast<int>(q % kWS);
-  constexpr uint32_t kBytes = kSeg * (sizeof(float4) + sizeof(int4));
+  constexpr uint32_t kBytes = kSeg * (sizeof(float4) + sizeof(int2));
   mbar_expect_tx(&s_bar[st], kBytes);
   bulk_g2s(&s_pos[st * kSeg], p.rec_pos32 + static_cast<size_t>(seg) * kSeg, kSeg * sizeof(float4), &s_bar[st]);
-  bulk_g2s(&s_meta[st * kSeg], p.rec_meta16 + static_cast<size_t>(seg) * kSeg, kSeg * sizeof(int4), &s_bar[st]);
+  bulk_g2s(&s_meta[st * kSeg], p.rec_meta + static_cast<size_t>(seg) * kSeg, kSeg * sizeof(int2), &s_bar[st]);
 }
 
 // acc += v when t < 0 (one predicated add)
@@ -168,13 +183,6 @@ __device__ __forceinline__ void fma_if_abs_lt(float &acc, float t, float lim, fl
   asm("{\n\t.reg .pred p;\n\tsetp.lt.f32 p, %1, %2;\n\t@p fma.rn.f32 %0, %3, %4, %0;\n\t}" : "+f"(acc)
       : "f"(fabsf(t)), "f"(lim), "f"(a), "f"(b));
 }
-// a += 1 and b += 1 when d2 < 64
-__device__ __forceinline__ void count_if_lt64(int &a, int &b, float d2) {
-  asm("{\n\t.reg .pred p;\n\tsetp.lt.f32 p, %2, 0f42800000;\n\t@p add.s32 %0, %0, 1;\n\t@p add.s32 %1, %1, 1;\n\t}"
-      : "+r"(a), "+r"(b)
-      : "f"(d2));
-}
-
 // soft-core LJ in FP32 (src/fitness.rs:57-70): eps*(q^2 - 2q) with
 // q = R6/(r^6 + R6/2), evaluated as 4 eps x (x - 1) = 4 eps (x^2 - x),
 // x = q/2 = 1/(r^6 2/R6 + 1); at d2 = 0 it is exactly 0
@@ -194,15 +202,12 @@ __device__ __forceinline__ float vdw_term(float d2, float2 tp) {
 // doubles) and whose FP32 term is exactly 0, so the sums are unchanged; the
 // guard band of the vdW cutoff is the one at 144.
 template <bool SERIAL, bool CLAMP>
-__device__ __forceinline__ void pair32(const float4 &r, int rtrow, int rser, const float2 *tab, float lx, float ly,
-                                       float lz, int lt, int lser, float gv, float ge, float gdd, float &av,
-                                       float &ae, int &lc, int &rc, bool &amb) {
-  const float d2 = d2f(r, lx, ly, lz);
-  const float2 tp = __ldg(&tab[rtrow + lt]);
+__device__ __forceinline__ void pair32(float d2, float qr, const float2 tp, bool same, float gv, float ge, float gdd,
+                                       float &av, float &ae, bool &amb) {
   const float tv = __fsub_rn(d2, 144.0f);  // d2 < 144  <=>  tv < 0
   if (SERIAL || CLAMP) {
     const float v = vdw_term<CLAMP>(d2, tp);
-    if (SERIAL) av += (tv < 0.0f && rser != lser) ? v : 0.0f;
+    if (SERIAL) av += (tv < 0.0f && !same) ? v : 0.0f;
     else add_if_lt0(av, tv, v);
   } else {
     // the well depth multiplies into the sum: one FMA (vdw_term without the
@@ -211,21 +216,8 @@ __device__ __forceinline__ void pair32(const float4 &r, int rtrow, int rser, con
     fma_if_lt0(av, tv, __fmaf_rn(x, x, -x), tp.y);
   }
   const float te = __fsub_rn(d2, 113.0f);  // 1 < d2 < 225  <=>  |te| < 112
-  fma_if_abs_lt(ae, te, 112.0f, r.w, rcp_approx(d2));
-  count_if_lt64(lc, rc, d2);
+  fma_if_abs_lt(ae, te, 112.0f, qr, rcp_approx(d2));
   amb = amb | (fabsf(__fsub_rn(fabsf(te), 112.0f)) < ge) | (fabsf(tv) < gv) | (fabsf(__fsub_rn(d2, 64.0f)) < gdd);
-}
-
-// One pair of a far row (no pair within the vdW cutoff): Coulomb only, the
-// same FP32 expressions and decision as pair32().  Every FP32 d2 of a far
-// row exceeds 144, where d2 - 113 and d2 - 225 are exact (Sterbenz) and
-// |d2 - 113| < 112 is d2 < 225: one bound, one band.
-__device__ __forceinline__ void pair32_elec(const float4 &r, float lx, float ly, float lz, float ge, float &ae,
-                                            bool &amb) {
-  const float d2 = d2f(r, lx, ly, lz);
-  const float tf = __fsub_rn(d2, 225.0f);
-  fma_if_lt0(ae, tf, r.w, rcp_approx(d2));
-  amb = amb | (fabsf(tf) < ge);
 }
 
 __device__ __forceinline__ bool near_band(float d2, float gv, float ge, float gdd) {
@@ -343,15 +335,17 @@ template <int S, int kAtoms, int MINB, bool SERIAL, bool CLAMP, int SPLIT>
 __global__ void __launch_bounds__(kWarps * 32, MINB) k_score_f32w(const BatchParams bp) {
   extern __shared__ __align__(128) unsigned char smem[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const WarpSmem L = warp_layout(bp.smem_cnt);
+  const WarpSmem L = warp_layout(bp.smem_cnt, kAtoms);
   unsigned char *base = smem + static_cast<size_t>(wib) * L.total;
   float4 *s_pos = reinterpret_cast<float4 *>(base + L.pos);
-  int4 *s_meta = reinterpret_cast<int4 *>(base + L.meta);
-  uint16_t *s_list = reinterpret_cast<uint16_t *>(base + L.list);  // kept rows per slot, as stage indices
-  uint16_t *s_fixq = reinterpret_cast<uint16_t *>(base + L.fixq);  // flagged steps: list position | slot << 8
-  unsigned *s_cmask = reinterpret_cast<unsigned *>(base + L.cmask);  // near rows' burial ballots (this segment)
-  uint16_t *s_cidx = reinterpret_cast<uint16_t *>(base + L.cidx);
-  int *s_lfix = reinterpret_cast<int *>(base + L.lfix);            // ligand burial corrections per slot and lane
+  int2 *s_meta = reinterpret_cast<int2 *>(base + L.meta);
+  uint32_t *s_list = reinterpret_cast<uint32_t *>(base + L.list);
+  uint16_t *s_fixq = reinterpret_cast<uint16_t *>(base + L.fixq);    // steps: list position | slot << 8 | rows << 12
+  unsigned *s_cmask = reinterpret_cast<unsigned *>(base + L.cmask);
+  uint16_t *s_cstep = reinterpret_cast<uint16_t *>(base + L.cstep);
+  float4 *s_lig = reinterpret_cast<float4 *>(base + L.lig);
+  uint16_t *s_lt = reinterpret_cast<uint16_t *>(base + L.lt);
+  int *s_lcnt = reinterpret_cast<int *>(base + L.lcnt);
   uint64_t *s_bar = reinterpret_cast<uint64_t *>(base + L.bars);
   ScoreParams *s_desc = reinterpret_cast<ScoreParams *>(base + L.desc);
   gd_pose_frame *s_frame = reinterpret_cast<gd_pose_frame *>(base + L.frame);
@@ -360,6 +354,10 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_score_f32w(const BatchPar
   int *s_rc = reinterpret_cast<int *>(base + L.rc);  // receptor burial counts of the current segment
   float4 *s_ssph = reinterpret_cast<float4 *>(base + L.ssph);
   uint16_t *s_segl = reinterpret_cast<uint16_t *>(base + L.segl);
+  // a list entry's parts (shared addresses fit 18 bits, type rows 12)
+  const uint32_t pos_at = smem_u32(s_pos), far_row = (pos_at + kFar * 16) << 12;
+  auto entry_atom = [&](uint32_t e) { return static_cast<int>(((e >> 12) - pos_at) >> 4); };
+  static_assert(kMaxTypes * kMaxTypes <= 4096, "a type row in 12 bits");
   const int gwarp = static_cast<int>(blockIdx.x) * kWarps + wib;
   uint8_t *cnt = bp.smem_cnt ? reinterpret_cast<uint8_t *>(base + L.cnt)
                              : bp.gcounts + static_cast<size_t>(gwarp) * bp.gcount_stride;
@@ -368,12 +366,11 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_score_f32w(const BatchPar
     for (int s = 0; s < kWS; ++s) mbar_init(&s_bar[s], 1);
     fence_mbar_init();
     s_pos[kFar] = make_float4(1.0e9f, 1.0e9f, 1.0e9f, 0.0f);  // far from real and idle ligand lanes
-    s_meta[kFar] = make_int4(0, 0, 0, 0);
+    s_meta[kFar] = make_int2(0, 0);
   }
   if (!SPLIT)
     for (int i = lane; i < bp.max_nr; i += 32) cnt[i] = 0;
   for (int i = lane; i < kSeg; i += 32) s_rc[i] = 0;
-  for (int i = lane; i < kMaxS * 32; i += 32) s_lfix[i] = 0;
   __syncwarp();
 
   static_assert(S >= 1 && S <= kMaxS, "one row-test round covers at most four slots");
@@ -484,9 +481,8 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_score_f32w(const BatchPar
       }
       auto seg_at = [&](int k) { return listed ? static_cast<int>(s_segl[k]) : rpart + k * R; };
       long long fv = 0, fe = 0;  // this item's vdW and Coulomb sums, 2^-32 fixed point
-      int lcnt[S];
 #pragma unroll
-      for (int s = 0; s < S; ++s) lcnt[s] = 0;
+      for (int s = 0; s < S; ++s) s_lcnt[s * 32 + lane] = 0;
       // an item without a segment in reach (the usual one of a pose apart from
       // the receptor, and of a receptor part) ends here
       if (nk > 0) {
@@ -495,35 +491,28 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_score_f32w(const BatchPar
             if (!(bp.drop_copy && item == 0 && ch == ch0 && k == 0))
               issue_seg(q + k, seg_at(k), p, s_pos, s_meta, s_bar);
         q_issued = q + min(nk, kWS);
-        float lx[S], ly[S], lz[S], lq[S];
-        int lt[S], lser[S];
 #pragma unroll
         for (int s = 0; s < S; ++s) {
           const int j = ch * kChunk + s * 32 + lane;
           const bool on = j < p.nl;
+          // (idle lanes: far from every receptor atom, including the padding at +1e9)
+          float4 l = make_float4(-1.0e9f, -1.0e9f, -1.0e9f, 0.0f);
+          int lt = 0;
           if (on) {
             const float3 c = atom32(p, f, pose, j);
-            lx[s] = c.x;
-            ly[s] = c.y;
-            lz[s] = c.z;
-            lq[s] = static_cast<float>(p.lig_rel[j].w);
-            lt[s] = p.lig_type[j];
-            if (!GD_DCHECK(bp.err, lt[s] >= 0 && lt[s] < p.nt, 6)) lt[s] = 0;
-            lser[s] = SERIAL ? p.lig_serial[j] : 0;
-          } else {
-            // far from every receptor atom, including the padding at +1e9
-            lx[s] = ly[s] = lz[s] = -1.0e9f;
-            lq[s] = 0.0f;
-            lt[s] = 0;
-            lser[s] = 0;
+            l = make_float4(c.x, c.y, c.z, static_cast<float>(p.lig_rel[j].w));
+            lt = p.lig_type[j];
+            if (!GD_DCHECK(bp.err, lt >= 0 && lt < p.nt, 6)) lt = 0;
           }
+          s_lig[s * 32 + lane] = l;
+          s_lt[s * 32 + lane] = static_cast<uint16_t>(lt);
           // bounding sphere of the slot's 32 atoms: with a rigid pose the
           // precomputed small enclosing sphere moved with it (s_ssph, smaller
           // than the centroid's sphere), else the centroid's of these atoms
           const unsigned on_mask = __ballot_sync(kFull, on);
           float cx = 0.0f, cy = 0.0f, cz = 0.0f, rr = 0.0f;
           if (!cull) {
-            cx = on ? lx[s] : 0.f, cy = on ? ly[s] : 0.f, cz = on ? lz[s] : 0.f;
+            cx = on ? l.x : 0.f, cy = on ? l.y : 0.f, cz = on ? l.z : 0.f;
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
               cx += __shfl_xor_sync(kFull, cx, o);
@@ -534,16 +523,16 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_score_f32w(const BatchPar
             cx *= inv;
             cy *= inv;
             cz *= inv;
-            rr = on ? sqrtf((lx[s] - cx) * (lx[s] - cx) + (ly[s] - cy) * (ly[s] - cy) + (lz[s] - cz) * (lz[s] - cz))
+            rr = on ? sqrtf((l.x - cx) * (l.x - cx) + (l.y - cy) * (l.y - cy) + (l.z - cz) * (l.z - cz))
                     : 0.0f;
             rr = warp_max(rr);
           }
           // axis-aligned bounding box of the same atoms (half-widths widened
           // like the radius so that FP32 rounding never shrinks it)
-          const float lo_x = warp_min(on ? lx[s] : 3.0e38f), lo_y = warp_min(on ? ly[s] : 3.0e38f),
-                      lo_z = warp_min(on ? lz[s] : 3.0e38f);
-          const float hi_x = warp_max(on ? lx[s] : -3.0e38f), hi_y = warp_max(on ? ly[s] : -3.0e38f),
-                      hi_z = warp_max(on ? lz[s] : -3.0e38f);
+          const float lo_x = warp_min(on ? l.x : 3.0e38f), lo_y = warp_min(on ? l.y : 3.0e38f),
+                      lo_z = warp_min(on ? l.z : 3.0e38f);
+          const float hi_x = warp_max(on ? l.x : -3.0e38f), hi_y = warp_max(on ? l.y : -3.0e38f),
+                      hi_z = warp_max(on ? l.z : -3.0e38f);
           if (lane == 0) {
             s_blob[s] = !on_mask ? make_float4(0.0f, 0.0f, 0.0f, -1.0e30f)
                                  : (cull ? s_ssph[s] : make_float4(cx, cy, cz, rr * 1.0001f + 0.01f));
@@ -564,7 +553,8 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_score_f32w(const BatchPar
         const float mlim = myb.w + reach;
         const float mlim2 = (myb.w >= 0.0f) ? mlim * mlim : -1.0f;  // empty slot: no row kept
         const float mnear = myb.w + reach_v, mnear2 = mnear * mnear;
-        // per segment: flagged steps (high 16 bits) and recorded near rows (low 16)
+        const float4 bx0 = s_box[2 * (my_s & (kMaxS - 1))], bx1 = s_box[2 * (my_s & (kMaxS - 1)) + 1];
+        // per segment: flagged steps (high 16 bits) and recorded ones (low 16)
         int seg_cnt = 0;
         for (int kk = 0; kk < nk; ++kk, ++q) {
           const int g = seg_at(kk);
@@ -583,7 +573,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_score_f32w(const BatchPar
           // front, near rows from the back; each run is padded with the far
           // dummy atom to whole steps.
           int nf_mine = 0, nn_mine = 0;  // far / near rows of this lane's slot
-          uint16_t *my_list = s_list + my_s * kList;
+          uint32_t *my_list = s_list + my_s * kList;
           for (int b0 = 0; b0 < na; b0 += kBlk) {
             const float4 ra = s_pos[sbase + b0 + my_a];  // atoms past nr are padding far away
             const float dx = ra.x - myb.x, dy = ra.y - myb.y, dz = ra.z - myb.z;
@@ -591,13 +581,13 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_score_f32w(const BatchPar
             // distance from the atom to the slot's box: a second lower bound on
             // every pair distance of the row (either bound may drop the row or
             // make it far)
-            const float4 bx0 = s_box[2 * (my_s & (kMaxS - 1))], bx1 = s_box[2 * (my_s & (kMaxS - 1)) + 1];
             const float ex = fmaxf(fabsf(ra.x - bx0.x) - bx0.w, 0.0f), ey = fmaxf(fabsf(ra.y - bx0.y) - bx1.x, 0.0f),
                         ez = fmaxf(fabsf(ra.z - bx0.z) - bx1.y, 0.0f);
             const float db2 = ex * ex + ey * ey + ez * ez;
             const bool keep = dc2 < mlim2 && db2 < reach2, nearr = dc2 < mnear2 && db2 < reach_v2;
             const unsigned Mf = __ballot_sync(kFull, keep && !nearr), Mn = __ballot_sync(kFull, keep && nearr);
-            const uint16_t idx = static_cast<uint16_t>(sbase + b0 + my_a);
+            const int at = sbase + b0 + my_a;
+            const uint32_t idx = (pos_at + static_cast<uint32_t>(at) * 16) << 12 | static_cast<uint32_t>(s_meta[at].x);
             // at most na <= kSeg rows per slot: far rows fill [0, nf), near rows
             // (kList - nn, kList - 1], with room for both paddings in between
             const int pf = nf_mine + __popc(Mf & my_group & lt_mask), pn = kList - 1 - nn_mine - __popc(Mn & my_group & lt_mask);
@@ -609,120 +599,157 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_score_f32w(const BatchPar
           }
           if (my_s < S && my_a < kAtoms &&
               GD_DCHECK(bp.err, nf_mine + my_a < kList && kList - 1 - nn_mine - my_a >= 0, 3)) {
-            my_list[nf_mine + my_a] = static_cast<uint16_t>(kFar);
-            my_list[kList - 1 - nn_mine - my_a] = static_cast<uint16_t>(kFar);
+            my_list[nf_mine + my_a] = far_row;
+            my_list[kList - 1 - nn_mine - my_a] = far_row;
           }
           __syncwarp();
 
-          // Phase 2: every term of the kept rows, kAtoms rows per step
+          // Phase 2: every term of the kept rows, kAtoms rows per step (two in
+          // the last one where two are left: a run of 13 rows wastes one, not
+          // three)
           float av = 0.0f, ae = 0.0f;  // ae: corrections from FP64 re-decisions (charge included)
-#pragma unroll
+#pragma unroll 1
           for (int s = 0; s < S; ++s) {
-            float aes = 0.0f;  // sum of q_r / d2 over this slot's kept pairs
             const int nf = __shfl_sync(kFull, nf_mine, s * 8), nn = __shfl_sync(kFull, nn_mine, s * 8);
-            const uint16_t *lst = s_list + s * kList;
-            // far rows: Coulomb only
-#pragma unroll 1
-            for (int k0 = 0; k0 < nf; k0 += kAtoms) {
-              int ix[kAtoms];
-              float4 r[kAtoms];
-#pragma unroll
-              for (int i = 0; i < kAtoms; ++i) {
-                ix[i] = lst[k0 + i];
-                if (!GD_DCHECK(bp.err, ix[i] <= kFar, 4)) ix[i] = kFar;
-                r[i] = s_pos[ix[i]];
+            const uint32_t *lst = s_list + s * kList;
+            const float4 l = s_lig[s * 32 + lane];
+            const float2 *tabl = tab + s_lt[s * 32 + lane];
+            const int lser = SERIAL && ch * kChunk + s * 32 + lane < p.nl ? p.lig_serial[ch * kChunk + s * 32 + lane] : 0;
+            float aes = 0.0f;  // sum of q_r / d2 over this slot's kept pairs
+            int lc = 0;        // the lane's pairs within 8 A
+            auto row = [&](uint32_t e) {
+              if (!GD_DCHECK(bp.err, entry_atom(e) >= 0 && entry_atom(e) <= kFar, 4)) e = far_row;
+              float4 r;
+              asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                           : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w)
+                           : "r"(e >> 12));
+              return r;
+            };
+            // N consecutive entries in one load (N = 4: k0 is a multiple of 4, N = 2: even)
+            auto entries = [&](int k0, uint32_t *e, auto count) {
+              constexpr int N = decltype(count)::value;
+              if constexpr (N == 4) {
+                const uint4 v = *reinterpret_cast<const uint4 *>(lst + k0);
+                e[0] = v.x;
+                e[1] = v.y;
+                e[2] = v.z;
+                e[3] = v.w;
+              } else if constexpr (N == 2) {
+                const uint2 v = *reinterpret_cast<const uint2 *>(lst + k0);
+                e[0] = v.x;
+                e[1] = v.y;
+              } else {
+                e[0] = lst[k0];
               }
+            };
+            auto flag = [&](bool amb, int k0, int rows) {
+              if (!__any_sync(kFull, amb)) return;
+              if (lane == 0 && GD_DCHECK(bp.err, (seg_cnt >> 16) < kMaxS * (kList / kAtoms + 2), 7))
+                s_fixq[seg_cnt >> 16] = static_cast<uint16_t>(k0 | s << 8 | rows << 12);
+              seg_cnt += 1 << 16;
+            };
+            // far rows: Coulomb only.  Every FP32 d2 of a far row exceeds 144,
+            // where d2 - 225 is exact (Sterbenz) and d2 < 225 is the whole
+            // decision: one bound, one band.
+            auto far_step = [&](int k0, auto count) {
+              constexpr int N = decltype(count)::value;
+              uint32_t e[N];
+              entries(k0, e, count);
               bool amb = false;
 #pragma unroll
-              for (int i = 0; i < kAtoms; ++i) pair32_elec(r[i], lx[s], ly[s], lz[s], ge, aes, amb);
-              if (__any_sync(kFull, amb)) {  // at most one entry per step: <= 4 * 18 per segment
-                if (lane == 0 && GD_DCHECK(bp.err, (seg_cnt >> 16) < kMaxS * kList, 7))
-                  s_fixq[seg_cnt >> 16] = static_cast<uint16_t>(k0 | (s << 8));
-                seg_cnt += 1 << 16;
+              for (int i = 0; i < N; ++i) {
+                const float4 r = row(e[i]);
+                const float d2 = d2f(r, l.x, l.y, l.z), tf = __fsub_rn(d2, 225.0f);
+                fma_if_lt0(aes, tf, r.w, rcp_approx(d2));
+                amb = amb | (fabsf(tf) < ge);
               }
-            }
-            // near rows: every term; the first step may start in the padding
-#pragma unroll 1
-            for (int k0 = kList - (nn + kAtoms - 1) / kAtoms * kAtoms; k0 < kList; k0 += kAtoms) {
-              int ix[kAtoms];
-              float4 r[kAtoms];
-              int rt[kAtoms], rs[kAtoms], rc[kAtoms];
+              flag(amb, k0, N);
+            };
+            // near rows: every term
+            auto near_step = [&](int k0, auto count) {
+              constexpr int N = decltype(count)::value;
+              uint32_t e[N];
+              entries(k0, e, count);
+              bool amb = false, in[N], any_in = false;
 #pragma unroll
-              for (int i = 0; i < kAtoms; ++i) {
-                ix[i] = lst[k0 + i];
-                if (!GD_DCHECK(bp.err, ix[i] <= kFar, 4)) ix[i] = kFar;
-                r[i] = s_pos[ix[i]];
-                const int4 mt = s_meta[ix[i]];
-                rt[i] = mt.x;
-                if (!GD_DCHECK(bp.err, rt[i] >= 0 && rt[i] + lt[s] < p.nt * p.nt, 5)) rt[i] = 0;
-                rs[i] = mt.y;
-                rc[i] = 0;
+              for (int i = 0; i < N; ++i) {
+                const float4 r = row(e[i]);
+                uint32_t rt = e[i] & 0xfffu;
+                if (!GD_DCHECK(bp.err, static_cast<int>(rt) + s_lt[s * 32 + lane] < p.nt * p.nt, 5)) rt = 0;
+                const float2 tp = __ldg(tabl + rt);
+                const float d2 = d2f(r, l.x, l.y, l.z);
+                const bool same = SERIAL && s_meta[entry_atom(e[i])].y == lser;
+                pair32<SERIAL, CLAMP>(d2, r.w, tp, same, gv, ge, gdd, av, aes, amb);
+                in[i] = d2 < 64.0f;
+                any_in = any_in || in[i];
               }
-              bool amb = false;
+              flag(amb, k0, N);
+              // burial: a step with no pair within 8 A (about half of them)
+              // has nothing to count; else the rows' ballots are recorded here
+              // and added up once per segment (below)
+              if (__any_sync(kFull, any_in)) {
+                const int at = (seg_cnt & 0xffff) * kAtoms;
 #pragma unroll
-              for (int i = 0; i < kAtoms; ++i)
-                pair32<SERIAL, CLAMP>(r[i], rt[i], rs[i], tab, lx[s], ly[s], lz[s], lt[s], lser[s], gv, ge, gdd, av,
-                                      aes, lcnt[s], rc[i], amb);
-              if (__any_sync(kFull, amb)) {  // at most one entry per step: <= 4 * 18 per segment
-                if (lane == 0 && GD_DCHECK(bp.err, (seg_cnt >> 16) < kMaxS * kList, 7))
-                  s_fixq[seg_cnt >> 16] = static_cast<uint16_t>(k0 | (s << 8));
-                seg_cnt += 1 << 16;
-              }
-              // receptor burial counts of the step's rows: their ballots are
-              // recorded here and added up once per segment (below); a step
-              // with no pair within 8 A (about half of them) records nothing
-              int any_rc = 0;
-#pragma unroll
-              for (int i = 0; i < kAtoms; ++i) any_rc |= rc[i];
-              if (__any_sync(kFull, any_rc != 0)) {
-#pragma unroll
-                for (int i = 0; i < kAtoms; ++i) {
-                  const unsigned bm = __ballot_sync(kFull, rc[i] != 0);
-                  if (lane == i && GD_DCHECK(bp.err, (seg_cnt & 0xffff) + i < kMaxS * kList, 8)) {
-                    s_cmask[(seg_cnt & 0xffff) + i] = bm;
-                    s_cidx[(seg_cnt & 0xffff) + i] = static_cast<uint16_t>(ix[i]);
-                  }
+                for (int i = 0; i < N; ++i) {
+                  const unsigned bm = __ballot_sync(kFull, in[i]);
+                  lc += in[i];
+                  if (lane == i && GD_DCHECK(bp.err, at + i < kMaxS * kList, 8)) s_cmask[at + i] = bm;
                 }
-                seg_cnt += kAtoms;
+                if (lane == 0) s_cstep[seg_cnt & 0xffff] = static_cast<uint16_t>(k0 | s << 8 | N << 12);
+                ++seg_cnt;
               }
+            };
+            using Step = std::integral_constant<int, kAtoms>;
+            using Two = std::integral_constant<int, 2>;
+            int k0 = 0;
+#pragma unroll 1
+            for (; nf - k0 > (kAtoms == 4 ? 2 : 0); k0 += kAtoms) far_step(k0, Step());
+            if (kAtoms == 4 && k0 < nf) far_step(k0, Two());
+            // the first near step starts in the padding
+            k0 = kList - (nn + kAtoms - 1) / kAtoms * kAtoms;
+            if (kAtoms == 4 && ((nn - 1) & 2) == 0 && nn > 0) {  // one or two rows over
+              near_step(k0 + 2, Two());
+              k0 += 4;
             }
-            ae = __fmaf_rn(aes, lq[s], ae);
+#pragma unroll 1
+            for (; k0 < kList; k0 += kAtoms) near_step(k0, Step());
+            ae = __fmaf_rn(aes, l.w, ae);
+            if (lc) s_lcnt[s * 32 + lane] += lc;
           }
           __syncwarp();
           // FP64 re-decisions of the flagged steps' pairs in the guard band
-          const int nfix = seg_cnt >> 16, ncm = seg_cnt & 0xffff;
+          const int nfix = seg_cnt >> 16, ncs = seg_cnt & 0xffff;
 #pragma unroll 1
           for (int t = 0; t < nfix; ++t) {
-            const int e = s_fixq[t], k0 = e & 255, s = e >> 8;
+            const int e = s_fixq[t], k0 = e & 255, s = (e >> 8) & 15, rows = e >> 12;
             const int j = ch * kChunk + s * 32 + lane;
             if (j >= p.nl) continue;
-            double X, Y, Z;
-            ligand_atom(p, f, pose, j, X, Y, Z);
-            // the lane's FP32 coordinates, as in the chunk set-up
-            const float3 c32 = atom32(p, f, pose, j);
-            const float fx = c32.x, fy = c32.y, fz = c32.z, fq = static_cast<float>(p.lig_rel[j].w);
-            const int ft = p.lig_type[j], fs = SERIAL ? p.lig_serial[j] : 0;
+            const float4 l = s_lig[s * 32 + lane];
 #pragma unroll 1
-            for (int i = 0; i < kAtoms; ++i) {
-              const int ixi = s_list[s * kList + k0 + i];
-              if (ixi == kFar || !GD_DCHECK(bp.err, ixi < kFar, 4)) continue;
+            for (int i = 0; i < rows; ++i) {
+              const int ixi = entry_atom(s_list[s * kList + k0 + i]);
+              if (ixi == kFar || !GD_DCHECK(bp.err, ixi >= 0 && ixi < kFar, 4)) continue;
               const float4 ri = s_pos[ixi];
-              if (!near_band(d2f(ri, fx, fy, fz), gv, ge, gdd)) continue;
-              const int4 mt = s_meta[ixi];
-              const FixOut fo = fix_pair<SERIAL, CLAMP>(p, X, Y, Z, ri, gbase + ixi - sbase, mt.x, mt.y, fx, fy, fz, fq,
-                                                        ft, fs);
+              if (!near_band(d2f(ri, l.x, l.y, l.z), gv, ge, gdd)) continue;
+              double X, Y, Z;
+              ligand_atom(p, f, pose, j, X, Y, Z);
+              const int2 mt = s_meta[ixi];
+              const FixOut fo = fix_pair<SERIAL, CLAMP>(p, X, Y, Z, ri, gbase + ixi - sbase, mt.x, mt.y, l.x, l.y, l.z, l.w,
+                                                        s_lt[s * 32 + lane], SERIAL ? p.lig_serial[j] : 0);
               av += fo.dv;
               ae += fo.de;
               if (fo.dl) {
-                s_lfix[s * 32 + lane] += fo.dl;
+                s_lcnt[s * 32 + lane] += fo.dl;
                 atomicAdd(&s_rc[ixi - sbase], fo.dl);
               }
             }
           }
           // receptor burial counts of the near rows (the far atom's ballots are 0)
-          for (int t = lane; t < ncm; t += 32) {
-            const unsigned bm = s_cmask[t];
-            if (bm) atomicAdd(&s_rc[s_cidx[t] - sbase], __popc(bm));
+          for (int t = lane; t < ncs * kAtoms; t += 32) {
+            const int e = s_cstep[t / kAtoms], i = t % kAtoms;
+            const unsigned bm = i < (e >> 12) ? s_cmask[t] : 0u;
+            if (bm)
+              atomicAdd(&s_rc[entry_atom(s_list[((e >> 8) & 15) * kList + (e & 255) + i]) - sbase], __popc(bm));
           }
           seg_cnt = 0;
           fv += fx_energy(av, bp.err);
@@ -760,13 +787,11 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_score_f32w(const BatchPar
       double dch = 0.0;
 #pragma unroll
       for (int s = 0; s < S; ++s) {
-        lcnt[s] += s_lfix[s * 32 + lane];  // burial corrections of FP64 re-decisions
-        s_lfix[s * 32 + lane] = 0;
-        const int j = ch * kChunk + s * 32 + lane;
+        const int lcnt = s_lcnt[s * 32 + lane], j = ch * kChunk + s * 32 + lane;
         if (R == 1) {
-          if (j < p.nl) dch += p.lig_desolv[static_cast<size_t>(j) * 11 + min(lcnt[s], 10)];
-        } else if (j < p.nl && lcnt[s] != 0 && GD_DCHECK(bp.err, j < bp.max_nl, 11)) {
-          atomicAdd(&bp.lcount[static_cast<size_t>(gp) * bp.max_nl + j], static_cast<unsigned>(lcnt[s]));
+          if (j < p.nl) dch += p.lig_desolv[static_cast<size_t>(j) * 11 + min(lcnt, 10)];
+        } else if (j < p.nl && lcnt != 0 && GD_DCHECK(bp.err, j < bp.max_nl, 11)) {
+          atomicAdd(&bp.lcount[static_cast<size_t>(gp) * bp.max_nl + j], static_cast<unsigned>(lcnt));
         }
       }
       if (SPLIT) {
@@ -893,6 +918,13 @@ cudaError_t with_variant(int tune, bool serial, bool clamp, F f) {
   }
 }
 
+// Rows per step of a variant.
+int variant_atoms(int tune, bool serial, bool clamp) {
+  if (tune == kSplitTune || tune == kSplitPartsTune) return 4;
+  if (serial || clamp || tune == 4) return 1;
+  return tune == 16 + 4 ? 2 : 4;
+}
+
 // The dynamic shared memory of a CTA can exceed the 48 KB default (receptors
 // near kCntSmemMax keep their burial counters there): the kernel's limit is
 // raised before the occupancy query, which otherwise reports an invalid
@@ -974,7 +1006,7 @@ static gd_status plan_batch(gd_context *ctx, const std::vector<ScoreParams> &des
   pl->tune = slots;
   auto fit = [&](int smem_cnt, int *per_sm) -> cudaError_t {
     pl->smem_cnt = smem_cnt;
-    pl->smem = warp_layout(smem_cnt).total * kWarps;
+    pl->smem = warp_layout(smem_cnt, variant_atoms(pl->tune, serial, clamp)).total * kWarps;
     cudaError_t e = occupancy_var(pl->tune, serial, clamp, pl->smem, per_sm);
     if (e == cudaSuccess && *per_sm < 1) e = cudaErrorInvalidConfiguration;
     return e;
@@ -1117,7 +1149,6 @@ static gd_status launch_args(gd_context *ctx, int ncx, const BatchPlan &pl, cons
   bp.gcount_stride = static_cast<int>(gs);
   bp.smem_cnt = pl.smem_cnt;
   bp.max_nr = pl.max_nr;
-  bp.warp_smem = static_cast<int>(warp_layout(pl.smem_cnt).total);
   bp.err = ctx->d_err;
   bp.split = pl.split;
   bp.drop_copy = ctx->tune_fault == 1;
