@@ -972,7 +972,7 @@ struct BatchPlan {
 };
 
 constexpr size_t kSplitScratchMax = size_t(4) << 30;  // split scratch beyond this: whole poses
-constexpr int kMaxRparts = 8;  // receptor parts per chunk, at most (GD_TUNE_RPARTS accepts 1..8)
+constexpr int kMaxRparts = 24;  // receptor parts per chunk, at most (GD_TUNE_RPARTS accepts 1..8)
 
 static size_t al256(size_t b) { return (b + 255) / 256 * 256; }
 
@@ -1014,14 +1014,19 @@ static gd_status plan_batch(gd_context *ctx, const std::vector<ScoreParams> &des
   int per_sm = 0;
   cudaError_t e = fit(pl->max_nr <= kCntSmemMax ? ((pl->max_nr + 15) / 16) * 16 : 0, &per_sm);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "batched scoring occupancy");
-  // receptor parts: a launch with fewer (pose, chunk) items than about two
-  // rounds of the split kernel's resident warps splits each chunk's receptor
-  // into R interleaved segment sets, so that the SMs fill, keeping at least
-  // two segments per part.  A part's item also pays the chunk's set-up, so
-  // for receptors of fewer than 16 segments the target shrinks in
-  // proportion (measured on receptors of 6, 40 and 107 segments at 150 to
-  // 1,200 poses).  GD_TUNE_RPARTS forces R.  The energies do not depend on R
-  // (fixed-point sums).
+  // receptor parts: R interleaved segment sets of each chunk, so that the SMs
+  // fill and the last items to finish are short.  A part's item pays the
+  // chunk's set-up again, and a receptor of g segments spreads that over
+  // about g/R segments, so R falls with the launch's rounds (items per
+  // resident warp, w) and grows with g: R = 1 + 0.75 sqrt(g) / w, rounded.
+  // The best R of 1..8, measured on receptors of 4 to 107 segments at w of
+  // 0.1 to 50, lies within one of it; R = 1 starts at w of 10 for 40
+  // segments, where both cost the same (4,800 poses: 6.51 and 6.50 ms; 1,200
+  // poses: 1.98 ms at R = 1, 1.83 at 3).  From 8 parts on more of them pay
+  // only in launches of a fraction of a round (one pose of 2,538 x 1,280
+  // atoms: 135 us at 8, 114 at 24; 150 poses: 371 at 8, 381 at 16), so there
+  // the slope is an eighth.  GD_TUNE_RPARTS forces R.  The energies do not
+  // depend on R (fixed-point sums).
   int split_per_sm = 0;
   {
     const int keep_tune = pl->tune;
@@ -1032,24 +1037,25 @@ static gd_status plan_batch(gd_context *ctx, const std::vector<ScoreParams> &des
     e = fit(pl->max_nr <= kCntSmemMax ? ((pl->max_nr + 15) / 16) * 16 : 0, &per_sm);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "batched scoring occupancy");
   }
-  const long long target = static_cast<long long>(std::min(2.0, max_nseg / 8.0) * split_per_sm * kWarps *
-                                                  ctx->sm_count);
-  int R = ctx->tune_rparts > 0 ? ctx->tune_rparts
-                               : static_cast<int>(std::min<long long>(
-                                     kMaxRparts, std::max<long long>(1, (target + std::max(chunk_items, 1LL) - 1) /
-                                                                            std::max(chunk_items, 1LL))));
-  if (ctx->tune_rparts <= 0) R = std::max(1, std::min(R, max_nseg / 2));
+  int R = ctx->tune_rparts;
+  if (R <= 0) {
+    const double rounds = static_cast<double>(std::max(chunk_items, 1LL)) / split_per_sm / kWarps / ctx->sm_count;
+    const double want = 1.5 + 0.75 * std::sqrt(static_cast<double>(max_nseg)) / rounds;
+    R = static_cast<int>(std::min({want, 7.0 + want / 8.0, static_cast<double>(std::max(1, std::min(kMaxRparts, max_nseg)))}));
+  }
   auto split_bytes = [&](int r, size_t *part_b, size_t *cnt_b, size_t *lcnt_b) {
     *part_b = static_cast<size_t>(poses) * pl->max_chunks * r * 96 * sizeof(double);
     *cnt_b = static_cast<size_t>(poses) * ((pl->max_nr + 1) / 2) * sizeof(unsigned);
     *lcnt_b = r > 1 ? static_cast<size_t>(poses) * std::max(pl->max_nl, 1) * sizeof(unsigned) : 0;
     const size_t b = al256(*part_b) + al256(*cnt_b) + al256(static_cast<size_t>(poses) * sizeof(int)) + al256(*lcnt_b);
-    return b <= kSplitScratchMax && (ctx->budget == 0 || ctx->in_use + b <= ctx->budget);
+    // (further parts leave half of what a budget has left)
+    const uint64_t left = ctx->budget == 0 ? UINT64_MAX : ctx->budget > ctx->in_use ? ctx->budget - ctx->in_use : 0;
+    return b <= kSplitScratchMax && b <= (r > 1 ? left / 2 : left);
   };
   size_t part_b = 0, cnt_b = 0, lcnt_b = 0;
   bool fits = split_bytes(R, &part_b, &cnt_b, &lcnt_b);
-  if (!fits && R > 1 && ctx->tune_rparts <= 0) {
-    R = 1;
+  while (!fits && R > 1 && ctx->tune_rparts <= 0) {
+    R /= 2;
     fits = split_bytes(R, &part_b, &cnt_b, &lcnt_b);
   }
   pl->split = 0;

@@ -132,9 +132,9 @@ gd_status gd_context_destroy(gd_context *ctx);
  *                      every pair in FP64), 1 = the FP64 one always.  Both
  *                      decide every atom pair exactly; the keys are identical.
  *   GD_TUNE_RPARTS:    receptor parts per ligand chunk of a split FP32
- *                      launch: 0 = automatic (more than one only when the
- *                      launch has too few (pose, chunk) items to fill the
- *                      GPU), 1..8 = that many.  The energies do not depend
+ *                      launch: 0 = automatic (1 to 24: the more, the fewer
+ *                      (pose, chunk) items the launch has and the longer the
+ *                      receptor is), 1..8 = that many.  The energies do not depend
  *                      on it (per-segment fixed-point sums).
  * Read-only (gd_context_get_tuning; set_tuning refuses them):
  *   GD_INFO_LAST_FCC:      pair counts of the context's last device

@@ -2,13 +2,13 @@
 (four rows, two for one or two rows left): k receptor atoms close to one ligand
 slot and m at 14 A from it, against the oracle and against every other variant
 of the kernel and the 16-pose, split and whole-pose forms, whose energies are
-the same bits."""
+the same bits; and the automatic number of receptor parts."""
 import numpy as np
 import pytest
 
 import gdock_gb300 as gd
 from conftest import make_mol, tatom
-from gdock_gb300 import _lib
+from gdock_gb300 import _lib, synth
 from test_gpu_scoring import F32_TOL, check
 
 pytestmark = pytest.mark.gpu
@@ -48,6 +48,23 @@ def test_remainders(oracle, near, far):
             ctx.set_tuning(_lib.GD_TUNE_SPLIT, 1)
             ctx.set_tuning(_lib.GD_TUNE_F32_SLOTS, tune)
             check(cx.score_poses(genes, gd.GD_PREC_F32), oracle.score_poses(R, L, [], genes), F32_TOL)
+    finally:
+        cx.close()
+        ctx.close()
+
+
+@pytest.mark.parametrize("rec,lig,n", [(12, 20, 1), (12, 20, 3000), (300, 60, 1), (300, 60, 150), (300, 60, 1500), (300, 60, 5000)])
+def test_automatic_receptor_parts(rec, lig, n):
+    """The automatic number of receptor parts (by the launch's items: from 24,
+    or one part a segment, down to 1) leaves the energies of whole poses."""
+    c = synth.make_complex(rec, lig, 4, seed=rec + n)
+    genes = synth.quaternion_genes(np.random.default_rng(n), n, half_box=15.0)
+    ctx = gd.Context(0)
+    cx = gd.Complex(c.receptor, gd.position_ligand(c.receptor, c.ligand), c.restraint_pairs, ctx=ctx)
+    try:
+        auto = cx.score_poses(genes, gd.GD_PREC_F32)
+        ctx.set_tuning(_lib.GD_TUNE_SPLIT, 1)
+        assert cx.score_poses(genes, gd.GD_PREC_F32).tobytes() == auto.tobytes()
     finally:
         cx.close()
         ctx.close()
