@@ -1808,9 +1808,6 @@ gd_status cluster_device(gd_complex *cx, const double *genes, int n, const gd_cl
   if (c0 > (1 << 30)) return GD_ERR_STATE;
   const long long words = pair_words(t), pairs = static_cast<long long>(t->GR) * t->GL;
   const int aw = (n + 31) / 32;
-  std::vector<gd_pose_frame> frames(n);
-  gd_make_frames(genes, n, frames.data());
-  const double maxd = max_displacement(genes, n);
   const size_t fb = al256(sizeof(gd_pose_frame) * n), cb = al256(sizeof(int) * n), ub = al256(sizeof(uint32_t) * words),
                bb = al256(sizeof(int) * words), adj_b = al256(sizeof(uint32_t) * static_cast<size_t>(n) * aw);
   // small calls (rows over every residue pair, and the adjacency, within 16
@@ -1829,6 +1826,15 @@ gd_status cluster_device(gd_complex *cx, const double *genes, int n, const gd_cl
   uint32_t *d_u, *d_lists;
   char *d_direct;
   auto t_step = std::chrono::steady_clock::now();
+  // the frames are staged behind the place of the greedy pass's results
+  const size_t res_b = n > kGreedyMax ? 0 : al256(greedy_bytes(n));
+  const bool staged = fb <= kStageMax;
+  if ((s = ensure_scratch(ctx, 0, staged ? res_b + fb : 0)) != GD_OK) return s;
+  std::vector<gd_pose_frame> pageable(staged ? 0 : n);
+  gd_pose_frame *frames =
+      staged ? reinterpret_cast<gd_pose_frame *>(static_cast<char *>(ctx->h_pinned) + res_b) : pageable.data();
+  double maxd = 0.0;
+  frames_and_max_disp(genes, n, frames, &maxd);
   for (;;) {
     const size_t lb = al256(sizeof(uint32_t) * static_cast<size_t>(n) * cap);
     s = ensure_scratch(ctx, fb + cb + ub + bb + 256 + lb + direct_b, 0);
@@ -1841,7 +1847,7 @@ gd_status cluster_device(gd_complex *cx, const double *genes, int n, const gd_cl
     d_info = reinterpret_cast<int *>(b + fb + cb + ub + bb);
     d_lists = reinterpret_cast<uint32_t *>(b + fb + cb + ub + bb + 256);
     d_direct = b + fb + cb + ub + bb + 256 + lb;
-    cudaError_t e = cudaMemcpyAsync(d_frames, frames.data(), sizeof(gd_pose_frame) * n, cudaMemcpyHostToDevice, st);
+    cudaError_t e = cudaMemcpyAsync(d_frames, frames, sizeof(gd_pose_frame) * n, cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "contacts setup");
     trace_step("cluster (device):   scratch + frames", st, t_step);
     s = launch_contacts(cx, t, d_frames, n, cfg.contact_distance, maxd, d_counts, d_lists, cap, d_u, st);

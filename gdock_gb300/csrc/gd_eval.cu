@@ -476,20 +476,30 @@ gd_status gd_evaluate_poses(gd_evaluator *ev, const double *genes, int32_t n, gd
   cudaSetDevice(ctx->device);
   const size_t fb = sizeof(gd_pose_frame) * n, ob = sizeof(gd_dock_metrics) * n;
   const size_t fb_al = (fb + 255) / 256 * 256;
-  gd_status s = ensure_scratch(ctx, fb_al + ob, 0);
+  const bool staged = fb_al + ob <= kStageMax;
+  gd_status s = ensure_scratch(ctx, fb_al + ob, staged ? fb_al + ob : 0);
   if (s != GD_OK) return s;
   gd_pose_frame *d_frames = static_cast<gd_pose_frame *>(ctx->d_scratch);
   gd_dock_metrics *d_out = reinterpret_cast<gd_dock_metrics *>(static_cast<char *>(ctx->d_scratch) + fb_al);
-  std::vector<gd_pose_frame> frames(n);
-  gd_make_frames(genes, n, frames.data());
+  std::vector<gd_pose_frame> pageable(staged ? 0 : n);
+  gd_pose_frame *frames = staged ? static_cast<gd_pose_frame *>(ctx->h_pinned) : pageable.data();
+  void *res = staged ? static_cast<char *>(ctx->h_pinned) + fb_al : static_cast<void *>(out);
+  gd_make_frames(genes, n, frames);
   cudaStream_t st = ctx->stream;
-  cudaError_t e = cudaMemcpyAsync(d_frames, frames.data(), fb, cudaMemcpyHostToDevice, st);
+  cudaError_t e = cudaMemcpyAsync(d_frames, frames, fb, cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "evaluator frames upload");
-  if ((s = gd_evaluate_frames_device(ev, d_frames, n, d_out, st)) != GD_OK) return s;
-  e = cudaMemcpyAsync(out, d_out, ob, cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  if (e != cudaSuccess) return cuda_fail(ctx, e, "evaluator");
-  return check_device_error(ctx);
+  s = gd_evaluate_frames_device(ev, d_frames, n, d_out, st);
+  if (s == GD_OK) {
+    e = cudaMemcpyAsync(res, d_out, ob, cudaMemcpyDeviceToHost, st);
+    if (e != cudaSuccess) s = cuda_fail(ctx, e, "evaluator");
+  }
+  if (s != GD_OK) {
+    cudaStreamSynchronize(st);
+    return s;
+  }
+  s = finish_stream(ctx, st, "evaluator");
+  if (s == GD_OK && staged) copy_out(out, res, ob);
+  return s;
 }
 
 }  // extern "C"

@@ -134,8 +134,7 @@ struct gd_context {
   uint64_t in_use = 0;
   cudaStream_t stream = nullptr;
   int sm_count = 0;
-  int *d_err = nullptr;
-  int *h_err = nullptr, *h_info = nullptr;  // pinned: the error word as last read; small results of a call
+  int *d_err = nullptr, *h_info = nullptr;  // pinned: the error word that kernels write; small results of a call
   std::string last_error;
   // grow-only scratch: device and pinned host staging
   void *d_scratch = nullptr;
@@ -214,11 +213,16 @@ gd_status dev_alloc(gd_context *ctx, uint64_t bytes, void **p);
 void dev_free(gd_context *ctx, void *p, uint64_t bytes);
 gd_status ensure_scratch(gd_context *ctx, size_t dev_bytes, size_t pinned_bytes);
 gd_status check_device_error(gd_context *ctx);
-// Wait for the stream and report its errors, the device error word (read on
-// the same stream, before the wait) included.
+// Wait for the stream and report its errors, the device error word included.
 gd_status finish_stream(gd_context *ctx, cudaStream_t stream, const char *what);
 Thresholds make_thresholds(double contact_cutoff);
 void make_frame(const double *g, gd_pose_frame *f);
+void frames_and_max_disp(const double *genes, int n, gd_pose_frame *frames, double *max_disp);
+void copy_out(void *dst, const void *src, size_t bytes);
+// Inputs up to this size go through the context's pinned staging buffer (which
+// keeps its size): a copy from pageable memory passes a driver buffer piece by
+// piece and holds the host until it has left.
+constexpr size_t kStageMax = size_t(64) << 20;
 void guard_widths(const gd_complex *cx, double max_disp, float *gv, float *ge, float *gd);
 gd_status launch_score(gd_complex *cx, const gd_pose_frame *d_frames, const double *d_models, int n,
                        gd_precision prec, gd_pose_energy *d_out, cudaStream_t stream, double max_disp,

@@ -1101,14 +1101,14 @@ static ArgLayout arg_layout(int ncx, const BatchPlan &pl, size_t gcount_bytes) {
   o += al256(sizeof(ScoreParams) * ncx);
   L.start = o;
   o += al256(sizeof(long long) * (ncx + 1));
-  L.queue = o;
-  o += al256(sizeof(unsigned long long));
   L.pstart = o;
   o += al256(sizeof(long long) * (ncx + 1));
   L.gcounts = o;
   o += al256(gcount_bytes);
   L.part = o;
   o += al256(pl.part_b);
+  L.queue = o;  // from here on cleared before every launch
+  o += al256(sizeof(unsigned long long));
   L.pcount = o;
   o += al256(pl.cnt_b);
   L.pdone = o;
@@ -1141,8 +1141,7 @@ static gd_status upload_args(gd_context *ctx, const std::vector<ScoreParams> &de
 // Reset the work counter (and the split-mode counters) and launch.
 static gd_status launch_args(gd_context *ctx, int ncx, const BatchPlan &pl, const ArgLayout &L, char *arg,
                              bool serial, bool clamp, cudaStream_t stream) {
-  cudaError_t e = cudaMemsetAsync(arg + L.queue, 0, sizeof(unsigned long long), stream);
-  if (e == cudaSuccess && pl.split) e = cudaMemsetAsync(arg + L.pcount, 0, L.total - L.pcount, stream);
+  cudaError_t e = cudaMemsetAsync(arg + L.queue, 0, pl.split ? L.total - L.queue : sizeof(unsigned long long), stream);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "batched scoring reset");
   BatchParams bp{};
   bp.descs = reinterpret_cast<const ScoreParams *>(arg + L.desc);
