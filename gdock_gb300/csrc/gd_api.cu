@@ -908,6 +908,8 @@ class HostPool {
   long long gen_ = 0;
 };
 
+void host_parallel(int tasks, const std::function<void(int)> &f) { HostPool::get().run(tasks, f); }
+
 // Frames of n poses, on the host pool from 4,096 poses, and the largest
 // |displacement| component among them (sizes the FP32 guard bands).
 void frames_and_max_disp(const double *genes, int n, gd_pose_frame *frames, double *max_disp) {

@@ -1012,9 +1012,13 @@ struct TopoPack {
 void group_atoms(const std::vector<uint8_t> &chain, const std::vector<int16_t> &res, const std::vector<uint8_t> &elem,
                  std::vector<int64_t> &gkey, std::vector<int> &goff, std::vector<int> &atoms) {
   std::map<int64_t, std::vector<int>> g;
+  int64_t last = -1;
+  std::vector<int> *at = nullptr;  // the last atom's residue (usually the next one's too)
   for (size_t i = 0; i < chain.size(); ++i) {
     if (elem[i] == GD_ELEM_H) continue;  // src/clustering.rs:67-70
-    g[(static_cast<int64_t>(chain[i]) << 16) | static_cast<uint16_t>(res[i])].push_back(static_cast<int>(i));
+    const int64_t key = (static_cast<int64_t>(chain[i]) << 16) | static_cast<uint16_t>(res[i]);
+    if (key != last) at = &g[last = key];
+    at->push_back(static_cast<int>(i));
   }
   goff.assign(1, 0);
   for (auto &kv : g) {
@@ -1084,35 +1088,40 @@ gd_status build_topo(gd_complex *cx, ClusterTopo **out) {
   for (size_t a = 0; a < rx.size(); ++a)
     r32[a] = make_float4(static_cast<float>(rx[a] - cx->ox), static_cast<float>(ry[a] - cx->oy),
                          static_cast<float>(rz[a] - cx->oz), 0.0f);
-  std::vector<float4> rsph(t->GR);
+  // Spheres enclosing the atoms of every residue, of blocks of kLigBlock
+  // consecutive ligand residues and of 32 receptor residues (each slightly
+  // widened), on the host pool: sixteen passes over every atom for each kind,
+  // half of a first call on a large complex when they ran on one thread.
+  const int nb = (t->GL + kLigBlock - 1) / kLigBlock, nrb = (t->GR + 31) / 32;
+  std::vector<float4> rsph(t->GR), rbsph(std::max(nrb, 1), make_float4(0, 0, 0, 0));
+  std::vector<D4> lsph(t->GL), lbsph(std::max(nb, 1), D4{0, 0, 0, 0});
   std::vector<uint8_t> rch(t->GR), lch(t->GL);
-  for (int g = 0; g < t->GR; ++g) {
+  for (int g = 0; g < t->GR; ++g) rch[g] = static_cast<uint8_t>(t->rg_key[g] >> 16);
+  for (int g = 0; g < t->GL; ++g) lch[g] = static_cast<uint8_t>(t->lg_key[g] >> 16);
+  auto ball = [](const std::vector<double> &x, const std::vector<double> &y, const std::vector<double> &z, int a0, int a1) {
     double c[3], r;
-    const int a0 = t->rg_off[g];
-    enclosing_ball(rx.data() + a0, ry.data() + a0, rz.data() + a0, nullptr, t->rg_off[g + 1] - a0, c, r);
-    rsph[g] = make_float4(static_cast<float>(c[0] - cx->ox), static_cast<float>(c[1] - cx->oy),
-                          static_cast<float>(c[2] - cx->oz), static_cast<float>(r * (1 + 1e-6) + 1e-3));
-    rch[g] = static_cast<uint8_t>(t->rg_key[g] >> 16);
-  }
-  std::vector<D4> lsph(t->GL);
-  for (int g = 0; g < t->GL; ++g) {
-    double c[3], r;
-    const int a0 = t->lg_off[g];
-    enclosing_ball(lx.data() + a0, ly.data() + a0, lz.data() + a0, nullptr, t->lg_off[g + 1] - a0, c, r);
-    lsph[g] = D4{c[0], c[1], c[2], r * (1 + 1e-6) + 1e-3};
-    lch[g] = static_cast<uint8_t>(t->lg_key[g] >> 16);
-  }
-  // blocks of kLigBlock consecutive ligand residues: a sphere enclosing all
-  // their atoms (with the same small widening)
-  const int nb = (t->GL + kLigBlock - 1) / kLigBlock;
-  std::vector<D4> lbsph(std::max(nb, 1), D4{0, 0, 0, 0});
-  for (int b = 0; b < nb; ++b) {
-    const int g0 = b * kLigBlock, g1 = std::min(t->GL, g0 + kLigBlock);
-    double c[3], r;
-    const int a0 = t->lg_off[g0];
-    enclosing_ball(lx.data() + a0, ly.data() + a0, lz.data() + a0, nullptr, t->lg_off[g1] - a0, c, r);
-    lbsph[b] = D4{c[0], c[1], c[2], r * (1 + 1e-6) + 1e-3};
-  }
+    enclosing_ball(x.data() + a0, y.data() + a0, z.data() + a0, nullptr, a1 - a0, c, r);
+    return D4{c[0], c[1], c[2], r * (1 + 1e-6) + 1e-3};
+  };
+  auto rec_ball = [&](int g0, int g1) {
+    const D4 v = ball(rx, ry, rz, t->rg_off[g0], t->rg_off[g1]);
+    return make_float4(static_cast<float>(v.x - cx->ox), static_cast<float>(v.y - cx->oy), static_cast<float>(v.z - cx->oz),
+                       static_cast<float>(v.w));
+  };
+  const int nt = rx.size() + lx.size() >= 2048 ? 32 : 1;
+  auto spheres = [&](int task) {
+    auto each = [&](int n, auto f) {
+      for (int i = static_cast<int>(static_cast<long long>(n) * task / nt); i < static_cast<long long>(n) * (task + 1) / nt; ++i) f(i);
+    };
+    each(t->GR, [&](int g) { rsph[g] = rec_ball(g, g + 1); });
+    each(nrb, [&](int b) { rbsph[b] = rec_ball(b * 32, std::min(t->GR, b * 32 + 32)); });
+    each(t->GL, [&](int g) { lsph[g] = ball(lx, ly, lz, t->lg_off[g], t->lg_off[g + 1]); });
+    each(nb, [&](int b) {
+      lbsph[b] = ball(lx, ly, lz, t->lg_off[b * kLigBlock], t->lg_off[std::min(t->GL, (b + 1) * kLigBlock)]);
+    });
+  };
+  if (nt == 1) spheres(0);
+  else host_parallel(nt, spheres);
   // the same relative to the rotation centre, as the contact kernel moves them
   auto rel = [&](const D4 &v) { return D4{v.x - cx->cx, v.y - cx->cy, v.z - cx->cz, v.w}; };
   auto rel32 = [&](const D4 &v) {
@@ -1124,17 +1133,6 @@ gd_status build_topo(gd_complex *cx, ClusterTopo **out) {
   for (int g = 0; g < t->GL; ++g) lgrel[g] = rel32(lsph[g]);
   for (int b = 0; b < nb; ++b) lbrel[b] = rel32(lbsph[b]);
   for (size_t a = 0; a < lx.size(); ++a) lrel[a] = rel(D4{lx[a], ly[a], lz[a], 0.0});
-  // groups of 32 consecutive receptor residues
-  const int nrb = (t->GR + 31) / 32;
-  std::vector<float4> rbsph(std::max(nrb, 1), make_float4(0, 0, 0, 0));
-  for (int b = 0; b < nrb; ++b) {
-    const int g0 = b * 32, g1 = std::min(t->GR, g0 + 32);
-    double c[3], r;
-    const int a0 = t->rg_off[g0];
-    enclosing_ball(rx.data() + a0, ry.data() + a0, rz.data() + a0, nullptr, t->rg_off[g1] - a0, c, r);
-    rbsph[b] = make_float4(static_cast<float>(c[0] - cx->ox), static_cast<float>(c[1] - cx->oy),
-                           static_cast<float>(c[2] - cx->oz), static_cast<float>(r * (1 + 1e-6) + 1e-3));
-  }
   // one allocation and one copy for every array of the topology
   TopoPack pack;
   pack.add(rbsph, &t->d_rb_sph);

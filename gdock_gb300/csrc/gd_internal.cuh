@@ -1,6 +1,7 @@
 // Internal declarations shared by the gdock_gb300 CUDA sources.
 #pragma once
 
+#include <functional>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -219,6 +220,7 @@ Thresholds make_thresholds(double contact_cutoff);
 void make_frame(const double *g, gd_pose_frame *f);
 void frames_and_max_disp(const double *genes, int n, gd_pose_frame *frames, double *max_disp);
 void copy_out(void *dst, const void *src, size_t bytes);
+void host_parallel(int tasks, const std::function<void(int)> &f);  // f(0) .. f(tasks - 1) on the host pool
 // Inputs up to this size go through the context's pinned staging buffer (which
 // keeps its size): a copy from pageable memory passes a driver buffer piece by
 // piece and holds the host until it has left.
