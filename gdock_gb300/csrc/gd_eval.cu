@@ -15,11 +15,11 @@
 //     identity (a docked contact counts once when it is native); ligand atoms
 //     with none of these are left out.
 // Device (k_dockq): the lanes of one warp (or of eight, for few poses) take a
-// pose's ligand atoms; per atom the difference from its partner is one chain
-// of fused multiply-adds, the distance its square root, the sums exact integer
-// ones; contacts are decided in FP32 outside a guard band and exactly (the
-// reference's transform and threshold) inside it, and distances that
-// cancellation would spoil (below 1/4 A) are redone in the reference's order.
+// pose's ligand atoms; transform, distance and sums are fixed-point integers
+// finer than FP64's rounding; contacts are decided in FP32 outside a guard band
+// and exactly (the reference's transform and threshold) inside it, and
+// distances that cancellation would spoil (below 1/4 A) or that leave the
+// fixed-point range are formed in FP64 in the reference's order.
 //   rmsd  = sqrt(sum over pairs of distance / |reference|)    (src/evaluator.rs:86-103;
 //   irmsd = likewise over the interface pairings               the sum is of distances)
 //   fnat  = docked native contacts / |native contacts|
@@ -33,6 +33,8 @@
 
 #include "gd_device.cuh"
 
+struct Fix3 { long long x, y, z, pad; };
+
 struct gd_evaluator {
   gd_complex *cx = nullptr;
   gd_context *ctx = nullptr;
@@ -42,9 +44,18 @@ struct gd_evaluator {
   int64_t counts[GD_EVAL_COUNTS] = {};    // as gd_evaluator_counts reports them
   const int *u_slot = nullptr;            // [n_u] device slot of each such ligand atom (interface atoms first)
   int n_if = 0;                           // the first n_if of them have an i-RMSD partner or native contacts
-  const D4 *u_x0 = nullptr;               // [n_u] ligand atom relative to the rotation centre
-  const D4 *u_ref = nullptr;              // [n_u] paired reference atom (w = 1) or none (w = 0)
-  const D4 *u_iref = nullptr;             // [n_if] likewise; w = 2: the same atom as u_ref
+  // [n_u] ligand atom relative to the rotation centre in two limbs a coordinate
+  // (x, y; z), then the paired reference atom relative to `origin` (x, y; z) in
+  // 2^-51 A; w2 of u_z: bit 0: there is one; u_z.w >> 1: an i-RMSD partner of its own
+  // (1), the same (2)
+  const int4 *u_xy = nullptr, *u_z = nullptr;
+  const longlong2 *u_qxy = nullptr;
+  const long long *u_qz = nullptr;
+  const D4 *u_ref = nullptr;              // [n_u] paired reference atom
+  const D4 *u_iref = nullptr;             // [n_if] i-RMSD partner
+  const Fix3 *u_iq = nullptr;             // [n_if] the same relative to `origin` in 2^-51 A
+  bool fixed = false;                     // every coordinate is within the fixed-point range
+  long long origin[3] = {0, 0, 0};        // the FP32 origin O rounded to whole Angstroms, in 2^-51 A
   const int *u_pbeg = nullptr;            // [n_if + 1] CSR offsets into p_rec
   const D4 *p_rec = nullptr;              // [n_p] receptor atoms whose contact with the ligand atom is native
   const float4 *p_rec32 = nullptr;        // [n_p] the same, FP32 relative to the origin O
@@ -59,7 +70,14 @@ namespace {
 struct EvalParams {
   ScoreParams p;  // ligand arrays, frames and the rotation centre
   const int *u_slot, *u_pbeg;
-  const D4 *u_x0, *u_ref, *u_iref, *p_rec;
+  const int4 *u_xy, *u_z;
+  const longlong2 *u_qxy;
+  const long long *u_qz;
+  const Fix3 *u_iq;
+  long long ox, oy, oz;  // the evaluator's origin in 2^-51 A
+  float fx, fy, fz;      // ... less the FP32 origin O
+  bool fixed;
+  const D4 *u_ref, *u_iref, *p_rec;
   const float4 *p_rec32;
   int n_u, n_if, n_ref, n_iref, n_native;
   double thr5;
@@ -69,7 +87,7 @@ struct EvalParams {
 };
 
 constexpr int kEvalWarps = 8;
-constexpr int kEvalCtas = 2;    // resident per SM (registers)
+constexpr int kEvalCtas = 3;    // resident per SM (registers)
 // distance sums: a resolution of 2^-96 A (at the native pose the distances
 // are rounding noise of some 1e-15 A), 2^31 A of room, single distances from
 // 2^14 A on kept apart
@@ -93,55 +111,166 @@ __device__ __noinline__ bool exact_contact(const ScoreParams &p, const gd_pose_f
   return exact_d2(a.x, a.y, a.z, X, Y, Z) <= thr5;
 }
 
-// sqrt(d2) for d2 in [1/16, 2^900): s (1 - e)^(-1/2) by its Taylor series to
-// the second order on the hardware's approximation y of d2^(-1/2), with
-// s = d2 y and e = 1 - s y (about 2^-20, so that the next term lies below the
-// FP64 rounding): five FP64 operations.
-__device__ __forceinline__ double sqrt64(double d2) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d2));
-  const double s = d2 * y, e = __fma_rn(-s, y, 1.0);
-  return __fma_rn(s, e * __fma_rn(e, 0.375, 0.5), s);
+// Fixed point.  Ligand atoms (relative to the rotation centre, below 512 A) are
+// integers of 2^-50 A in two limbs h 2^29 + l, matrix entries (at most 1.5) of
+// 2^-59 likewise; positions and differences are 2^-51 A, translations and
+// reference atoms within 768 A of the origin, so that a difference stays below
+// 2^12 A.
+constexpr double kFixAtom = 512.0, kFixFar = 768.0;
+struct Limbs { int h, l; };
+__host__ __device__ __forceinline__ Limbs limbs(long long v) {
+  return Limbs{static_cast<int>(v >> 29), static_cast<int>(v & ((1 << 29) - 1))};
 }
 
-// What bounds it: the FP64 pipe.  The reference's transform, difference,
-// square and correctly rounded root cost about 60 FP64 operations per atom;
-// this form takes 12 for the difference, 3 and 5 for square and root and adds
-// in integers.  WPP warps per pose: one where the poses fill the GPU, else the
-// whole CTA (150 poses of one warp each kept 38 of the 152 SMs waiting on
-// FP64 latency).
+// One coordinate of the rotated atom: nine 32 x 32 -> 64 multiply-adds of
+// three products, the low limbs' dropped (three units of 2^-51 A at most; an
+// FP64 chain of multiply-adds errs by ten times as much at 60 A).
+__device__ __forceinline__ long long rotate(const Limbs &a, const Limbs &b, const Limbs &c, const int4 &xy, const int4 &z) {
+  long long hi = static_cast<long long>(a.h) * xy.x, mid = static_cast<long long>(a.h) * xy.y;
+  hi += static_cast<long long>(b.h) * xy.z;
+  mid += static_cast<long long>(a.l) * xy.x;
+  hi += static_cast<long long>(c.h) * z.x;
+  mid += static_cast<long long>(b.h) * xy.w;
+  mid += static_cast<long long>(b.l) * xy.z;
+  mid += static_cast<long long>(c.h) * z.y;
+  mid += static_cast<long long>(c.l) * z.x;
+  return hi + (mid >> 29);
+}
+
+// The length of (x, y, z) added to c 2^33 + r units of 2^-57 A, 2^-55 of it off
+// at most (2^-51 from 64 A on); false below 1/4 A.  The squared length D (in
+// 2^-68 A^2) differs from the square of its FP32 root s by R = D - s^2, some
+// 2^-20 of it, formed exactly modulo 2^64; then
+// sqrt(s^2 + R) = s + R / 2s - R^2 / 8s^3 + ... (the next term is 2^-60 of s),
+// R / 2s as a multiple q of 2^20 units and an FP32 remainder.  Lengths with a
+// coordinate from 64 A on are taken in 2^-45 A.  Conversions are of 32 bits:
+// those of 64 run on the FP64 unit (seven of them an atom kept it 82 % busy and
+// the kernel at 1.27 ms for 65,536 poses).
+struct Length {
+  unsigned s;  // 2^-24 A
+  int q, tail;
+  int far;     // all of them times 2^6
+};
+__device__ __forceinline__ bool fix_length(long long x, long long y, long long z, Length &o) {
+  auto high = [](long long v) { return static_cast<int>((v + 0x80000000ll) >> 32); };
+  auto size = [](int h) { return static_cast<unsigned>(h ^ (h >> 31)); };
+  o.far = (size(high(x)) | size(high(y)) | size(high(z))) >= 64u << 19;
+  if (o.far) {
+    x = (x + 32) >> 6;
+    y = (y + 32) >> 6;
+    z = (z + 32) >> 6;
+  }
+  auto f32 = [](long long v) { return __int2float_rn(static_cast<int>((v + (1 << 26)) >> 27)); };  // in 2^-24 A
+  const float gx = f32(x), gy = f32(y), gz = f32(z);
+  const float d2 = __fmul_rn(__fmaf_rn(gz, gz, __fmaf_rn(gy, gy, __fmul_rn(gx, gx))), 0x1p-48f);
+  if (!(d2 >= 0.0625f)) return false;
+  float rs;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rs) : "f"(d2));
+  o.s = __float2uint_rn(__fmul_rn(__fmul_rn(d2, rs), 16777216.0f));
+  const int hx = high(x), hy = high(y), hz = high(z), lx = static_cast<int>(x), ly = static_cast<int>(y),
+            lz = static_cast<int>(z);
+  const long long hl = static_cast<long long>(hx) * lx + static_cast<long long>(hy) * ly + static_cast<long long>(hz) * lz;
+  const unsigned long long hh = static_cast<long long>(hx) * hx + static_cast<long long>(hy) * hy + static_cast<long long>(hz) * hz;
+  const unsigned long long ll = static_cast<unsigned long long>(static_cast<long long>(lx) * lx) +
+                                static_cast<unsigned long long>(static_cast<long long>(ly) * ly) +
+                                static_cast<unsigned long long>(static_cast<long long>(lz) * lz);
+  const unsigned long long D = static_cast<unsigned long long>(hl >> 1) + (ll >> 34) + (hh << 30);
+  // R to 2^-64 of d2: 46 bits in two exact FP32 parts
+  const int up = (__float_as_int(d2) >> 23) - 127 + 4;
+  const long long R = static_cast<long long>(D - ((static_cast<unsigned long long>(o.s) * o.s) << 20)) >> up;
+  const float rh = __fmul_rn(__int2float_rn(static_cast<int>(R >> 22)), 4194304.0f);
+  const float rl = __int2float_rn(static_cast<int>(R) & 0x3fffff);
+  const float w = __fmul_rn(__fmul_rn(rs, 0x1p-12f), __int_as_float((127 + up) << 23));
+  const float s12 = __fmul_rn(__fmul_rn(__uint2float_rn(o.s), 0x1p-12f), __int_as_float((127 - up) << 23));
+  o.q = __float2int_rn(__fmul_rn(__fmul_rn(rh, w), 0x1p-20f));
+  const float qf = __fmul_rn(__int2float_rn(o.q), 0x1p20f);
+  const float rem = __fadd_rn(__fmaf_rn(-qf, s12, rh), rl);
+  o.tail = __float2int_rn(__fmaf_rn(rem, w, -__fmul_rn(__fmul_rn(qf, qf), __fmul_rn(rs, 0x1p-58f))));
+  return true;
+}
+
+struct FarSum { __int128 v; double nf; };
+
+// A thread's distance sums: fix_length()'s in registers, those formed in FP64
+// (few, or all of a pose out of range) in shared memory, touched when there is
+// one.
+struct PoseSum {
+  unsigned long long c = 0;
+  long long r = 0;
+  __device__ __forceinline__ void add(const Length &d) {
+    const int unit = d.far ? 64 : 1;
+    c += static_cast<unsigned long long>(d.s) * static_cast<unsigned>(unit);
+    r += static_cast<long long>(d.q) * (unit << 20);
+    r += static_cast<long long>(d.tail) * unit;
+  }
+  __device__ __forceinline__ DistSum close(const FarSum &far, bool used) const {
+    DistSum d;
+    if (used) {
+      d.v = far.v;
+      d.nf = far.nf;
+    }
+    d.v += ((static_cast<__int128>(c) << 33) + r) << (kDistBits - 57);
+    return d;
+  }
+};
+// A finished pose, until its warp has 32.
+struct Held {
+  __int128 l, i;
+  double nf_l, nf_i;
+  int common, pose;
+};
+
+// What bounds it: instruction issue and the integer multiply-add unit.  FP64
+// issues once in 64 cycles, so the FP64 form (12 operations for an atom's
+// difference from its partner, 8 for square and root) kept that pipe 85 % busy;
+// in fixed point an atom is some 230 integer and FP32 instructions on units
+// thirty times as fast, and the result is closer.  Three CTAs an SM measured
+// best (two: 3 % slower, four: spills, 5 %).  WPP warps per pose: one where the
+// poses fill the GPU, else the whole CTA (150 poses of one warp each kept 38 of
+// the 152 SMs waiting).
 // 65,536 poses of 2,538 x 1,280 atoms (the whole call, host frames and copies
-// included) 10.8 -> 4.32 ms; the kernel on 150 poses of 1,074 x 741 atoms 99 ->
-// 18 us.
+// included): 10.8 ms in the reference's operation order, 4.18 as FP64
+// multiply-add chains (the kernel 3.53), 1.69 in fixed point (0.99).
 template <int WPP>
 __global__ void __launch_bounds__(kEvalWarps * 32, kEvalCtas) k_dockq(const EvalParams e) {
   if (e.skip && *e.skip) return;
   __shared__ gd_pose_frame s_f[kEvalWarps / WPP];
+  __shared__ Limbs s_m[kEvalWarps][9];
+  __shared__ long long s_t[kEvalWarps][3];
   __shared__ __int128 s_sum[kEvalWarps][2];
   __shared__ double s_nf[kEvalWarps][2];
   __shared__ int s_common[kEvalWarps];
+  __shared__ Held s_held[WPP == 1 ? kEvalWarps * 32 : 32];
+  __shared__ FarSum s_far[kEvalWarps * 32][2];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int step = gridDim.x * (kEvalWarps / WPP);
   const int t0 = WPP == 1 ? lane : static_cast<int>(threadIdx.x);
   gd_pose_frame &f = s_f[WPP == 1 ? warp : 0];
-  // lane k keeps the k-th pose's sums until the warp has 32 of them: the
-  // divisions and roots of the metrics then run on all lanes
-  DistSum my_l, my_i;
-  int my_common = 0, my_pose = -1, held = 0;
+  // a warp keeps the poses' sums until it has 32 of them: the divisions and
+  // roots of the metrics then run on all lanes
+  Held *my = s_held + (WPP == 1 ? warp * 32 : 0);
+  int held = 0;
   auto finish = [&]() {
-    if (my_pose >= 0) {
+    __syncwarp();
+    if (lane < held) {
       // src/evaluator.rs:68-84, without contraction into fused multiply-adds
-      const double sl = my_l.value(kDistBits), si = my_i.value(kDistBits);
+      const Held &h = my[lane];
+      DistSum l, i;
+      l.v = h.l;
+      l.nf = h.nf_l;
+      i.v = h.i;
+      i.nf = h.nf_i;
+      const double sl = l.value(kDistBits), si = i.value(kDistBits);
       const double rmsd = e.n_ref ? __dsqrt_rn(__ddiv_rn(sl, static_cast<double>(e.n_ref))) : 0.0;
       const double irmsd = e.n_iref ? __dsqrt_rn(__ddiv_rn(si, static_cast<double>(e.n_iref))) : 0.0;
-      const double fnat = e.n_native ? __ddiv_rn(static_cast<double>(my_common), static_cast<double>(e.n_native)) : 0.0;
+      const double fnat = e.n_native ? __ddiv_rn(static_cast<double>(h.common), static_cast<double>(e.n_native)) : 0.0;
       const double a = __ddiv_rn(irmsd, 1.5), b = __ddiv_rn(rmsd, 8.5);
       const double is = __ddiv_rn(1.0, __dadd_rn(1.0, __dmul_rn(a, a)));
       const double ls = __ddiv_rn(1.0, __dadd_rn(1.0, __dmul_rn(b, b)));
       const double dockq = __ddiv_rn(__dadd_rn(__dadd_rn(fnat, is), ls), 3.0);
-      e.out[my_pose] = gd_dock_metrics{rmsd, irmsd, fnat, dockq};
+      e.out[h.pose] = gd_dock_metrics{rmsd, irmsd, fnat, dockq};
     }
-    my_pose = -1;
+    __syncwarp();
     held = 0;
   };
   for (int pose = blockIdx.x * (kEvalWarps / WPP) + (WPP == 1 ? warp : 0); pose < e.p.n_poses; pose += step) {
@@ -150,99 +279,126 @@ __global__ void __launch_bounds__(kEvalWarps * 32, kEvalCtas) k_dockq(const Eval
     if (t0 < 16) reinterpret_cast<double *>(&f)[t0] = reinterpret_cast<const double *>(e.p.frames + pose)[t0];
     if (WPP == 1) __syncwarp();
     else __syncthreads();
-    // moved atom = R x0 + (centre + displacement)
-    const double m00 = f.ca * f.cb, m01 = f.m01, m02 = f.m02, m10 = f.sa * f.cb, m11 = f.m11, m12 = f.m12;
-    const double m20 = -f.sb, m21 = f.cb * f.sg, m22 = f.cb * f.cg;
-    const double tx = e.p.cx + f.dx, ty = e.p.cy + f.dy, tz = e.p.cz + f.dz;
-    // the FP32 guard band of the contact test, as for the contact bitmaps
+    // the rotation (src/structure.rs:80-131) and the centre + displacement in
+    // fixed point, an entry a lane; fix: all of them are in range
+    bool ok = true;
+    if (lane < 9) {
+      const double a = lane == 0 ? f.ca : lane == 1 ? f.m01 : lane == 2 ? f.m02 : lane == 3 ? f.sa : lane == 4 ? f.m11
+                       : lane == 5 ? f.m12 : lane == 6 ? -f.sb : f.cb;
+      const double b = lane == 0 || lane == 3 ? f.cb : lane == 7 ? f.sg : lane == 8 ? f.cg : 1.0;
+      const double m = __dmul_rn(a, b);
+      ok = fabs(m) <= 1.5;
+      s_m[warp][lane] = limbs(ok ? __double2ll_rn(m * 0x1p59) : 0);
+    } else if (lane < 12) {
+      const double t = lane == 9 ? e.p.cx + f.dx : lane == 10 ? e.p.cy + f.dy : e.p.cz + f.dz;
+      const long long o = lane == 9 ? e.ox : lane == 10 ? e.oy : e.oz;
+      ok = fabs(t) < 4000.0;
+      const long long v = ok ? __double2ll_rn(t * 0x1p51) - o : 0;
+      ok = ok && llabs(v) < static_cast<long long>(kFixFar * 0x1p51);
+      s_t[warp][lane - 9] = v;
+    }
+    const bool fix = __all_sync(kFull, ok) && e.fixed;
+    __syncwarp();
+    Limbs m[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) m[k] = s_m[warp][k];
+    const long long tx = s_t[warp][0], ty = s_t[warp][1], tz = s_t[warp][2];
+    // the FP32 guard band of the contact test, as for the contact lists
     // (M bounds the coordinates; twice it covers the sum that forms them)
     const float M = 2.0f * (e.extent + fmaxf(fabsf(static_cast<float>(f.dx)),
                                              fmaxf(fabsf(static_cast<float>(f.dy)), fabsf(static_cast<float>(f.dz)))));
     const float guard = 4.0f * (17.33f * (2.0f * M + 5.0f) + 100.0f) * 0x1p-24f + 1e-6f;
-    const bool band_ok = guard < 1.0f;
-    DistSum sl, si;
+    const bool band_ok = guard < 1.0f && fix;
+    PoseSum sl, si;
     int common = 0;
+    FarSum *far = s_far[threadIdx.x];
+    bool used = false;
+    auto add_far = [&](double d, bool to_l, bool to_i) {
+      if (!used) far[0] = far[1] = FarSum{0, 0.0};
+      used = true;
+      DistSum v;
+      v.add(d, kDistBits);
+      for (int k = 0; k < 2; ++k)
+        if (k == 0 ? to_l : to_i) {
+          far[k].v += v.v;
+          far[k].nf += v.nf;
+        }
+    };
 #pragma unroll 1
     for (int u = t0; u < e.n_u; u += 32 * WPP) {
-      const D4 a = e.u_x0[u], r = e.u_ref[u];
-      auto from = [&](const D4 &q, double &dx, double &dy, double &dz) {
-        dx = __fma_rn(m00, a.x, __fma_rn(m01, a.y, __fma_rn(m02, a.z, tx - q.x)));
-        dy = __fma_rn(m10, a.x, __fma_rn(m11, a.y, __fma_rn(m12, a.z, ty - q.y)));
-        dz = __fma_rn(m20, a.x, __fma_rn(m21, a.y, __fma_rn(m22, a.z, tz - q.z)));
+      const int4 xy = e.u_xy[u], z = e.u_z[u];
+      const long long px = rotate(m[0], m[1], m[2], xy, z) + tx, py = rotate(m[3], m[4], m[5], xy, z) + ty,
+                      pz = rotate(m[6], m[7], m[8], xy, z) + tz;
+      auto slot = [&]() {
+        const int sl = e.u_slot[u];
+        return GD_DCHECK(e.p.err, sl >= 0 && sl < e.p.nl, 40) ? sl : 0;
       };
-      auto distance = [&](const D4 &q, double dx, double dy, double dz) {
-        const double d2 = __fma_rn(dz, dz, __fma_rn(dy, dy, dx * dx));
-        const int hi = __double2hiint(d2);
-        if (hi < 0x3fb00000 || hi >= 0x78300000) {  // below 1/16, or from 2^900 (and NaN) on
-          int slot = e.u_slot[u];
-          if (!GD_DCHECK(e.p.err, slot >= 0 && slot < e.p.nl, 40)) slot = 0;
-          return exact_distance(e.p, f, pose, slot, q.x, q.y, q.z);
+      const int iw = z.w >> 1;
+      if (z.w & 1) {
+        const longlong2 q = e.u_qxy[u];
+        Length d;
+        if (fix && fix_length(px - q.x, py - q.y, pz - e.u_qz[u], d)) {
+          sl.add(d);
+          if (iw == 2) si.add(d);
+        } else {
+          const D4 a = e.u_ref[u];
+          add_far(exact_distance(e.p, f, pose, slot(), a.x, a.y, a.z), true, iw == 2);
         }
-        return sqrt64(d2);
-      };
-      double dx, dy, dz;
-      from(r, dx, dy, dz);
-      double d = 0.0;
-      if (r.w != 0.0) {
-        d = distance(r, dx, dy, dz);
-        sl.add(d, kDistBits);
       }
       if (u < e.n_if) {
-        const D4 q = e.u_iref[u];
-        if (q.w == 2.0) {
-          si.add(d, kDistBits);
-        } else if (q.w != 0.0) {
-          double ex, ey, ez;
-          from(q, ex, ey, ez);
-          si.add(distance(q, ex, ey, ez), kDistBits);
+        if (iw == 1) {
+          const Fix3 q = e.u_iq[u];
+          Length d;
+          if (fix && fix_length(px - q.x, py - q.y, pz - q.z, d)) {
+            si.add(d);
+          } else {
+            const D4 a = e.u_iref[u];
+            add_far(exact_distance(e.p, f, pose, slot(), a.x, a.y, a.z), false, true);
+          }
         }
         int k = e.u_pbeg[u];
         const int k1 = e.u_pbeg[u + 1];
         if (k < k1) {
-          const float lx = static_cast<float>(dx) + static_cast<float>(r.x - e.p.ox),
-                      ly = static_cast<float>(dy) + static_cast<float>(r.y - e.p.oy),
-                      lz = static_cast<float>(dz) + static_cast<float>(r.z - e.p.oz);
+          auto f32 = [](long long v, float o) {
+            const int h = static_cast<int>((v + 0x80000000ll) >> 32);
+            return __fmaf_rn(__int2float_rn(static_cast<int>(v)), 0x1p-51f, __fmaf_rn(__int2float_rn(h), 0x1p-19f, o));
+          };
+          const float lx = f32(px, e.fx), ly = f32(py, e.fy), lz = f32(pz, e.fz);
           for (; k < k1; ++k) {
             const float t = d2f(__ldg(&e.p_rec32[k]), lx, ly, lz) - 25.0f;
             bool hit = t < 0.0f;
-            if (!(band_ok && fabsf(t) > guard)) {
-              int slot = e.u_slot[u];
-              if (!GD_DCHECK(e.p.err, slot >= 0 && slot < e.p.nl, 40)) slot = 0;
-              hit = exact_contact(e.p, f, pose, slot, e.p_rec[k], e.thr5);
-            }
+            if (!(band_ok && fabsf(t) > guard)) hit = exact_contact(e.p, f, pose, slot(), e.p_rec[k], e.thr5);
             common += hit;
           }
         }
       }
     }
-    sl.warp_total();
-    si.warp_total();
+    DistSum dl = sl.close(far[0], used), di = si.close(far[1], used);
+    dl.warp_total();
+    di.warp_total();
     common = __reduce_add_sync(kFull, common);
     if (WPP > 1) {
       if (lane == 0) {
-        s_sum[warp][0] = sl.v;
-        s_sum[warp][1] = si.v;
-        s_nf[warp][0] = sl.nf;
-        s_nf[warp][1] = si.nf;
+        s_sum[warp][0] = dl.v;
+        s_sum[warp][1] = di.v;
+        s_nf[warp][0] = dl.nf;
+        s_nf[warp][1] = di.nf;
         s_common[warp] = common;
       }
       __syncthreads();
       if (warp == 0) {
         for (int w = 1; w < WPP; ++w) {
-          sl.v += s_sum[w][0];
-          si.v += s_sum[w][1];
-          sl.nf += s_nf[w][0];
-          si.nf += s_nf[w][1];
+          dl.v += s_sum[w][0];
+          di.v += s_sum[w][1];
+          dl.nf += s_nf[w][0];
+          di.nf += s_nf[w][1];
           common += s_common[w];
         }
       }
     }
     if (WPP == 1 || warp == 0) {
-      if (lane == held) {
-        my_l = sl;
-        my_i = si;
-        my_common = common;
-        my_pose = pose;
+      if (lane == 0) {
+        my[held] = Held{dl.v, di.v, dl.nf, di.nf, common, pose};
       }
       if (++held == 32) finish();
     }
@@ -266,7 +422,18 @@ gd_status launch_dockq(gd_evaluator *ev, const gd_pose_frame *d_frames, int n, g
   ep.p = make_params(ev->cx, d_frames, nullptr, n, nullptr, 0.0);
   ep.u_slot = ev->u_slot;
   ep.u_pbeg = ev->u_pbeg;
-  ep.u_x0 = ev->u_x0;
+  ep.u_xy = ev->u_xy;
+  ep.u_z = ev->u_z;
+  ep.u_qxy = ev->u_qxy;
+  ep.u_qz = ev->u_qz;
+  ep.u_iq = ev->u_iq;
+  ep.ox = ev->origin[0];
+  ep.oy = ev->origin[1];
+  ep.oz = ev->origin[2];
+  ep.fx = static_cast<float>(std::ldexp(static_cast<double>(ev->origin[0]), -51) - ev->cx->ox);
+  ep.fy = static_cast<float>(std::ldexp(static_cast<double>(ev->origin[1]), -51) - ev->cx->oy);
+  ep.fz = static_cast<float>(std::ldexp(static_cast<double>(ev->origin[2]), -51) - ev->cx->oz);
+  ep.fixed = ev->fixed;
   ep.u_ref = ev->u_ref;
   ep.u_iref = ev->u_iref;
   ep.p_rec = ev->p_rec;
@@ -373,20 +540,57 @@ gd_status gd_evaluator_create(gd_complex *cx, const gd_atoms *reference, const u
   int n_if = 0;
   while (n_if < nu && group(order[n_if]) == 0) ++n_if;
   std::vector<int> u_slot(nu), u_pbeg(n_if + 1, 0);
-  std::vector<D4> u_x0(nu), u_ref(nu), u_iref(n_if), p_rec;
+  std::vector<D4> u_ref(nu), u_iref(n_if), p_rec;
+  std::vector<int4> u_xy(nu, make_int4(0, 0, 0, 0)), u_z(nu, make_int4(0, 0, 0, 0));
+  std::vector<longlong2> u_qxy(nu, longlong2{0, 0});
+  std::vector<long long> u_qz(nu, 0);
+  std::vector<Fix3> u_iq(n_if, Fix3{0, 0, 0, 0});
+  // the fixed-point images, as long as every coordinate is in range
+  bool fixed = std::max({std::fabs(cx->ox), std::fabs(cx->oy), std::fabs(cx->oz)}) < 3000.0;
+  const double whole[3] = {fixed ? std::nearbyint(cx->ox) : 0.0, fixed ? std::nearbyint(cx->oy) : 0.0,
+                           fixed ? std::nearbyint(cx->oz) : 0.0};
+  long long origin[3];
+  for (int k = 0; k < 3; ++k) origin[k] = std::llrint(std::ldexp(whole[k], 51));
+  auto fix_ref = [&](const D4 &v) {
+    if (!(std::fabs(v.x) < 4000.0 && std::fabs(v.y) < 4000.0 && std::fabs(v.z) < 4000.0)) {
+      fixed = false;
+      return Fix3{0, 0, 0, 0};
+    }
+    const Fix3 q{std::llrint(std::ldexp(v.x, 51)) - origin[0], std::llrint(std::ldexp(v.y, 51)) - origin[1],
+                 std::llrint(std::ldexp(v.z, 51)) - origin[2], 0};
+    const long long lim = std::llrint(std::ldexp(kFixFar, 51));
+    fixed = fixed && std::llabs(q.x) < lim && std::llabs(q.y) < lim && std::llabs(q.z) < lim;
+    return q;
+  };
   std::vector<float4> p_rec32;
   p_rec.reserve(n_p);
   p_rec32.reserve(n_p);
   for (int u = 0; u < nu; ++u) {
     const int j = order[u];
     u_slot[u] = cx->h_lig_slot[j];
-    u_x0[u] = D4{cx->h_lx[j] - cx->cx, cx->h_ly[j] - cx->cy, cx->h_lz[j] - cx->cz, 0.0};
+    const double x0[3] = {cx->h_lx[j] - cx->cx, cx->h_ly[j] - cx->cy, cx->h_lz[j] - cx->cz};
+    if (std::fabs(x0[0]) < kFixAtom && std::fabs(x0[1]) < kFixAtom && std::fabs(x0[2]) < kFixAtom) {
+      const Limbs x = limbs(std::llrint(std::ldexp(x0[0], 50))), y = limbs(std::llrint(std::ldexp(x0[1], 50))),
+                  z = limbs(std::llrint(std::ldexp(x0[2], 50)));
+      u_xy[u] = make_int4(x.h, x.l, y.h, y.l);
+      u_z[u] = make_int4(z.h, z.l, 0, 0);
+    } else {
+      fixed = false;
+    }
     u_ref[u] = l_ref[j];
+    if (l_ref[j].w != 0.0) {
+      const Fix3 q = fix_ref(l_ref[j]);
+      u_qxy[u] = longlong2{q.x, q.y};
+      u_qz[u] = q.z;
+      u_z[u].w = 1;
+    }
     if (u >= n_if) continue;
     u_iref[u] = l_iref[j];
-    if (l_ref[j].w != 0.0 && l_iref[j].w != 0.0 && l_ref[j].x == l_iref[j].x && l_ref[j].y == l_iref[j].y &&
-        l_ref[j].z == l_iref[j].z)
-      u_iref[u].w = 2.0;
+    if (l_iref[j].w != 0.0) {
+      u_iq[u] = fix_ref(l_iref[j]);
+      const bool same = l_ref[j].w != 0.0 && l_ref[j].x == l_iref[j].x && l_ref[j].y == l_iref[j].y && l_ref[j].z == l_iref[j].z;
+      u_z[u].w |= same ? 4 : 2;
+    }
     for (int a : l_rec[j]) {
       p_rec.push_back(D4{cx->h_rx[a], cx->h_ry[a], cx->h_rz[a], 0.0});
       p_rec32.push_back(make_float4(static_cast<float>(cx->h_rx[a] - cx->ox), static_cast<float>(cx->h_ry[a] - cx->oy),
@@ -403,6 +607,8 @@ gd_status gd_evaluator_create(gd_complex *cx, const gd_atoms *reference, const u
   ev->n_iref = static_cast<int>(ref_i.size());
   ev->n_native = n_native;
   ev->n_p = n_p;
+  ev->fixed = fixed;
+  std::copy(origin, origin + 3, ev->origin);
   ev->thr5 = make_thresholds(5.0).contact_le;
   const int64_t cnt[GD_EVAL_COUNTS] = {static_cast<int64_t>(rec_if.size()), static_cast<int64_t>(ref_if.size()),
                                        n_native, nu, std::min(nl, nf),
@@ -410,9 +616,9 @@ gd_status gd_evaluator_create(gd_complex *cx, const gd_atoms *reference, const u
   std::copy(cnt, cnt + GD_EVAL_COUNTS, ev->counts);
   auto al = [](size_t b) { return (std::max<size_t>(b, 1) + 255) / 256 * 256; };
   const size_t b_slot = al(sizeof(int) * nu), b_beg = al(sizeof(int) * (n_if + 1)), b_ref = al(sizeof(D4) * nu),
-               b_iref = al(sizeof(D4) * n_if), b_prec = al(sizeof(D4) * p_rec.size()),
+               b_iref = al(sizeof(D4) * n_if), b_x = al(sizeof(int4) * nu), b_qz = al(sizeof(long long) * nu), b_prec = al(sizeof(D4) * p_rec.size()),
                b_prec32 = al(sizeof(float4) * p_rec32.size());
-  ev->bytes = b_slot + b_beg + 2 * b_ref + b_iref + b_prec + b_prec32;
+  ev->bytes = b_slot + b_beg + b_ref + 2 * b_iref + 3 * b_x + b_qz + b_prec + b_prec32;
   gd_status s = dev_alloc(ctx, ev->bytes, &ev->block);
   if (s != GD_OK) {
     delete ev;
@@ -428,7 +634,11 @@ gd_status gd_evaluator_create(gd_complex *cx, const gd_atoms *reference, const u
   };
   ev->u_slot = reinterpret_cast<const int *>(put(u_slot.data(), sizeof(int) * nu, b_slot));
   ev->u_pbeg = reinterpret_cast<const int *>(put(u_pbeg.data(), sizeof(int) * (n_if + 1), b_beg));
-  ev->u_x0 = reinterpret_cast<const D4 *>(put(u_x0.data(), sizeof(D4) * nu, b_ref));
+  ev->u_xy = reinterpret_cast<const int4 *>(put(u_xy.data(), sizeof(int4) * nu, b_x));
+  ev->u_z = reinterpret_cast<const int4 *>(put(u_z.data(), sizeof(int4) * nu, b_x));
+  ev->u_qxy = reinterpret_cast<const longlong2 *>(put(u_qxy.data(), sizeof(longlong2) * nu, b_x));
+  ev->u_qz = reinterpret_cast<const long long *>(put(u_qz.data(), sizeof(long long) * nu, b_qz));
+  ev->u_iq = reinterpret_cast<const Fix3 *>(put(u_iq.data(), sizeof(Fix3) * n_if, b_iref));
   ev->u_ref = reinterpret_cast<const D4 *>(put(u_ref.data(), sizeof(D4) * nu, b_ref));
   ev->u_iref = reinterpret_cast<const D4 *>(put(u_iref.data(), sizeof(D4) * n_if, b_iref));
   ev->p_rec = reinterpret_cast<const D4 *>(put(p_rec.data(), sizeof(D4) * p_rec.size(), b_prec));
