@@ -103,6 +103,21 @@ static __device__ __forceinline__ double exact_d2(double ax, double ay, double a
   return __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
 }
 
+// Ligand coordinates relative to the FP32 origin O, in FP64, as the FP32 images
+// are rounded from: one chain of multiply-adds on the precomputed offset from
+// the rotation centre, 9 FP64 operations in place of the 31 of the reference's
+// order, from which it differs by some 1e-15 A (decisions inside the guard
+// bands take the exact coordinates).  FP64 issues at 1/64 of the FP32 rate, and
+// with receptor parts every part's item moves its ligand atoms: 150 poses of
+// 1,074 x 741 atoms apart from each other took 147 us, 58 of them the FP64
+// pipe's; with this and without the items that have no segment in reach, 97 us.
+static __device__ __forceinline__ void relative_atom(const ScoreParams &p, const gd_pose_frame &f, const D4 &r, double &x,
+                                                     double &y, double &z) {
+  const double tx = (p.cx + f.dx) - p.ox, ty = (p.cy + f.dy) - p.oy, tz = (p.cz + f.dz) - p.oz;
+  x = __fma_rn(f.ca * f.cb, r.x, __fma_rn(f.m01, r.y, __fma_rn(f.m02, r.z, tx)));
+  y = __fma_rn(f.sa * f.cb, r.x, __fma_rn(f.m11, r.y, __fma_rn(f.m12, r.z, ty)));
+  z = __fma_rn(-f.sb, r.x, __fma_rn(f.cb * f.sg, r.y, __fma_rn(f.cb * f.cg, r.z, tz)));
+}
 static __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
@@ -129,6 +144,30 @@ struct ExactSum {
     const unsigned __int128 t = sh >= 0 ? static_cast<unsigned __int128>(m) << sh
                                         : static_cast<unsigned __int128>(m >> min(-sh, 63));
     v += static_cast<long long>(b) < 0 ? -static_cast<__int128>(t) : static_cast<__int128>(t);
+  }
+  // The same for the usual term, of 2^(53 - bits) to 2^(117 - bits), in some
+  // two dozen instructions: the significand shifted by less than 64, two's
+  // complement by the sign, one carry chain.
+  __device__ __forceinline__ void add_term(double x, int bits) {
+    const unsigned lo = static_cast<unsigned>(__double2loint(x)), hi = static_cast<unsigned>(__double2hiint(x));
+    const int sh = static_cast<int>(hi << 1 >> 21) - 1075 + bits;
+    if (static_cast<unsigned>(sh) < 64u) {
+      const unsigned mh = (hi & 0xfffffu) | 0x100000u, g = static_cast<unsigned>(static_cast<int>(hi) >> 31);
+      const unsigned w0 = lo << (sh & 31), w1 = __funnelshift_l(lo, mh, sh), w2 = __funnelshift_l(mh, 0u, sh);
+      const bool up = (sh & 32) != 0;
+      const unsigned t0 = (up ? 0u : w0) ^ g, t1 = (up ? w0 : w1) ^ g, t2 = (up ? w1 : w2) ^ g, t3 = (up ? w2 : 0u) ^ g;
+      unsigned a0 = static_cast<unsigned>(v), a1 = static_cast<unsigned>(static_cast<unsigned __int128>(v) >> 32),
+               a2 = static_cast<unsigned>(static_cast<unsigned __int128>(v) >> 64),
+               a3 = static_cast<unsigned>(static_cast<unsigned __int128>(v) >> 96);
+      asm("{\n\t.reg .u32 c;\n\tadd.cc.u32 c, %8, %8;\n\taddc.cc.u32 %0, %0, %4;\n\taddc.cc.u32 %1, %1, %5;\n\t"
+          "addc.cc.u32 %2, %2, %6;\n\taddc.u32 %3, %3, %7;\n\t}"
+          : "+r"(a0), "+r"(a1), "+r"(a2), "+r"(a3)
+          : "r"(t0), "r"(t1), "r"(t2), "r"(t3), "r"(g));
+      v = static_cast<__int128>(static_cast<unsigned __int128>(static_cast<unsigned long long>(a3) << 32 | a2) << 64 |
+                                (static_cast<unsigned long long>(a1) << 32 | a0));
+    } else if ((lo | hi << 1) != 0u) {
+      add(x, bits);
+    }
   }
   // every lane: the sum over the warp
   __device__ __forceinline__ void warp_total() {

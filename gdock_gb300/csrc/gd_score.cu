@@ -10,19 +10,21 @@
 //   1. The ligand's atoms are moved in FP64 with the reference's operation
 //      order (coordinates bit-identical to gdock's) into shared memory, each
 //      CTA of the cluster a share, the others copied from its shared memory.
-//   2. Work units of one 32-atom ligand slot x a run of receptor atoms are taken by the cluster's warps from one counter.  A unit finds
-//      its pairs within reach in FP32 (bounding spheres of the slot and of the
-//      receptor segments, then each pair's distance, all with the FP32 guard
-//      band added, so that only pairs whose every term is exactly zero are
-//      dropped) and lists them in shared memory; every 32 listed pairs are
-//      evaluated in FP64, one per lane: near pairs (within 12 A) every term,
-//      far ones Coulomb only.  Decisions are exact: the squared distance's
-//      high word settles them, and pairs next to a cutoff are decided on d2
-//      in the reference's operation order against the exact thresholds.
+//   2. Work units of one 32-atom ligand slot x a run of receptor atoms are
+//      taken by the cluster's warps from one counter.  A unit finds its pairs
+//      within reach in FP32 (bounding spheres of the slot and of the receptor
+//      segments, then each pair's distance, all with the FP32 guard band
+//      added, so that only pairs whose every term is exactly zero are dropped)
+//      and lists them in shared memory; every 32 listed pairs are evaluated to
+//      FP64 accuracy, one per lane: near pairs (within 12 A) every term, far
+//      ones Coulomb only.  Distances and reciprocals are formed in integers,
+//      which issue beside the slow FP64 pipe.  Decisions are exact: the squared
+//      distance's high word settles them, and pairs next to a cutoff are
+//      decided on d2 in the reference's operation order against the exact
+//      thresholds.
 //   3. Every term is added as a 128-bit fixed-point integer.  Integer sums are
 //      exact, so the energies do not depend on which lane, warp or CTA took
-//      which pair, nor on the launch's other poses; the integer adds issue
-//      beside the FP64 pipe, which is the bound.
+//      which pair, nor on the launch's other poses.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -40,13 +42,14 @@ constexpr int kNW = kNT / 32;
 constexpr int kLigBits = 10;
 constexpr int kLigCap = 1 << kLigBits;  // ligand atoms held in shared memory at once (longer ligands: in turns)
 constexpr int kRows = 4;              // rows searched per step
+constexpr int kRowBuf = 32 + kRows;   // rows waiting per warp: fewer than a step and 32 more
 constexpr int kQueue = 32 * (kRows + 1);  // listed pairs per warp and kind: 31 left over + 32 of each row
 constexpr int kRowsMin = 8, kRowsMax = 128;  // receptor atoms of a unit (a power of two)
 constexpr int kMaxCluster = 16;
 constexpr int kTinyHi = 0x2b000000;   // high word of 2^-335: below it r^6 may underflow
 
 struct F64Smem {
-  size_t x, y, z, q, fx, fy, fz, lt, sph, rcnt, lcnt, queue, red, nf, frame, misc, total;
+  size_t x, y, z, q, fx, fy, fz, lt, sph, rcnt, lcnt, queue, row, red, nf, frame, misc, total;
 };
 
 __host__ __device__ inline F64Smem f64_smem(int nr, int nl) {
@@ -70,6 +73,7 @@ __host__ __device__ inline F64Smem f64_smem(int nr, int nl) {
   L.rcnt = take(2 * (static_cast<size_t>(nr) + 1));  // 16-bit burial counts, two a word
   L.lcnt = take(2 * (static_cast<size_t>(nl) + 1));
   L.queue = take(2 * sizeof(uint32_t) * kQueue * kNW);
+  L.row = take(sizeof(float4) * kRowBuf * kNW);
   L.red = take(3 * sizeof(__int128) * kNW);
   L.nf = take(3 * sizeof(double) * kNW);
   L.frame = take(sizeof(gd_pose_frame));
@@ -90,6 +94,30 @@ __device__ __forceinline__ double rcp64(double d) {
   e = __fma_rn(e, e, e);
   return __fma_rn(x, e, x);
 }
+
+// 1/d in integers, for normal d from 2^-1022 to 2^1021: with the significand
+// M / 2^53 and the hardware's FP32 approximation Y / 2^23 of its reciprocal, the
+// residual E = 2^76 - M Y is exact modulo 2^64 (it is below 2^55), and the
+// reciprocal is Y (1 + e + e^2 + ...) with e = E / 2^76 below 2^-21, formed to
+// 2^-57 and rounded once (0.51 units in the last place).  Some 33 integer
+// instructions beside the FP64 pipe, in place of three on it.
+__device__ __forceinline__ double rcp_int(double d) {
+  const unsigned lo = static_cast<unsigned>(__double2loint(d)), hi = static_cast<unsigned>(__double2hiint(d));
+  const unsigned mh = (hi & 0xfffffu) | 0x100000u;
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint_as_float(__funnelshift_l(lo, mh, 3) + 0x3e800000u)));
+  const unsigned Y = min(__float_as_uint(y) - 0x3f000000u, 0xffffffu);
+  const long long E = -static_cast<long long>(static_cast<unsigned long long>(lo) * Y + (static_cast<unsigned long long>(mh * Y) << 32));
+  const int eh = static_cast<int>(E >> 31);
+  const unsigned el = static_cast<unsigned>(E >> 7) & 0xffffffu;
+  const long long t = static_cast<long long>(eh) * static_cast<int>(Y) + __umulhi(Y << 8, el);
+  const int s = eh >> 8;
+  const unsigned q = __umulhi(static_cast<unsigned>(s * s), Y << 8) >> 11;
+  const unsigned long long V = (static_cast<unsigned long long>(Y) << 39) + (t >> 6) + q;
+  return __longlong_as_double(static_cast<long long>(((V + 512) >> 10) + (static_cast<unsigned long long>(2044 - (hi >> 20)) << 52)));
+}
+// ... and for any other d (infinite, undefined, next to the range's ends)
+__device__ __noinline__ double rcp_rare(double d) { return rcp64(d); }
 
 // min(count, 10) is all that is read: a count that has reached 10 is left
 // alone, which also keeps the 16 bits from overflowing (at most 10 + one
@@ -221,25 +249,31 @@ struct PairEval {
         // softcore_lj_potential (src/fitness.rs:57-70) as 4 eps (x^2 - x) with
         // x = 1 / (r^6 2/R6 + 1), half the reference's ratio
         const double2 tp = __ldg(reinterpret_cast<const double2 *>(p.tab64) + m.x + lt[k]);
-        const double u = rcp64(__fma_rn(d2 * d2 * d2, tp.x, 1.0));
+        const double w = __fma_rn(d2 * d2 * d2, tp.x, 1.0);
+        const double u = static_cast<unsigned>(__double2hiint(w)) < 0x7fc00000u ? rcp_int(w) : rcp_rare(w);
         double v = tp.y * __fma_rn(u, u, -u);
         if (CLAMP) v = v < -50.0 ? -50.0 : (v > 500.0 ? 500.0 : v);
-        vdw.add(v, p.fx_vdw);
+        vdw.add_term(v, p.fx_vdw);
       }
     }
     // elec_energy term (src/fitness.rs:296) without its constant, which
     // multiplies the pose's sum
-    if (pe) elec.add(rq * q[k] * rcp64(d2), p.fx_elec);
+    if (pe) elec.add_term(rq * q[k] * rcp_int(d2), p.fx_elec);
   }
 };
 
-// What bounds it: the FP64 pipe, two lanes' operations per clock and SM.  The
-// form that evaluated every pair spent about 35 of them on each pair, though
-// only 13 % of the pairs of a scan have a term; a listed pair costs 18 (near)
-// or 11 (far), and the FP32 search runs beside the FP64 pipe; d2 from integers
-// takes another 6 off.  On receptors of 2,538 and ligands of 1,280 atoms: 2,048
-// poses 348 -> 28.7 -> 18.0 ms (every pair; listed pairs; integers), 150 poses
-// 29.0 -> 2.38 -> 1.72 ms; one pose of 411 x 649 atoms 1,746 -> 89 -> 75 us a call.
+// What bounds it: the FP64 pipe (two lanes' operations per clock and SM; 55 %
+// busy) and instruction issue (63 %), at the 24 warps an SM that the registers
+// allow.  The form that evaluated every pair spent about 35 FP64 operations on
+// each pair, though only 13 % of the pairs of a scan have a term; a listed pair
+// cost 18 (near) or 11 (far), 6 fewer with d2 from integers, and with the
+// reciprocals in integers too it is 7 or 2.  The FP32 search takes some 25
+// instructions a row of 32 pairs: rows wait in shared memory as position and
+// list entry, and two of five of its pairs are listed.  On receptors of 2,538
+// and ligands of 1,280 atoms: 2,048 poses 348 -> 28.7 -> 18.7 -> 12.4 ms (every
+// pair; listed pairs; d2 from integers; reciprocals, short sums, row buffer), 150
+// poses 29.0 -> 2.38 -> 1.72 -> 1.40 ms; one pose of 411 x 649 atoms 1,746 -> 89
+// -> 53 us a call.
 template <bool FIX, bool SERIAL, bool CLAMP>
 __global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const int unit_rows) {
   if (p.skip && *p.skip) return;
@@ -264,6 +298,7 @@ __global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned lt_mask = (1u << lane) - 1u;
   uint32_t *q_near = reinterpret_cast<uint32_t *>(smem + L.queue) + warp * 2 * kQueue, *q_far = q_near + kQueue;
+  float4 *s_row = reinterpret_cast<float4 *>(smem + L.row) + warp * kRowBuf;
 
   if (!p.models && tid < 16)
     reinterpret_cast<double *>(s_frame)[tid] = reinterpret_cast<const double *>(p.frames + pose)[tid];
@@ -312,7 +347,8 @@ __global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const
         s_fy[k] = fy;
         s_fz[k] = fz;
       }
-      // a sphere around the slot: centre of its bounding box, farthest atom
+      // a sphere around the slot: the precomputed smallest one moved with the
+      // pose, else the bounding box's centre and farthest atom
       float lo[3] = {on ? fx : 3.0e38f, on ? fy : 3.0e38f, on ? fz : 3.0e38f},
             hi[3] = {on ? fx : -3.0e38f, on ? fy : -3.0e38f, on ? fz : -3.0e38f};
 #pragma unroll
@@ -327,7 +363,17 @@ __global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const
       const bool odd = __any_sync(kFull, !(rr < 3.0e38f));  // not finite: a sphere that keeps everything
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) rr = fmaxf(rr, __shfl_xor_sync(kFull, rr, o));
-      if (lane == 0) s_sph[s] = make_float4(cx, cy, cz, odd ? INFINITY : rr * 1.0001f + 0.01f);
+      if (lane == 0) {
+        float4 sp = make_float4(cx, cy, cz, odd ? INFINITY : rr * 1.0001f + 0.01f);
+        if (!p.models && !odd) {
+          const D4 v = p.lig_slot_sph[(l0 >> 5) + s];
+          double x, y, z;
+          relative_atom(p, f, v, x, y, z);
+          const float r = static_cast<float>(v.w) * 1.0001f + 0.01f;
+          if (r < sp.w) sp = make_float4(static_cast<float>(x), static_cast<float>(y), static_cast<float>(z), r);
+        }
+        s_sph[s] = sp;
+      }
     }
     for (int k = tid; k < nl; k += kNT) {
       int t = p.lig_type[l0 + k];
@@ -369,54 +415,74 @@ __global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const
       const float lx = on ? s_fx[k] : 0.0f, ly = on ? s_fy[k] : 0.0f, lz = on ? s_fz[k] : 0.0f;
       const float4 sp = s_sph[slot];
       const float lim_s = sp.w + reach, lim_s2 = lim_s * lim_s;
+      int nrow = 0;  // rows waiting
+      // kRows waiting rows (n of them real) against the lane's atom: their
+      // loads, distances and votes overlap
+      auto step = [&](int at, int n) {
+        float4 r[kRows];
+        float d2[kRows];
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) r[i] = s_row[at + i];
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) d2[i] = d2f(r[i], lx, ly, lz);
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) {
+          const bool reached = on && i < n && !(d2[i] > lim_e), close = reached && !(d2[i] > lim_v);
+          const unsigned Mn = __ballot_sync(kFull, close), Mf = __ballot_sync(kFull, reached && !close);
+          const int to = (close ? nn : kQueue + nf) + __popc((close ? Mn : Mf) & lt_mask);
+          if (reached) q_near[to] = __float_as_uint(r[i].w) | static_cast<uint32_t>(k);
+          nn += __popc(Mn);
+          nf += __popc(Mf);
+        }
+        if (nn >= 32 || nf >= 32) {
+          __syncwarp();
+          for (; nn >= 32; nn -= 32) ev.template eval<true>(true, q_near[nn - 32 + lane], vdw, elec);
+          for (; nf >= 32; nf -= 32) ev.template eval<false>(true, q_far[nf - 32 + lane], vdw, elec);
+          __syncwarp();
+        }
+      };
 #pragma unroll 1
-      for (int a0 = r0 & ~31; a0 < r1; a0 += 32) {
-        {
-          const float4 sg = __ldg(&p.rec_seg[a0 / kRecSeg]);
-          const float dx = sg.x - sp.x, dy = sg.y - sp.y, dz = sg.z - sp.z;
-          const float lim = sg.w + sp.w + reach + 0.1f + 1e-3f * (sg.w + sp.w);
-          if (dx * dx + dy * dy + dz * dz > lim * lim) {
-            a0 |= 32;  // the segment's second half too
-            continue;
+      for (int a0 = r0 & ~31;; a0 += 32) {
+        const bool last = a0 >= r1;
+        if (!last) {
+          {
+            const float4 sg = __ldg(&p.rec_seg[a0 / kRecSeg]);
+            const float dx = sg.x - sp.x, dy = sg.y - sp.y, dz = sg.z - sp.z;
+            const float lim = sg.w + sp.w + reach + 0.1f + 1e-3f * (sg.w + sp.w);
+            if (dx * dx + dy * dy + dz * dz > lim * lim) {
+              a0 |= 32;  // the segment's second half too
+              continue;
+            }
           }
+          // rows: receptor atoms within reach of the slot's sphere
+          bool keep = a0 + lane >= r0 && a0 + lane < r1;
+          float4 r = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          if (keep) {
+            r = __ldg(&p.rec_pos32[a0 + lane]);
+            const float dx = r.x - sp.x, dy = r.y - sp.y, dz = r.z - sp.z;
+            keep = !(dx * dx + dy * dy + dz * dz > lim_s2);
+          }
+          const unsigned rows = __ballot_sync(kFull, keep);
+          if (keep) {
+            r.w = __uint_as_float(static_cast<uint32_t>(a0 + lane) << kLigBits);
+            s_row[nrow + __popc(rows & lt_mask)] = r;
+          }
+          nrow += __popc(rows);
+          __syncwarp();
         }
-        // rows: receptor atoms within reach of the slot's sphere
-        bool keep = a0 + lane >= r0 && a0 + lane < r1;
-        if (keep) {
-          const float4 r = __ldg(&p.rec_pos32[a0 + lane]);
-          const float dx = r.x - sp.x, dy = r.y - sp.y, dz = r.z - sp.z;
-          keep = !(dx * dx + dy * dy + dz * dz > lim_s2);
+        int at = 0;
+        for (; at + kRows <= nrow; at += kRows) step(at, kRows);
+        if (last) {
+          if (at < nrow) step(at, nrow - at);
+          break;
         }
-        unsigned rows = __ballot_sync(kFull, keep);
-        // kRows rows a step (past the last: a row that lists nothing), so that
-        // their loads and votes overlap
-        while (rows) {
-          int a[kRows];
-          float d2[kRows];
-#pragma unroll
-          for (int i = 0; i < kRows; ++i) {
-            a[i] = rows ? a0 + __ffs(rows) - 1 : -1;
-            rows &= rows - 1;
-            d2[i] = d2f(__ldg(&p.rec_pos32[max(a[i], a0)]), lx, ly, lz);
-          }
-#pragma unroll
-          for (int i = 0; i < kRows; ++i) {
-            const bool reached = on && a[i] >= 0 && !(d2[i] > lim_e), close = reached && !(d2[i] > lim_v);
-            const unsigned Mn = __ballot_sync(kFull, close), Mf = __ballot_sync(kFull, reached && !close);
-            const uint32_t e = static_cast<uint32_t>(a[i]) << kLigBits | static_cast<uint32_t>(k);
-            if (close) q_near[nn + __popc(Mn & lt_mask)] = e;
-            else if (reached) q_far[nf + __popc(Mf & lt_mask)] = e;
-            nn += __popc(Mn);
-            nf += __popc(Mf);
-          }
-          if (nn >= 32 || nf >= 32) {
-            __syncwarp();
-            for (; nn >= 32; nn -= 32) ev.template eval<true>(true, q_near[nn - 32 + lane], vdw, elec);
-            for (; nf >= 32; nf -= 32) ev.template eval<false>(true, q_far[nf - 32 + lane], vdw, elec);
-            __syncwarp();
-          }
+        if (at > 0) {  // fewer than a step are left
+          nrow -= at;
+          __syncwarp();
+          if (lane < nrow) s_row[lane] = s_row[at + lane];
         }
       }
+      __syncwarp();
     }
     // the rest of both lists, together when they fit one round (the near
     // evaluation decides every term itself)
@@ -501,17 +567,18 @@ cudaError_t launch_f64(Kern kern, const ScoreParams &p, int sm_count, cudaStream
   // CTAs per pose: the more the fewer poses there are, as far as the pose's
   // rows (receptor atom x ligand slot) go round.  Poses differ widely in work,
   // so splitting them pays beyond the point where they fill the SMs, the less
-  // so the more CTAs a cluster must find places for at once.  Measured on
-  // 2,538 x 1,280 atoms, us at 1 / 2 / 4 / 8 / 16 CTAs: 40 poses 3695 / 1937 /
-  // 1028 / 657 / 640, 300 poses 4930 / 3879 / 3312 / 3150 / 3786, 1,200 poses
-  // 12547 / 11307 / 11067 / 11648 / 14676; on 411 x 649 atoms 2,400 poses 3242 /
-  // 3062 / 3265 / 3809 / 5719, 9,600 poses 10759 / 10954 / 12225 / 14601 / 22295.
+  // so the more CTAs a cluster must find places for at once.  Measured (the
+  // call), us at 1 / 2 / 4 / 8 / 16 CTAs: 2,538 x 1,280 atoms, 40 poses 2714 /
+  // 1461 / 776 / 495 / 529, 300 poses 3515 / 2811 / 2414 / 2382 / 3169, 1,200
+  // poses 8544 / 7867 / 7850 / 8810 / 12327; 411 x 649 atoms, 2,400 poses 2165 /
+  // 2244 / 2648 / 3216 / 5165, 9,600 poses 7189 / 7996 / 9966 / 12375 / 20207;
+  // 253 x 170 atoms, one pose 69 / 53 / 42 / 40 / 39.
   const long long rows = static_cast<long long>(std::max(1, (std::min(p.nl, kLigCap) + 31) / 32)) * std::max(1, p.nr);
   constexpr int kPerSm[] = {64, 32, 16, 4};  // CTAs per SM up to which poses are split in 2, 4, 8, 16
   int nc = 1;
   for (int k = 0; k < 4 && nc < kMaxCluster; ++k)
     if (static_cast<long long>(p.n_poses) * (2 << k) <= static_cast<long long>(kPerSm[k]) * sm_count &&
-        rows > 64 * kNW * (2 << k))
+        rows > 16 * kNW * (2 << k))
       nc = 2 << k;
   // rows per unit: 32 units or more for every warp, so that the last ones
   // leave few warps waiting (8 to 128 units a warp made no difference)

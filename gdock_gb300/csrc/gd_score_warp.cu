@@ -225,21 +225,6 @@ __device__ __forceinline__ bool near_band(float d2, float gv, float ge, float gd
   return (fabsf(__fsub_rn(fabsf(te), 112.0f)) < ge) | (fabsf(tv) < gv) | (fabsf(__fsub_rn(d2, 64.0f)) < gdd);
 }
 
-// Ligand coordinates relative to the FP32 origin O, in FP64, as the FP32 images
-// are rounded from: one chain of multiply-adds on the precomputed offset from
-// the rotation centre, 9 FP64 operations in place of the 31 of the reference's
-// order, from which it differs by some 1e-15 A (decisions inside the guard
-// bands take the exact coordinates).  FP64 issues at 1/64 of the FP32 rate, and
-// with receptor parts every part's item moves its ligand atoms: 150 poses of
-// 1,074 x 741 atoms apart from each other took 147 us, 58 of them the FP64
-// pipe's; with this and without the items that have no segment in reach, 97 us.
-__device__ __forceinline__ void relative_atom(const ScoreParams &p, const gd_pose_frame &f, const D4 &r, double &x,
-                                              double &y, double &z) {
-  const double tx = (p.cx + f.dx) - p.ox, ty = (p.cy + f.dy) - p.oy, tz = (p.cz + f.dz) - p.oz;
-  x = __fma_rn(f.ca * f.cb, r.x, __fma_rn(f.m01, r.y, __fma_rn(f.m02, r.z, tx)));
-  y = __fma_rn(f.sa * f.cb, r.x, __fma_rn(f.m11, r.y, __fma_rn(f.m12, r.z, ty)));
-  z = __fma_rn(-f.sb, r.x, __fma_rn(f.cb * f.sg, r.y, __fma_rn(f.cb * f.cg, r.z, tz)));
-}
 __device__ __forceinline__ float3 atom32(const ScoreParams &p, const gd_pose_frame &f, int pose, int j) {
   double x, y, z;
   if (p.models) {
