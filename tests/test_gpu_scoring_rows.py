@@ -68,3 +68,22 @@ def test_automatic_receptor_parts(rec, lig, n):
     finally:
         cx.close()
         ctx.close()
+
+
+@pytest.mark.parametrize("rec,lig,n", [(12, 20, 1), (40, 60, 33), (300, 60, 1), (120, 60, 1500)])
+def test_shared_serials_in_chunks(oracle, rec, lig, n):
+    """Receptor and ligand numbered from 1: the split kernels for equal serials
+    give the whole-pose kernel's energies, and the oracle's."""
+    c = synth.make_complex(rec, lig, 4, seed=rec + n, overlap_serials=True)
+    L = gd.position_ligand(c.receptor, c.ligand)
+    genes = synth.quaternion_genes(np.random.default_rng(n), n, half_box=15.0)
+    ctx = gd.Context(0)
+    cx = gd.Complex(c.receptor, L, c.restraint_pairs, ctx=ctx)
+    try:
+        auto = cx.score_poses(genes, gd.GD_PREC_F32)
+        check(auto[:8], oracle.score_poses(c.receptor, L, c.restraint_pairs, genes[:8]), F32_TOL)
+        ctx.set_tuning(_lib.GD_TUNE_SPLIT, 1)
+        assert cx.score_poses(genes, gd.GD_PREC_F32).tobytes() == auto.tobytes()
+    finally:
+        cx.close()
+        ctx.close()
