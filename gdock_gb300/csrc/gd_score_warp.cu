@@ -86,6 +86,7 @@ struct BatchParams {
   int split;
   const long long *pose_start;    // first batch-wide pose index of each complex
   int max_chunks;                 // partial slots per pose (chunks x rparts)
+  double2 *air;                   // [pose] restraint energy and satisfied restraints (rparts > 1)
   double *part;                   // [pose][chunk * rparts + part][vdw, elec (fixed point), ligand desolvation][32 lanes]
   unsigned *pcount;               // [pose][(max_nr + 1) / 2] receptor burial counts, two 16-bit counts a word
   int *pdone;                     // [pose] items finished
@@ -786,6 +787,16 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_score_f32w(const BatchPar
         reinterpret_cast<long long *>(pt)[lane] = fv;
         reinterpret_cast<long long *>(pt)[32 + lane] = fe;
         pt[64 + lane] = dch;
+        if (SPLIT == 2 && rem == 0) {
+          // with receptor parts the pose's first item adds its restraint
+          // energy, beside other items' pairs and not at the end of the launch
+          // (one pose of 2,538 x 1,280 atoms 95 -> 91 us; 65,536 in chunks
+          // alone were 0.8 % slower with it)
+          double air;
+          int sat;
+          warp_air(p, f, pose, lane, air, sat);
+          if (lane == 0) bp.air[gp] = make_double2(air, static_cast<double>(sat));
+        }
       } else {
         vdw_i += fv;
         elec_i += fe;
@@ -811,48 +822,94 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_score_f32w(const BatchPar
       done = __shfl_sync(kFull, done, 0);
       if (done != per_pose - 1) continue;
       __threadfence();
-      for (int c = 0; c < per_pose; ++c) {
-        const long long *pi =
-            reinterpret_cast<const long long *>(bp.part + (static_cast<size_t>(gp) * bp.max_chunks + c) * 96);
-        vdw_i += __ldcg(pi + lane);
-        elec_i += __ldcg(pi + 32 + lane);
-      }
-      // ligand desolvation chunk by chunk, in the same order and arithmetic
-      // as whole-pose items
-      for (int c = 0; c < nchunks; ++c) {
-        if (R == 1) {
-          desolv_t += __ldcg(bp.part + (static_cast<size_t>(gp) * bp.max_chunks + c) * 96 + 64 + lane);
-        } else {
-          double dc = 0.0, t[S];
+      if constexpr (SPLIT == 2) {
+        // every loop here waits for L2 once or twice per round; with receptor
+        // parts (launches of few poses) nothing runs beside the last poses'
+        // rounds, so theirs hold more loads: one pose of 6,800 x 2,500 atoms 151 ->
+        // 139 us.  The sums keep their order.
+        constexpr int kP = 8, kC = 3, kR = 16;
+        const double *pose_part = bp.part + static_cast<size_t>(gp) * bp.max_chunks * 96;
+        for (int c0 = 0; c0 < per_pose; c0 += kP) {
+          long long v[kP], e[kP];
 #pragma unroll
-          for (int s = 0; s < S; ++s) {
-            const int j = c * kChunk + s * 32 + lane;
-            t[s] = 0.0;
-            if (j < p.nl) {
-              const unsigned n = __ldcg(&bp.lcount[static_cast<size_t>(gp) * bp.max_nl + j]);
-              t[s] = p.lig_desolv[static_cast<size_t>(j) * 11 + (n < 10u ? n : 10u)];
+          for (int u = 0; u < kP; ++u) {
+            const long long *pi = reinterpret_cast<const long long *>(pose_part + min(c0 + u, per_pose - 1) * 96);
+            v[u] = __ldcg(pi + lane);
+            e[u] = __ldcg(pi + 32 + lane);
+          }
+#pragma unroll
+          for (int u = 0; u < kP; ++u) {
+            if (c0 + u < per_pose) {
+              vdw_i += v[u];
+              elec_i += e[u];
+            }
+          }
+        }
+        // ligand desolvation chunk by chunk, in the same order and arithmetic
+        // as whole-pose items
+        for (int c0 = 0; c0 < nchunks; c0 += kC) {
+          unsigned n[kC * S];
+          double t[kC * S];
+#pragma unroll
+          for (int u = 0; u < kC * S; ++u) {
+            const int j = c0 * kChunk + u * 32 + lane;
+            n[u] = j < p.nl ? __ldcg(&bp.lcount[static_cast<size_t>(gp) * bp.max_nl + j]) : 0u;
+          }
+#pragma unroll
+          for (int u = 0; u < kC * S; ++u) {
+            const int j = c0 * kChunk + u * 32 + lane;
+            t[u] = j < p.nl ? p.lig_desolv[static_cast<size_t>(j) * 11 + (n[u] < 10u ? n[u] : 10u)] : 0.0;
+          }
+#pragma unroll
+          for (int u = 0; u < kC; ++u) {
+            double dc = 0.0;
+#pragma unroll
+            for (int s = 0; s < S; ++s) dc += t[u * S + s];
+            if (c0 + u < nchunks) desolv_t += dc;
+          }
+        }
+        for (int i0 = 0; i0 < p.nr; i0 += 32 * kR) {
+          unsigned w[kR];
+          double t[kR];
+#pragma unroll
+          for (int u = 0; u < kR; ++u) {
+            const int i = i0 + u * 32 + lane;
+            w[u] = i < p.nr ? __ldcg(&bp.pcount[static_cast<size_t>(gp) * ((bp.max_nr + 1) >> 1) + (i >> 1)]) : 0u;
+          }
+#pragma unroll
+          for (int u = 0; u < kR; ++u) {
+            const int i = i0 + u * 32 + lane;
+            const unsigned c = (w[u] >> ((lane & 1) * 16)) & 0xffffu;
+            t[u] = i < p.nr ? p.rec_desolv[static_cast<size_t>(i) * 11 + (c < 10u ? c : 10u)] : 0.0;
+          }
+#pragma unroll
+          for (int u = 0; u < kR; ++u) desolv_t += t[u];
+        }
+      } else {
+        for (int c = 0; c < per_pose; ++c) {
+          const long long *pi =
+              reinterpret_cast<const long long *>(bp.part + (static_cast<size_t>(gp) * bp.max_chunks + c) * 96);
+          vdw_i += __ldcg(pi + lane);
+          elec_i += __ldcg(pi + 32 + lane);
+        }
+        for (int c = 0; c < nchunks; ++c)
+          desolv_t += __ldcg(bp.part + (static_cast<size_t>(gp) * bp.max_chunks + c) * 96 + 64 + lane);
+        // four rounds' loads in flight, added in order
+        for (int i0 = 0; i0 < p.nr; i0 += 128) {
+          double t[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int i = i0 + u * 32 + lane;
+            t[u] = 0.0;
+            if (i < p.nr) {
+              const unsigned w = __ldcg(&bp.pcount[static_cast<size_t>(gp) * ((bp.max_nr + 1) >> 1) + (i >> 1)]);
+              const unsigned c = (w >> ((i & 1) * 16)) & 0xffffu;
+              t[u] = p.rec_desolv[static_cast<size_t>(i) * 11 + (c < 10u ? c : 10u)];
             }
           }
 #pragma unroll
-          for (int s = 0; s < S; ++s) dc += t[s];
-          desolv_t += dc;
+          for (int u = 0; u < 4; ++u) desolv_t += t[u];
         }
-      }
-      // four rounds' loads in flight, added in order
-      for (int i0 = 0; i0 < p.nr; i0 += 128) {
-        double t[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int i = i0 + u * 32 + lane;
-          t[u] = 0.0;
-          if (i < p.nr) {
-            const unsigned w = __ldcg(&bp.pcount[static_cast<size_t>(gp) * ((bp.max_nr + 1) >> 1) + (i >> 1)]);
-            const unsigned c = (w >> ((i & 1) * 16)) & 0xffffu;
-            t[u] = p.rec_desolv[static_cast<size_t>(i) * 11 + (c < 10u ? c : 10u)];
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) desolv_t += t[u];
       }
     } else {
       // receptor burial -> desolvation; reset the counters for the next item
@@ -867,7 +924,13 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_score_f32w(const BatchPar
     desolv_t = warp_sum(desolv_t);
     double air;
     int sat;
-    warp_air(p, f, pose, lane, air, sat);
+    if (SPLIT == 2) {
+      const double2 a = __ldcg(&bp.air[gp]);
+      air = a.x;
+      sat = static_cast<int>(a.y);
+    } else {
+      warp_air(p, f, pose, lane, air, sat);
+    }
     if (lane == 0) write_pose(p, pose, vdw_t, elec_t, desolv_t, air, sat);
     __syncwarp();
   }
@@ -954,7 +1017,7 @@ struct BatchPlan {
   std::vector<long long> pose_start;  // pose prefix per complex
   int split = 0, max_chunks = 1;
   int rparts = 1, max_nl = 0;  // receptor parts per chunk (split mode), longest ligand
-  size_t part_b = 0, cnt_b = 0, done_b = 0, lcnt_b = 0;  // split-mode scratch
+  size_t part_b = 0, cnt_b = 0, done_b = 0, lcnt_b = 0, air_b = 0;  // split-mode scratch
 };
 
 constexpr size_t kSplitScratchMax = size_t(4) << 30;  // split scratch beyond this: whole poses
@@ -1037,7 +1100,8 @@ static gd_status plan_batch(gd_context *ctx, const std::vector<ScoreParams> &des
     *part_b = static_cast<size_t>(poses) * pl->max_chunks * r * 96 * sizeof(double);
     *cnt_b = static_cast<size_t>(poses) * ((pl->max_nr + 1) / 2) * sizeof(unsigned);
     *lcnt_b = r > 1 ? static_cast<size_t>(poses) * std::max(pl->max_nl, 1) * sizeof(unsigned) : 0;
-    const size_t b = al256(*part_b) + al256(*cnt_b) + al256(static_cast<size_t>(poses) * sizeof(int)) + al256(*lcnt_b);
+    const size_t b = al256(*part_b) + al256(*cnt_b) + al256(static_cast<size_t>(poses) * sizeof(int)) + al256(*lcnt_b) +
+                     (r > 1 ? al256(static_cast<size_t>(poses) * sizeof(double2)) : 0);
     // (further parts leave half of what a budget has left)
     const uint64_t left = ctx->budget == 0 ? UINT64_MAX : ctx->budget > ctx->in_use ? ctx->budget - ctx->in_use : 0;
     return b <= kSplitScratchMax && b <= (r > 1 ? left / 2 : left);
@@ -1058,12 +1122,13 @@ static gd_status plan_batch(gd_context *ctx, const std::vector<ScoreParams> &des
     pl->cnt_b = cnt_b;
     pl->lcnt_b = lcnt_b;
     pl->done_b = static_cast<size_t>(poses) * sizeof(int);
+    pl->air_b = R > 1 ? static_cast<size_t>(poses) * sizeof(double2) : 0;
     pl->tune = R > 1 ? kSplitPartsTune : kSplitTune;
     e = fit(0, &per_sm);  // burial counters live in the split scratch
     if (e != cudaSuccess) return cuda_fail(ctx, e, "batched scoring occupancy");
   } else {
     pl->rparts = 1;
-    pl->part_b = pl->cnt_b = pl->done_b = pl->lcnt_b = 0;
+    pl->part_b = pl->cnt_b = pl->done_b = pl->lcnt_b = pl->air_b = 0;
   }
   for (int c = 0; c < ncx; ++c) {
     const long long per_pose =
@@ -1081,7 +1146,7 @@ static gd_status plan_batch(gd_context *ctx, const std::vector<ScoreParams> &des
 // items), split-mode partials, receptor burial counts, item counters and
 // (receptor parts) ligand burial counts.
 struct ArgLayout {
-  size_t desc, start, queue, pstart, gcounts, part, pcount, pdone, lcount, total;
+  size_t desc, start, queue, pstart, gcounts, part, air, pcount, pdone, lcount, total;
 };
 
 static ArgLayout arg_layout(int ncx, const BatchPlan &pl, size_t gcount_bytes) {
@@ -1097,6 +1162,8 @@ static ArgLayout arg_layout(int ncx, const BatchPlan &pl, size_t gcount_bytes) {
   o += al256(gcount_bytes);
   L.part = o;
   o += al256(pl.part_b);
+  L.air = o;
+  o += al256(pl.air_b);
   L.queue = o;  // from here on cleared before every launch
   o += al256(sizeof(unsigned long long));
   L.pcount = o;
@@ -1150,6 +1217,7 @@ static gd_status launch_args(gd_context *ctx, int ncx, const BatchPlan &pl, cons
   bp.pose_start = reinterpret_cast<const long long *>(arg + L.pstart);
   bp.max_chunks = pl.max_chunks * pl.rparts;
   bp.part = pl.split ? reinterpret_cast<double *>(arg + L.part) : nullptr;
+  bp.air = pl.split && pl.rparts > 1 ? reinterpret_cast<double2 *>(arg + L.air) : nullptr;
   bp.pcount = pl.split ? reinterpret_cast<unsigned *>(arg + L.pcount) : nullptr;
   bp.pdone = pl.split ? reinterpret_cast<int *>(arg + L.pdone) : nullptr;
   bp.rparts = pl.split ? pl.rparts : 1;
