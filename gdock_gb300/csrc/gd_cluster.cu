@@ -1316,10 +1316,14 @@ long long pair_words(const ClusterTopo *t) {
   return std::max<long long>(1, (static_cast<long long>(t->GR) * t->GL + 31) / 32);
 }
 
-// List entries per pose: 2,048 cover docked poses of most complexes (a pose
-// with more makes the pass run again), fewer where the lists would pass 4 GiB.
+// List entries per pose (a pose with more makes the pass run again): 2,048
+// cover docked poses of most complexes; large ones get up to 8,192, as many as
+// a bit per residue pair would take (poses sunk into a receptor of 2,000
+// residues pass 2,048, and the second pass took 8.5 ms of 22 for 4,096 poses).
+// Fewer where the lists would pass 4 GiB.
 int list_cap(const ClusterTopo *t, int n) {
-  long long cap = std::min<long long>(std::max<long long>(static_cast<long long>(t->GR) * t->GL, 1), 2048);
+  const long long pairs = std::max<long long>(static_cast<long long>(t->GR) * t->GL, 1);
+  long long cap = std::min(pairs, std::max(2048LL, std::min(8192LL, pairs / 32)));
   while (cap > 64 && cap * n * static_cast<long long>(sizeof(uint32_t)) > (4LL << 30)) cap /= 2;
   return static_cast<int>(cap);
 }
