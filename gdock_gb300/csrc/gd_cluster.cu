@@ -358,6 +358,8 @@ struct ContactListParams {
   uint32_t *lists;   // [n][cap], entries rg * GL + lg in any order
   int cap;
   uint32_t *ubits;   // union of all poses' contacts, bit rg * GL + lg; may be null
+  uint32_t *rows;    // [n][row_words] each pose's contacts, the same bits; may be null
+  long long row_words;
   int *err;          // the context's error word (index checks of the debug library)
 };
 
@@ -431,6 +433,7 @@ __global__ void __launch_bounds__(kContactWarps * 32) k_contacts(const ContactLi
       const uint32_t v = s_out[wib][k];
       if (at + k < p.cap) p.lists[static_cast<size_t>(pose) * p.cap + at + k] = v;
       if (p.ubits) atomicOr(&p.ubits[v >> 5], 1u << (v & 31));
+      if (p.rows) atomicOr(&p.rows[pose * p.row_words + (v >> 5)], 1u << (v & 31));
     }
     __syncwarp();
     nout = 0;
@@ -1320,11 +1323,16 @@ long long pair_words(const ClusterTopo *t) {
 // cover docked poses of most complexes; large ones get up to 8,192, as many as
 // a bit per residue pair would take (poses sunk into a receptor of 2,000
 // residues pass 2,048, and the second pass took 8.5 ms of 22 for 4,096 poses).
-// Fewer where the lists would pass 4 GiB.
-int list_cap(const ClusterTopo *t, int n) {
+// Fewer where the lists would pass 4 GiB or half of what a budget has left.
+int list_cap(const gd_context *ctx, const ClusterTopo *t, int n) {
   const long long pairs = std::max<long long>(static_cast<long long>(t->GR) * t->GL, 1);
   long long cap = std::min(pairs, std::max(2048LL, std::min(8192LL, pairs / 32)));
-  while (cap > 64 && cap * n * static_cast<long long>(sizeof(uint32_t)) > (4LL << 30)) cap /= 2;
+  long long most = 4LL << 30;
+  if (ctx->budget) {
+    const uint64_t used = ctx->in_use - std::min<uint64_t>(ctx->in_use, ctx->d_scratch_bytes);
+    most = std::min<long long>(most, static_cast<long long>(ctx->budget - std::min(ctx->budget, used)) / 2);
+  }
+  while (cap > 64 && cap * n * static_cast<long long>(sizeof(uint32_t)) > most) cap /= 2;
   return static_cast<int>(cap);
 }
 
@@ -1339,7 +1347,8 @@ double max_displacement(const double *genes, int n) {
 // union, too when given).  maxd bounds the poses' |displacement| components
 // (it sizes the FP32 guard band, as for the scoring kernels).
 gd_status launch_contacts(gd_complex *cx, ClusterTopo *t, const gd_pose_frame *d_frames, int n, double cutoff,
-                          double maxd, int *d_counts, uint32_t *d_lists, int cap, uint32_t *d_ubits, cudaStream_t st) {
+                          double maxd, int *d_counts, uint32_t *d_lists, int cap, uint32_t *d_ubits, cudaStream_t st,
+                          uint32_t *d_rows = nullptr, long long row_words = 0) {
   gd_context *ctx = cx->ctx;
   cudaError_t e = cudaMemsetAsync(d_counts, 0, sizeof(int) * static_cast<size_t>(n), st);
   if (e == cudaSuccess && d_ubits) e = cudaMemsetAsync(d_ubits, 0, sizeof(uint32_t) * pair_words(t), st);
@@ -1388,6 +1397,8 @@ gd_status launch_contacts(gd_complex *cx, ClusterTopo *t, const gd_pose_frame *d
   p.lists = d_lists;
   p.cap = cap;
   p.ubits = d_ubits;
+  p.rows = d_rows;
+  p.row_words = row_words;
   p.err = ctx->d_err;
   // whole blocks of ligand residues per unit, halves where the blocks give
   // every resident warp less than six and quarters where less than one (whole
@@ -1415,9 +1426,24 @@ static gd_status contacts_fast(gd_complex *cx, ClusterTopo *t, const std::vector
   cudaStream_t st = ctx->stream;
   const size_t fb = al256(sizeof(gd_pose_frame) * n), cb = al256(sizeof(int) * n), ob = al256(sizeof(long long) * (n + 1));
   std::vector<int> counts(n);
-  for (int cap = list_cap(t, n);;) {
+  for (int cap = list_cap(ctx, t, n);;) {
     const size_t lb = al256(sizeof(uint32_t) * static_cast<size_t>(n) * cap);
     gd_status s = ensure_scratch(ctx, fb + cb + ob + lb, 0);
+    if (s == GD_ERR_OOM && n > 64) {  // half of the poses at a time
+      std::vector<gd_pose_frame> part(frames.begin(), frames.begin() + n / 2);
+      s = contacts_fast(cx, t, part, n / 2, cutoff, maxd, flat, loffs);
+      if (s != GD_OK) return s;
+      std::vector<uint32_t> more;
+      std::vector<long long> offs;
+      part.assign(frames.begin() + n / 2, frames.begin() + n);
+      s = contacts_fast(cx, t, part, n - n / 2, cutoff, maxd, more, offs);
+      if (s != GD_OK) return s;
+      const long long at = loffs.back();
+      flat.insert(flat.end(), more.begin(), more.end());
+      for (size_t i = 1; i < offs.size(); ++i) loffs.push_back(at + offs[i]);
+      ctx->last_error.clear();  // the refused allocation is not this call's failure
+      return GD_OK;
+    }
     if (s != GD_OK) return s;
     char *base = static_cast<char *>(ctx->d_scratch);
     gd_pose_frame *d_frames = reinterpret_cast<gd_pose_frame *>(base);
@@ -1767,6 +1793,53 @@ gd_status cluster_sets(gd_context *ctx, const int64_t *keys, const int64_t *offs
   return GD_OK;
 }
 
+// Clusters of n poses from a bit per residue pair and pose, without lists and
+// the universe: for contexts whose budget has no room for those.  The pair
+// counts run over every residue pair, so it is the slower form.
+static gd_status cluster_bits(gd_complex *cx, ClusterTopo *t, const gd_pose_frame *frames, int n, double maxd,
+                              const gd_cluster_cfg &cfg, int c0, int32_t *n_clusters, int32_t *centers, int32_t *sizes,
+                              int32_t *members) {
+  gd_context *ctx = cx->ctx;
+  cudaStream_t st = ctx->stream;
+  const long long pairs = static_cast<long long>(t->GR) * t->GL;
+  if (pairs > INT32_MAX) return GD_ERR_OOM;
+  const int wide = std::max(1, static_cast<int>((pairs + 63) / 64)), aw = (n + 31) / 32;
+  const size_t fb = al256(sizeof(gd_pose_frame) * n), cb = al256(sizeof(int) * n),
+               rb = al256(sizeof(unsigned long long) * static_cast<size_t>(wide) * n),
+               adj_b = al256(sizeof(uint32_t) * static_cast<size_t>(n) * aw);
+  gd_status s = ensure_scratch(ctx, fb + cb + 256 + rb + adj_b + greedy_bytes(n), 0);
+  if (s != GD_OK) return s;
+  char *b = static_cast<char *>(ctx->d_scratch);
+  gd_pose_frame *d_frames = reinterpret_cast<gd_pose_frame *>(b);
+  FccParams fp{};
+  int *d_counts = reinterpret_cast<int *>(b + fb), *d_info = reinterpret_cast<int *>(b + fb + cb);
+  fp.sizes = d_counts;
+  fp.info = d_info;
+  fp.bits = reinterpret_cast<unsigned long long *>(b + fb + cb + 256);
+  fp.adj = reinterpret_cast<uint32_t *>(b + fb + cb + 256 + rb);
+  fp.n = n;
+  fp.stride = wide;
+  fp.c = cfg.fcc_cutoff;
+  fp.cs = cfg.fcc_cutoff * cfg.strictness;
+  fp.adj_words = aw;
+  fp.c0 = c0;
+  ctx->h_info[0] = static_cast<int>(pairs);
+  cudaError_t e = cudaMemcpyAsync(d_frames, frames, sizeof(gd_pose_frame) * n, cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(d_info, ctx->h_info, sizeof(int), cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(b + fb + cb + 256, 0, rb, st);
+  if (e != cudaSuccess) return cuda_fail(ctx, e, "contacts setup");
+  s = launch_contacts(cx, t, d_frames, n, cfg.contact_distance, maxd, d_counts, nullptr, 0, nullptr, st,
+                      reinterpret_cast<uint32_t *>(b + fb + cb + 256), 2LL * wide);
+  if (s != GD_OK) return s;
+  if ((e = launch_fcc(fp, st)) != cudaSuccess) return cuda_fail(ctx, e, "FCC on the device");
+  s = greedy_clusters(ctx, fp.adj, n, aw, cfg.min_cluster_size, b + fb + cb + 256 + rb + adj_b, n_clusters, centers, sizes, members);
+  if (s != GD_OK) return s;
+  ctx->last_contacts = 2;
+  ctx->last_fcc = 1;
+  ctx->last_error.clear();  // the refused allocation is not this call's failure
+  return GD_OK;
+}
+
 // cluster_structures on the device for receptors and ligands that share no
 // residue: contact lists, their union, FCC over bitsets or postings, greedy
 // clustering.  Returns GD_ERR_STATE when the topology calls for the general
@@ -1822,7 +1895,7 @@ gd_status cluster_device(gd_complex *cx, const double *genes, int n, const gd_cl
                                        greedy_bytes(n)
                                  : 0;
   cudaStream_t st = ctx->stream;
-  int cap = list_cap(t, n), info[2] = {0, 0};
+  int cap = list_cap(ctx, t, n), info[2] = {0, 0};
   gd_pose_frame *d_frames;
   int *d_counts, *d_base, *d_info;
   uint32_t *d_u, *d_lists;
@@ -1840,6 +1913,8 @@ gd_status cluster_device(gd_complex *cx, const double *genes, int n, const gd_cl
   for (;;) {
     const size_t lb = al256(sizeof(uint32_t) * static_cast<size_t>(n) * cap);
     s = ensure_scratch(ctx, fb + cb + ub + bb + 256 + lb + direct_b, 0);
+    if (s == GD_ERR_OOM)
+      return cluster_bits(cx, t, frames, n, maxd, cfg, static_cast<int>(c0), n_clusters, centers, sizes, members);
     if (s != GD_OK) return s;
     char *b = static_cast<char *>(ctx->d_scratch);
     d_frames = reinterpret_cast<gd_pose_frame *>(b);
@@ -1971,6 +2046,8 @@ gd_status cluster_device(gd_complex *cx, const double *genes, int n, const gd_cl
     }
     if (s != GD_OK) {
       if (pre) dev_free(ctx, pre, pre_b);
+      if (s == GD_ERR_OOM && !postings)
+        return cluster_bits(cx, t, frames, n, maxd, cfg, static_cast<int>(c0), n_clusters, centers, sizes, members);
       return s;
     }
     ctx->last_fcc = postings ? 2 : 1;

@@ -65,3 +65,30 @@ def test_more_contacts_than_room(oracle):
     for a, b in zip(cx.pose_contacts(genes), sets):
         np.testing.assert_array_equal(a, b)
     assert [(r.center_idx, r.members) for r in cx.cluster(genes)] == oracle.cluster(sets)
+
+
+def test_lists_within_a_budget():
+    """2,000 poses whose lists of 2,048 entries would take 16 MB, with 7 MB left
+    in the context's budget: shorter lists, or a bit per residue pair, or half
+    of the poses at a time, the same clusters and contacts."""
+    from gdock_gb300 import synth
+    c = synth.make_complex(50, 76, 0, seed=5)
+    lig = gd.position_ligand(c.receptor, c.ligand)
+    genes = synth.quaternion_genes(np.random.default_rng(3), 2000, half_box=12.0)
+    out = []
+    for budget in (0, 1):
+        ctx = gd.Context(0)
+        cx = gd.Complex(c.receptor, lig, [], ctx=ctx)
+        if budget:
+            resident = ctx.bytes_in_use
+            cx.close()
+            ctx.close()
+            ctx = gd.Context(0, hbm_budget_bytes=resident + (7 << 20))
+            cx = gd.Complex(c.receptor, lig, [], ctx=ctx)
+        try:
+            keys = cx.pose_contacts(genes)
+            out.append(([(r.center_idx, r.members) for r in cx.cluster(genes)], [k.tobytes() for k in keys]))
+        finally:
+            cx.close()
+            ctx.close()
+    assert out[0] == out[1]
