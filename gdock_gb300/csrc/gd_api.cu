@@ -958,12 +958,6 @@ gd_status gd_make_frames(const double *genes, int32_t n, gd_pose_frame *frames) 
   return GD_OK;
 }
 
-// Up to this many poses the kernel reads the frames from, and writes the
-// energies to, the pinned staging buffers themselves: 5 us less per call than
-// with two copies (one pose of 430 x 651 atoms, FP32: 60 us for 64; 150 poses:
-// 116 for 121; 1,000: 333 for 340); from 4,000 poses on both cost the same.
-constexpr int kDirectPoses = 1024;
-
 gd_status gd_score_poses(gd_complex *cx, const double *genes, int32_t n, gd_precision prec, gd_pose_energy *out) {
   gd::NvtxRange nvtx_range("gd_score_poses");
   if (!cx) return GD_ERR_INVALID_ARG;

@@ -317,10 +317,10 @@ cudaError_t launch_fcc(const FccParams &p, cudaStream_t st) {
   // small launches in small tiles, to fill the SMs (whole calls on 1,074 x 741
   // atoms, tiles of 16 / 64: 183 poses 138 / 150 us, 1,024 poses 337 / 349,
   // 2,048 poses 560 / 552; the kernel on 183 poses 68 -> 7 us)
-  cudaError_t e = cudaMemsetAsync(p.adj, 0, sizeof(uint32_t) * static_cast<size_t>(p.n) * p.adj_words, st);
-  if (e != cudaSuccess) return e;
-  const int T = p.n <= 1024 ? 16 : 64;
-  const dim3 grid((p.n + T - 1) / T, (p.n + T - 1) / T);
+  // Every word of the matrix is stored by some tile (tiles of 16 go on to a
+  // whole word), so it is not cleared first.
+  const int T = p.n <= 1024 ? 16 : 64, tiles = T == 16 ? 2 * p.adj_words : (p.n + T - 1) / T;
+  const dim3 grid(tiles, tiles);
   if (T == 16) k_fcc<16><<<grid, 256, 0, st>>>(p);
   else k_fcc<64><<<grid, 256, 0, st>>>(p);
   return cudaGetLastError();
@@ -583,10 +583,10 @@ __global__ void __launch_bounds__(kContactWarps * 32) k_contacts(const ContactLi
 
 // Exclusive prefix sums (one CTA): of the set bits of a bitmap's words, or of
 // counts; *total receives the sum.  With counts2 given, *max2 receives the
-// largest of its n2 entries.
+// largest of its n2 entries, and host_info (pinned) both.
 template <bool BITS>
 __global__ void __launch_bounds__(1024) k_scan(const uint32_t *v, long long words, int *base, int *total,
-                                               const int *counts2, int n2, int *max2) {
+                                               const int *counts2, int n2, int *max2, int *host_info) {
   __shared__ int s_w[32];
   __shared__ int s_run;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -640,7 +640,10 @@ __global__ void __launch_bounds__(1024) k_scan(const uint32_t *v, long long word
     run += s_run;
     __syncthreads();
   }
-  if (t == 0) *total = run;
+  if (t == 0) {
+    *total = run;
+    if (host_info) host_info[0] = run;
+  }
   if (counts2) {
     int m = 0;
     for (int k = t; k < n2; k += 1024) m = max(m, counts2[k]);
@@ -649,7 +652,10 @@ __global__ void __launch_bounds__(1024) k_scan(const uint32_t *v, long long word
     __syncthreads();
     if (warp == 0) {
       m = __reduce_max_sync(kFull, s_w[lane]);
-      if (lane == 0) *max2 = m;
+      if (lane == 0) {
+        *max2 = m;
+        host_info[1] = m;
+      }
     }
   }
 }
@@ -1239,6 +1245,13 @@ size_t al256(size_t b) { return (b + 255) / 256 * 256; }
 // Device bytes of a greedy pass's results: cluster count, labels, centres.
 size_t greedy_bytes(int n) { return 256 + 2 * al256(sizeof(int) * static_cast<size_t>(n)); }
 
+// Up to this many elements k_greedy writes its results, a word or two an
+// element, to pinned memory itself.  With that, the universe's size written
+// there by k_scan, one clearing pass instead of three and frames read in place,
+// a call on 183 poses of 1,074 x 741 atoms went from 138 to 112 us (on 4,096 of
+// 2,000 x 500 residues from 2,104 to 2,094).
+constexpr int kGreedyDirect = 4096;
+
 // Greedy clustering of the adjacency matrix d_adj (rows of `words`), its
 // results through d_buf (greedy_bytes) into the caller's arrays; waits for the
 // stream and reports device-side errors.
@@ -1264,6 +1277,13 @@ gd_status greedy_clusters(gd_context *ctx, const uint32_t *d_adj, int n, int wor
       *d_center = reinterpret_cast<int *>(b + 256 + lb);
   gd_status s = ensure_scratch(ctx, 0, total);
   if (s != GD_OK) return s;
+  char *h = static_cast<char *>(ctx->h_pinned);
+  const bool direct = n <= kGreedyDirect;
+  if (direct) {
+    d_k = reinterpret_cast<int *>(h);
+    d_label = reinterpret_cast<int *>(h + 256);
+    d_center = reinterpret_cast<int *>(h + 256 + lb);
+  }
   const size_t smem = greedy_smem(n).total;
   if (smem > 40 * 1024)
     e = cudaFuncSetAttribute(k_greedy, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
@@ -1282,8 +1302,7 @@ gd_status greedy_clusters(gd_context *ctx, const uint32_t *d_adj, int n, int wor
     lc.numAttrs = 1;
     e = cudaLaunchKernelEx(&lc, k_greedy, d_adj, n, words, min_size, d_label, d_center, d_k);
   }
-  char *h = static_cast<char *>(ctx->h_pinned);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(h, b, total, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess && !direct) e = cudaMemcpyAsync(h, b, total, cudaMemcpyDeviceToHost, st);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "greedy clustering");
   if ((s = finish_stream(ctx, st, "FCC on the device")) != GD_OK) return s;
   *n_clusters = order_clusters(reinterpret_cast<int *>(h + 256), reinterpret_cast<int *>(h + 256 + lb),
@@ -1350,8 +1369,11 @@ gd_status launch_contacts(gd_complex *cx, ClusterTopo *t, const gd_pose_frame *d
                           double maxd, int *d_counts, uint32_t *d_lists, int cap, uint32_t *d_ubits, cudaStream_t st,
                           uint32_t *d_rows = nullptr, long long row_words = 0) {
   gd_context *ctx = cx->ctx;
-  cudaError_t e = cudaMemsetAsync(d_counts, 0, sizeof(int) * static_cast<size_t>(n), st);
-  if (e == cudaSuccess && d_ubits) e = cudaMemsetAsync(d_ubits, 0, sizeof(uint32_t) * pair_words(t), st);
+  // counts and union in one pass where the union follows the counts
+  const size_t cb = al256(sizeof(int) * static_cast<size_t>(n)), ub = sizeof(uint32_t) * pair_words(t);
+  const bool joined = d_ubits && reinterpret_cast<char *>(d_ubits) == reinterpret_cast<char *>(d_counts) + cb;
+  cudaError_t e = cudaMemsetAsync(d_counts, 0, joined ? cb + ub : sizeof(int) * static_cast<size_t>(n), st);
+  if (e == cudaSuccess && d_ubits && !joined) e = cudaMemsetAsync(d_ubits, 0, ub, st);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "contacts setup");
   if (t->GR == 0 || t->GL == 0 || n == 0) return GD_OK;
   ContactListParams p{};
@@ -1924,16 +1946,17 @@ gd_status cluster_device(gd_complex *cx, const double *genes, int n, const gd_cl
     d_info = reinterpret_cast<int *>(b + fb + cb + ub + bb);
     d_lists = reinterpret_cast<uint32_t *>(b + fb + cb + ub + bb + 256);
     d_direct = b + fb + cb + ub + bb + 256 + lb;
-    cudaError_t e = cudaMemcpyAsync(d_frames, frames, sizeof(gd_pose_frame) * n, cudaMemcpyHostToDevice, st);
+    cudaError_t e = cudaSuccess;
+    if (n <= kDirectPoses && staged) d_frames = frames;  // read in place
+    else e = cudaMemcpyAsync(d_frames, frames, sizeof(gd_pose_frame) * n, cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "contacts setup");
     trace_step("cluster (device):   scratch + frames", st, t_step);
     s = launch_contacts(cx, t, d_frames, n, cfg.contact_distance, maxd, d_counts, d_lists, cap, d_u, st);
     if (s != GD_OK) return s;
     ctx->last_contacts = 2;
     trace_step("cluster (device):   k_contacts", st, t_step);
-    k_scan<true><<<1, 1024, 0, st>>>(d_u, words, d_base, d_info, d_counts, n, d_info + 1);
+    k_scan<true><<<1, 1024, 0, st>>>(d_u, words, d_base, d_info, d_counts, n, d_info + 1, ctx->h_info);
     e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaMemcpyAsync(ctx->h_info, d_info, sizeof(info), cudaMemcpyDeviceToHost, st);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "contact union");
     trace_step("cluster (device):   union scan", st, t_step);
     FccParams fp{};
@@ -2062,7 +2085,7 @@ gd_status cluster_device(gd_complex *cx, const double *genes, int n, const gd_cl
       e = cudaMemsetAsync(d_cur, 0, kc_b, st);
       if (e == cudaSuccess) e = cudaMemsetAsync(d_common, 0, common_b + adj_b, st);
       if (e == cudaSuccess) {
-        k_scan<false><<<1, 1024, 0, st>>>(reinterpret_cast<const uint32_t *>(d_kc), U, d_offs, d_offs + U, nullptr, 0, nullptr);
+        k_scan<false><<<1, 1024, 0, st>>>(reinterpret_cast<const uint32_t *>(d_kc), U, d_offs, d_offs + U, nullptr, 0, nullptr, nullptr);
         k_post_fill<<<std::min(n, ctx->sm_count * 16), 256, 0, st>>>(d_lists, d_counts, cap, d_u, d_base, n, d_offs, d_cur,
                                                                      d_list);
         k_post_pairs<<<std::max(1, std::min((U + 7) / 8, ctx->sm_count * 16)), 256, 0, st>>>(d_offs, d_kc, d_list, U, n,

@@ -696,10 +696,11 @@ gd_status gd_evaluate_poses(gd_evaluator *ev, const double *genes, int32_t n, gd
   void *res = staged ? static_cast<char *>(ctx->h_pinned) + fb_al : static_cast<void *>(out);
   gd_make_frames(genes, n, frames);
   cudaStream_t st = ctx->stream;
-  cudaError_t e = cudaMemcpyAsync(d_frames, frames, fb, cudaMemcpyHostToDevice, st);
+  const bool direct = staged && n <= kDirectPoses;  // frames and metrics in the staging buffer itself
+  cudaError_t e = direct ? cudaSuccess : cudaMemcpyAsync(d_frames, frames, fb, cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "evaluator frames upload");
-  s = gd_evaluate_frames_device(ev, d_frames, n, d_out, st);
-  if (s == GD_OK) {
+  s = gd_evaluate_frames_device(ev, direct ? frames : d_frames, n, direct ? static_cast<gd_dock_metrics *>(res) : d_out, st);
+  if (s == GD_OK && !direct) {
     e = cudaMemcpyAsync(res, d_out, ob, cudaMemcpyDeviceToHost, st);
     if (e != cudaSuccess) s = cuda_fail(ctx, e, "evaluator");
   }
