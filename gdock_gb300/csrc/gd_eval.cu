@@ -450,10 +450,12 @@ gd_status launch_dockq(gd_evaluator *ev, const gd_pose_frame *d_frames, int n, g
   ep.extent = static_cast<float>(m * (1.0 + 1e-6));
   ep.skip = skip;
   ep.out = d_out;
-  // one warp per pose when the poses give every resident warp one, else a CTA
-  // per pose
+  // one warp per pose when the poses give two of three resident warps one, else
+  // a CTA per pose (2,538 x 1,280 atoms, the call with its host frames: 1,500
+  // poses 169 us a warp each, 154 a CTA each, 2,500 poses 248 and 253, 5,000
+  // poses 249 and 313; 841 x 170 atoms, 1,000 poses 83 and 93)
   const int warps = kEvalCtas * kEvalWarps * ev->ctx->sm_count;
-  if (n >= warps)
+  if (n >= warps * 2 / 3)
     k_dockq<1><<<std::min((n + kEvalWarps - 1) / kEvalWarps, warps / kEvalWarps), kEvalWarps * 32, 0, stream>>>(ep);
   else
     k_dockq<kEvalWarps><<<n, kEvalWarps * 32, 0, stream>>>(ep);
