@@ -691,6 +691,24 @@ gd_status gd_complex_create(gd_context *ctx, const gd_atoms *rec, const gd_atoms
     rad = std::max(rad, std::sqrt(dx * dx + dy * dy + dz * dz));
   }
   cx->lig_radius = rad;
+  // the fixed-point images of the FP32 kernel's transform
+  std::vector<int4> lfix(2 * static_cast<size_t>(lig->n), make_int4(0, 0, 0, 0));
+  cx->fix32 = std::max({std::fabs(o[0]), std::fabs(o[1]), std::fabs(o[2])}) < 4000.0;
+  for (int k = 0; k < lig->n; ++k) {
+    const D4 &r = lrel[k];
+    if (!(std::fabs(r.x) < kFixAtom && std::fabs(r.y) < kFixAtom && std::fabs(r.z) < kFixAtom)) {
+      cx->fix32 = false;
+      break;
+    }
+    const Limbs x = limbs(std::llrint(std::ldexp(r.x, 50))), y = limbs(std::llrint(std::ldexp(r.y, 50))),
+                z = limbs(std::llrint(std::ldexp(r.z, 50)));
+    const float q = static_cast<float>(r.w);
+    int qb;
+    std::memcpy(&qb, &q, 4);
+    lfix[2 * static_cast<size_t>(k)] = make_int4(x.h, x.l, y.h, y.l);
+    lfix[2 * static_cast<size_t>(k) + 1] = make_int4(z.h, z.l, qb, ltp[k]);
+  }
+  for (int k = 0; k < 3; ++k) cx->ofix[k] = cx->fix32 ? std::llrint(std::ldexp(o[k], 51)) : 0;
   {
     const double m = std::max({std::fabs(c[0]), std::fabs(c[1]), std::fabs(c[2])}) + rad;
     cx->abs_max = std::isfinite(m) ? std::max(cx->abs_max, m) : INFINITY;
@@ -776,6 +794,7 @@ gd_status gd_complex_create(gd_context *ctx, const gd_atoms *rec, const gd_atoms
   pack.add(lz, &cx->lig_z);
   pack.add(lq, &cx->lig_q);
   pack.add(lrel, &cx->lig_rel);
+  pack.add(lfix, &cx->lig_fix);
   pack.add(ltp, &cx->lig_type);
   pack.add(lser, &cx->lig_serial);
   pack.add(ldes, &cx->lig_desolv);

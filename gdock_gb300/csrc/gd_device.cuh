@@ -104,13 +104,11 @@ static __device__ __forceinline__ double exact_d2(double ax, double ay, double a
 }
 
 // Ligand coordinates relative to the FP32 origin O, in FP64, as the FP32 images
-// are rounded from: one chain of multiply-adds on the precomputed offset from
-// the rotation centre, 9 FP64 operations in place of the 31 of the reference's
-// order, from which it differs by some 1e-15 A (decisions inside the guard
-// bands take the exact coordinates).  FP64 issues at 1/64 of the FP32 rate, and
-// with receptor parts every part's item moves its ligand atoms: 150 poses of
-// 1,074 x 741 atoms apart from each other took 147 us, 58 of them the FP64
-// pipe's; with this and without the items that have no segment in reach, 97 us.
+// are rounded from where fixed point does not reach, and for the slots' spheres:
+// one chain of multiply-adds on the precomputed offset from the rotation centre,
+// 9 FP64 operations in place of the 31 of the reference's order, from which it
+// differs by some 1e-15 A (decisions inside the guard bands take the exact
+// coordinates).
 static __device__ __forceinline__ void relative_atom(const ScoreParams &p, const gd_pose_frame &f, const D4 &r, double &x,
                                                      double &y, double &z) {
   const double tx = (p.cx + f.dx) - p.ox, ty = (p.cy + f.dy) - p.oy, tz = (p.cz + f.dz) - p.oz;
@@ -118,6 +116,27 @@ static __device__ __forceinline__ void relative_atom(const ScoreParams &p, const
   y = __fma_rn(f.sa * f.cb, r.x, __fma_rn(f.m11, r.y, __fma_rn(f.m12, r.z, ty)));
   z = __fma_rn(-f.sb, r.x, __fma_rn(f.cb * f.sg, r.y, __fma_rn(f.cb * f.cg, r.z, tz)));
 }
+// One coordinate of the rotated atom: nine 32 x 32 -> 64 multiply-adds of
+// three products, the low limbs' dropped (three units of 2^-51 A at most; an
+// FP64 chain of multiply-adds errs by ten times as much at 60 A).
+static __device__ __forceinline__ long long rotate(const Limbs &a, const Limbs &b, const Limbs &c, const int4 &xy, const int4 &z) {
+  long long hi = static_cast<long long>(a.h) * xy.x, mid = static_cast<long long>(a.h) * xy.y;
+  hi += static_cast<long long>(b.h) * xy.z;
+  mid += static_cast<long long>(a.l) * xy.x;
+  hi += static_cast<long long>(c.h) * z.x;
+  mid += static_cast<long long>(b.h) * xy.w;
+  mid += static_cast<long long>(b.l) * xy.z;
+  mid += static_cast<long long>(c.h) * z.y;
+  mid += static_cast<long long>(c.l) * z.x;
+  return hi + (mid >> 29);
+}
+
+// The nearest float to v 2^-51 (v below 2^63): two exact parts and one rounding.
+static __device__ __forceinline__ float fix_float(long long v) {
+  const float hi = __int2float_rn(static_cast<int>(v >> 40)), lo = __uint2float_rn(static_cast<unsigned>(v >> 8));
+  return __fmul_rn(__fmaf_rn(lo, 0x1p-32f, hi), 0x1p-11f);
+}
+
 static __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);

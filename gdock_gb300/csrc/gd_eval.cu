@@ -111,32 +111,6 @@ __device__ __noinline__ bool exact_contact(const ScoreParams &p, const gd_pose_f
   return exact_d2(a.x, a.y, a.z, X, Y, Z) <= thr5;
 }
 
-// Fixed point.  Ligand atoms (relative to the rotation centre, below 512 A) are
-// integers of 2^-50 A in two limbs h 2^29 + l, matrix entries (at most 1.5) of
-// 2^-59 likewise; positions and differences are 2^-51 A, translations and
-// reference atoms within 768 A of the origin, so that a difference stays below
-// 2^12 A.
-constexpr double kFixAtom = 512.0, kFixFar = 768.0;
-struct Limbs { int h, l; };
-__host__ __device__ __forceinline__ Limbs limbs(long long v) {
-  return Limbs{static_cast<int>(v >> 29), static_cast<int>(v & ((1 << 29) - 1))};
-}
-
-// One coordinate of the rotated atom: nine 32 x 32 -> 64 multiply-adds of
-// three products, the low limbs' dropped (three units of 2^-51 A at most; an
-// FP64 chain of multiply-adds errs by ten times as much at 60 A).
-__device__ __forceinline__ long long rotate(const Limbs &a, const Limbs &b, const Limbs &c, const int4 &xy, const int4 &z) {
-  long long hi = static_cast<long long>(a.h) * xy.x, mid = static_cast<long long>(a.h) * xy.y;
-  hi += static_cast<long long>(b.h) * xy.z;
-  mid += static_cast<long long>(a.l) * xy.x;
-  hi += static_cast<long long>(c.h) * z.x;
-  mid += static_cast<long long>(b.h) * xy.w;
-  mid += static_cast<long long>(b.l) * xy.z;
-  mid += static_cast<long long>(c.h) * z.y;
-  mid += static_cast<long long>(c.l) * z.x;
-  return hi + (mid >> 29);
-}
-
 // The length of (x, y, z) added to c 2^33 + r units of 2^-57 A, 2^-55 of it off
 // at most (2^-51 from 64 A on); false below 1/4 A.  The squared length D (in
 // 2^-68 A^2) differs from the square of its FP32 root s by R = D - s^2, some

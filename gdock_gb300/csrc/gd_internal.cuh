@@ -82,6 +82,17 @@ struct Thresholds {
   double contact_le;// dist <= 5   <=>  d2 <= contact_le (per call's cutoff)
 };
 
+// Fixed point.  Ligand atoms (relative to the rotation centre, below 512 A) are
+// integers of 2^-50 A in two limbs h 2^29 + l, matrix entries (at most 1.5) of
+// 2^-59 likewise; positions and differences are 2^-51 A, translations and
+// reference atoms within 768 A of the origin, so that a difference stays below
+// 2^12 A.
+constexpr double kFixAtom = 512.0, kFixFar = 768.0;
+struct Limbs { int h, l; };
+__host__ __device__ __forceinline__ Limbs limbs(long long v) {
+  return Limbs{static_cast<int>(v >> 29), static_cast<int>(v & ((1 << 29) - 1))};
+}
+
 struct ScoreParams {
   // receptor, sorted by atom type, padded to a multiple of kTile
   const float4 *rec_pos32;  // (x-O, y-O, z-O, 332.0636*q) FP32
@@ -95,6 +106,9 @@ struct ScoreParams {
   // ligand in slot order (spatially compact runs of 32 atoms)
   const int *lig_perm;      // slot position -> original atom index
   const D4 *lig_slot_sph;   // per 32-atom slot: bounding sphere (centre relative to the rotation centre, radius)
+  const int4 *lig_fix;      // the same in fixed point: two limbs a coordinate, the FP32 charge, the type
+  int fix32;                // ... when every coordinate is in range
+  long long ofix[3];        // the FP32 origin O in 2^-51 A
   const D4 *lig_rel;        // ligand atoms relative to the rotation centre, and their charge
   const double *lig_x, *lig_y, *lig_z;
   const double *lig_q;
@@ -183,6 +197,9 @@ struct gd_complex {
   int *lig_perm = nullptr;  // slot position -> original ligand atom index
   float4 *rec_seg = nullptr;  // receptor segment spheres (FP32, relative to O)
   D4 *lig_slot_sph = nullptr;  // ligand slot spheres (relative to the rotation centre)
+  int4 *lig_fix = nullptr;     // ... in fixed point, with FP32 charge and type
+  bool fix32 = false;
+  long long ofix[3] = {0, 0, 0};
   D4 *lig_rel = nullptr;       // ligand atoms relative to the rotation centre, and their charge
   int nseg = 0;
   std::vector<void *> allocs;

@@ -625,6 +625,9 @@ ScoreParams make_params(gd_complex *cx, const gd_pose_frame *d_frames, const dou
   p.lig_perm = cx->lig_perm;
   p.lig_slot_sph = cx->lig_slot_sph;
   p.lig_rel = cx->lig_rel;
+  p.lig_fix = cx->lig_fix;
+  p.fix32 = cx->fix32;
+  std::copy(cx->ofix, cx->ofix + 3, p.ofix);
   p.rec_seg = cx->rec_seg;
   p.nseg = cx->nseg;
   p.lig_x = cx->lig_x;

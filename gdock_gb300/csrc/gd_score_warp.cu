@@ -7,8 +7,9 @@
 //
 // Per work item a warp
 //   1. copies the complex's descriptor and the pose frame to its shared memory;
-//   2. for each chunk of 32*S ligand atoms: moves them in FP64 (one
-//      multiply-add chain a coordinate; src/structure.rs:80-131), keeps FP32
+//   2. for each chunk of 32*S ligand atoms: moves them in fixed point (nine
+//      32-bit multiply-adds a coordinate, closer than FP64; out of its range in
+//      FP64; src/structure.rs:80-131), keeps FP32
 //      copies in shared memory (S slots of 32 atoms, one per lane; the ligand
 //      is stored in spatially compact slot order) and a bounding sphere and
 //      box per slot;
@@ -99,7 +100,7 @@ struct BatchParams {
 };
 
 struct WarpSmem {
-  size_t pos, meta, list, fixq, cmask, cstep, lig, lt, lcnt, bars, desc, frame, blob, box, rc, ssph, segl, cnt, total;
+  size_t pos, meta, list, fixq, cmask, cstep, lig, lt, lcnt, bars, desc, frame, fixm, blob, box, rc, ssph, segl, cnt, total;
 };
 
 // atoms: rows per step of the kernel variant
@@ -142,6 +143,9 @@ __host__ __device__ inline WarpSmem warp_layout(int smem_cnt, int atoms) {
   al(16);
   L.frame = o;
   o += sizeof(gd_pose_frame);
+  L.fixm = o;  // the frame in fixed point: nine matrix entries, the translation
+  o += 9 * sizeof(Limbs) + 3 * sizeof(long long);
+  al(16);
   L.blob = o;
   o += sizeof(float4) * 8;
   L.box = o;
@@ -335,6 +339,8 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_score_f32w(const BatchPar
   uint64_t *s_bar = reinterpret_cast<uint64_t *>(base + L.bars);
   ScoreParams *s_desc = reinterpret_cast<ScoreParams *>(base + L.desc);
   gd_pose_frame *s_frame = reinterpret_cast<gd_pose_frame *>(base + L.frame);
+  Limbs *s_fm = reinterpret_cast<Limbs *>(base + L.fixm);
+  long long *s_ft = reinterpret_cast<long long *>(s_fm + 9);
   float4 *s_blob = reinterpret_cast<float4 *>(base + L.blob);
   float4 *s_box = reinterpret_cast<float4 *>(base + L.box);  // per slot: (centre, hx), (hy, hz, -, -)
   int *s_rc = reinterpret_cast<int *>(base + L.rc);  // receptor burial counts of the current segment
@@ -477,7 +483,31 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_score_f32w(const BatchPar
             if (!(bp.drop_copy && item == 0 && ch == ch0 && k == 0))
               issue_seg(q + k, seg_at(k), p, s_pos, s_meta, s_bar);
         q_issued = q + min(nk, kWS);
-#pragma unroll
+        // the frame in fixed point, an entry a lane.  With receptor parts every
+        // part's item moves its ligand atoms, and in FP64 that kept its pipe 30 %
+        // busy and the warps waiting: 150 poses of 2,538 x 1,280 atoms 347 ->
+        // 330 us, of 1,074 x 741 176 -> 160, of 411 x 649 116 -> 103
+        bool fix = p.fix32 && !p.models;
+        if (fix) {
+          bool ok = true;
+          if (lane < 9) {
+            const double a = lane == 0 ? f.ca : lane == 1 ? f.m01 : lane == 2 ? f.m02 : lane == 3 ? f.sa : lane == 4 ? f.m11
+                             : lane == 5 ? f.m12 : lane == 6 ? -f.sb : f.cb;
+            const double b = lane == 0 || lane == 3 ? f.cb : lane == 7 ? f.sg : lane == 8 ? f.cg : 1.0;
+            const double m = __dmul_rn(a, b);
+            ok = fabs(m) <= 1.5;
+            s_fm[lane] = limbs(ok ? __double2ll_rn(m * 0x1p59) : 0);
+          } else if (lane < 12) {
+            const double t = lane == 9 ? p.cx + f.dx : lane == 10 ? p.cy + f.dy : p.cz + f.dz;
+            ok = fabs(t) < 4000.0;
+            const long long v = ok ? __double2ll_rn(t * 0x1p51) - p.ofix[lane - 9] : 0;
+            ok = ok && llabs(v) < static_cast<long long>(kFixFar * 0x1p51);
+            s_ft[lane - 9] = v;
+          }
+          fix = __all_sync(kFull, ok);
+          __syncwarp();
+        }
+#pragma unroll 1
         for (int s = 0; s < S; ++s) {
           const int j = ch * kChunk + s * 32 + lane;
           const bool on = j < p.nl;
@@ -485,9 +515,18 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_score_f32w(const BatchPar
           float4 l = make_float4(-1.0e9f, -1.0e9f, -1.0e9f, 0.0f);
           int lt = 0;
           if (on) {
-            const float3 c = atom32(p, f, pose, j);
-            l = make_float4(c.x, c.y, c.z, static_cast<float>(p.lig_rel[j].w));
-            lt = p.lig_type[j];
+            if (fix) {
+              const int4 xy = __ldg(&p.lig_fix[2 * j]), z = __ldg(&p.lig_fix[2 * j + 1]);
+              l.x = fix_float(rotate(s_fm[0], s_fm[1], s_fm[2], xy, z) + s_ft[0]);
+              l.y = fix_float(rotate(s_fm[3], s_fm[4], s_fm[5], xy, z) + s_ft[1]);
+              l.z = fix_float(rotate(s_fm[6], s_fm[7], s_fm[8], xy, z) + s_ft[2]);
+              l.w = __int_as_float(z.z);
+              lt = z.w;
+            } else {
+              const float3 c = atom32(p, f, pose, j);
+              l = make_float4(c.x, c.y, c.z, static_cast<float>(p.lig_rel[j].w));
+              lt = p.lig_type[j];
+            }
             if (!GD_DCHECK(bp.err, lt >= 0 && lt < p.nt, 6)) lt = 0;
           }
           s_lig[s * 32 + lane] = l;
