@@ -137,6 +137,26 @@ static __device__ __forceinline__ float fix_float(long long v) {
   return __fmul_rn(__fmaf_rn(lo, 0x1p-32f, hi), 0x1p-11f);
 }
 
+// The squared length of d (2^-51 A, below 16 A) in 2^-56 A^2: exact squares,
+// truncated.
+static __device__ __forceinline__ unsigned long long fix_d2(const long long *d) {
+  long long H = 0, M = 0;
+  unsigned lo = 0;
+  // d = h 2^32 + l with a signed l: d^2 = h^2 2^64 + h l 2^33 + l^2
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const int l = static_cast<int>(d[a]);
+    const int h = static_cast<int>(d[a] >> 32) + static_cast<int>(static_cast<unsigned>(l) >> 31);
+    H += static_cast<long long>(h) * h;
+    M += static_cast<long long>(h) * l;
+    lo += static_cast<unsigned>(__mulhi(l, l)) >> 2;  // three of them fit 32 bits
+  }
+  return (static_cast<unsigned long long>(H) << 18) + (M >> 13) + (lo >> 12);
+}
+// A fixed-point d2's high word (2^-24 A^2) next to that of the squared cutoff
+// c2: within 6e-8 A^2, where integers and doubles differ by some 1e-14.
+static __device__ __forceinline__ bool near_fix(unsigned hw, unsigned c2) { return hw - ((c2 << 24) - 1u) <= 1u; }
+
 static __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);

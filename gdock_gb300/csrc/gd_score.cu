@@ -153,10 +153,6 @@ __device__ __noinline__ ExactPair exact_pair(const ScoreParams &p, const gd_pose
 __device__ __forceinline__ bool near_hi(int hi, double t) {
   return static_cast<unsigned>(hi - (__double2hiint(t) - 1)) <= 2u;
 }
-// A fixed-point d2's high word (2^-24 A^2) next to that of the squared cutoff
-// c2: within 6e-8 A^2, where integers and doubles differ by some 1e-14.
-__device__ __forceinline__ bool near_fix(unsigned hw, unsigned c2) { return hw - ((c2 << 24) - 1u) <= 1u; }
-
 // FIX: d2 from integer coordinates.  The differences and the three squares are
 // exact and d2 is truncated below 2^-56 A^2, so its error is the coordinates'
 // rounding to 2^-52 A, less than theirs as doubles above 4 A.  It takes about
@@ -186,18 +182,7 @@ struct PairEval {
       rq = __longlong_as_double(rzq.y);
       const long long d[3] = {rxy.x - static_cast<const long long *>(x)[k], rxy.y - static_cast<const long long *>(y)[k],
                               rzq.x - static_cast<const long long *>(z)[k]};
-      long long H = 0, M = 0;
-      unsigned lo = 0;
-      // d = h 2^32 + l with a signed l: d^2 = h^2 2^64 + h l 2^33 + l^2
-#pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        const int l = static_cast<int>(d[a]);
-        const int h = static_cast<int>(d[a] >> 32) + static_cast<int>(static_cast<unsigned>(l) >> 31);
-        H += static_cast<long long>(h) * h;
-        M += static_cast<long long>(h) * l;
-        lo += static_cast<unsigned>(__mulhi(l, l)) >> 2;  // three of them fit 32 bits
-      }
-      const unsigned long long D = (static_cast<unsigned long long>(H) << 18) + (M >> 13) + (lo >> 12);  // 2^-56 A^2
+      const unsigned long long D = fix_d2(d);  // 2^-56 A^2
       const unsigned hw = static_cast<unsigned>(D >> 32);
       // to a double, rounded: the leading bit at 63 - n (n = 0 from 128 A^2 on)
       const int n = NEAR ? __clz(hw) : 0;

@@ -35,10 +35,10 @@
 //      position and its row of the pair table.  That took 150 poses of
 //      2,538 x 1,280 atoms from 419 to 376 us and 65,536 of them from 83.4
 //      to 81.4 ms;
-//   6. re-decides in FP64, once per segment, the pairs of flagged steps whose
-//      FP32 d2 lies within the guard band of a cutoff (1, 8, 12, 15 A), so
-//      all decisions equal the FP64 ones; a flagged step computes exact
-//      coordinates only for the pairs that lie in a band;
+//   6. re-decides, once per segment, the pairs of flagged steps whose FP32 d2
+//      lies within the guard band of a cutoff (1, 8, 12, 15 A): on integer
+//      distances, and in the reference's FP64 order where those lie next to
+//      the cutoff, so all decisions equal the FP64 ones;
 //   7. reduces exactly: each segment's FP32 vdW and Coulomb partials become
 //      2^-32 fixed-point integers summed per lane (integer sums do not depend
 //      on their order, so neither do the energies on how segments, chunks and
@@ -255,18 +255,32 @@ __device__ __forceinline__ float warp_max(float v) {
   return r;
 }
 
-// Corrections of one pair's FP32 contributions after its FP64 re-decision.
+// Corrections of one pair's FP32 contributions after its exact re-decision.
 struct FixOut {
   float dv, de;
   int dl;
 };
 
-// FP64 re-decision of one flagged pair (exact ligand coordinates X, Y, Z):
-// recomputes the FP32 d2 and decisions bit-identically to pair32() and
-// returns the corrections where the exact decision differs.
+// A pair's decisions in the reference's arithmetic: bit 0 vdW, 1 Coulomb, 2
+// burial.  Out of line: a handful of pairs come here.
+__device__ __noinline__ int exact_flags(const ScoreParams &p, const gd_pose_frame &f, int pose, int j, int ridx) {
+  const D4 r64 = p.rec_pos64[ridx];
+  double X, Y, Z;
+  ligand_atom(p, f, pose, j, X, Y, Z);
+  const double d2x = exact_d2(r64.x, r64.y, r64.z, X, Y, Z);
+  return (d2x > 0.0 && d2x < p.thr.vdw_lt) | (d2x > p.thr.elec_gt && d2x < p.thr.elec_lt) << 1 | (d2x < p.thr.desolv_lt) << 2;
+}
+
+// Re-decision of one flagged pair (the lane's ligand atom j): recomputes the
+// FP32 d2 and decisions bit-identically to pair32() and returns the corrections
+// where the exact decision differs.  With the frame in fixed point (fm, ft) the
+// integer d2 decides all but pairs within 6e-8 A^2 of a cutoff, which take the
+// reference's FP64 order (some 45 FP64 operations, each 64 cycles apart): one
+// pose of 2,538 x 1,280 atoms 88 -> 86 us, 65,536 poses 82.9 -> 82.6 ms.
 template <bool SERIAL, bool CLAMP>
-__device__ __forceinline__ FixOut fix_pair(const ScoreParams &p, double X, double Y, double Z, float4 r, int ridx,
-                                        int rtrow, int rser, float lx, float ly, float lz, float lq, int lt, int lser) {
+__device__ __forceinline__ FixOut fix_pair(const ScoreParams &p, const gd_pose_frame &f, int pose, int j, bool fix,
+                                           const Limbs *fm, const long long *ft, float4 r, int ridx, int rtrow, int rser,
+                                           float lx, float ly, float lz, float lq, int lt, int lser) {
   FixOut o{0.0f, 0.0f, 0};
   const float d2 = d2f(r, lx, ly, lz);
   const float te = __fsub_rn(d2, 113.0f);
@@ -274,12 +288,28 @@ __device__ __forceinline__ FixOut fix_pair(const ScoreParams &p, double X, doubl
   if (SERIAL) pv32 = pv32 && (rser != lser);
   const bool pe32 = fabsf(te) < 112.0f;
   const bool pd32 = d2 < 64.0f;
-  const D4 r64 = p.rec_pos64[ridx];
-  const double d2x = exact_d2(r64.x, r64.y, r64.z, X, Y, Z);
-  bool pv64 = d2x > 0.0 && d2x < p.thr.vdw_lt;
+  bool pv64 = false, pe64 = false, pd64 = false, decided = false;
+  if (fix) {
+    const int4 xy = __ldg(&p.lig_fix[2 * j]), z = __ldg(&p.lig_fix[2 * j + 1]);
+    const longlong2 *rp = reinterpret_cast<const longlong2 *>(p.rec_fix + ridx);
+    const longlong2 rxy = __ldg(rp);
+    const long long rz = __ldg(reinterpret_cast<const long long *>(rp + 1));
+    const long long d[3] = {rxy.x - p.ofix[0] - ft[0] - rotate(fm[0], fm[1], fm[2], xy, z),
+                            rxy.y - p.ofix[1] - ft[1] - rotate(fm[3], fm[4], fm[5], xy, z),
+                            rz - p.ofix[2] - ft[2] - rotate(fm[6], fm[7], fm[8], xy, z)};
+    const unsigned hw = static_cast<unsigned>(fix_d2(d) >> 32);
+    decided = !(near_fix(hw, 225u) | near_fix(hw, 144u) | near_fix(hw, 64u) | near_fix(hw, 1u) | (hw == 0u));
+    pv64 = hw < (144u << 24);
+    pd64 = hw < (64u << 24);
+    pe64 = hw >= (1u << 24) && hw < (225u << 24);
+  }
+  if (!decided) {
+    const int e = exact_flags(p, f, pose, j, ridx);
+    pv64 = e & 1;
+    pe64 = e & 2;
+    pd64 = e & 4;
+  }
   if (SERIAL) pv64 = pv64 && (rser != lser);
-  const bool pe64 = d2x > p.thr.elec_gt && d2x < p.thr.elec_lt;
-  const bool pd64 = d2x < p.thr.desolv_lt;
   if (pv64 != pv32) {
     const float v = vdw_term<CLAMP>(d2, __ldg(reinterpret_cast<const float2 *>(p.tab32) + rtrow + lt));
     o.dv = pv64 ? v : -v;
@@ -632,7 +662,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_score_f32w(const BatchPar
           // Phase 2: every term of the kept rows, kAtoms rows per step (two in
           // the last one where two are left: a run of 13 rows wastes one, not
           // three)
-          float av = 0.0f, ae = 0.0f;  // ae: corrections from FP64 re-decisions (charge included)
+          float av = 0.0f, ae = 0.0f;  // ae: corrections from exact re-decisions (charge included)
 #pragma unroll 1
           for (int s = 0; s < S; ++s) {
             const int nf = __shfl_sync(kFull, nf_mine, s * 8), nn = __shfl_sync(kFull, nn_mine, s * 8);
@@ -742,7 +772,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_score_f32w(const BatchPar
             if (lc) s_lcnt[s * 32 + lane] += lc;
           }
           __syncwarp();
-          // FP64 re-decisions of the flagged steps' pairs in the guard band
+          // exact re-decisions of the flagged steps' pairs in the guard band
           const int nfix = seg_cnt >> 16, ncs = seg_cnt & 0xffff;
 #pragma unroll 1
           for (int t = 0; t < nfix; ++t) {
@@ -756,10 +786,8 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_score_f32w(const BatchPar
               if (ixi == kFar || !GD_DCHECK(bp.err, ixi >= 0 && ixi < kFar, 4)) continue;
               const float4 ri = s_pos[ixi];
               if (!near_band(d2f(ri, l.x, l.y, l.z), gv, ge, gdd)) continue;
-              double X, Y, Z;
-              ligand_atom(p, f, pose, j, X, Y, Z);
               const int2 mt = s_meta[ixi];
-              const FixOut fo = fix_pair<SERIAL, CLAMP>(p, X, Y, Z, ri, gbase + ixi - sbase, mt.x, mt.y, l.x, l.y, l.z, l.w,
+              const FixOut fo = fix_pair<SERIAL, CLAMP>(p, f, pose, j, fix && p.fix, s_fm, s_ft, ri, gbase + ixi - sbase, mt.x, mt.y, l.x, l.y, l.z, l.w,
                                                         s_lt[s * 32 + lane], SERIAL ? p.lig_serial[j] : 0);
               av += fo.dv;
               ae += fo.de;
