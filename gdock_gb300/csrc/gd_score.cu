@@ -317,8 +317,11 @@ __global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const
         fy = static_cast<float>(Y - p.oy);
         fz = static_cast<float>(Z - p.oz);
         if (FIX) {
-          // (a coordinate that is not a number: no pair has a term)
-          if (!(fabsf(fx) + fabsf(fy) + fabsf(fz) < 3.0e38f)) fx = INFINITY;
+          // an atom with a coordinate that is not finite has no pair with a term:
+          // all three images infinite keep it out of the search, whose tests
+          // keep an undefined distance for an FP64 decision that the integers
+          // cannot make
+          if (!(fabsf(fx) + fabsf(fy) + fabsf(fz) < 3.0e38f)) fx = fy = fz = INFINITY;
           constexpr double kOne = 1LL << kFixBits;
           s_x[k] = __longlong_as_double(__double2ll_rn(X * kOne));
           s_y[k] = __longlong_as_double(__double2ll_rn(Y * kOne));

@@ -75,3 +75,31 @@ def test_coincident_atoms_and_vanishing_radii(oracle):
     cx = gd.Complex(rec, lig, [])
     xyz = np.stack([lig.xyz(), lig.xyz() + 1.0e-160, lig.xyz() + [0.0, 1.0e-9, 0.0]])
     check_nan(cx.score_models(xyz), oracle.score_models(rec, lig, [], xyz))
+
+
+@pytest.mark.parametrize("gene", range(6))
+def test_one_undefined_gene(oracle, big, gene):
+    """A NaN gene and nothing else out of range: that pose has no pair terms,
+    the others keep their bits."""
+    rec, lig = _first_atoms(big.receptor, 120), _first_atoms(big.ligand, 90)
+    lig = gd.position_ligand(rec, lig)
+    genes = synth.random_genes(np.random.default_rng(6), 5, max_displacement=5.0)
+    cx = gd.Complex(rec, lig, big.restraint_pairs)
+    before = cx.score_poses(genes)
+    genes[2, gene] = np.nan
+    got = cx.score_poses(genes)
+    check_nan(got, oracle.score_poses(rec, lig, big.restraint_pairs, genes))
+    keep = [0, 1, 3, 4]
+    assert got[keep].tobytes() == before[keep].tobytes()
+
+
+@pytest.mark.parametrize("axis", range(3))
+def test_one_undefined_model_coordinate(oracle, big, axis):
+    """One NaN coordinate of one atom of a model: the atom's pairs have no
+    term, the model's other atoms and the other models theirs."""
+    rec, lig = _first_atoms(big.receptor, 120), _first_atoms(big.ligand, 90)
+    lig = gd.position_ligand(rec, lig)
+    xyz = lig.xyz()[None] + np.random.default_rng(7).normal(0, 3.0, (4, 1, 3))
+    xyz[1, 40, axis] = np.nan
+    cx = gd.Complex(rec, lig, big.restraint_pairs)
+    check_nan(cx.score_models(xyz), oracle.score_models(rec, lig, big.restraint_pairs, xyz))
