@@ -185,11 +185,8 @@ void make_frame(const double *g, gd_pose_frame *f) {
 // most M*2^-24 rounding (M bounds |x - O|); for a pair at distance c the
 // computed d2 is then off by at most ~2c*sqrt(3)*(2M*2^-24 + c*2^-24) +
 // 4c^2*2^-24.  Four times that is the band.
-void guard_widths(const gd_complex *cx, double max_disp, float *gv, float *ge, float *gdd) {
+void guard_bands(double M, float *gv, float *ge, float *gdd) {
   const double u = std::ldexp(1.0, -24);
-  const double lig = std::max({std::fabs(cx->cx - cx->ox), std::fabs(cx->cy - cx->oy), std::fabs(cx->cz - cx->oz)}) +
-                     cx->lig_radius + max_disp;
-  const double M = std::max(cx->rec_extent, lig) + 1.0;
   auto band = [&](double c) {
     const double err = 2.0 * c * std::sqrt(3.0) * (2.0 * M * u + c * u) + 4.0 * c * c * u;
     return static_cast<float>(4.0 * err + 1e-6);
@@ -197,6 +194,11 @@ void guard_widths(const gd_complex *cx, double max_disp, float *gv, float *ge, f
   *gv = band(12.0);
   *ge = band(15.0);
   *gdd = band(8.0);
+}
+void guard_widths(const gd_complex *cx, double max_disp, float *gv, float *ge, float *gdd) {
+  const double lig = std::max({std::fabs(cx->cx - cx->ox), std::fabs(cx->cy - cx->oy), std::fabs(cx->cz - cx->oz)}) +
+                     cx->lig_radius + max_disp;
+  guard_bands(std::max(cx->rec_extent, lig) + 1.0, gv, ge, gdd);
 }
 
 static double asp_of(uint8_t e) {  // src/fitness.rs:129-138
@@ -644,10 +646,9 @@ gd_status gd_complex_create(gd_context *ctx, const gd_atoms *rec, const gd_atoms
                           static_cast<float>(rec->z[i] - o[2]), static_cast<float>(332.0636 * rec->charge[i]));
     rp64[k] = D4{rec->x[i], rec->y[i], rec->z[i], rec->charge[i]};
     {
-      const double m = std::max({std::fabs(rec->x[i]), std::fabs(rec->y[i]), std::fabs(rec->z[i])});
-      const bool fin = std::isfinite(rec->x[i]) && std::isfinite(rec->y[i]) && std::isfinite(rec->z[i]);
-      cx->abs_max = fin ? std::max(cx->abs_max, m) : INFINITY;
-      if (fin && m <= kFixMax)
+      const bool in = std::fabs(rec->x[i]) <= kFixMax && std::fabs(rec->y[i]) <= kFixMax && std::fabs(rec->z[i]) <= kFixMax;
+      cx->fix64 = cx->fix64 && in;
+      if (in)
         rfix[k] = FixAtom{std::llrint(std::ldexp(rec->x[i], kFixBits)), std::llrint(std::ldexp(rec->y[i], kFixBits)),
                           std::llrint(std::ldexp(rec->z[i], kFixBits)), rec->charge[i]};
     }
@@ -709,10 +710,6 @@ gd_status gd_complex_create(gd_context *ctx, const gd_atoms *rec, const gd_atoms
     lfix[2 * static_cast<size_t>(k) + 1] = make_int4(z.h, z.l, qb, ltp[k]);
   }
   for (int k = 0; k < 3; ++k) cx->ofix[k] = cx->fix32 ? std::llrint(std::ldexp(o[k], 51)) : 0;
-  {
-    const double m = std::max({std::fabs(c[0]), std::fabs(c[1]), std::fabs(c[2])}) + rad;
-    cx->abs_max = std::isfinite(m) ? std::max(cx->abs_max, m) : INFINITY;
-  }
   // bounding sphere of each 32-atom slot in the positioned frame: a pose moves
   // it rigidly, so its transformed centre and the same radius bound the
   // slot's atoms in every pose

@@ -25,7 +25,8 @@ struct alignas(32) FixAtom {
   double q;
 };
 constexpr int kFixBits = 51;
-constexpr double kFixMax = 4000.0;  // |coordinate| up to which the integers are used (they hold 4,096)
+constexpr double kFixMax = 4000.0;   // receptor |coordinate| up to which the integers are used (they hold 4,096)
+constexpr double kFixHold = 4095.0;  // ligand |coordinate| they take; beyond, no receptor atom is near
 
 // The receptor's arrays are padded to a multiple of this many atoms.
 constexpr int kTile = 256;
@@ -98,7 +99,7 @@ struct ScoreParams {
   const float4 *rec_pos32;  // (x-O, y-O, z-O, 332.0636*q) FP32
   const D4 *rec_pos64; // (x, y, z, q) FP64
   const FixAtom *rec_fix;   // the same as integers
-  int fix;                  // every coordinate of the launch lies within kFixMax
+  int fix;                  // every receptor coordinate lies within kFixMax
   const int2 *rec_meta;     // (type, serial)
   const double *rec_desolv; // [nr * 11] energy contribution at burial count 0..10
   const float4 *rec_seg;    // per kRecSeg-atom segment: bounding sphere (centre - O, radius) FP32
@@ -184,7 +185,7 @@ struct gd_complex {
   float4 *rec_pos32 = nullptr;
   D4 *rec_pos64 = nullptr;
   gd::FixAtom *rec_fix = nullptr;
-  double abs_max = 0;     // max |x| over receptor atoms and (ligand centroid + radius); inf when not finite
+  bool fix64 = true;      // every receptor coordinate lies within kFixMax
   int2 *rec_meta = nullptr;
   double *rec_desolv = nullptr;
   double *lig_x = nullptr, *lig_y = nullptr, *lig_z = nullptr, *lig_q = nullptr;
@@ -247,6 +248,7 @@ constexpr size_t kStageMax = size_t(64) << 20;
 // with two copies (one pose of 430 x 651 atoms, FP32: 60 us for 64; 150 poses:
 // 116 for 121; 1,000: 333 for 340); from 4,000 poses on both cost the same.
 constexpr int kDirectPoses = 1024;
+void guard_bands(double M, float *gv, float *ge, float *gd);
 void guard_widths(const gd_complex *cx, double max_disp, float *gv, float *ge, float *gd);
 gd_status launch_score(gd_complex *cx, const gd_pose_frame *d_frames, const double *d_models, int n,
                        gd_precision prec, gd_pose_energy *d_out, cudaStream_t stream, double max_disp,

@@ -309,6 +309,7 @@ __global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const
     for (int s = rank + nc * warp; s < nslot; s += nc * kNW) {
       const int k = s * 32 + lane, j = l0 + k;
       const bool on = k < nl;
+      bool held = on;  // in the sphere
       float fx = 0.0f, fy = 0.0f, fz = 0.0f;
       if (on) {
         double X, Y, Z;
@@ -317,11 +318,16 @@ __global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const
         fy = static_cast<float>(Y - p.oy);
         fz = static_cast<float>(Z - p.oz);
         if (FIX) {
-          // an atom with a coordinate that is not finite has no pair with a term:
-          // all three images infinite keep it out of the search, whose tests
-          // keep an undefined distance for an FP64 decision that the integers
-          // cannot make
-          if (!(fabsf(fx) + fabsf(fy) + fabsf(fz) < 3.0e38f)) fx = fy = fz = INFINITY;
+          // The receptor lies within kFixMax, so an atom with a coordinate beyond
+          // kFixHold, or one that is not a number, has no pair with a term: images
+          // at infinity keep it out of the search.  A property of the atom alone:
+          // the launch's other poses, and what their displacements are said to
+          // be, change nothing.
+          held = fabs(X) < kFixHold && fabs(Y) < kFixHold && fabs(Z) < kFixHold;
+          if (!held) {
+            X = Y = Z = 0.0;
+            fx = fy = fz = INFINITY;
+          }
           constexpr double kOne = 1LL << kFixBits;
           s_x[k] = __longlong_as_double(__double2ll_rn(X * kOne));
           s_y[k] = __longlong_as_double(__double2ll_rn(Y * kOne));
@@ -337,8 +343,8 @@ __global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const
       }
       // a sphere around the slot: the precomputed smallest one moved with the
       // pose, else the bounding box's centre and farthest atom
-      float lo[3] = {on ? fx : 3.0e38f, on ? fy : 3.0e38f, on ? fz : 3.0e38f},
-            hi[3] = {on ? fx : -3.0e38f, on ? fy : -3.0e38f, on ? fz : -3.0e38f};
+      float lo[3] = {held ? fx : 3.0e38f, held ? fy : 3.0e38f, held ? fz : 3.0e38f},
+            hi[3] = {held ? fx : -3.0e38f, held ? fy : -3.0e38f, held ? fz : -3.0e38f};
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
@@ -347,7 +353,7 @@ __global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const
           hi[a] = fmaxf(hi[a], __shfl_xor_sync(kFull, hi[a], o));
         }
       const float cx = 0.5f * (lo[0] + hi[0]), cy = 0.5f * (lo[1] + hi[1]), cz = 0.5f * (lo[2] + hi[2]);
-      float rr = on ? sqrtf((fx - cx) * (fx - cx) + (fy - cy) * (fy - cy) + (fz - cz) * (fz - cz)) : 0.0f;
+      float rr = held ? sqrtf((fx - cx) * (fx - cx) + (fy - cy) * (fy - cy) + (fz - cz) * (fz - cz)) : 0.0f;
       const bool odd = __any_sync(kFull, !(rr < 3.0e38f));  // not finite: a sphere that keeps everything
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) rr = fmaxf(rr, __shfl_xor_sync(kFull, rr, o));
@@ -606,7 +612,7 @@ ScoreParams make_params(gd_complex *cx, const gd_pose_frame *d_frames, const dou
   p.rec_pos32 = cx->rec_pos32;
   p.rec_pos64 = cx->rec_pos64;
   p.rec_fix = cx->rec_fix;
-  p.fix = cx->abs_max + max_disp <= kFixMax;
+  p.fix = cx->fix64;
   p.rec_meta = cx->rec_meta;
   p.rec_desolv = cx->rec_desolv;
   p.nr = cx->nr;
@@ -667,9 +673,12 @@ gd_status launch_score(gd_complex *cx, const gd_pose_frame *d_frames, const doub
   if (prec == GD_PREC_F32)
     return launch_score_batch_f32(ctx, std::vector<ScoreParams>{p}, serial, clamp,
                                   ctx->tune_f32_slots ? ctx->tune_f32_slots : kDefaultF32Tune, stream);
-  // the band is first order in the coordinates' FP32 rounding: beyond 1 A^2
-  // (coordinates some 40,000 A from the origin, or not finite) FP32 drops
-  // nothing and every pair is decided in FP64
+  // Here the bands only keep FP32 from dropping a pair that has a term, and such
+  // a pair's ligand atom lies within 15 A of the receptor's extent, wherever the
+  // launch's poses are.  They are first order in the coordinates' FP32 rounding:
+  // beyond 1 A^2 (receptor coordinates some 40,000 A from the origin, or not
+  // finite) FP32 drops nothing and every pair is decided in FP64.
+  guard_bands(cx->rec_extent + 17.0, &p.guard_v, &p.guard_e, &p.guard_d);
   if (!(p.guard_e <= 1.0f)) p.guard_e = p.guard_v = INFINITY;
   cudaError_t e;
   const int sm = ctx->sm_count;

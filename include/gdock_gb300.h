@@ -187,8 +187,9 @@ gd_status gd_score_poses(gd_complex *cx, const double *genes, int32_t n, gd_prec
 
 /* Same, on device-resident frames and outputs, enqueued on `stream`
  * (a cudaStream_t; NULL = the context's stream).  max_displacement bounds
- * |dx|, |dy|, |dz| over the frames (it sizes the FP32 guard bands).  Returns
- * after the launch; errors of the device run are reported by gd_sync. */
+ * |dx|, |dy|, |dz| over the frames: it sizes the guard bands of the FP32 form,
+ * whose energies rely on it; the FP64 form does not read it.  Returns after
+ * the launch; errors of the device run are reported by gd_sync. */
 gd_status gd_score_frames_device(gd_complex *cx, const gd_pose_frame *d_frames, int32_t n,
                                  gd_precision prec, double max_displacement, gd_pose_energy *d_out,
                                  void *stream);

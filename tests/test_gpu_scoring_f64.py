@@ -103,3 +103,46 @@ def test_one_undefined_model_coordinate(oracle, big, axis):
     xyz[1, 40, axis] = np.nan
     cx = gd.Complex(rec, lig, big.restraint_pairs)
     check_nan(cx.score_models(xyz), oracle.score_models(rec, lig, big.restraint_pairs, xyz))
+
+
+@pytest.mark.parametrize("far", [3000.0, 3990.0, 4200.0, 1.0e6, 1.0e300, np.inf, np.nan])
+def test_a_pose_beside_one_far_away(oracle, big, far):
+    """A pose's record does not depend on the call's other poses, however far
+    away they are; nor a model's on the other models."""
+    rec, lig = _first_atoms(big.receptor, 120), _first_atoms(big.ligand, 90)
+    lig = gd.position_ligand(rec, lig)
+    genes = synth.random_genes(np.random.default_rng(8), 6, max_displacement=5.0)
+    cx = gd.Complex(rec, lig, big.restraint_pairs)
+    alone = cx.score_poses(genes)
+    beside = np.concatenate([genes, genes[:1]])
+    beside[6, 4] = far
+    got = cx.score_poses(beside)
+    assert got[:6].tobytes() == alone.tobytes()
+    check_nan(got, oracle.score_poses(rec, lig, big.restraint_pairs, beside))
+    xyz = lig.xyz()[None] + genes[:, None, 3:]
+    models = np.concatenate([xyz, xyz[:1]])
+    models[6, 7:70, 1] += far  # some of a model's atoms only
+    got = cx.score_models(models)
+    assert got[:6].tobytes() == cx.score_models(xyz).tobytes()
+    check_nan(got, oracle.score_models(rec, lig, big.restraint_pairs, models))
+
+
+@pytest.mark.parametrize("stated", [0.0, 8.9, 1.0e4, 1.0e300])
+def test_the_stated_displacement_does_not_matter(big, stated):
+    """gd_score_frames_device in the FP64 form: max_displacement sizes the FP32
+    form's guard bands, FP64 energies are the same bits whatever it says."""
+    torch = pytest.importorskip("torch")
+    from gdock_gb300 import _lib
+    rec, lig = _first_atoms(big.receptor, 120), _first_atoms(big.ligand, 90)
+    lig = gd.position_ligand(rec, lig)
+    genes = synth.random_genes(np.random.default_rng(9), 40, max_displacement=9.0)
+    genes[7, 3] = 5000.0
+    cx = gd.Complex(rec, lig, big.restraint_pairs)
+    want = cx.score_poses(genes)
+    frames = torch.from_numpy(_lib.make_frames(genes)).to("cuda")
+    out = torch.zeros((len(genes), 6), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    cx.ctx.check(cx.lib.gd_score_frames_device(cx.h, frames.data_ptr(), len(genes), gd.GD_PREC_F64, stated,
+                                               out.data_ptr(), None))
+    cx.ctx.sync()
+    assert out.cpu().numpy().tobytes() == want.tobytes()
