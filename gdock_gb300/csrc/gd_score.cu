@@ -71,7 +71,7 @@ __host__ __device__ inline F64Smem f64_smem(int nr, int nl) {
   L.lt = take(cap);
   L.sph = take(sizeof(float4) * (cap / 32));
   L.rcnt = take(2 * (static_cast<size_t>(nr) + 1));  // 16-bit burial counts, two a word
-  L.lcnt = take(2 * (static_cast<size_t>(nl) + 1));
+  L.lcnt = take(2 * (cap + 1));  // of a turn's ligand atoms
   L.queue = take(2 * sizeof(uint32_t) * kQueue * kNW);
   L.row = take(sizeof(float4) * kRowBuf * kNW);
   L.red = take(3 * sizeof(__int128) * kNW);
@@ -169,7 +169,7 @@ struct PairEval {
   uint32_t *rcnt, *lcnt;
   int base;  // ligand atom of the shared arrays' first entry
 
-  // one listed pair per lane (on): w = receptor atom, ligand entry
+  // one listed pair per lane (on): w = receptor atom, ligand entry of the turn
   template <bool NEAR>
   __device__ __forceinline__ void eval(bool on, uint32_t w, ExactSum<> &vdw, ExactSum<> &elec) const {
     if (!on) return;
@@ -228,7 +228,7 @@ struct PairEval {
       if (SERIAL) pv = pv && m.y != __ldg(p.lig_serial + base + k);
       if (pd) {
         bury(rcnt, ri);
-        bury(lcnt, base + k);
+        bury(lcnt, k);
       }
       if (pv) {
         // softcore_lj_potential (src/fitness.rs:57-70) as 4 eps (x^2 - x) with
@@ -288,7 +288,11 @@ __global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const
   if (!p.models && tid < 16)
     reinterpret_cast<double *>(s_frame)[tid] = reinterpret_cast<const double *>(p.frames + pose)[tid];
   for (int i = tid; i < (p.nr + 1) / 2; i += kNT) s_rcnt[i] = 0;
-  for (int i = tid; i < (p.nl + 1) / 2; i += kNT) s_lcnt[i] = 0;
+  for (int i = tid; i < (min(p.nl, kLigCap) + 1) / 2; i += kNT) s_lcnt[i] = 0;
+  if (lane == 0) {
+    s_red[warp * 3 + 2] = 0;
+    s_nf[warp * 3 + 2] = 0.0;
+  }
   if (tid == 0) *s_next = 0;
   __syncthreads();
   const gd_pose_frame &f = *s_frame;
@@ -302,7 +306,30 @@ __global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const
   ExactSum<> vdw, elec;
   int first = 0;  // unit counter at the start of this turn
 
+  // desolvation of n atoms from the cluster's summed burial counts, a share per CTA
+  auto desolvate = [&](ExactSum<> &sum, uint32_t *cnt, const double *tab, int n) {
+    for (int i = rank * kNT + tid; i < n; i += nc * kNT) {
+      unsigned c = 0;
+      for (int r = 0; r < nc; ++r) {
+        const uint32_t *o = nc > 1 ? cluster.map_shared_rank(cnt, r) : cnt;
+        c += (o[i >> 1] >> ((i & 1) * 16)) & 0xffffu;
+      }
+      sum.add(tab[static_cast<size_t>(i) * 11 + min(c, 10u)], p.fx_desolv);
+    }
+  };
+  // ... added to the warp's sum in shared memory
+  auto keep_desolv = [&](ExactSum<> &sum) {
+    sum.warp_total();
+    if (lane == 0) {
+      s_red[warp * 3 + 2] += sum.v;
+      s_nf[warp * 3 + 2] += sum.nf;
+    }
+  };
+
+  // Ligands of more than kLigCap atoms in turns of equal length: a turn's atoms
+  // meet every receptor atom, so their burial counts are complete at its end.
   const int turns = (p.nl + kLigCap - 1) / kLigCap, turn = turns ? ((p.nl + turns - 1) / turns + 31) / 32 * 32 : 0;
+  const int l_last = turn ? (p.nl - 1) / turn * turn : 0;  // first atom of the last turn
   for (int l0 = 0; l0 < p.nl; l0 += turn) {
     const int nl = min(turn, p.nl - l0), nslot = (nl + 31) / 32, nunit = nslot * ngrp;
     // the CTA's share of the slots: one warp per slot, one atom per lane
@@ -490,9 +517,15 @@ __global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const
     __syncwarp();
     // every warp of the cluster drew one unit number past the last
     first += nunit + nc * kNW;
-    if (l0 + turn < p.nl) {
-      if (nc > 1) cluster.sync();  // nobody reads this turn's ligand atoms any more
+    if (l0 < l_last) {
+      if (nc > 1) cluster.sync();  // the counts are complete, nobody reads this turn's ligand atoms any more
       else __syncthreads();
+      ExactSum<> part;
+      desolvate(part, s_lcnt, p.lig_desolv + static_cast<size_t>(l0) * 11, nl);
+      keep_desolv(part);
+      if (nc > 1) cluster.sync();
+      else __syncthreads();
+      for (int i = tid; i < (nl + 1) / 2; i += kNT) s_lcnt[i] = 0;
     }
   }
 
@@ -508,31 +541,17 @@ __global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const
   }
   if (nc > 1) cluster.sync();
   else __syncthreads();
-  // desolvation from the cluster's summed burial counts, a share per CTA
   ExactSum<> desolv;
-  for (int side = 0; side < 2; ++side) {
-    const int n = side ? p.nl : p.nr;
-    const double *tab = side ? p.lig_desolv : p.rec_desolv;
-    uint32_t *cnt = side ? s_lcnt : s_rcnt;
-    for (int i = rank * kNT + tid; i < n; i += nc * kNT) {
-      unsigned c = 0;
-      for (int r = 0; r < nc; ++r) {
-        const uint32_t *o = nc > 1 ? cluster.map_shared_rank(cnt, r) : cnt;
-        c += (o[i >> 1] >> ((i & 1) * 16)) & 0xffffu;
-      }
-      desolv.add(tab[static_cast<size_t>(i) * 11 + min(c, 10u)], p.fx_desolv);
-    }
-  }
+  desolvate(desolv, s_rcnt, p.rec_desolv, p.nr);
+  desolvate(desolv, s_lcnt, p.lig_desolv + static_cast<size_t>(l_last) * 11, p.nl - l_last);
+  keep_desolv(desolv);
   vdw.warp_total();
   elec.warp_total();
-  desolv.warp_total();
   if (lane == 0) {
     s_red[warp * 3] = vdw.v;
     s_red[warp * 3 + 1] = elec.v;
-    s_red[warp * 3 + 2] = desolv.v;
     s_nf[warp * 3] = vdw.nf;
     s_nf[warp * 3 + 1] = elec.nf;
-    s_nf[warp * 3 + 2] = desolv.nf;
   }
   if (nc > 1) cluster.sync();
   else __syncthreads();

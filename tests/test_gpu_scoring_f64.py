@@ -146,3 +146,16 @@ def test_the_stated_displacement_does_not_matter(big, stated):
                                                out.data_ptr(), None))
     cx.ctx.sync()
     assert out.cpu().numpy().tobytes() == want.tobytes()
+
+
+@pytest.mark.parametrize("nr,nl,n", [(40, 90000, 1), (40, 90000, 3), (5, 120001, 2)])
+def test_long_ligands(oracle, big, nr, nl, n):
+    """Ligands of any length: their burial counts are held a turn at a time."""
+    from conftest import make_mol, tatom
+    rng = np.random.default_rng(nl)
+    rec = make_mol([tatom(*x, "CNO"[k % 3], charge=0.3, serial=k + 1) for k, x in enumerate(rng.normal(0, 4.0, (nr, 3)))])
+    lig = make_mol([tatom(*x, "CNO"[k % 3], charge=0.2, serial=1000 + k, chain="B")
+                    for k, x in enumerate(rng.uniform(-30, 30, (nl, 3)))])
+    genes = synth.random_genes(rng, n, max_displacement=9.0)
+    cx = gd.Complex(rec, lig, [])
+    check(cx.score_poses(genes), oracle.score_poses(rec, lig, [], genes), F64_TOL)
