@@ -38,6 +38,9 @@ gd_status fail(gd_context *ctx, gd_status s, const std::string &msg) {
 }
 
 gd_status cuda_fail(gd_context *ctx, cudaError_t e, const char *what) {
+  // reported here: cleared, so that the check after a later launch does not
+  // read it back (errors that end the context stay)
+  (void)cudaGetLastError();
   std::string m = std::string(what) + ": " + cudaGetErrorName(e) + " (" + cudaGetErrorString(e) + ")";
   return fail(ctx, e == cudaErrorMemoryAllocation ? GD_ERR_OOM : GD_ERR_CUDA, m);
 }
@@ -51,10 +54,6 @@ gd_status dev_alloc(gd_context *ctx, uint64_t bytes, void **p) {
   cudaError_t e = cudaMalloc(p, bytes);
   if (e != cudaSuccess) {
     *p = nullptr;
-    // a failed allocation is not a sticky error: clear it, so that a caller
-    // that falls back to a smaller plan does not read it back from
-    // cudaGetLastError() after its next launch
-    (void)cudaGetLastError();
     return cuda_fail(ctx, e, "cudaMalloc");
   }
   ctx->in_use += bytes;

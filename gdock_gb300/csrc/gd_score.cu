@@ -712,7 +712,18 @@ gd_status launch_score(gd_complex *cx, const gd_pose_frame *d_frames, const doub
     else e = clamp ? launch_f64(k_score_f64<false, false, true>, p, sm, stream)
                    : launch_f64(k_score_f64<false, false, false>, p, sm, stream);
   }
-  if (e != cudaSuccess) return cuda_fail(ctx, e, "score kernel launch");
+  if (e != cudaSuccess) {
+    // the one size that the form does not take: the receptor's burial counts
+    const size_t need = f64_smem(p.nr, p.nl).total;
+    int most = 0;
+    if (cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device) == cudaSuccess &&
+        need > static_cast<size_t>(most)) {
+      const std::string what = "score kernel launch: a receptor of " + std::to_string(p.nr) + " atoms takes " +
+                               std::to_string(need) + " bytes of shared memory a block, there are " + std::to_string(most);
+      return cuda_fail(ctx, e, what.c_str());
+    }
+    return cuda_fail(ctx, e, "score kernel launch");
+  }
   return GD_OK;
 }
 

@@ -159,3 +159,21 @@ def test_long_ligands(oracle, big, nr, nl, n):
     genes = synth.random_genes(rng, n, max_displacement=9.0)
     cx = gd.Complex(rec, lig, [])
     check(cx.score_poses(genes), oracle.score_poses(rec, lig, [], genes), F64_TOL)
+
+
+def test_a_refused_receptor_leaves_no_error_behind(oracle, big):
+    """A receptor whose counts do not fit a CTA's shared memory is refused;
+    the next calls are not (a launch's check reads no older error)."""
+    from conftest import make_mol, tatom
+    xyz = np.random.default_rng(11).uniform(-90, 90, (150000, 3))
+    rec = make_mol([tatom(*x, serial=k + 1) for k, x in enumerate(xyz)])
+    lig = make_mol([tatom(0, 0, 0, charge=0.2, serial=200000, chain="B")])
+    cx = gd.Complex(rec, lig, [])
+    with pytest.raises(Exception, match="shared memory"):
+        cx.score_poses(np.zeros((1, 6)))
+    rec, lig = _first_atoms(big.receptor, 120), _first_atoms(big.ligand, 90)
+    lig = gd.position_ligand(rec, lig)
+    genes = synth.random_genes(np.random.default_rng(12), 3, max_displacement=5.0)
+    ok = gd.Complex(rec, lig, [])
+    assert len(ok.pose_contacts(genes)) == 3
+    check(ok.score_poses(genes), oracle.score_poses(rec, lig, [], genes), F64_TOL)
