@@ -47,6 +47,7 @@ constexpr int kQueue = 32 * (kRows + 1);  // listed pairs per warp and kind: 31 
 constexpr int kRowsMin = 8, kRowsMax = 128;  // receptor atoms of a unit (a power of two)
 constexpr int kMaxCluster = 16;
 constexpr int kTinyHi = 0x2b000000;   // high word of 2^-335: below it r^6 may underflow
+constexpr unsigned kFixCoarse = 1u << 21;  // 1/8 A^2 as a fixed-point d2's high word
 
 struct F64Smem {
   size_t x, y, z, q, fx, fy, fz, lt, sph, rcnt, lcnt, queue, row, red, nf, frame, misc, total;
@@ -153,11 +154,13 @@ __device__ __noinline__ ExactPair exact_pair(const ScoreParams &p, const gd_pose
 __device__ __forceinline__ bool near_hi(int hi, double t) {
   return static_cast<unsigned>(hi - (__double2hiint(t) - 1)) <= 2u;
 }
-// FIX: d2 from integer coordinates.  The differences and the three squares are
-// exact and d2 is truncated below 2^-56 A^2, so its error is the coordinates'
-// rounding to 2^-52 A, less than theirs as doubles above 4 A.  It takes about
-// 45 integer instructions a pair, which issue beside the FP64 pipe, in place of
-// 6 FP64 ones.
+// FIX: d2 from integer coordinates of 2^-51 A.  Doubles from 2 A on lie on that
+// grid; a smaller coordinate moves by 2^-52 A at most, of the order of what the
+// transform's own roundings leave.  The differences and the three squares are
+// exact and d2 is truncated below 2^-56 A^2, half a unit in a double's last place
+// from 1/8 A^2 on; closer pairs (a few in a million) are formed in FP64 in the
+// reference's order.  It takes about 45 integer instructions a pair, which issue
+// beside the FP64 pipe, in place of 6 FP64 ones.
 template <bool FIX, bool SERIAL, bool CLAMP>
 struct PairEval {
   const ScoreParams &p;
@@ -195,7 +198,7 @@ struct PairEval {
         pv = hw < (144u << 24);
         pd = hw < (64u << 24);
         pe = pe && hw >= (1u << 24);
-        rare = rare | near_fix(hw, 144u) | near_fix(hw, 64u) | near_fix(hw, 1u) | (hw == 0u);
+        rare = rare | near_fix(hw, 144u) | near_fix(hw, 64u) | near_fix(hw, 1u) | (hw < kFixCoarse);
       }
     } else {
       const double2 *rp = reinterpret_cast<const double2 *>(p.rec_pos64 + ri);

@@ -177,3 +177,21 @@ def test_a_refused_receptor_leaves_no_error_behind(oracle, big):
     ok = gd.Complex(rec, lig, [])
     assert len(ok.pose_contacts(genes)) == 3
     check(ok.score_poses(genes), oracle.score_poses(rec, lig, [], genes), F64_TOL)
+
+
+@pytest.mark.parametrize("square", [1e-4, 0.01, 0.1, 0.1249, 0.1251])
+def test_small_distances(oracle, square):
+    """Pairs of narrow atoms 0.01 to 0.4 A apart, where the integers' step of
+    2^-56 A^2 is coarser than a double's."""
+    from conftest import make_mol, tatom
+    rmin = 0.05 * np.sqrt(square)
+    rec = make_mol([tatom(50.0, 3.0, 7.0, charge=0.5, epsilon=-4.0, rmin2=rmin)])
+    lig = make_mol([tatom(50.0, 3.0, 7.0, charge=0.3, epsilon=-4.0, rmin2=rmin, serial=9, chain="B")])
+    xyz = np.tile(np.array([50.0, 3.0, 7.0]), (20, 1, 1))
+    u = np.random.default_rng(10).normal(size=(20, 1, 3))
+    xyz += u / np.linalg.norm(u, axis=2)[..., None] * np.sqrt(square)
+    got = gd.Complex(rec, lig, []).score_models(xyz)["vdw"]
+    ref = oracle.score_models(rec, lig, [], xyz)[:, 1]
+    # one term: a dozen FP64 roundings of the reference's and of this form's,
+    # 6 r times d2's for r^6
+    assert np.abs(got / ref - 1.0).max() <= 2.0 ** -49
