@@ -117,10 +117,13 @@ static __device__ __forceinline__ void relative_atom(const ScoreParams &p, const
   z = __fma_rn(-f.sb, r.x, __fma_rn(f.cb * f.sg, r.y, __fma_rn(f.cb * f.cg, r.z, tz)));
 }
 // One coordinate of the rotated atom: nine 32 x 32 -> 64 multiply-adds of
-// three products, the low limbs' dropped (three units of 2^-51 A at most; an
-// FP64 chain of multiply-adds errs by ten times as much at 60 A).
+// three products, the low limbs' dropped.  Those are of either sign and the sum
+// is rounded, so that the error, five quarters of a unit of 2^-51 A at most, is as
+// often up as down and averages out over a pose's atoms (limbs from 0 up and a
+// sum rounded down put every atom 5e-16 A to one side on average).  An FP64 chain
+// of multiply-adds errs by ten times as much at 60 A.
 static __device__ __forceinline__ long long rotate(const Limbs &a, const Limbs &b, const Limbs &c, const int4 &xy, const int4 &z) {
-  long long hi = static_cast<long long>(a.h) * xy.x, mid = static_cast<long long>(a.h) * xy.y;
+  long long hi = static_cast<long long>(a.h) * xy.x, mid = static_cast<long long>(a.h) * xy.y + (1 << 28);
   hi += static_cast<long long>(b.h) * xy.z;
   mid += static_cast<long long>(a.l) * xy.x;
   hi += static_cast<long long>(c.h) * z.x;

@@ -260,14 +260,17 @@ __global__ void __launch_bounds__(kEvalWarps * 32, kEvalCtas) k_dockq(const Eval
       const double a = lane == 0 ? f.ca : lane == 1 ? f.m01 : lane == 2 ? f.m02 : lane == 3 ? f.sa : lane == 4 ? f.m11
                        : lane == 5 ? f.m12 : lane == 6 ? -f.sb : f.cb;
       const double b = lane == 0 || lane == 3 ? f.cb : lane == 7 ? f.sg : lane == 8 ? f.cg : 1.0;
-      const double m = __dmul_rn(a, b);
+      // (the product with what its rounding drops, which every atom would share)
+      const double m = __dmul_rn(a, b), rest = __fma_rn(a, b, -m);
       ok = fabs(m) <= 1.5;
-      s_m[warp][lane] = limbs(ok ? __double2ll_rn(m * 0x1p59) : 0);
+      s_m[warp][lane] = limbs(ok ? __double2ll_rn(m * 0x1p59) + __double2ll_rn(rest * 0x1p59) : 0);
     } else if (lane < 12) {
-      const double t = lane == 9 ? e.p.cx + f.dx : lane == 10 ? e.p.cy + f.dy : e.p.cz + f.dz;
+      // (centre and displacement converted apart: their FP64 sum is rounded, again
+      // for every atom alike)
+      const double c = lane == 9 ? e.p.cx : lane == 10 ? e.p.cy : e.p.cz, d = lane == 9 ? f.dx : lane == 10 ? f.dy : f.dz;
       const long long o = lane == 9 ? e.ox : lane == 10 ? e.oy : e.oz;
-      ok = fabs(t) < 4000.0;
-      const long long v = ok ? __double2ll_rn(t * 0x1p51) - o : 0;
+      ok = fabs(c) < 4000.0 && fabs(d) < 4000.0 && fabs(c + d) < 4000.0;
+      const long long v = ok ? __double2ll_rn(c * 0x1p51) + __double2ll_rn(d * 0x1p51) - o : 0;
       ok = ok && llabs(v) < static_cast<long long>(kFixFar * 0x1p51);
       s_t[warp][lane - 9] = v;
     }

@@ -84,14 +84,15 @@ struct Thresholds {
 };
 
 // Fixed point.  Ligand atoms (relative to the rotation centre, below 512 A) are
-// integers of 2^-50 A in two limbs h 2^29 + l, matrix entries (at most 1.5) of
-// 2^-59 likewise; positions and differences are 2^-51 A, translations and
+// integers of 2^-50 A in two limbs h 2^29 + l, l of either sign, matrix entries
+// (at most 1.5) of 2^-59 likewise; positions and differences are 2^-51 A, translations and
 // reference atoms within 768 A of the origin, so that a difference stays below
 // 2^12 A.
 constexpr double kFixAtom = 512.0, kFixFar = 768.0;
 struct Limbs { int h, l; };
 __host__ __device__ __forceinline__ Limbs limbs(long long v) {
-  return Limbs{static_cast<int>(v >> 29), static_cast<int>(v & ((1 << 29) - 1))};
+  const long long h = (v + (1 << 28)) >> 29;
+  return Limbs{static_cast<int>(h), static_cast<int>(v - (h << 29))};
 }
 
 struct ScoreParams {

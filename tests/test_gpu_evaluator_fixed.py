@@ -48,3 +48,35 @@ def test_range(oracle, arm, at):
                     tatom(at - arm, 3, 2, resseq=1, chain="B")])
     genes = np.concatenate([np.zeros((1, 6)), rng.uniform(0, 6, (4, 6)), [[1, 2, 3, 760.0, 0, 0], [1, 2, 3, 0, -775.0, 0]]])
     run(oracle, rec, lig, ref, genes)
+
+
+@pytest.mark.parametrize("n", [64, 3000])
+def test_near_native_sums_have_no_bias(n):
+    """Poses 0.3 to 1 A from the reference structure, the centre at hundreds of
+    A: an error that all atoms share does not average out of the RMSD.  Against
+    extended precision from the same frames.  Tolerance: centre and displacement
+    rounded to 2^-51 A, 8e-16 A on the distance, over 0.25 A and halved by the
+    root, and 2.2e-16 for sum, division and root."""
+    from gdock_gb300 import _lib
+    if np.finfo(np.longdouble).eps > 2e-19:
+        pytest.skip("no extended precision here")
+    rng = np.random.default_rng(n)
+    at = np.array([500.0, -300.0, 200.0])
+    rec = make_mol([tatom(*x, resseq=1 + k // 8, chain="A", serial=k + 1)
+                    for k, x in enumerate(np.round(at + rng.normal(0, 9, (40, 3)), 3))])
+    xyz = np.round(at + rng.normal(0, 8, (300, 3)), 3)
+    lig = make_mol([tatom(*x, resseq=1 + k // 8, chain="B", serial=50 + k) for k, x in enumerate(xyz)])
+    genes = rng.normal(0, 0.002, (n, 6))
+    genes[:, 3:] = rng.uniform(0.25, 0.5, (n, 3)) * rng.choice([-1, 1], (n, 3))
+    got = gd.Evaluator(gd.Complex(rec, lig, []), lig).eval_metrics(genes)["rmsd"]
+    f = _lib.make_frames(genes).astype(np.longdouble)[:40]  # ca sa cb sb cg sg m01 m02 m11 m12 dx dy dz
+    ca, sa, cb, sb, cg, sg, m01, m02, m11, m12 = f[:, :10].T
+    rot = np.array([[ca * cb, m01, m02], [sa * cb, m11, m12], [-sb, cb * sg, cb * cg]])  # 3 x 3 x poses
+    c = np.array([np.cumsum(v)[-1] / len(v) for v in (lig.x, lig.y, lig.z)]).astype(np.longdouble)
+    x = xyz.astype(np.longdouble) - c
+    moved = [sum(rot[i, j][:, None] * x[None, :, j] for j in range(3)) + c[i] + f[:, 10 + i, None] for i in range(3)]
+    d = np.sqrt(sum((moved[i] - xyz[None, :, i]) ** 2 for i in range(3)))
+    assert d.min() > 0.25
+    want = np.sqrt(d.sum(axis=1) / len(xyz))
+    err = np.abs(got[:40] / want - 1)
+    assert err.max() <= 2e-15, float(err.max())
