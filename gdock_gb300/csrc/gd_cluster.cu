@@ -840,7 +840,9 @@ __global__ void __launch_bounds__(kGreedyThreads)
       label[e0 + r] = -1;
     }
   }
-  __syncthreads();
+  // (every CTA has started before its s_best is written to)
+  if (nc > 1) cluster.sync();
+  else __syncthreads();
   int k = 0;
   for (;; ++k) {
     // the unused element with the largest count, lower index on ties: the
