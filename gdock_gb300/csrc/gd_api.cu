@@ -92,19 +92,25 @@ gd_status ensure_scratch(gd_context *ctx, size_t dev_bytes, size_t pinned_bytes)
   return GD_OK;
 }
 
-gd_status ensure_batch_scratch(gd_context *ctx, size_t dev_bytes) {
-  if (dev_bytes <= ctx->d_batch_bytes) return GD_OK;
-  if (ctx->d_batch) {
+static gd_status grow(gd_context *ctx, void **p, size_t *have, size_t dev_bytes) {
+  if (dev_bytes <= *have) return GD_OK;
+  if (*p) {
     cudaStreamSynchronize(ctx->stream);
-    dev_free(ctx, ctx->d_batch, ctx->d_batch_bytes);
+    dev_free(ctx, *p, *have);
   }
-  ctx->d_batch = nullptr;
-  ctx->d_batch_bytes = 0;
+  *p = nullptr;
+  *have = 0;
   const size_t want = std::max(dev_bytes, static_cast<size_t>(1) << 20);
-  gd_status s = dev_alloc(ctx, want, &ctx->d_batch);
+  gd_status s = dev_alloc(ctx, want, p);
   if (s != GD_OK) return s;
-  ctx->d_batch_bytes = want;
+  *have = want;
   return GD_OK;
+}
+gd_status ensure_batch_scratch(gd_context *ctx, size_t dev_bytes) {
+  return grow(ctx, &ctx->d_batch, &ctx->d_batch_bytes, dev_bytes);
+}
+gd_status ensure_cluster_scratch(gd_context *ctx, size_t dev_bytes) {
+  return grow(ctx, &ctx->d_cluster, &ctx->d_cluster_bytes, dev_bytes);
 }
 
 // The context's error word after a wait for the work that may set it: it lies
@@ -486,6 +492,7 @@ gd_status gd_context_destroy(gd_context *ctx) {
   cudaStreamSynchronize(ctx->stream);
   if (ctx->d_scratch) cudaFree(ctx->d_scratch);
   if (ctx->d_batch) cudaFree(ctx->d_batch);
+  if (ctx->d_cluster) cudaFree(ctx->d_cluster);
   if (ctx->h_pinned) cudaFreeHost(ctx->h_pinned);
   if (ctx->d_err) cudaFreeHost(ctx->d_err);
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);

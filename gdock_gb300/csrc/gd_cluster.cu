@@ -2051,12 +2051,13 @@ gd_status cluster_device(gd_complex *cx, const double *genes, int n, const gd_cl
                  list_b = al256(sizeof(int) * std::max<size_t>(memberships, 1)),
                  common_b = al256(sizeof(uint32_t) * static_cast<size_t>(n) * n);
     size_t extra_b = (postings ? off_b + kc_b + list_b + common_b : rows_b) + adj_b + greedy_bytes(n);
-    // up to 64 MiB from the context's kept scratch, else for this call alone
-    const bool kept = !postings && extra_b <= (size_t(64) << 20);
+    // up to 64 MiB from scratch that the context keeps for this (not where a
+    // budget bounds what it may hold), else for this call alone
+    const bool kept = !postings && ctx->budget == 0 && extra_b <= (size_t(64) << 20);
     void *extra = nullptr;
     if (kept) {
-      s = ensure_batch_scratch(ctx, extra_b);
-      extra = ctx->d_batch;
+      s = ensure_cluster_scratch(ctx, extra_b);
+      extra = ctx->d_cluster;
     } else {
       s = dev_alloc(ctx, extra_b, &extra);
     }

@@ -158,9 +158,14 @@ struct gd_context {
   size_t d_scratch_bytes = 0;
   void *h_pinned = nullptr;
   size_t h_pinned_bytes = 0;
-  // argument blocks of batched launches (descriptors, queue, counters)
+  // argument blocks of batched launches (descriptors, queue, counters): such a
+  // launch may still be running, on a stream of the caller's, when its call has
+  // returned, so nothing else may use it
   void *d_batch = nullptr;
   size_t d_batch_bytes = 0;
+  // rows, adjacency and results of clustering calls (contexts without a budget)
+  void *d_cluster = nullptr;
+  size_t d_cluster_bytes = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   int tune_f32_slots = 0;  // 0: automatic (kDefaultF32Tune)
   int tune_split = 0;      // GD_TUNE_SPLIT: 0 automatic, 1 whole poses, 2 always split
@@ -262,6 +267,7 @@ void enclosing_ball(const double *x, const double *y, const double *z, const int
                     double &r);
 std::vector<int> compact_runs(const double *x, const double *y, const double *z, int n, int unit, int sub);
 gd_status ensure_batch_scratch(gd_context *ctx, size_t dev_bytes);
+gd_status ensure_cluster_scratch(gd_context *ctx, size_t dev_bytes);
 ScoreParams make_params(gd_complex *cx, const gd_pose_frame *d_frames, const double *d_models, int n,
                         gd_pose_energy *d_out, double max_disp);
 gd_status launch_score_batch_f32(gd_context *ctx, const std::vector<ScoreParams> &descs, bool serial, bool clamp,

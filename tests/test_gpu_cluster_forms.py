@@ -92,3 +92,43 @@ def test_lists_within_a_budget():
             cx.close()
             ctx.close()
     assert out[0] == out[1]
+
+
+def test_beside_scoring_on_a_stream():
+    """An FP32 gd_score_frames_device call returns before its launch has run, so
+    a clustering call made right after it must not use that launch's memory:
+    energies and clusters are those of the calls alone."""
+    torch = pytest.importorskip("torch")
+    from gdock_gb300 import _lib, synth
+    c = synth.make_complex(300, 150, 4, seed=8)
+    ctx = gd.Context(0)
+    cx = gd.Complex(c.receptor, gd.position_ligand(c.receptor, c.ligand), c.restraint_pairs, ctx=ctx)
+    try:
+        genes = synth.quaternion_genes(np.random.default_rng(4), 20000, half_box=20.0)
+        poses = genes[:3000]  # rows past what small calls keep beside the contact lists
+        frames = torch.from_numpy(_lib.make_frames(genes)).to("cuda")
+        out = torch.zeros((len(genes), 6), dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        stream = torch.cuda.Stream()
+
+        def score():
+            ctx.check(ctx.lib.gd_score_frames_device(cx.h, frames.data_ptr(), len(genes), gd.GD_PREC_F32, 20.0,
+                                                     out.data_ptr(), stream.cuda_stream))
+
+        def clusters():
+            return [(r.center_idx, r.members) for r in cx.cluster(poses, gd.ClusteringConfig(min_cluster_size=1))]
+
+        score()
+        stream.synchronize()
+        energies, alone = out.cpu().numpy().tobytes(), clusters()
+        for _ in range(3):
+            out.zero_()
+            torch.cuda.synchronize()
+            score()
+            assert clusters() == alone
+            stream.synchronize()
+            ctx.sync()
+            assert out.cpu().numpy().tobytes() == energies
+    finally:
+        cx.close()
+        ctx.close()
