@@ -243,15 +243,16 @@ __device__ __forceinline__ float3 atom32(const ScoreParams &p, const gd_pose_fra
   return make_float3(static_cast<float>(x), static_cast<float>(y), static_cast<float>(z));
 }
 
-// Warp-wide minimum and maximum, one instruction each.
+// Warp-wide minimum and maximum, one instruction each (volatile: every lane takes
+// part, so the compiler must not sink them into a branch).
 __device__ __forceinline__ float warp_min(float v) {
   float r;
-  asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
   return r;
 }
 __device__ __forceinline__ float warp_max(float v) {
   float r;
-  asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
   return r;
 }
 

@@ -41,3 +41,23 @@ def test_blocks_have_started_before_their_shared_memory_is_touched(file, name, b
             uses = [end + later.index(s) for s in (m.group(1) + "(", "map_shared_rank") if s in later]
             first = min(uses)
     assert "cluster.sync()" in body[:first], name
+
+
+def collectives():
+    """(file, statement) of every inline assembly statement that all lanes of a
+    warp, or threads of a block, take part in."""
+    for f in sorted([*CSRC.glob("*.cu"), *CSRC.glob("*.cuh")]):
+        src = re.sub(r"//[^\n]*", "", f.read_text())
+        for m in re.finditer(r"\basm\b", src):
+            stmt = src[m.start():src.index(";\n", m.start())]
+            if re.search(r"\.sync\b|\bbar\.|\bbarrier\.", stmt):
+                yield f.name, stmt
+
+
+def test_collective_assembly_stays_where_it_is_written():
+    """A statement that is not volatile may be moved, or sunk into a branch that
+    some lanes do not take, as if it were a function of its operands alone."""
+    found = list(collectives())
+    assert found
+    for file, stmt in found:
+        assert re.match(r"asm\s+volatile\b", stmt), (file, stmt)
