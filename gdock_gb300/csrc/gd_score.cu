@@ -41,19 +41,26 @@ constexpr int kNT = 256;              // threads per CTA of k_score_f64
 constexpr int kNW = kNT / 32;
 constexpr int kLigBits = 10;
 constexpr int kLigCap = 1 << kLigBits;  // ligand atoms held in shared memory at once (longer ligands: in turns)
+// Ligands up to this many atoms have their burial counts in shared memory from
+// first to last; longer ones a turn at a time, in a variant of its own: the turn's
+// end in the common one cost its pairs 2.5 % (registers), and the counts of longer
+// ligands in shared memory cost a resident CTA.  300 poses on 2,538 atoms, all
+// counts / a turn's: ligands of 3,000 atoms 2.16 / 2.38 ms, 4,200 2.87 / 3.18, 6,000
+// 4.37 / 3.87, 20,000 11.3 / 9.6.
+constexpr int kLigCounts = 4096;
 constexpr int kRows = 4;              // rows searched per step
 constexpr int kRowBuf = 32 + kRows;   // rows waiting per warp: fewer than a step and 32 more
 constexpr int kQueue = 32 * (kRows + 1);  // listed pairs per warp and kind: 31 left over + 32 of each row
 constexpr int kRowsMin = 8, kRowsMax = 128;  // receptor atoms of a unit (a power of two)
 constexpr int kMaxCluster = 16;
-constexpr int kTinyHi = 0x2b000000;   // high word of 2^-335: below it r^6 may underflow
 constexpr unsigned kFixCoarse = 1u << 21;  // 1/8 A^2 as a fixed-point d2's high word
+constexpr int kTinyHi = 0x2b000000;   // high word of 2^-335: below it r^6 may underflow
 
 struct F64Smem {
   size_t x, y, z, q, fx, fy, fz, lt, sph, rcnt, lcnt, queue, row, red, nf, frame, misc, total;
 };
 
-__host__ __device__ inline F64Smem f64_smem(int nr, int nl) {
+__host__ __device__ inline F64Smem f64_smem(int nr, int nl, bool turns) {
   F64Smem L;
   size_t o = 0;
   const size_t cap = nl < kLigCap ? (static_cast<size_t>(nl) + 31) / 32 * 32 : kLigCap;
@@ -72,7 +79,7 @@ __host__ __device__ inline F64Smem f64_smem(int nr, int nl) {
   L.lt = take(cap);
   L.sph = take(sizeof(float4) * (cap / 32));
   L.rcnt = take(2 * (static_cast<size_t>(nr) + 1));  // 16-bit burial counts, two a word
-  L.lcnt = take(2 * (cap + 1));  // of a turn's ligand atoms
+  L.lcnt = take(2 * ((turns ? cap : static_cast<size_t>(nl)) + 1));
   L.queue = take(2 * sizeof(uint32_t) * kQueue * kNW);
   L.row = take(sizeof(float4) * kRowBuf * kNW);
   L.red = take(3 * sizeof(__int128) * kNW);
@@ -161,7 +168,7 @@ __device__ __forceinline__ bool near_hi(int hi, double t) {
 // from 1/8 A^2 on; closer pairs (a few in a million) are formed in FP64 in the
 // reference's order.  It takes about 45 integer instructions a pair, which issue
 // beside the FP64 pipe, in place of 6 FP64 ones.
-template <bool FIX, bool SERIAL, bool CLAMP>
+template <bool FIX, bool SERIAL, bool CLAMP, bool TURNS>
 struct PairEval {
   const ScoreParams &p;
   const gd_pose_frame &f;
@@ -172,7 +179,7 @@ struct PairEval {
   uint32_t *rcnt, *lcnt;
   int base;  // ligand atom of the shared arrays' first entry
 
-  // one listed pair per lane (on): w = receptor atom, ligand entry of the turn
+  // one listed pair per lane (on): w = receptor atom, ligand entry
   template <bool NEAR>
   __device__ __forceinline__ void eval(bool on, uint32_t w, ExactSum<> &vdw, ExactSum<> &elec) const {
     if (!on) return;
@@ -231,7 +238,7 @@ struct PairEval {
       if (SERIAL) pv = pv && m.y != __ldg(p.lig_serial + base + k);
       if (pd) {
         bury(rcnt, ri);
-        bury(lcnt, k);
+        bury(lcnt, TURNS ? k : base + k);
       }
       if (pv) {
         // softcore_lj_potential (src/fitness.rs:57-70) as 4 eps (x^2 - x) with
@@ -262,11 +269,11 @@ struct PairEval {
 // pair; listed pairs; d2 from integers; reciprocals, short sums, row buffer), 150
 // poses 29.0 -> 2.38 -> 1.72 -> 1.40 ms; one pose of 411 x 649 atoms 1,746 -> 89
 // -> 53 us a call.
-template <bool FIX, bool SERIAL, bool CLAMP>
+template <bool FIX, bool SERIAL, bool CLAMP, bool TURNS>
 __global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const int unit_rows) {
   if (p.skip && *p.skip) return;
   extern __shared__ __align__(128) unsigned char smem[];
-  const F64Smem L = f64_smem(p.nr, p.nl);
+  const F64Smem L = f64_smem(p.nr, p.nl, TURNS);
   double *s_x = reinterpret_cast<double *>(smem + L.x), *s_y = reinterpret_cast<double *>(smem + L.y),
          *s_z = reinterpret_cast<double *>(smem + L.z), *s_q = reinterpret_cast<double *>(smem + L.q);
   float *s_fx = reinterpret_cast<float *>(smem + L.fx), *s_fy = reinterpret_cast<float *>(smem + L.fy),
@@ -291,8 +298,8 @@ __global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const
   if (!p.models && tid < 16)
     reinterpret_cast<double *>(s_frame)[tid] = reinterpret_cast<const double *>(p.frames + pose)[tid];
   for (int i = tid; i < (p.nr + 1) / 2; i += kNT) s_rcnt[i] = 0;
-  for (int i = tid; i < (min(p.nl, kLigCap) + 1) / 2; i += kNT) s_lcnt[i] = 0;
-  if (lane == 0) {
+  for (int i = tid; i < ((TURNS ? min(p.nl, kLigCap) : p.nl) + 1) / 2; i += kNT) s_lcnt[i] = 0;
+  if (TURNS && lane == 0) {
     s_red[warp * 3 + 2] = 0;
     s_nf[warp * 3 + 2] = 0.0;
   }
@@ -309,30 +316,7 @@ __global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const
   ExactSum<> vdw, elec;
   int first = 0;  // unit counter at the start of this turn
 
-  // desolvation of n atoms from the cluster's summed burial counts, a share per CTA
-  auto desolvate = [&](ExactSum<> &sum, uint32_t *cnt, const double *tab, int n) {
-    for (int i = rank * kNT + tid; i < n; i += nc * kNT) {
-      unsigned c = 0;
-      for (int r = 0; r < nc; ++r) {
-        const uint32_t *o = nc > 1 ? cluster.map_shared_rank(cnt, r) : cnt;
-        c += (o[i >> 1] >> ((i & 1) * 16)) & 0xffffu;
-      }
-      sum.add(tab[static_cast<size_t>(i) * 11 + min(c, 10u)], p.fx_desolv);
-    }
-  };
-  // ... added to the warp's sum in shared memory
-  auto keep_desolv = [&](ExactSum<> &sum) {
-    sum.warp_total();
-    if (lane == 0) {
-      s_red[warp * 3 + 2] += sum.v;
-      s_nf[warp * 3 + 2] += sum.nf;
-    }
-  };
-
-  // Ligands of more than kLigCap atoms in turns of equal length: a turn's atoms
-  // meet every receptor atom, so their burial counts are complete at its end.
   const int turns = (p.nl + kLigCap - 1) / kLigCap, turn = turns ? ((p.nl + turns - 1) / turns + 31) / 32 * 32 : 0;
-  const int l_last = turn ? (p.nl - 1) / turn * turn : 0;  // first atom of the last turn
   for (int l0 = 0; l0 < p.nl; l0 += turn) {
     const int nl = min(turn, p.nl - l0), nslot = (nl + 31) / 32, nunit = nslot * ngrp;
     // the CTA's share of the slots: one warp per slot, one atom per lane
@@ -425,7 +409,7 @@ __global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const
     }
     __syncthreads();
 
-    const PairEval<FIX, SERIAL, CLAMP> ev{p, f, pose, s_x, s_y, s_z, s_q, s_lt, s_rcnt, s_lcnt, l0};
+    const PairEval<FIX, SERIAL, CLAMP, TURNS> ev{p, f, pose, s_x, s_y, s_z, s_q, s_lt, s_rcnt, s_lcnt, l0};
     int *next = nc > 1 ? cluster.map_shared_rank(s_next, 0) : s_next;
     int nn = 0, nf = 0;  // listed near and far pairs of this warp
     for (;;) {
@@ -520,15 +504,26 @@ __global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const
     __syncwarp();
     // every warp of the cluster drew one unit number past the last
     first += nunit + nc * kNW;
-    if (l0 < l_last) {
-      if (nc > 1) cluster.sync();  // the counts are complete, nobody reads this turn's ligand atoms any more
+    if (l0 + turn < p.nl) {
+      if (nc > 1) cluster.sync();  // nobody reads this turn's ligand atoms any more
       else __syncthreads();
-      ExactSum<> part;
-      desolvate(part, s_lcnt, p.lig_desolv + static_cast<size_t>(l0) * 11, nl);
-      keep_desolv(part);
-      if (nc > 1) cluster.sync();
-      else __syncthreads();
-      for (int i = tid; i < (nl + 1) / 2; i += kNT) s_lcnt[i] = 0;
+      if constexpr (TURNS) {
+        // a turn's atoms have met every receptor atom: their counts are complete
+        ExactSum<> part;
+        for (int i = rank * kNT + tid; i < nl; i += nc * kNT) {
+          unsigned c = 0;
+          for (int r = 0; r < nc; ++r) c += (cluster.map_shared_rank(s_lcnt, r)[i >> 1] >> ((i & 1) * 16)) & 0xffffu;
+          part.add(p.lig_desolv[static_cast<size_t>(l0 + i) * 11 + min(c, 10u)], p.fx_desolv);
+        }
+        part.warp_total();
+        if (lane == 0) {
+          s_red[warp * 3 + 2] += part.v;
+          s_nf[warp * 3 + 2] += part.nf;
+        }
+        if (nc > 1) cluster.sync();
+        else __syncthreads();
+        for (int i = tid; i < (nl + 1) / 2; i += kNT) s_lcnt[i] = 0;
+      }
     }
   }
 
@@ -544,17 +539,36 @@ __global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const
   }
   if (nc > 1) cluster.sync();
   else __syncthreads();
+  // desolvation from the cluster's summed burial counts, a share per CTA
   ExactSum<> desolv;
-  desolvate(desolv, s_rcnt, p.rec_desolv, p.nr);
-  desolvate(desolv, s_lcnt, p.lig_desolv + static_cast<size_t>(l_last) * 11, p.nl - l_last);
-  keep_desolv(desolv);
+  const int l_left = TURNS && turn ? (p.nl - 1) / turn * turn : 0;  // first ligand atom not summed yet
+  for (int side = 0; side < 2; ++side) {
+    const int n = side ? p.nl - l_left : p.nr;
+    const double *tab = side ? p.lig_desolv + static_cast<size_t>(l_left) * 11 : p.rec_desolv;
+    uint32_t *cnt = side ? s_lcnt : s_rcnt;
+    for (int i = rank * kNT + tid; i < n; i += nc * kNT) {
+      unsigned c = 0;
+      for (int r = 0; r < nc; ++r) {
+        const uint32_t *o = nc > 1 ? cluster.map_shared_rank(cnt, r) : cnt;
+        c += (o[i >> 1] >> ((i & 1) * 16)) & 0xffffu;
+      }
+      desolv.add(tab[static_cast<size_t>(i) * 11 + min(c, 10u)], p.fx_desolv);
+    }
+  }
   vdw.warp_total();
   elec.warp_total();
+  desolv.warp_total();
   if (lane == 0) {
+    if (TURNS) {
+      desolv.v += s_red[warp * 3 + 2];
+      desolv.nf += s_nf[warp * 3 + 2];
+    }
     s_red[warp * 3] = vdw.v;
     s_red[warp * 3 + 1] = elec.v;
+    s_red[warp * 3 + 2] = desolv.v;
     s_nf[warp * 3] = vdw.nf;
     s_nf[warp * 3 + 1] = elec.nf;
+    s_nf[warp * 3 + 2] = desolv.nf;
   }
   if (nc > 1) cluster.sync();
   else __syncthreads();
@@ -576,8 +590,8 @@ __global__ void __launch_bounds__(kNT, 3) k_score_f64(const ScoreParams p, const
 // ------------------------------------------------------------ dispatch ----
 
 template <typename Kern>
-cudaError_t launch_f64(Kern kern, const ScoreParams &p, int sm_count, cudaStream_t stream) {
-  const size_t smem = f64_smem(p.nr, p.nl).total;
+cudaError_t launch_f64(Kern kern, const ScoreParams &p, bool turns, int sm_count, cudaStream_t stream) {
+  const size_t smem = f64_smem(p.nr, p.nl, turns).total;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return e;
   // CTAs per pose: the more the fewer poses there are, as far as the pose's
@@ -704,20 +718,24 @@ gd_status launch_score(gd_complex *cx, const gd_pose_frame *d_frames, const doub
   if (!(p.guard_e <= 1.0f)) p.guard_e = p.guard_v = INFINITY;
   cudaError_t e;
   const int sm = ctx->sm_count;
-  if (p.fix) {
-    if (serial) e = clamp ? launch_f64(k_score_f64<true, true, true>, p, sm, stream)
-                          : launch_f64(k_score_f64<true, true, false>, p, sm, stream);
-    else e = clamp ? launch_f64(k_score_f64<true, false, true>, p, sm, stream)
-                   : launch_f64(k_score_f64<true, false, false>, p, sm, stream);
+  if (p.nl > kLigCounts) {
+    // (one variant: the tests of the others change nothing where they are not needed)
+    e = p.fix ? launch_f64(k_score_f64<true, true, true, true>, p, true, sm, stream)
+              : launch_f64(k_score_f64<false, true, true, true>, p, true, sm, stream);
+  } else if (p.fix) {
+    if (serial) e = clamp ? launch_f64(k_score_f64<true, true, true, false>, p, false, sm, stream)
+                          : launch_f64(k_score_f64<true, true, false, false>, p, false, sm, stream);
+    else e = clamp ? launch_f64(k_score_f64<true, false, true, false>, p, false, sm, stream)
+                   : launch_f64(k_score_f64<true, false, false, false>, p, false, sm, stream);
   } else {
-    if (serial) e = clamp ? launch_f64(k_score_f64<false, true, true>, p, sm, stream)
-                          : launch_f64(k_score_f64<false, true, false>, p, sm, stream);
-    else e = clamp ? launch_f64(k_score_f64<false, false, true>, p, sm, stream)
-                   : launch_f64(k_score_f64<false, false, false>, p, sm, stream);
+    if (serial) e = clamp ? launch_f64(k_score_f64<false, true, true, false>, p, false, sm, stream)
+                          : launch_f64(k_score_f64<false, true, false, false>, p, false, sm, stream);
+    else e = clamp ? launch_f64(k_score_f64<false, false, true, false>, p, false, sm, stream)
+                   : launch_f64(k_score_f64<false, false, false, false>, p, false, sm, stream);
   }
   if (e != cudaSuccess) {
     // the one size that the form does not take: the receptor's burial counts
-    const size_t need = f64_smem(p.nr, p.nl).total;
+    const size_t need = f64_smem(p.nr, p.nl, p.nl > kLigCounts).total;
     int most = 0;
     if (cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device) == cudaSuccess &&
         need > static_cast<size_t>(most)) {

@@ -148,9 +148,10 @@ def test_the_stated_displacement_does_not_matter(big, stated):
     assert out.cpu().numpy().tobytes() == want.tobytes()
 
 
-@pytest.mark.parametrize("nr,nl,n", [(40, 90000, 1), (40, 90000, 3), (5, 120001, 2)])
+@pytest.mark.parametrize("nr,nl,n", [(40, 4096, 2), (40, 4097, 2), (40, 90000, 1), (40, 90000, 3), (5, 120001, 2)])
 def test_long_ligands(oracle, big, nr, nl, n):
-    """Ligands of any length: their burial counts are held a turn at a time."""
+    """Ligands of any length: past 4,096 atoms their burial counts are held a turn
+    at a time, in a variant of the kernel that checks serials and clamps."""
     from conftest import make_mol, tatom
     rng = np.random.default_rng(nl)
     rec = make_mol([tatom(*x, "CNO"[k % 3], charge=0.3, serial=k + 1) for k, x in enumerate(rng.normal(0, 4.0, (nr, 3)))])
