@@ -121,9 +121,9 @@ static __device__ __forceinline__ void relative_atom(const ScoreParams &p, const
 // is rounded, so that the error, five quarters of a unit of 2^-51 A at most, is as
 // often up as down and averages out over a pose's atoms (limbs from 0 up and a
 // sum rounded down put every atom 5e-16 A to one side on average).  An FP64 chain
-// of multiply-adds errs by ten times as much at 60 A.
-static __device__ __forceinline__ long long rotate(const Limbs &a, const Limbs &b, const Limbs &c, const int4 &xy, const int4 &z) {
-  long long hi = static_cast<long long>(a.h) * xy.x, mid = static_cast<long long>(a.h) * xy.y + (1 << 28);
+// of multiply-adds errs by ten times as much at 60 A.  half: what rounds the sum.
+static __device__ __forceinline__ long long rotate(const Limbs &a, const Limbs &b, const Limbs &c, const int4 &xy, const int4 &z, long long half = 1 << 28) {
+  long long hi = static_cast<long long>(a.h) * xy.x, mid = static_cast<long long>(a.h) * xy.y + half;
   hi += static_cast<long long>(b.h) * xy.z;
   mid += static_cast<long long>(a.l) * xy.x;
   hi += static_cast<long long>(c.h) * z.x;
