@@ -87,3 +87,29 @@ def test_shared_serials_in_chunks(oracle, rec, lig, n):
     finally:
         cx.close()
         ctx.close()
+
+
+def test_seven_near_and_six_far_rows(oracle):
+    """7 near and 6 far rows (three left over after a step, two after another)
+    with charges of one sign, so that no sum cancels."""
+    rng = np.random.default_rng(76)
+    rec = [tatom(*rng.normal(0, 1.5, 3), "CNO"[k % 3], charge=0.3, serial=k + 1) for k in range(7)]
+    rec += [tatom(14.5, *rng.normal(0, 0.7, 2), "O", charge=0.4, serial=100 + k) for k in range(6)]
+    lig = [tatom(*rng.normal(0, 1.0, 3), "CNO"[k % 3], charge=0.2, serial=1000 + k, chain="B") for k in range(32)]
+    R, L = make_mol(rec), make_mol(lig)
+    xyz = np.stack([L.xyz() + rng.normal(0, 0.2, 3) for _ in range(3)])
+    genes = np.zeros((16, 6))
+    genes[:, 3:] = rng.normal(0, 0.2, (16, 3))
+    ctx = gd.Context(0)
+    cx = gd.Complex(R, L, [], ctx=ctx)
+    try:
+        check(cx.score_models(xyz, gd.GD_PREC_F32), oracle.score_models(R, L, [], xyz), F32_TOL)
+        pose = cx.score_poses(genes, gd.GD_PREC_F32)
+        check(pose, oracle.score_poses(R, L, [], genes), F32_TOL)
+        for tune, split in ((324, 1), (68, 1), (324, 2)):
+            ctx.set_tuning(_lib.GD_TUNE_F32_SLOTS, tune)
+            ctx.set_tuning(_lib.GD_TUNE_SPLIT, split)
+            assert cx.score_poses(genes, gd.GD_PREC_F32).tobytes() == pose.tobytes(), (tune, split)
+    finally:
+        cx.close()
+        ctx.close()
