@@ -382,7 +382,7 @@ __device__ __noinline__ bool exact_contact(const ContactListParams &p, int pose,
 // residue pair, every block's atoms moved in the reference's 34 FP64
 // operations) kept the FP64 pipe 77 % busy and wrote bitmaps over all residue
 // pairs, whose clearing, union and compaction moved 2 GB for 4,096 poses of
-// 2,000 x 500 residues: contacts and union CONTACTS_US.
+// 2,000 x 500 residues: contacts and union 3.0 -> 0.81 ms.
 __global__ void __launch_bounds__(kContactWarps * 32) k_contacts(const ContactListParams p) {
   __shared__ double s_m[12];  // rotation by rows, then centre + displacement - O
   __shared__ float s_m32[12];

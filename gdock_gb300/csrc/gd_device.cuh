@@ -134,7 +134,8 @@ static __device__ __forceinline__ long long rotate(const Limbs &a, const Limbs &
   return hi + (mid >> 29);
 }
 
-// The nearest float to v 2^-51 (v below 2^63): two exact parts and one rounding.
+// v 2^-51 as a float (v below 2^63): off by the rounding of the sum and, the low
+// part having been rounded to 24 bits first, by another 2^-36 A at most.
 static __device__ __forceinline__ float fix_float(long long v) {
   const float hi = __int2float_rn(static_cast<int>(v >> 40)), lo = __uint2float_rn(static_cast<unsigned>(v >> 8));
   return __fmul_rn(__fmaf_rn(lo, 0x1p-32f, hi), 0x1p-11f);

@@ -202,10 +202,10 @@ __device__ __forceinline__ float vdw_term(float d2, float2 tp) {
 
 // One pair's FP32 terms.  The Coulomb sum accumulates q_r / d2 (scaled by
 // the lane's ligand charge once per segment).  The vdW decision is d2 < 144
-// alone: the reference's 0 < r excludes only coincident atoms, whose FP32
-// d2 is then exactly 0 too (the FP32 coordinates are roundings of the same
-// doubles) and whose FP32 term is exactly 0, so the sums are unchanged; the
-// guard band of the vdW cutoff is the one at 144.
+// alone: the reference's 0 < r excludes only coincident atoms, whose FP32 d2 is
+// 0 (models) or within the rounding of the two images (poses, moved in fixed
+// point: some 1e-11 A^2), where r^6 vanishes beside R6 and x^2 - x is exactly 0,
+// so the sums are unchanged; the guard band of the vdW cutoff is the one at 144.
 template <bool SERIAL, bool CLAMP>
 __device__ __forceinline__ void pair32(float d2, float qr, const float2 tp, bool same, float gv, float ge, float gdd,
                                        float &av, float &ae, bool &amb) {
