@@ -46,6 +46,7 @@ struct ClusterTopo {
   // receptor heavy atoms grouped by residue (canonical ids), ligand likewise
   int GR = 0, GL = 0;
   std::vector<int64_t> rg_key, lg_key;  // (chain << 16) | uint16(resseq)
+  std::vector<int> rg_rank, lg_rank;    // the keys' ranks among their molecule's
   std::vector<int> rg_off, lg_off;      // atom ranges
   std::vector<int> r_atoms, l_atoms;    // original atom indices, grouped
   bool multi_chain_rec = false, multi_chain_lig = false;
@@ -1041,9 +1042,11 @@ void group_atoms(const std::vector<uint8_t> &chain, const std::vector<int16_t> &
 
 // Residue groups put into spatially compact runs of `unit` (and, within, of
 // `sub`) by their centroids, so that a block of consecutive groups has a small
-// enclosing sphere whatever the chain's course.
-void compact_groups(const std::vector<double> &x, const std::vector<double> &y, const std::vector<double> &z,
-                    std::vector<int64_t> &gkey, std::vector<int> &goff, std::vector<int> &atoms, int unit, int sub) {
+// enclosing sphere whatever the chain's course.  Returns each group's index before
+// (by key: its rank).
+std::vector<int> compact_groups(const std::vector<double> &x, const std::vector<double> &y, const std::vector<double> &z,
+                                std::vector<int64_t> &gkey, std::vector<int> &goff, std::vector<int> &atoms, int unit,
+                                int sub) {
   const int G = static_cast<int>(gkey.size());
   std::vector<double> c[3];
   for (int g = 0; g < G; ++g) {
@@ -1066,6 +1069,7 @@ void compact_groups(const std::vector<double> &x, const std::vector<double> &y, 
   gkey.swap(key);
   goff.swap(off);
   atoms.swap(at);
+  return order;
 }
 
 gd_status build_topo(gd_complex *cx, ClusterTopo **out) {
@@ -1082,8 +1086,8 @@ gd_status build_topo(gd_complex *cx, ClusterTopo **out) {
     std::set_intersection(a.begin(), a.end(), b.begin(), b.end(), std::back_inserter(both));
     t->mixed = !both.empty();
   }
-  compact_groups(cx->h_rx, cx->h_ry, cx->h_rz, t->rg_key, t->rg_off, t->r_atoms, 32, 8);
-  compact_groups(cx->h_lx, cx->h_ly, cx->h_lz, t->lg_key, t->lg_off, t->l_atoms, kLigBlock, kLigBlock / 4);
+  t->rg_rank = compact_groups(cx->h_rx, cx->h_ry, cx->h_rz, t->rg_key, t->rg_off, t->r_atoms, 32, 8);
+  t->lg_rank = compact_groups(cx->h_lx, cx->h_ly, cx->h_lz, t->lg_key, t->lg_off, t->l_atoms, kLigBlock, kLigBlock / 4);
   std::vector<double> rx, ry, rz, lx, ly, lz;
   for (int i : t->r_atoms) {
     rx.push_back(cx->h_rx[i]);
@@ -1508,6 +1512,58 @@ static gd_status contacts_fast(gd_complex *cx, ClusterTopo *t, const std::vector
   }
 }
 
+// Orders the contacts of poses of two molecules of one chain each: keys by the
+// residues of the smaller chain, then by the other's.  A pose's contacts are set
+// as bits at their keys' ranks and read off in order; where the bits would be many
+// more than the contacts, the keys are sorted.  The lists come in no order: with a
+// sort for every pose 200 poses of 50 x 76 residues took 3.2 ms, with lists in the
+// order of the residues and a sort of those 1.4, so 0.88.
+class KeyOrder {
+ public:
+  explicit KeyOrder(const ClusterTopo *t) : t_(t), rec_first_((t->rg_key[0] >> 16) < (t->lg_key[0] >> 16)) {
+    hi_.resize(rec_first_ ? t->GR : t->GL);
+    lo_.resize(rec_first_ ? t->GL : t->GR);
+    auto put = [](std::vector<int64_t> &v, const std::vector<int64_t> &key, const std::vector<int> &rank, int shift) {
+      for (size_t g = 0; g < v.size(); ++g)
+        v[rank[g]] = ((key[g] >> 16) << (16 + shift)) | ((key[g] & 0xffff) << shift);
+    };
+    put(hi_, rec_first_ ? t->rg_key : t->lg_key, rec_first_ ? t->rg_rank : t->lg_rank, 32);
+    put(lo_, rec_first_ ? t->lg_key : t->rg_key, rec_first_ ? t->lg_rank : t->rg_rank, 0);
+    row_ = (lo_.size() + 63) / 64;
+  }
+  void append(const uint32_t *v, size_t n, std::vector<uint64_t> &bits, std::vector<int64_t> &out) const {
+    const uint32_t GL = static_cast<uint32_t>(t_->GL);
+    const size_t words = hi_.size() * row_;
+    const bool by_bits = words <= 16 * n;
+    if (by_bits) bits.resize(words, 0);  // (all zero between poses)
+    const size_t from = out.size();
+    for (size_t k = 0; k < n; ++k) {
+      const uint32_t rg = v[k] / GL, lg = v[k] % GL;
+      const size_t a = rec_first_ ? t_->rg_rank[rg] : t_->lg_rank[lg], b = rec_first_ ? t_->lg_rank[lg] : t_->rg_rank[rg];
+      if (by_bits) bits[a * row_ + (b >> 6)] |= uint64_t(1) << (b & 63);
+      else out.push_back(hi_[a] | lo_[b]);
+    }
+    if (!by_bits) {
+      std::sort(out.begin() + from, out.end());
+      return;
+    }
+    out.resize(from + n);
+    size_t at = from;
+    for (size_t a = 0; a < hi_.size(); ++a)
+      for (size_t w = 0; w < row_; ++w) {
+        uint64_t &word = bits[a * row_ + w];
+        for (uint64_t x = word; x; x &= x - 1) out[at++] = hi_[a] | lo_[w * 64 + __builtin_ctzll(x)];
+        word = 0;
+      }
+  }
+
+ private:
+  const ClusterTopo *t_;
+  bool rec_first_;
+  std::vector<int64_t> hi_, lo_;  // a key's halves by rank
+  size_t row_;                    // words a row of bits
+};
+
 // Contact keys of n poses (sorted per pose) into a host vector + offsets:
 // through k_contacts when the topology allows it (and GD_TUNE_CONTACTS does not
 // ask for the other), else through k_contacts_rl.  Both decide every atom pair
@@ -1618,6 +1674,30 @@ gd_status pose_contacts_host(gd_complex *cx, const double *genes, int n, double 
   const int nth = n >= 256 ? static_cast<int>(std::max(1u, std::min(16u, std::thread::hardware_concurrency()))) : 1;
   std::vector<std::vector<int64_t>> part(nth);
   std::vector<int64_t> cnt(n, 0);
+  if (fast && pairs > 0) {
+    const KeyOrder order(t);
+    auto work = [&](int q) {
+      const int i0 = static_cast<int>(static_cast<long long>(n) * q / nth),
+                i1 = static_cast<int>(static_cast<long long>(n) * (q + 1) / nth);
+      std::vector<uint64_t> bits;
+      part[q].reserve(static_cast<size_t>(loffs[i1] - loffs[i0]));
+      for (int i = i0; i < i1; ++i)
+        order.append(flat.data() + loffs[i], static_cast<size_t>(loffs[i + 1] - loffs[i]), bits, part[q]);
+    };
+    if (nth == 1) {
+      work(0);
+      keys.swap(part[0]);
+    } else {
+      std::vector<std::thread> th;
+      for (int q = 0; q < nth; ++q) th.emplace_back(work, q);
+      for (auto &x : th) x.join();
+      keys.clear();
+      keys.reserve(static_cast<size_t>(loffs[n]));
+      for (const auto &v : part) keys.insert(keys.end(), v.begin(), v.end());
+    }
+    offs.assign(loffs.begin(), loffs.end());
+    return GD_OK;
+  }
   auto work = [&](int q) {
     const int i0 = static_cast<int>(static_cast<long long>(n) * q / nth),
               i1 = static_cast<int>(static_cast<long long>(n) * (q + 1) / nth);

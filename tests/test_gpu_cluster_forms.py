@@ -132,3 +132,20 @@ def test_beside_scoring_on_a_stream():
     finally:
         cx.close()
         ctx.close()
+
+
+@pytest.mark.parametrize("chains", ["AB", "BA", "AA"])
+@pytest.mark.parametrize("rec,lig", [([5] * 40, [4] * 70), ([3] * 300, [3] * 130), ([30], [4] * 64), ([4] * 65, [30])])
+def test_order_of_contact_keys(oracle, chains, rec, lig):
+    """Keys read off as bits (many contacts for the residue pairs there are) and
+    sorted (few), the smaller chain's residues first, numbers from negative on."""
+    rng = np.random.default_rng(len(rec) + len(lig))
+    R, L = residues(rng, rec, chains[0], np.zeros(3)), residues(rng, lig, chains[1], np.zeros(3))
+    R.resseq[:] = R.resseq * 3 - 60
+    L.resseq[:] = L.resseq * 5 - 31 + (1 << 13)
+    genes = np.concatenate([rng.uniform(0, 6.28, (300, 3)), rng.normal(0, 4.0, (300, 3))], axis=1)
+    genes[::3, 3] += 17.0  # a few contacts only
+    cx = gd.Complex(R, L, [])
+    for n in (7, 300):  # one host thread, several
+        for a, b in zip(cx.pose_contacts(genes[:n]), oracle.pose_contacts_many(R, L, genes[:n])):
+            np.testing.assert_array_equal(a, b)
