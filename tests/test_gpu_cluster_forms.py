@@ -149,3 +149,21 @@ def test_order_of_contact_keys(oracle, chains, rec, lig):
     for n in (7, 300):  # one host thread, several
         for a, b in zip(cx.pose_contacts(genes[:n]), oracle.pose_contacts_many(R, L, genes[:n])):
             np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("n", [3, 200, 886, 887, 1300])
+@pytest.mark.parametrize("min_size", [0, 1, 2, 3])
+@pytest.mark.parametrize("cutoff,strictness", [(0.6, 0.75), (1.0, 1.0), (0.6, 1.8), (1.1, 1.0)])
+def test_clusters_of_one(oracle, n, min_size, cutoff, strictness):
+    """Poses with no, few and equal contacts, most alone in their cluster: where
+    the greedy pass stops and the rest is numbered on the host.  Cutoffs that no
+    ratio meets leave every pose without an edge, its own included."""
+    rng = np.random.default_rng(n)
+    sets = [np.zeros(0, np.int64) if k % 11 == 3 else np.unique(rng.integers(0, 10 ** 6, int(rng.integers(1, 9)))) for k in range(n)]
+    for k in range(0, n - 30, 29):  # pairs, one of three
+        sets[k + 17] = sets[k].copy()
+        if k % 58 == 0:
+            sets[k + 29] = sets[k].copy()
+    cfg = gd.ClusteringConfig(fcc_cutoff=cutoff, strictness=strictness, min_cluster_size=min_size)
+    want = oracle.cluster(sets, fcc_cutoff=cutoff, strictness=strictness, min_size=min_size)
+    assert [(r.center_idx, r.members) for r in gd.cluster_sets(sets, cfg)] == want
