@@ -655,8 +655,8 @@ gd_status gd_complex_create(gd_context *ctx, const gd_atoms *rec, const gd_atoms
       const bool in = std::fabs(rec->x[i]) <= kFixMax && std::fabs(rec->y[i]) <= kFixMax && std::fabs(rec->z[i]) <= kFixMax;
       cx->fix64 = cx->fix64 && in;
       if (in)
-        rfix[k] = FixAtom{std::llrint(std::ldexp(rec->x[i], kFixBits)), std::llrint(std::ldexp(rec->y[i], kFixBits)),
-                          std::llrint(std::ldexp(rec->z[i], kFixBits)), rec->charge[i]};
+        rfix[k] = FixAtom{fix_int(rec->x[i], kFixOne), fix_int(rec->y[i], kFixOne),
+                          fix_int(rec->z[i], kFixOne), rec->charge[i]};
     }
     rmeta[k] = make_int2(rtype[i] * nt, rec->serial[i]);
     desolv_row(rec->element[i], rec->vdw_radius[i], &rdes[static_cast<size_t>(k) * 11]);
@@ -707,15 +707,15 @@ gd_status gd_complex_create(gd_context *ctx, const gd_atoms *rec, const gd_atoms
       cx->fix32 = false;
       break;
     }
-    const Limbs x = limbs(std::llrint(std::ldexp(r.x, 50))), y = limbs(std::llrint(std::ldexp(r.y, 50))),
-                z = limbs(std::llrint(std::ldexp(r.z, 50)));
+    const Limbs x = limbs(fix_int(r.x, 0x1p50)), y = limbs(fix_int(r.y, 0x1p50)),
+                z = limbs(fix_int(r.z, 0x1p50));
     const float q = static_cast<float>(r.w);
     int qb;
     std::memcpy(&qb, &q, 4);
     lfix[2 * static_cast<size_t>(k)] = make_int4(x.h, x.l, y.h, y.l);
     lfix[2 * static_cast<size_t>(k) + 1] = make_int4(z.h, z.l, qb, ltp[k]);
   }
-  for (int k = 0; k < 3; ++k) cx->ofix[k] = cx->fix32 ? std::llrint(std::ldexp(o[k], 51)) : 0;
+  for (int k = 0; k < 3; ++k) cx->ofix[k] = cx->fix32 ? fix_int(o[k], 0x1p51) : 0;
   // bounding sphere of each 32-atom slot in the positioned frame: a pose moves
   // it rigidly, so its transformed centre and the same radius bound the
   // slot's atoms in every pose

@@ -542,15 +542,15 @@ gd_status gd_evaluator_create(gd_complex *cx, const gd_atoms *reference, const u
   const double whole[3] = {fixed ? std::nearbyint(cx->ox) : 0.0, fixed ? std::nearbyint(cx->oy) : 0.0,
                            fixed ? std::nearbyint(cx->oz) : 0.0};
   long long origin[3];
-  for (int k = 0; k < 3; ++k) origin[k] = std::llrint(std::ldexp(whole[k], 51));
+  for (int k = 0; k < 3; ++k) origin[k] = fix_int(whole[k], 0x1p51);
   auto fix_ref = [&](const D4 &v) {
     if (!(std::fabs(v.x) < 4000.0 && std::fabs(v.y) < 4000.0 && std::fabs(v.z) < 4000.0)) {
       fixed = false;
       return Fix3{0, 0, 0, 0};
     }
-    const Fix3 q{std::llrint(std::ldexp(v.x, 51)) - origin[0], std::llrint(std::ldexp(v.y, 51)) - origin[1],
-                 std::llrint(std::ldexp(v.z, 51)) - origin[2], 0};
-    const long long lim = std::llrint(std::ldexp(kFixFar, 51));
+    const Fix3 q{fix_int(v.x, 0x1p51) - origin[0], fix_int(v.y, 0x1p51) - origin[1],
+                 fix_int(v.z, 0x1p51) - origin[2], 0};
+    const long long lim = fix_int(kFixFar, 0x1p51);
     fixed = fixed && std::llabs(q.x) < lim && std::llabs(q.y) < lim && std::llabs(q.z) < lim;
     return q;
   };
@@ -562,8 +562,8 @@ gd_status gd_evaluator_create(gd_complex *cx, const gd_atoms *reference, const u
     u_slot[u] = cx->h_lig_slot[j];
     const double x0[3] = {cx->h_lx[j] - cx->cx, cx->h_ly[j] - cx->cy, cx->h_lz[j] - cx->cz};
     if (std::fabs(x0[0]) < kFixAtom && std::fabs(x0[1]) < kFixAtom && std::fabs(x0[2]) < kFixAtom) {
-      const Limbs x = limbs(std::llrint(std::ldexp(x0[0], 50))), y = limbs(std::llrint(std::ldexp(x0[1], 50))),
-                  z = limbs(std::llrint(std::ldexp(x0[2], 50)));
+      const Limbs x = limbs(fix_int(x0[0], 0x1p50)), y = limbs(fix_int(x0[1], 0x1p50)),
+                  z = limbs(fix_int(x0[2], 0x1p50));
       u_xy[u] = make_int4(x.h, x.l, y.h, y.l);
       u_z[u] = make_int4(z.h, z.l, 0, 0);
     } else {

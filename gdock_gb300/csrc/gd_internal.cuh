@@ -25,6 +25,7 @@ struct alignas(32) FixAtom {
   double q;
 };
 constexpr int kFixBits = 51;
+constexpr double kFixOne = 0x1p51;
 constexpr double kFixMax = 4000.0;   // receptor |coordinate| up to which the integers are used (they hold 4,096)
 constexpr double kFixHold = 4095.0;  // ligand |coordinate| they take; beyond, no receptor atom is near
 
@@ -89,6 +90,10 @@ struct Thresholds {
 // reference atoms within 768 A of the origin, so that a difference stays below
 // 2^12 A.
 constexpr double kFixAtom = 512.0, kFixFar = 768.0;
+// v in units of 1 / one (a power of two), rounded, on the host: two calls to the
+// mathematics library a coordinate (ldexp, llrint) took 10 us of 380 at the creation
+// of a complex of 430 x 651 atoms.
+inline long long fix_int(double v, double one) { return static_cast<long long>(__builtin_rint(v * one)); }
 struct Limbs { int h, l; };
 __host__ __device__ __forceinline__ Limbs limbs(long long v) {
   const long long h = (v + (1 << 28)) >> 29;
