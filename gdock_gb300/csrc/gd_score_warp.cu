@@ -290,7 +290,9 @@ __device__ __forceinline__ FixOut fix_pair(const ScoreParams &p, const gd_pose_f
   const bool pe32 = fabsf(te) < 112.0f;
   const bool pd32 = d2 < 64.0f;
   bool pv64 = false, pe64 = false, pd64 = false, decided = false;
-  if (fix) {
+  // (integers hold d2 below 256 A^2; pairs farther off come here where a pose of
+  // the launch is so far away that the bands cover every distance)
+  if (fix && d2 < 240.0f) {
     const int4 xy = __ldg(&p.lig_fix[2 * j]), z = __ldg(&p.lig_fix[2 * j + 1]);
     const longlong2 *rp = reinterpret_cast<const longlong2 *>(p.rec_fix + ridx);
     const longlong2 rxy = __ldg(rp);

@@ -27,3 +27,19 @@ def test_range(oracle, at, arm):
     genes[5, 3], genes[6, 4], genes[7, 5] = 767.0, 769.0, -5000.0
     e = gd.Complex(R, L, []).score_poses(genes, gd.GD_PREC_F32)
     check(e, oracle.score_poses(R, L, [], genes), F32_TOL)
+
+
+@pytest.mark.parametrize("far", [5.0e4, 3.0e6, 1.0e8, np.inf])
+def test_poses_beside_one_far_away(oracle, far):
+    """A pose so far away that the launch's guard bands cover every distance:
+    all pairs of the other poses are re-decided, those beyond 16 A not on
+    integers."""
+    from gdock_gb300 import synth
+    c = synth.make_complex(50, 76, 6, seed=1)
+    lig = gd.position_ligand(c.receptor, c.ligand)
+    genes = synth.quaternion_genes(np.random.default_rng(2), 24, half_box=12.0)
+    genes[7, 3] = far
+    e = gd.Complex(c.receptor, lig, c.restraint_pairs).score_poses(genes, gd.GD_PREC_F32)
+    ref = oracle.score_poses(c.receptor, lig, c.restraint_pairs, genes)
+    keep = np.arange(24) != 7
+    check(e[keep], ref[keep], F32_TOL)
