@@ -48,6 +48,9 @@ gd_status cuda_fail(gd_context *ctx, cudaError_t e, const char *what) {
 gd_status dev_alloc(gd_context *ctx, uint64_t bytes, void **p) {
   *p = nullptr;
   if (bytes == 0) bytes = 16;
+  // scratch that a large clustering call left, with no call in it now, does not
+  // stand in the way of other allocations
+  if (ctx->budget && ctx->in_use + bytes > ctx->budget && ctx->scratch_use == 0) (void)trim_scratch(ctx, 0);
   if (ctx->budget && ctx->in_use + bytes > ctx->budget)
     return fail(ctx, GD_ERR_OOM, "HBM budget exceeded: " + std::to_string(ctx->in_use + bytes) + " > " +
                                      std::to_string(ctx->budget) + " bytes");
@@ -90,6 +93,15 @@ gd_status ensure_scratch(gd_context *ctx, size_t dev_bytes, size_t pinned_bytes)
     ctx->h_pinned_bytes = want;
   }
   return GD_OK;
+}
+
+bool trim_scratch(gd_context *ctx, size_t need) {
+  if (!ctx->d_scratch || ctx->d_scratch_bytes <= std::max(need, static_cast<size_t>(1) << 20)) return false;
+  cudaStreamSynchronize(ctx->stream);
+  dev_free(ctx, ctx->d_scratch, ctx->d_scratch_bytes);
+  ctx->d_scratch = nullptr;
+  ctx->d_scratch_bytes = 0;
+  return need == 0 || ensure_scratch(ctx, need, 0) == GD_OK;
 }
 
 static gd_status grow(gd_context *ctx, void **p, size_t *have, size_t dev_bytes) {
@@ -993,13 +1005,12 @@ gd_status gd_score_poses(gd_complex *cx, const double *genes, int32_t n, gd_prec
   if (prec != GD_PREC_F32 && prec != GD_PREC_F64) return fail(ctx, GD_ERR_INVALID_ARG, "bad precision");
   if (n == 0) return GD_OK;
   cudaSetDevice(ctx->device);
+  const ScratchUse use(ctx);
   const size_t fb = sizeof(gd_pose_frame) * n, ob = sizeof(gd_pose_energy) * n;
   gd_status s = ensure_scratch(ctx, fb + ob + 256, fb + ob + 256);
   if (s != GD_OK) return s;
   gd_pose_frame *h_frames = static_cast<gd_pose_frame *>(ctx->h_pinned);
   gd_pose_energy *h_out = reinterpret_cast<gd_pose_energy *>(static_cast<char *>(ctx->h_pinned) + ((fb + 255) / 256) * 256);
-  gd_pose_frame *d_frames = static_cast<gd_pose_frame *>(ctx->d_scratch);
-  gd_pose_energy *d_out = reinterpret_cast<gd_pose_energy *>(static_cast<char *>(ctx->d_scratch) + ((fb + 255) / 256) * 256);
   // phase times on stderr with GD_TRACE (host frames, launch set-up, device
   // work and copies, result copy)
   const bool tr = trace_on();
@@ -1014,9 +1025,15 @@ gd_status gd_score_poses(gd_complex *cx, const double *genes, int32_t n, gd_prec
   frames_and_max_disp(genes, n, h_frames, &maxd);
   lap("score_poses: frames (host)");
   const bool direct = n <= kDirectPoses;
-  cudaError_t e = direct ? cudaSuccess : cudaMemcpyAsync(d_frames, h_frames, fb, cudaMemcpyHostToDevice, ctx->stream);
-  if (e != cudaSuccess) return cuda_fail(ctx, e, "H2D frames");
-  s = launch_score(cx, direct ? h_frames : d_frames, nullptr, n, prec, direct ? h_out : d_out, ctx->stream, maxd);
+  cudaError_t e = cudaSuccess;
+  gd_pose_energy *d_out = nullptr;
+  do {  // (once more where the launch's memory is refused and the scratch holds more than this call needs)
+    gd_pose_frame *d_frames = static_cast<gd_pose_frame *>(ctx->d_scratch);
+    d_out = reinterpret_cast<gd_pose_energy *>(static_cast<char *>(ctx->d_scratch) + ((fb + 255) / 256) * 256);
+    if (!direct) e = cudaMemcpyAsync(d_frames, h_frames, fb, cudaMemcpyHostToDevice, ctx->stream);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "H2D frames");
+    s = launch_score(cx, direct ? h_frames : d_frames, nullptr, n, prec, direct ? h_out : d_out, ctx->stream, maxd);
+  } while (s == GD_ERR_OOM && trim_scratch(ctx, fb + ob + 256) && (ctx->last_error.clear(), true));
   if (s == GD_OK && !direct) {
     e = cudaMemcpyAsync(h_out, d_out, ob, cudaMemcpyDeviceToHost, ctx->stream);
     if (e != cudaSuccess) s = cuda_fail(ctx, e, "D2H energies");
@@ -1114,10 +1131,9 @@ gd_status gd_score_models(gd_complex *cx, const double *lig_xyz, int32_t n_model
   const size_t ob = sizeof(gd_pose_energy) * n_models;
   const size_t mb_al = ((mb + 255) / 256) * 256;
   const bool staged = mb <= kStageMax;
+  const ScratchUse use(ctx);
   gd_status s = ensure_scratch(ctx, mb_al + ob, (staged ? mb_al : 0) + ob);
   if (s != GD_OK) return s;
-  double *d_models = static_cast<double *>(ctx->d_scratch);
-  gd_pose_energy *d_out = reinterpret_cast<gd_pose_energy *>(static_cast<char *>(ctx->d_scratch) + mb_al);
   double *h_models = static_cast<double *>(ctx->h_pinned);
   gd_pose_energy *h_out = reinterpret_cast<gd_pose_energy *>(static_cast<char *>(ctx->h_pinned) + (staged ? mb_al : 0));
   // one pass on the host: into the pinned staging buffer, and the displacement
@@ -1139,10 +1155,16 @@ gd_status gd_score_models(gd_complex *cx, const double *lig_xyz, int32_t n_model
   if (nt == 1) pass(0);
   else HostPool::get().run(nt, pass);
   const double m = *std::max_element(part, part + nt);
-  cudaError_t e = cudaMemcpyAsync(d_models, staged ? h_models : lig_xyz, mb, cudaMemcpyHostToDevice, ctx->stream);
-  if (e != cudaSuccess) return cuda_fail(ctx, e, "H2D models");
   const bool direct = n_models <= kDirectPoses;
-  s = launch_score(cx, nullptr, d_models, n_models, prec, direct ? h_out : d_out, ctx->stream, m);
+  cudaError_t e = cudaSuccess;
+  gd_pose_energy *d_out = nullptr;
+  do {  // (as in gd_score_poses)
+    double *d_models = static_cast<double *>(ctx->d_scratch);
+    d_out = reinterpret_cast<gd_pose_energy *>(static_cast<char *>(ctx->d_scratch) + mb_al);
+    e = cudaMemcpyAsync(d_models, staged ? h_models : lig_xyz, mb, cudaMemcpyHostToDevice, ctx->stream);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "H2D models");
+    s = launch_score(cx, nullptr, d_models, n_models, prec, direct ? h_out : d_out, ctx->stream, m);
+  } while (s == GD_ERR_OOM && trim_scratch(ctx, mb_al + ob) && (ctx->last_error.clear(), true));
   if (s == GD_OK && !direct) {
     e = cudaMemcpyAsync(h_out, d_out, ob, cudaMemcpyDeviceToHost, ctx->stream);
     if (e != cudaSuccess) s = cuda_fail(ctx, e, "D2H energies");

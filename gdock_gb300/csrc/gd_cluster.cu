@@ -1519,6 +1519,17 @@ static gd_status contacts_fast(gd_complex *cx, ClusterTopo *t, const std::vector
     void *d_flat = nullptr;
     const size_t flat_b = sizeof(uint32_t) * flat.size();
     s = dev_alloc(ctx, flat_b, &d_flat);
+    if (s == GD_ERR_OOM) {  // no room to gather them on the device: the lists up to the longest one
+      std::vector<uint32_t> all(static_cast<size_t>(n) * most);
+      e = cudaMemcpy2DAsync(all.data(), sizeof(uint32_t) * most, d_lists, sizeof(uint32_t) * cap, sizeof(uint32_t) * most, n,
+                            cudaMemcpyDeviceToHost, st);
+      if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+      if (e != cudaSuccess) return cuda_fail(ctx, e, "contact lists");
+      for (int i = 0; i < n; ++i)
+        std::copy_n(all.begin() + static_cast<size_t>(i) * most, counts[i], flat.begin() + loffs[i]);
+      ctx->last_error.clear();  // the refused allocation is not this call's failure
+      return GD_OK;
+    }
     if (s != GD_OK) return s;
     e = cudaMemcpyAsync(d_offs, loffs.data(), sizeof(long long) * (n + 1), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) {
@@ -2114,7 +2125,12 @@ gd_status cluster_device(gd_complex *cx, const double *genes, int n, const gd_cl
     const size_t kc_b = al256(sizeof(int) * static_cast<size_t>(std::max(U, 1))), pre_b = kc_b + 256;
     if (ctx->tune_fcc != 1 && n <= 16384 && (ctx->tune_fcc == 2 || bits_work > 2e10)) {
       s = dev_alloc(ctx, pre_b, &pre);
-      if (s != GD_OK) return s;
+      if (s != GD_OK && (s != GD_ERR_OOM || ctx->tune_fcc == 2)) return s;
+    }
+    if (s != GD_OK) {  // no room to count the postings: the bitsets
+      ctx->last_error.clear();
+      s = GD_OK;
+    } else if (pre) {
       int *d_kc = static_cast<int *>(pre);
       unsigned long long *d_work = reinterpret_cast<unsigned long long *>(static_cast<char *>(pre) + kc_b), work = 0;
       e = cudaMemsetAsync(pre, 0, pre_b, st);
@@ -2232,6 +2248,7 @@ gd_status gd_pose_contacts(gd_complex *cx, const double *genes, int32_t n, int64
   if (n < 0 || (n > 0 && (!genes || !offsets)) || cap < 0 || (cap > 0 && !keys))
     return fail(ctx, GD_ERR_INVALID_ARG, "bad genes/keys/offsets");
   cudaSetDevice(ctx->device);
+  const ScratchUse use(ctx);
   std::vector<int64_t> k, o;
   gd_status s = pose_contacts_host(cx, genes, n, 5.0, k, o);
   if (s != GD_OK) return s;
@@ -2252,6 +2269,7 @@ gd_status gd_cluster(gd_complex *cx, const double *genes, int32_t n, const gd_cl
   *n_clusters = 0;
   if (n == 0) return GD_OK;  // cluster_structures on no structures
   cudaSetDevice(ctx->device);
+  const ScratchUse use(ctx);
   gd_status s = cluster_device(cx, genes, n, c, n_clusters, centers, sizes, members);
   if (s != GD_ERR_STATE) return s;
   // multi-chain molecules or shared residues: contact keys on the host path
@@ -2271,6 +2289,7 @@ gd_status gd_cluster_sets(gd_context *ctx, const int64_t *keys, const int64_t *o
   if (n > 0 && offsets[n] > 0 && !keys) return fail(ctx, GD_ERR_INVALID_ARG, "null keys");
   cudaSetDevice(ctx->device);
   const gd_cluster_cfg c = cfg ? *cfg : default_cfg();
+  const ScratchUse use(ctx);
   return cluster_sets(ctx, keys, offsets, n, c, n_clusters, centers, sizes, members);
 }
 

@@ -679,6 +679,7 @@ gd_status gd_evaluate_poses(gd_evaluator *ev, const double *genes, int32_t n, gd
   const size_t fb = sizeof(gd_pose_frame) * n, ob = sizeof(gd_dock_metrics) * n;
   const size_t fb_al = (fb + 255) / 256 * 256;
   const bool staged = fb_al + ob <= kStageMax;
+  const ScratchUse use(ctx);
   gd_status s = ensure_scratch(ctx, fb_al + ob, staged ? fb_al + ob : 0);
   if (s != GD_OK) return s;
   gd_pose_frame *d_frames = static_cast<gd_pose_frame *>(ctx->d_scratch);

@@ -1279,7 +1279,6 @@ gd_status server_admit(gd_server *S) {
     }
     const gd_atoms ra = job->rec.view(), la = job->lig.view();
     gd_complex *cx = nullptr;
-    const uint64_t before = ctx->in_use;
     const auto ta = Clock::now();
     s = gd_complex_create(ctx, &ra, &la, job->pairs.empty() ? nullptr : job->pairs.data(),
                           static_cast<int32_t>(job->pairs.size() / 2), &job->w, &cx);
@@ -1288,7 +1287,7 @@ gd_status server_admit(gd_server *S) {
       s = GD_OK;
       break;
     }
-    const uint64_t bytes = ctx->in_use - before;
+    const uint64_t bytes = s == GD_OK ? cx->bytes : 0;
     if (s == GD_OK && S->cfg.hbm_budget && S->job_bytes + bytes > S->cfg.hbm_budget && S->job_bytes > 0) {
       gd_complex_destroy(cx);  // over the server's budget: admit later
       break;

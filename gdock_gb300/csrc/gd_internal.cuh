@@ -161,6 +161,7 @@ struct gd_context {
   // grow-only scratch: device and pinned host staging
   void *d_scratch = nullptr;
   size_t d_scratch_bytes = 0;
+  int scratch_use = 0;  // calls that hold d_scratch (0: an allocation that a budget refuses may take it back)
   void *h_pinned = nullptr;
   size_t h_pinned_bytes = 0;
   // argument blocks of batched launches (descriptors, queue, counters): such a
@@ -242,6 +243,16 @@ gd_status cuda_fail(gd_context *ctx, cudaError_t e, const char *what);
 gd_status dev_alloc(gd_context *ctx, uint64_t bytes, void **p);
 void dev_free(gd_context *ctx, void *p, uint64_t bytes);
 gd_status ensure_scratch(gd_context *ctx, size_t dev_bytes, size_t pinned_bytes);
+// Give back what the scratch holds beyond `need` bytes; false when that is nothing.
+bool trim_scratch(gd_context *ctx, size_t need);
+// A call that keeps data in d_scratch, from entry to return.
+struct ScratchUse {
+  gd_context *ctx;
+  explicit ScratchUse(gd_context *c) : ctx(c) { ++ctx->scratch_use; }
+  ~ScratchUse() { --ctx->scratch_use; }
+  ScratchUse(const ScratchUse &) = delete;
+  ScratchUse &operator=(const ScratchUse &) = delete;
+};
 gd_status check_device_error(gd_context *ctx);
 // Wait for the stream and report its errors, the device error word included.
 gd_status finish_stream(gd_context *ctx, cudaStream_t stream, const char *what);

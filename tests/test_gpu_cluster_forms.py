@@ -167,3 +167,42 @@ def test_clusters_of_one(oracle, n, min_size, cutoff, strictness):
     cfg = gd.ClusteringConfig(fcc_cutoff=cutoff, strictness=strictness, min_cluster_size=min_size)
     want = oracle.cluster(sets, fcc_cutoff=cutoff, strictness=strictness, min_size=min_size)
     assert [(r.center_idx, r.members) for r in gd.cluster_sets(sets, cfg)] == want
+
+
+@pytest.mark.parametrize("mib", [8, 12, 32])
+@pytest.mark.parametrize("backwards", [False, True])
+def test_calls_one_after_another_within_a_budget(mib, backwards):
+    """What a clustering call keeps does not stand in the way of the calls after
+    it, in either order, and contact keys need no second copy of the lists."""
+    from gdock_gb300 import synth
+    c = synth.make_complex(50, 76, 0, seed=9)
+    lig = gd.position_ligand(c.receptor, c.ligand)
+    genes = synth.quaternion_genes(np.random.default_rng(3), 3000, half_box=12.0)
+    cfg = gd.ga_default_cfg(pop_size=100, max_generations=3, early_stopping=0, seed=1)
+
+    def calls(ctx, cx):
+        run = [lambda: cx.score_poses(genes, "f32").tobytes(), lambda: cx.score_poses(genes[:200], "f64").tobytes(),
+               lambda: [(r.center_idx, r.members) for r in cx.cluster(genes)],
+               lambda: [k.tobytes() for k in cx.pose_contacts(genes)],
+               lambda: gd.run_ga([cx], cfg, "f32", ctx=ctx).genes.tobytes(),
+               lambda: gd.Complex(c.receptor, lig, [], ctx=ctx).close()]
+        out = [f() for f in (run[::-1] if backwards else run)]
+        return out[::-1] if backwards else out
+
+    got = []
+    for budget in (0, 1):
+        ctx = gd.Context(0)
+        cx = gd.Complex(c.receptor, lig, [], ctx=ctx)
+        if budget:
+            resident = ctx.bytes_in_use
+            cx.close()
+            ctx.close()
+            ctx = gd.Context(0, hbm_budget_bytes=resident + (mib << 20))
+            cx = gd.Complex(c.receptor, lig, [], ctx=ctx)
+        try:
+            got.append(calls(ctx, cx))
+            assert ctx.lib.gd_last_error(ctx.h) == b""
+        finally:
+            cx.close()
+            ctx.close()
+    assert got[0] == got[1]
