@@ -49,6 +49,12 @@ struct ClusterTopo {
   std::vector<int> rg_rank, lg_rank;    // the keys' ranks among their molecule's
   std::vector<int> rg_off, lg_off;      // atom ranges
   std::vector<int> r_atoms, l_atoms;    // original atom indices, grouped
+  // the residues of a molecule of several chains in the order of their keys, for
+  // the contacts within it
+  struct Groups {
+    std::vector<int64_t> key;
+    std::vector<int> off, atoms;
+  } r_by_key, l_by_key;
   bool multi_chain_rec = false, multi_chain_lig = false;
   bool mixed = false;  // a (chain, resseq) residue with atoms in both molecules
   float4 *d_r32 = nullptr;  // receptor heavy atoms (x-O, y-O, z-O, 0) FP32, grouped
@@ -1094,6 +1100,8 @@ gd_status build_topo(gd_complex *cx, ClusterTopo **out) {
     std::set_intersection(a.begin(), a.end(), b.begin(), b.end(), std::back_inserter(both));
     t->mixed = !both.empty();
   }
+  if (t->multi_chain_rec) t->r_by_key = {t->rg_key, t->rg_off, t->r_atoms};
+  if (t->multi_chain_lig) t->l_by_key = {t->lg_key, t->lg_off, t->l_atoms};
   t->rg_rank = compact_groups(cx->h_rx, cx->h_ry, cx->h_rz, t->rg_key, t->rg_off, t->r_atoms, 32, 8);
   t->lg_rank = compact_groups(cx->h_lx, cx->h_ly, cx->h_lz, t->lg_key, t->lg_off, t->l_atoms, kLigBlock, kLigBlock / 4);
   std::vector<double> rx, ry, rz, lx, ly, lz;
@@ -1610,7 +1618,7 @@ gd_status pose_contacts_host(gd_complex *cx, const double *genes, int n, double 
   const Thresholds thr = make_thresholds(cutoff);
   if (t->multi_chain_rec && t->rr_cutoff != cutoff) {
     t->rr_keys.clear();
-    intra_contacts(t->rg_key, t->rg_off, t->r_atoms, cx->h_rx.data(), cx->h_ry.data(), cx->h_rz.data(),
+    intra_contacts(t->r_by_key.key, t->r_by_key.off, t->r_by_key.atoms, cx->h_rx.data(), cx->h_ry.data(), cx->h_rz.data(),
                    thr.contact_le, t->rr_keys);
     t->rr_cutoff = cutoff;
   }
@@ -1748,7 +1756,7 @@ gd_status pose_contacts_host(gd_complex *cx, const double *genes, int n, double 
         tz.resize(cx->nl);
         for (int a : t->l_atoms)
           xform_host(frames[i], cx->cx, cx->cy, cx->cz, cx->h_lx[a], cx->h_ly[a], cx->h_lz[a], tx[a], ty[a], tz[a]);
-        intra_contacts(t->lg_key, t->lg_off, t->l_atoms, tx.data(), ty.data(), tz.data(), thr.contact_le, pk);
+        intra_contacts(t->l_by_key.key, t->l_by_key.off, t->l_by_key.atoms, tx.data(), ty.data(), tz.data(), thr.contact_le, pk);
       }
       std::sort(pk.begin(), pk.end());
       pk.erase(std::unique(pk.begin(), pk.end()), pk.end());
@@ -1997,7 +2005,7 @@ gd_status cluster_device(gd_complex *cx, const double *genes, int n, const gd_cl
   if (t->multi_chain_rec) {
     if (t->rr_cutoff != cfg.contact_distance) {
       t->rr_keys.clear();
-      intra_contacts(t->rg_key, t->rg_off, t->r_atoms, cx->h_rx.data(), cx->h_ry.data(), cx->h_rz.data(),
+      intra_contacts(t->r_by_key.key, t->r_by_key.off, t->r_by_key.atoms, cx->h_rx.data(), cx->h_ry.data(), cx->h_rz.data(),
                      thr.contact_le, t->rr_keys);
       t->rr_cutoff = cfg.contact_distance;
     }
@@ -2007,7 +2015,7 @@ gd_status cluster_device(gd_complex *cx, const double *genes, int n, const gd_cl
     if (t->ll_cutoff != cfg.contact_distance) {
       std::vector<int64_t> ll;
       bool unstable = false;
-      intra_contacts(t->lg_key, t->lg_off, t->l_atoms, cx->h_lx.data(), cx->h_ly.data(), cx->h_lz.data(),
+      intra_contacts(t->l_by_key.key, t->l_by_key.off, t->l_by_key.atoms, cx->h_lx.data(), cx->h_ly.data(), cx->h_lz.data(),
                      thr.contact_le, ll, &unstable);
       t->ll_count = static_cast<long long>(ll.size());
       t->ll_unstable = unstable;
